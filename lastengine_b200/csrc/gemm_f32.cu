@@ -1,83 +1,325 @@
 // True 32-bit matrix product on the CUDA cores:  C[M,N] (+)= A[M,K] . W[N,K]^T.
 //
-// FFMA only: no tensor cores, no TF32, no reduced-precision mode of any kind.  Every output
-// element is one thread's sum over k = 0..K-1 in ascending order, whatever M is, so a row's
-// result does not depend on which other rows share the launch: a token gives the same bits
-// in a prompt, alone, or in a batch.  (The reference's all-float path is its CPU forward,
-// src/dense.rs:94-102, one dot product per output row.)
+// FFMA only: no tensor cores, no TF32, no reduced-precision mode of any kind.  An output element is
+// summed in one fixed order whatever M is and whichever kernel runs: k is cut into chunks of F32_CHUNK, a
+// chunk is one chain of fused multiply-adds in ascending k from zero, and the chunks' sums are added in
+// ascending order.  A row's result therefore does not depend on which other rows share the launch: a
+// token gives the same bits in a prompt, alone, or in a batch.  The cut lets warps work on several chunks
+// of one element at a time, and its error against 64 bits is smaller than that of one chain over K.  (The
+// reference's all-float path is its CPU forward, src/dense.rs:94-102, one dot product per output row.)
 //
 // Weights are [N,K] row-major as in the reference (src/dense.rs:96).  With group_offsets the
 // rows of A and C are grouped by expert: group e owns rows [off[e], off[e+1]) and the weight
 // matrix W + e * w_group_stride.
-#include "common.cuh"
+#include "stream_common.cuh"
 
-#define F32_BM 64
-#define F32_BN 64
-#define F32_BK 16
+#define F32_CHUNK 128
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
-                int M, int N, int K, int lda, int ldc, int accumulate,
-                const int* __restrict__ group_offsets, size_t w_group_stride) {
-  __shared__ float As[F32_BK][F32_BM + 4];
-  __shared__ float Ws[F32_BK][F32_BN + 4];
+// ---- up to 16 rows: the weights are streamed ---------------------------------------------------------
+// A decode step's product is bound by reading W once.  A block owns 16 weight rows at a time; a warp owns
+// two chunks of k of all 16 (a lane is one weight row in one chunk and holds the sums of every row of A), so
+// eight warps cover 2,048 k per round, and after a round 16 x M threads add the round's 16 chunk sums to
+// their element in order.  W and the same k of A come through a ring of cp.async stages per warp (32 k: 4 KB of
+// W), which runs on across rounds and tiles; segments of 32 floats lie 36 apart, so the lanes' 16-byte loads
+// of different rows meet no bank twice.  K = 2,048: 17.5 us for 2 rows x 11,264 (92 MB: 0.8 of the copy rate) where
+// the tiles of 64 x 64 took 209; from 8 rows on the multiply-adds and the loads of A (one per row of A and 4 k) weigh in:
+// 25 us for 8 rows, 45 for 16, against 54 for 16 rows in tiles.
+#define F32S_SEG 36
+#define F32S_ROWS 16
+template <int MT> struct F32Stream {
+  static constexpr int STAGE = (32 + 2 * MT) * F32S_SEG;          // floats of a warp's stage: W, then A
+  static constexpr int STAGES = MT <= 4 ? 4 : (MT <= 8 ? 3 : 2);
+  static constexpr int SMEM = (8 * STAGES * STAGE + 2 * 16 * MT * F32S_ROWS) * 4;
+};
+
+template <int MT>
+__global__ void __launch_bounds__(256, 1)
+gemm_f32_stream_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                       int M, int N, int K, int lda, int ldc, int accumulate, int tiles) {
+  constexpr int STAGES = F32Stream<MT>::STAGES, STAGE = F32Stream<MT>::STAGE;
+  extern __shared__ __align__(16) float smem[];
+  float* part = smem + 8 * STAGES * STAGE;                         // [2][chunk of the round][row of A][weight row]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float* ring = smem + warp * STAGES * STAGE;
+  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+  const int chunks = (K + F32_CHUNK - 1) / F32_CHUNK, rounds = (chunks + 15) / 16;
+  const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int steps = mine * rounds * 4;
+
+  auto k_of = [&](int s, int half) { return ((((s >> 2) % rounds) * 16 + warp * 2 + half) * F32_CHUNK) + (s & 3) * 32; };
+  auto issue_w = [&](int s) {
+    const int n0 = (blockIdx.x + (s / (4 * rounds)) * gridDim.x) * F32S_ROWS;
+    const uint32_t dst = ring_s + (s % STAGES) * STAGE * 4;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int p = lane + 32 * j, seg = p >> 3, k = k_of(s, seg >> 4) + (p & 7) * 4, n = n0 + (seg & 15);
+      const bool in = n < N && k < K;
+      st_cp16(dst + (seg * F32S_SEG + (p & 7) * 4) * 4, in ? W + (size_t)n * K + k : W, in ? 16 : 0);
+    }
+  };
+  auto issue_a = [&](int s) {
+    const uint32_t dst = ring_s + ((s % STAGES) * STAGE + 32 * F32S_SEG) * 4;
+#pragma unroll
+    for (int j = 0; j < (MT + 1) / 2; j++) {
+      const int p = lane + 32 * j, seg = p >> 3, m = seg >> 1, k = k_of(s, seg & 1) + (p & 7) * 4;
+      if (m >= MT) break;
+      const bool in = m < M && k < K;
+      st_cp16(dst + (seg * F32S_SEG + (p & 7) * 4) * 4, in ? A + (size_t)m * lda + k : A, in ? 16 : 0);
+    }
+  };
+
+  for (int s = 0; s < STAGES - 1; s++)
+    if (s < steps) issue_w(s);      // the weights do not depend on the kernel before this one
+  pdl_wait();
+  for (int s = 0; s < STAGES - 1; s++) {
+    if (s < steps) issue_a(s);
+    st_commit();
+  }
+  float acc[MT], total = 0.f;
+#pragma unroll
+  for (int m = 0; m < MT; m++) acc[m] = 0.f;
+  int buf = 0;
+  for (int s = 0; s < steps; s++) {
+    const int ahead = s + STAGES - 1;
+    if (ahead < steps) {
+      issue_w(ahead);
+      issue_a(ahead);
+    }
+    st_commit();
+    st_wait<STAGES - 1>();
+    __syncwarp();
+    const float* w = ring + (s % STAGES) * STAGE + lane * F32S_SEG;
+    const float* a = ring + (s % STAGES) * STAGE + (32 + (lane >> 4)) * F32S_SEG;
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++) {
+      const float4 wv = load4(w + kk * 4);
+#pragma unroll
+      for (int m = 0; m < MT; m++) {
+        const float4 av = load4(a + m * 2 * F32S_SEG + kk * 4);
+        acc[m] = fmaf(av.x, wv.x, acc[m]);
+        acc[m] = fmaf(av.y, wv.y, acc[m]);
+        acc[m] = fmaf(av.z, wv.z, acc[m]);
+        acc[m] = fmaf(av.w, wv.w, acc[m]);
+      }
+    }
+    __syncwarp();
+    if ((s & 3) == 3) {
+      const int round = (s >> 2) % rounds;
+      float* p = part + buf * 16 * MT * F32S_ROWS;
+#pragma unroll
+      for (int m = 0; m < MT; m++) {
+        p[((warp * 2 + (lane >> 4)) * MT + m) * F32S_ROWS + (lane & 15)] = acc[m];
+        acc[m] = 0.f;
+      }
+      __syncthreads();
+      // the sums of a round are read before the barrier of the next, and written over after it
+      if (tid < F32S_ROWS * MT) {
+        const int m = tid >> 4, r = tid & 15, c1 = min(16, chunks - round * 16);
+        for (int c = 0; c < c1; c++) total += p[(c * MT + m) * F32S_ROWS + r];
+        if (round == rounds - 1) {
+          const int n = (blockIdx.x + (s / (4 * rounds)) * gridDim.x) * F32S_ROWS + r;
+          if (m < M && n < N) {
+            float* c = C + (size_t)m * ldc + n;
+            *c = accumulate ? *c + total : total;
+          }
+          total = 0.f;
+        }
+      }
+      buf ^= 1;
+    }
+  }
+}
+
+// ---- more rows: tiles ----------------------------------------------------------------------------------
+// 256 threads; a block's tile is BM x BN, and its eight warps are WM x WN x WK: WM x WN parts of the tile, and WK chunks
+// of k at a time (WK 1 for many rows; more where the tiles would leave SMs idle: a small tile over eight chunks gives a
+// few dozen rows as many blocks as a stream of the weights has).  A lane of a warp's 8 x 4 holds TM x TN sums, rows 8
+// apart and columns side by side.  Both operands lie in shared memory as rows of 32 k at a pitch of 36 floats, where
+// the 16-byte loads of eight lanes meet no bank twice, and come through a ring of cp.async stages that runs on
+// across chunks and tiles, so only a block's first loads are waited for.  Bound by the FMA pipes and the shared loads beside
+// them: 37 TFLOP/s of the 72 the pipes have at 2,048 rows x 11,264 x 2,048 (2.5 ms, 3.7 ms before in tiles of 64 x 64 with
+// 4 x 4 sums a thread); 523 rows x 2,048 x 5,632 570 -> 436 us.  Twice the warps over the largest tile (half the
+// sums a thread, half again as many shared loads) took 2.75 ms; fma.rn.f32x2 in place of single multiply-adds takes 2.4
+// cycles for two against 2.0 and gives the pipes nothing.
+template <int BM, int BN, int WK>
+struct F32Tile {
+  static constexpr int ROWS = WK * (BM + BN);                       // rows of 32 k in a stage
+  static constexpr int STAGE = ROWS * F32S_SEG;
+  static constexpr int PART = WK > 1 ? WK * BM * (BN + 4) : 0;      // chunk sums on their way to being added up
+  static constexpr int STAGES = (3 * STAGE + PART) * 4 <= 220 * 1024 ? 3 : 2;
+  static constexpr int SMEM = (STAGES * STAGE + PART) * 4;
+};
+
+__device__ __forceinline__ void f32_cp4(uint32_t dst, const float* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
+template <int BM, int BN, int WM, int WN, int WK, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN * WK, 1)
+gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                     int M, int N, int K, int lda, int ldc, int accumulate,
+                     const int* __restrict__ group_offsets, size_t w_group_stride) {
+  using T = F32Tile<BM, BN, WK>;
+  constexpr int TM = BM / WM / 8, TN = BN / WN / 4, STAGES = T::STAGES, THREADS = 32 * WM * WN * WK;
+  constexpr int SUMS = WK > 1 ? BM * BN / THREADS : 1;
+  static_assert(TN % 4 == 0 && BM * BN % THREADS == 0 && T::ROWS * 8 % THREADS == 0, "whole vectors and equal shares");
+  extern __shared__ __align__(16) float smem[];
+  float* part = smem + STAGES * T::STAGE;
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lm = lane & 7, ln = lane >> 3;
+  const int wk = warp % WK, wn = warp / WK % WN, wm = warp / (WK * WN);
+  pdl_wait();
   int row_begin = 0, row_end = M;
   if (group_offsets) {
     row_begin = group_offsets[blockIdx.z];
     row_end = group_offsets[blockIdx.z + 1];
     W += (size_t)blockIdx.z * w_group_stride;
   }
-  const int m0 = row_begin + blockIdx.y * F32_BM;
-  if (m0 >= row_end) return;
-  const int n0 = blockIdx.x * F32_BN;
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int lrow = tid >> 2, lk = (tid & 3) * 4;  // loader: row of the tile, first of 4 k
+  // tiles in order of their rows first, so that blocks that run together share their weights
+  const int tiles_m = (row_end - row_begin + BM - 1) / BM, tiles = tiles_m * ((N + BN - 1) / BN);
+  const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int chunks = (K + F32_CHUNK - 1) / F32_CHUNK, rounds = (chunks + WK - 1) / WK;
+  const int steps = mine * rounds * 4;      // stages of 32 k: four to a chunk
 
-  float acc[4][4];
+  auto issue = [&](int s) {
+    const int tile = blockIdx.x + (s / (4 * rounds)) * gridDim.x;
+    const int m0 = row_begin + tile % tiles_m * BM, n0 = tile / tiles_m * BN;
+    const uint32_t dst = ring + (s % STAGES) * T::STAGE * 4;
+    const int k0 = ((s >> 2) % rounds) * WK * F32_CHUNK + (s & 3) * 32;
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+    for (int j = 0; j < T::ROWS * 8 / THREADS; j++) {
+      const int p = tid + THREADS * j, row = p >> 3, c = row / (BM + BN), r = row % (BM + BN);
+      const int k = k0 + c * F32_CHUNK + (p & 7) * 4;
+      const int g = r < BM ? m0 + r : n0 + r - BM;
+      const bool in = g < (r < BM ? row_end : N);
+      const float* src = r < BM ? A + (size_t)g * lda : W + (size_t)g * K;
+      const uint32_t d = dst + (row * F32S_SEG + (p & 7) * 4) * 4;
+      if (VEC) {
+        st_cp16(d, in && k < K ? src + k : W, in && k < K ? 16 : 0);
+      } else {
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+        for (int e = 0; e < 4; e++) f32_cp4(d + e * 4, in && k + e < K ? src + k + e : W, in && k + e < K);
+      }
+    }
+  };
 
-  for (int k0 = 0; k0 < K; k0 += F32_BK) {
-    {
-      const int r = m0 + lrow;
-      const float* src = A + (size_t)r * lda + k0 + lk;
-#pragma unroll
-      for (int e = 0; e < 4; e++) As[lk + e][lrow] = (r < row_end && k0 + lk + e < K) ? src[e] : 0.f;
-      const int n = n0 + lrow;
-      const float* wsrc = W + (size_t)n * K + k0 + lk;
-#pragma unroll
-      for (int e = 0; e < 4; e++) Ws[lk + e][lrow] = (n < N && k0 + lk + e < K) ? wsrc[e] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < F32_BK; kk++) {
-      float a[4], w[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) w[j] = Ws[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int s = 0; s < STAGES - 1; s++) {
+    if (s < steps) issue(s);
+    st_commit();
   }
+  float acc[TM][TN], total[WK > 1 ? 1 : TM][WK > 1 ? 1 : TN], sum[SUMS];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int r = m0 + ty * 4 + i;
-    if (r >= row_end) continue;
+  for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float* c = C + (size_t)r * ldc + n;
-      *c = accumulate ? *c + acc[i][j] : acc[i][j];
+    for (int j = 0; j < TN; j++) acc[i][j] = total[WK > 1 ? 0 : i][WK > 1 ? 0 : j] = 0.f;
+#pragma unroll
+  for (int i = 0; i < SUMS; i++) sum[i] = 0.f;
+  for (int s = 0; s < steps; s++) {
+    st_wait<STAGES - 2>();
+    __syncthreads();      // stage s has arrived for everyone, and everyone is done with the one before it
+    if (s + STAGES - 1 < steps) issue(s + STAGES - 1);
+    st_commit();
+    const float* a = smem + (s % STAGES) * T::STAGE + (wk * (BM + BN) + wm * (BM / WM) + lm) * F32S_SEG;
+    const float* w = smem + (s % STAGES) * T::STAGE + (wk * (BM + BN) + BM + wn * (BN / WN) + ln * TN) * F32S_SEG;
+#pragma unroll
+    for (int kk = 0; kk < 32; kk += 4) {
+      float4 av[TM];
+#pragma unroll
+      for (int i = 0; i < TM; i++) av[i] = load4(a + i * 8 * F32S_SEG + kk);
+#pragma unroll
+      for (int j = 0; j < TN; j++) {
+        const float4 wv = load4(w + j * F32S_SEG + kk);
+#pragma unroll
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(av[i].x, wv.x, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(av[i].y, wv.y, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(av[i].z, wv.z, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(av[i].w, wv.w, acc[i][j]);
+      }
+    }
+    if ((s & 3) != 3) continue;
+    // a chunk (or WK of them) is done
+    const int round = (s >> 2) % rounds, tile = blockIdx.x + (s / (4 * rounds)) * gridDim.x;
+    const int m0 = row_begin + tile % tiles_m * BM, n0 = tile / tiles_m * BN;
+    if (WK == 1) {
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+          total[WK > 1 ? 0 : i][WK > 1 ? 0 : j] += acc[i][j];
+          acc[i][j] = 0.f;
+        }
+      if (round < rounds - 1) continue;
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+        const int r = m0 + wm * (BM / WM) + lm + 8 * i;
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+          const int n = n0 + wn * (BN / WN) + ln * TN + j;
+          float& t = total[WK > 1 ? 0 : i][WK > 1 ? 0 : j];
+          if (r < row_end && n < N) {
+            float* c = C + (size_t)r * ldc + n;
+            *c = accumulate ? *c + t : t;
+          }
+          t = 0.f;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j += 4) {
+          store4(part + (wk * BM + wm * (BM / WM) + lm + 8 * i) * (BN + 4) + wn * (BN / WN) + ln * TN + j,
+                 make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]));
+          acc[i][j] = acc[i][j + 1] = acc[i][j + 2] = acc[i][j + 3] = 0.f;
+        }
+      __syncthreads();      // the next write to `part` comes after the barriers of the stages between
+      const int c1 = min(WK, chunks - round * WK);
+#pragma unroll
+      for (int i = 0; i < SUMS; i++) {
+        const int e = tid + THREADS * i, m = e / BN, n = e % BN;
+        for (int c = 0; c < c1; c++) sum[i] += part[(c * BM + m) * (BN + 4) + n];
+        if (round == rounds - 1) {
+          if (m0 + m < row_end && n0 + n < N) {
+            float* c = C + (size_t)(m0 + m) * ldc + n0 + n;
+            *c = accumulate ? *c + sum[i] : sum[i];
+          }
+          sum[i] = 0.f;
+        }
+      }
     }
   }
+}
+
+template <int MT>
+static int launch_f32_stream(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldc,
+                             int accumulate, cudaStream_t st) {
+  constexpr int smem = F32Stream<MT>::SMEM;
+  static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_stream_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  LEB_REQUIRE(set == cudaSuccess, "leb_gemm_f32: %s", cudaGetErrorString(set));
+  const int tiles = ceil_div(N, F32S_ROWS), sms = sm_count();
+  const int blocks = ceil_div(tiles, ceil_div(tiles, sms));        // as many tiles for every block
+  leb_launch(gemm_f32_stream_kernel<MT>, dim3(blocks), dim3(256), smem, st, C, A, W, M, N, K, lda, ldc, accumulate, tiles);
+  LEB_CHECK_LAUNCH("leb_gemm_f32");
+  return 0;
+}
+
+template <int BM, int BN, int WM, int WN, int WK, bool VEC>
+static int launch_f32_tile(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldc, int accumulate,
+                           const int* group_offsets, int groups, size_t w_group_stride, cudaStream_t st) {
+  constexpr int smem = F32Tile<BM, BN, WK>::SMEM;
+  auto kernel = gemm_f32_tile_kernel<BM, BN, WM, WN, WK, VEC>;
+  static const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  LEB_REQUIRE(set == cudaSuccess, "leb_gemm_f32: %s", cudaGetErrorString(set));
+  const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, BN);
+  LEB_REQUIRE(tiles < (1ll << 24) && groups <= 65535, "leb_gemm_f32: too many tiles (%lld) or groups (%d)", tiles, groups);
+  const int sms = sm_count(), blocks = ceil_div((int)tiles, ceil_div((int)tiles, sms));
+  leb_launch(kernel, dim3(blocks, 1, groups), dim3(32 * WM * WN * WK), smem, st, C, A, W, M, N, K, lda, ldc, accumulate, group_offsets,
+             w_group_stride);
+  LEB_CHECK_LAUNCH("leb_gemm_f32");
+  return 0;
 }
 
 LEB_API int leb_gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda,
@@ -85,10 +327,38 @@ LEB_API int leb_gemm_f32(float* C, const float* A, const float* W, int M, int N,
                          size_t w_group_stride, cudaStream_t st) {
   if (M <= 0 || N <= 0) return 0;
   LEB_REQUIRE(K > 0, "leb_gemm_f32: K must be positive");
-  dim3 grid(ceil_div(N, F32_BN), ceil_div(M, F32_BM), group_offsets ? n_groups : 1);
-  LEB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "leb_gemm_f32: too many row tiles (%u) or groups (%u)", grid.y, grid.z);
-  gemm_f32_kernel<<<grid, 256, 0, st>>>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets,
-                                        w_group_stride);
-  LEB_CHECK_LAUNCH("leb_gemm_f32");
-  return 0;
+  // 16-byte loads: rows of both operands begin on 16 bytes and hold whole vectors
+  const bool vec = K % 4 == 0 && lda % 4 == 0 && w_group_stride % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+  if (!group_offsets && M <= 16 && vec) {
+    if (M == 1) return launch_f32_stream<1>(C, A, W, M, N, K, lda, ldc, accumulate, st);
+    if (M == 2) return launch_f32_stream<2>(C, A, W, M, N, K, lda, ldc, accumulate, st);
+    if (M <= 4) return launch_f32_stream<4>(C, A, W, M, N, K, lda, ldc, accumulate, st);
+    if (M <= 8) return launch_f32_stream<8>(C, A, W, M, N, K, lda, ldc, accumulate, st);
+    return launch_f32_stream<16>(C, A, W, M, N, K, lda, ldc, accumulate, st);
+  }
+  const int groups = group_offsets ? n_groups : 1;
+  int pick = 0;
+  if (group_offsets) {
+    pick = M <= 32 * groups ? 4 : M <= 128 * groups ? 2 : 1;      // by the rows a group has on average
+  } else {
+    // The tile whose waves of one block per SM take least; the weights are a wave's measured microseconds per
+    // 2,048 of K.  (2,048 rows x 5,632 x 2,048 runs fastest in the largest tiles, 64 rows x 2,048 x 2,048
+    // in 28 us in tiles of 32 x 32, 31 in 64 x 16, 79 in 64 x 64 and 235 in 128 x 128.)
+    const int bm[5] = {128, 64, 32, 64, 32}, bn[5] = {128, 64, 32, 16, 16}, cost[5] = {2400, 790, 265, 275, 168};
+    long long best = -1;
+    for (int i = 0; i < 5; i++) {
+      const long long tiles = (long long)ceil_div(M, bm[i]) * ceil_div(N, bn[i]);
+      const long long t = (tiles + sm_count() - 1) / sm_count() * cost[i];
+      if (best < 0 || t < best) best = t, pick = i;
+    }
+  }
+#define LEB_F32_TILE(BM, BN, WM, WN, WK)                                                                                     \
+  return vec ? launch_f32_tile<BM, BN, WM, WN, WK, true>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st) \
+             : launch_f32_tile<BM, BN, WM, WN, WK, false>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st)
+  if (pick == 0) LEB_F32_TILE(128, 128, 2, 4, 1);
+  if (pick == 1) LEB_F32_TILE(64, 64, 1, 2, 4);
+  if (pick == 2) LEB_F32_TILE(32, 32, 1, 2, 8);
+  if (pick == 3) LEB_F32_TILE(64, 16, 1, 1, 8);
+  LEB_F32_TILE(32, 16, 1, 1, 8);
+#undef LEB_F32_TILE
 }

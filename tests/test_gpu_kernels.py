@@ -93,6 +93,35 @@ def test_linear_f32(M, N, K_):
     assert torch.equal(one.cpu()[0], out.cpu()[M - 1])
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 8, 9, 16, 17, 32, 33, 64, 65, 129, 300])
+@pytest.mark.parametrize("N,K_", [(17, 4), (50, 124), (2400, 128), (36, 132), (130, 2052), (4111, 260), (33, 4100), (40, 301)])
+def test_linear_f32_sums(M, N, K_):
+    """Every kernel of the 32-bit product (the stream up to 16 rows, tiles of five sizes, sizes without whole 16-byte
+    vectors): part tiles, part chunks of k, more chunks than a round holds, rows with a stride, and the same bits
+    whatever the row count.  A chunk of up to 128 products and a sum over K/128 chunks: each rounding is at most 2^-24
+    of a partial sum, so 2^-24 * (128 + K/128) of sum |x w| bounds every element."""
+    x, w = gen(M, K_ + 12, seed=6)[:, :K_], gen(N, K_, seed=7)
+    want = x.double() @ w.double().T
+    bound = 2.0 ** -24 * (min(K_, 128) + K_ / 128 + 2) * (x.double().abs() @ w.double().abs().T)
+    xd, wd = gen(M, K_ + 12, seed=6).to(DEV)[:, :K_], w.to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K().linear(out, xd, wd)
+    assert bool(((out.cpu().double() - want).abs() <= bound).all())
+    base = gen(M, N, seed=8).to(DEV)
+    b0 = base.clone()
+    K().linear(base, xd, wd, K().ACCUMULATE)
+    assert torch.equal(base, b0 + out)
+    one = torch.empty(1, N, device=DEV)
+    K().linear(one, xd[M - 1:], wd)
+    assert torch.equal(one[0], out[M - 1])
+    # rows grouped by expert: each group against its own weights, an empty group among them
+    offs = torch.tensor([0, M // 3, M // 3, M], dtype=torch.int32, device=DEV)
+    w3 = torch.stack([wd, wd * 2, wd * 0.5])
+    grouped = torch.full((M, N), float("nan"), device=DEV)
+    K().linear(grouped, xd, w3, group_offsets=offs)
+    assert torch.equal(grouped[:M // 3], out[:M // 3]) and torch.equal(grouped[M // 3:], out[M // 3:] * 0.5)
+
+
 @pytest.mark.parametrize("M", [1, 5, 8, 9, 33, 64, 65, 200])
 @pytest.mark.parametrize("N,K_", [(48, 72), (100, 200), (17, 40)])
 def test_linear_bf16_small(M, N, K_):
