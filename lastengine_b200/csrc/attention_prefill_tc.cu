@@ -16,8 +16,18 @@
 // 128-byte swizzle straight from the paged cache: no gather, no transposition.
 //
 // Roles: warps 0-3 softmax (thread r owns row r of S, P and O), warp 4 TMA producer, warp 5 issues
-// the MMAs.  S and P are double-buffered in tensor memory, so the product of the next page's
-// scores runs while this page's exponentials are taken; two blocks per SM overlap the rest.
+// the MMAs.  What bounds it is the special function unit: 64 exponentials a row and page are 512 cycles of a
+// scheduler's share, more than the products (320) or the other instructions of the row.  The unit stays busy where
+// enough rows are in their exponentials, so three blocks share an SM (112 registers a thread, 128 columns of
+// tensor memory, 64 KB of shared memory), and a row's chain is kept short: a row of S is taken into registers
+// whole, whereupon the next page's scores are issued into the same columns, and P goes to the second product
+// through shared memory (swizzled as the TMA tiles are); the thread that issues the products takes what they need from
+// uniform registers.  Per layer of 32 heads over 8: 16,384 rows 2.13 -> 1.75 ms (629 TFLOP/s), 8,192 0.54 -> 0.49,
+// 2,048 55.7 -> 52 us, against two blocks per SM with two buffers of S and P in tensor memory.  Measured beside it:
+// four blocks of 80 registers that read S in halves 0.50 ms at 8,192 rows; P over S in tensor memory 0.53 (three
+// blocks) and 0.67 (four, with spills); weights against the maximum so far before this page's is known: no change.
+// Weights as two bfloat16 terms (WIDE) go back to tensor memory over the scores they came from; those kernels run two
+// blocks per SM with two buffers of S.
 // The running maximum is only moved when it grew by more than 8 (a factor 256): exponentials stay
 // bounded, the row sum uses the same reference, and the quotient at the end is exact; moving it
 // means rescaling O in tensor memory, which then happens a few times per row instead of once
@@ -32,7 +42,13 @@
 #include "tc_common.cuh"
 
 #define ATC_THREADS 192
-#define ATC_STAGES 4
+template <bool WIDE>
+struct AtcShape {
+  static constexpr int BLOCKS = WIDE ? 2 : 3;        // per SM
+  static constexpr int STAGES = WIDE ? 4 : 2;        // pages of keys and values on their way
+  static constexpr int S_BUFS = WIDE ? 2 : 1;
+  static constexpr int COLUMNS = WIDE ? 256 : 128;   // of tensor memory
+};
 #define ATC_NEG (-1e30f)
 
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
@@ -44,6 +60,22 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
         "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
         "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
         "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -61,6 +93,37 @@ __device__ __forceinline__ float ex2(float x) {   // 2^x, one special-function s
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+__device__ __forceinline__ bool elect_lane() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// two floats at a time (one issue slot for both)
+__device__ __forceinline__ uint64_t f2(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float2 halves(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -82,7 +145,7 @@ __device__ __forceinline__ int atc_blocks_seen(int qpos, int window, int pool) {
 // WIDE: the weights as two terms as POOLED has them, for layers without pooled blocks too.
 // GS query heads per kv head (1, 2, 4, 8): a tile is GS heads x 128/GS positions; VD: width of a value head (64 or 32)
 template <int GS, bool POOLED, bool WIDE, int VD>
-__global__ void __launch_bounds__(ATC_THREADS, 2)
+__global__ void __launch_bounds__(ATC_THREADS, AtcShape<WIDE>::BLOCKS)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_pk,
                             const __grid_constant__ CUtensorMap map_pv, bf16* __restrict__ out,
@@ -93,19 +156,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int nh, int nkv, int window, int chunk, int pool, float scale, const float* __restrict__ head_scale,
                             const float* __restrict__ freq_v, const float* __restrict__ slopes,
                             const float* __restrict__ sinks, int* __restrict__ status) {
-  constexpr int HD = 64, PAGE = 64, TP = 128 / GS, NS = ATC_STAGES;
+  constexpr int HD = 64, PAGE = 64, TP = 128 / GS, NS = AtcShape<WIDE>::STAGES, SB = AtcShape<WIDE>::S_BUFS;
   constexpr int Q_BYTES = 128 * HD * 2, KV_BYTES = PAGE * HD * 2, V_BYTES = VD * PAGE * 2;
   extern __shared__ uint8_t atc_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)atc_raw + 1023) & ~(uintptr_t)1023);   // swizzled tiles want 1024
   uint8_t* sq = smem;
   uint8_t* sk = sq + Q_BYTES;
   uint8_t* sv = sk + NS * KV_BYTES;
-  __shared__ uint64_t q_full, k_full[NS], v_full[NS], kv_empty[NS], s_full[2], p_full[2], pv_done[2];
+  uint8_t* sp = sv + NS * V_BYTES;                 // P (not WIDE)
+  __shared__ uint64_t q_full, k_full[NS], v_full[NS], k_empty[NS], v_empty[NS], s_full[SB], s_free, p_full[SB], pv_done[SB];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_s;
   volatile int* abort_flag = &abort_s;
 
-  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // blocks start in the order x, y, z: kv heads vary fastest, and the tiles with the longest key
   // range come first, for all heads, so that the short ones fill the gaps at the end
@@ -144,9 +207,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     for (int s = 0; s < NS; s++) {
       mbar_init(&k_full[s], 1);
       mbar_init(&v_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+      mbar_init(&k_empty[s], 1);
+      mbar_init(&v_empty[s], 1);
     }
-    for (int i = 0; i < 2; i++) {
+    mbar_init(&s_free, 4);
+    for (int i = 0; i < SB; i++) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);
       mbar_init(&pv_done[i], 1);
@@ -154,15 +219,18 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 4) {
-    tmem_alloc(&tmem_slot, 256);
+    tmem_alloc(&tmem_slot, AtcShape<WIDE>::COLUMNS);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();      // barriers and tensor memory are set up; now q and the cache must be complete
+  // Barriers and tensor memory are set up (a block of the next kernel, let in from here on, cannot take the columns
+  // this one still waits for); now q and the cache must be complete.
+  pdl_wait();
   const uint32_t tmem = tmem_slot;
-  const uint32_t t_o = tmem, t_s0 = tmem + 64, t_p0 = tmem + 192;   // O | S0 S1 | P0 P1 (columns)
+  // O | S (WIDE: S0 S1) in columns; WIDE has P over the S it came from
+  const uint32_t t_o = tmem, t_s0 = tmem + 64;
   // instruction descriptor: float accumulate, bfloat16 operands, both K-major, N = 64, M = 128
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
   constexpr uint32_t IDESC_PV = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)VD >> 3) << 17) | ((128u >> 4) << 24);   // N = VD
@@ -180,55 +248,67 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int s = i % NS;
         int page = next_page;
         if (i + 1 < n_it) next_page = page_of(i + 1);   // asked for before the wait below
-        if (!mbar_wait(&kv_empty[s], ((i / NS) & 1) ^ 1, abort_flag)) { atomicExch(status, 11); ok = false; break; }
+        if (!mbar_wait(&k_empty[s], ((i / NS) & 1) ^ 1, abort_flag)) { atomicExch(status, 11); ok = false; break; }
         if (page < 0) page = 0;   // a page the window has left behind: every key of it is masked
         const int y = (page * nkv + kvh) * PAGE;
         const bool pooled = POOLED && i < npp;
         mbar_expect_tx(&k_full[s], KV_BYTES);
         tma_load_2d(sk + s * KV_BYTES, pooled ? &map_pk : &map_k, &k_full[s], 0, y);
+        if (!mbar_wait(&v_empty[s], ((i / NS) & 1) ^ 1, abort_flag)) { atomicExch(status, 21); ok = false; break; }
         mbar_expect_tx(&v_full[s], V_BYTES);
         tma_load_2d(sv + s * V_BYTES, pooled ? &map_pv : &map_v, &v_full[s], 0, (page * nkv + kvh) * VD);
       }
     }
   } else if (warp == 5) {
-    // ---- MMA issuer ----
-    if (lane == 0) {
-      auto scores = [&](int i) -> bool {
-        const int s = i % NS;
-        if (!mbar_wait(&k_full[s], (i / NS) & 1, abort_flag)) { atomicExch(status, 12); return false; }
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sq), ka = smem_u32(sk + s * KV_BYTES);
+    // ---- MMA issuer: the whole warp walks the loop, so that what the products take is uniform across it (values of a
+    // divergent branch have to be moved to uniform registers one by one before every instruction); one lane issues ----
+    const int n = __shfl_sync(0xffffffffu, n_it, 0);
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint64_t q_desc = make_desc(smem_u32(sq)), k_desc = make_desc(smem_u32(sk)), v_desc = make_desc(smem_u32(sv)), p_desc = make_desc(smem_u32(sp));
+    auto arrived = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+      const bool in = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+      if (!in && lane == 0) atomicExch(status, code);
+      return in;
+    };
+    auto scores = [&](int i) -> bool {
+      const int s = i % NS;
+      if (!arrived(&k_full[s], (i / NS) & 1, 12)) return false;
+      tc_fence_after();
+      if (elect_lane()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; kk++)
-          umma_bf16(t_s0 + 64 * (i & 1), make_desc(qa + kk * 32), make_desc(ka + kk * 32), IDESC, kk > 0);
-        umma_commit(&s_full[i & 1]);
-        return true;
-      };
-      if (!mbar_wait(&q_full, 0, abort_flag)) { atomicExch(status, 13); ok = false; }
-      if (ok) ok = scores(0);
-      for (int i = 0; i < n_it && ok; i++) {
-        if (i + 1 < n_it && !scores(i + 1)) { ok = false; break; }
-        const int s = i % NS;
-        if (!mbar_wait(&p_full[i & 1], (i >> 1) & 1, abort_flag)) { atomicExch(status, 14); ok = false; break; }
-        if (!mbar_wait(&v_full[s], (i / NS) & 1, abort_flag)) { atomicExch(status, 15); ok = false; break; }
-        tc_fence_after();
-        const uint32_t va = smem_u32(sv + s * V_BYTES);
+          umma_bf16(tm + 64 + 64 * (i & (SB - 1)), q_desc + kk * 2, k_desc + s * (KV_BYTES / 16) + kk * 2, IDESC, kk > 0);
+        umma_commit(&k_empty[s]);
+        umma_commit(&s_full[i & (SB - 1)]);
+      }
+      __syncwarp();
+      return true;
+    };
+    ok = arrived(&q_full, 0, 13) && scores(0);
+    for (int i = 0; i < n && ok; i++) {
+      // with one S the next scores wait until every softmax warp holds its rows of these
+      if (SB == 1 && i + 1 < n && !arrived(&s_free, i & 1, 22)) { ok = false; break; }
+      if (i + 1 < n && !scores(i + 1)) { ok = false; break; }
+      const int s = i % NS;
+      if (!arrived(&v_full[s], (i / NS) & 1, 15)) { ok = false; break; }
+      if (!arrived(&p_full[i & (SB - 1)], (i / SB) & 1, 14)) { ok = false; break; }
+      tc_fence_after();
+      if (elect_lane()) {
+        const uint64_t va = v_desc + s * (V_BYTES / 16);
         if (WIDE) {
-          const uint32_t t_p = t_s0 + 64 * (i & 1);   // hi in the scores' first 32 columns, lo in the next 32
+          const uint32_t t_p = tm + 64 + 64 * (i & 1);   // hi in the scores' first 32 columns, lo in the next 32
 #pragma unroll
-          for (int kk = 0; kk < PAGE / 16; kk++)
-            umma_bf16_ts(t_o, t_p + kk * 8, make_desc(va + kk * 32), IDESC_PV, (i > 0 || kk > 0));
+          for (int kk = 0; kk < PAGE / 16; kk++) umma_bf16_ts(tm, t_p + kk * 8, va + kk * 2, IDESC_PV, (i > 0 || kk > 0));
 #pragma unroll
-          for (int kk = 0; kk < PAGE / 16; kk++)
-            umma_bf16_ts(t_o, t_p + 32 + kk * 8, make_desc(va + kk * 32), IDESC_PV, 1);
+          for (int kk = 0; kk < PAGE / 16; kk++) umma_bf16_ts(tm, t_p + 32 + kk * 8, va + kk * 2, IDESC_PV, 1);
         } else {
 #pragma unroll
-          for (int kk = 0; kk < PAGE / 16; kk++)
-            umma_bf16_ts(t_o, t_p0 + 32 * (i & 1) + kk * 8, make_desc(va + kk * 32), IDESC_PV, (i > 0 || kk > 0));
+          for (int kk = 0; kk < PAGE / 16; kk++) umma_bf16(tm, p_desc + kk * 2, va + kk * 2, IDESC_PV, (i > 0 || kk > 0));
         }
-        umma_commit(&kv_empty[s]);
-        umma_commit(&pv_done[i & 1]);
+        umma_commit(&v_empty[s]);
+        umma_commit(&pv_done[i & (SB - 1)]);
       }
+      __syncwarp();
     }
   } else {
     // ---- softmax: thread r owns row r = (head r / TP, position r % TP) ----
@@ -247,36 +327,41 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     float m_used = ATC_NEG, l = 0.f;
     for (int i = 0; i < n_it && ok; i++) {
       const bool pooled = POOLED && i < npp;
-      const int key0 = pooled ? i * PAGE : (jb0 + i - npp) * PAGE, bsel = i & 1, s = i % NS;
-      if (!mbar_wait(&s_full[bsel], (i >> 1) & 1, abort_flag)) { atomicExch(status, 16); ok = false; break; }
+      const int key0 = pooled ? i * PAGE : (jb0 + i - npp) * PAGE, bsel = i & (SB - 1), s = i % NS;
+      if (!mbar_wait(&s_full[bsel], (i / SB) & 1, abort_flag)) { atomicExch(status, 16); ok = false; break; }
       tc_fence_after();
-      uint32_t v[64];
-      tmem_ld32(t_s0 + 64 * bsel + lane_base, v);
-      tmem_ld32(t_s0 + 64 * bsel + lane_base + 32, v + 32);
+      const uint32_t t_s = t_s0 + 64 * bsel + lane_base;
+      // columns [c_lo, c_hi] of this page are keys this row may see
+      const int c_lo = pooled ? 0 : max(0, key_lo_row - key0);
+      const int c_hi = row_valid ? min(PAGE - 1, (pooled ? nb_row - 1 : qpos) - key0) : -1;
+      // The scores stay as the product left them; the scale goes into the exponent's multiply-add.
+      uint32_t v[PAGE];
+      tmem_ld32(t_s, v);
+      tmem_ld32(t_s + 32, v + 32);
       tmem_ld_wait();
+      if (SB == 1) {      // the next scores may come
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free);
+      }
       if (sloped) {
         const float at0 = slope2 * (float)(key0 - qpos);
 #pragma unroll
         for (int c = 0; c < PAGE; c++)
           v[c] = __float_as_uint(fmaf(__uint_as_float(v[c]), scale2, fmaf(slope2, (float)c, at0)));
       }
-      // columns [c_lo, c_hi] of this page are keys this row may see
-      const int c_lo = pooled ? 0 : max(0, key_lo_row - key0);
-      const int c_hi = row_valid ? min(PAGE - 1, (pooled ? nb_row - 1 : qpos) - key0) : -1;
-      // The scores stay as the product left them; the scale goes into the exponent's multiply-add.
-      float rm[4] = {ATC_NEG, ATC_NEG, ATC_NEG, ATC_NEG};   // four chains instead of one of 64 steps
-      if (c_lo == 0 && c_hi == PAGE - 1) {
+      if (c_lo > 0 || c_hi < PAGE - 1) {
 #pragma unroll
-        for (int c = 0; c < PAGE; c++) rm[c & 3] = fmaxf(rm[c & 3], __uint_as_float(v[c]));
-      } else {
-#pragma unroll
-        for (int c = 0; c < PAGE; c++) {
-          const float sc = (c >= c_lo && c <= c_hi) ? __uint_as_float(v[c]) : ATC_NEG;
-          v[c] = __float_as_uint(sc);
-          rm[c & 3] = fmaxf(rm[c & 3], sc);
-        }
+        for (int c = 0; c < PAGE; c++)
+          if (c < c_lo || c > c_hi) v[c] = __float_as_uint(ATC_NEG);
       }
-      const float rmax = fmaxf(fmaxf(rm[0], rm[1]), fmaxf(rm[2], rm[3]));
+      float rm[2] = {ATC_NEG, ATC_NEG};
+#pragma unroll
+      for (int c = 0; c < PAGE; c += 4) {
+        rm[0] = max3(rm[0], __uint_as_float(v[c]), __uint_as_float(v[c + 1]));
+        rm[1] = max3(rm[1], __uint_as_float(v[c + 2]), __uint_as_float(v[c + 3]));
+      }
+      const float rmax = fmaxf(rm[0], rm[1]);
       // maxima are kept times scale * log2(e); a row with no key in this page keeps what it had
       const float m_new = rmax > 0.5f * ATC_NEG ? fmaxf(m_used, rmax * scale_after) : m_used;
       bool move = false;
@@ -284,48 +369,51 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       else if (m_new > m_used + 8.f) move = true;   // the reference maximum has to follow
       if (__any_sync(0xffffffffu, move)) {
         // O holds pages < i; the product of page i waits for this warp's P, so O is still once page i-1 is in
-        if (!mbar_wait(&pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, abort_flag)) { atomicExch(status, 17); ok = false; break; }
+        if (!mbar_wait(&pv_done[(i - 1) & (SB - 1)], ((i - 1) / SB) & 1, abort_flag)) { atomicExch(status, 17); ok = false; break; }
         tc_fence_after();
         const float f = move ? ex2(m_used - m_new) : 1.f;
 #pragma unroll
-        for (int hcol = 0; hcol < VD; hcol += 32) {
-          uint32_t o[32];
-          tmem_ld32(t_o + lane_base + hcol, o);
+        for (int hcol = 0; hcol < VD; hcol += 16) {
+          uint32_t o[16];
+          tmem_ld16(t_o + lane_base + hcol, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < 32; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * f);
-          tmem_st32(t_o + lane_base + hcol, o);
+          for (int c = 0; c < 16; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * f);
+          tmem_st16(t_o + lane_base + hcol, o);
         }
         tmem_st_wait();
         l *= f;
         if (move) m_used = m_new;
       }
+      // P of the pages before (WIDE: of page i-2, which lay where this one goes) has been read
+      if (i >= SB && !mbar_wait(&pv_done[bsel], ((i - SB) / SB) & 1, abort_flag)) { atomicExch(status, 18); ok = false; break; }
+      uint32_t pk[WIDE ? 32 : 4], pl[WIDE ? 32 : 1];
       const float m_ref = m_used > 0.5f * ATC_NEG ? m_used : 0.f;
-      uint32_t pk[32], pl[WIDE ? 32 : 1];
-      float ps[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint64_t scale_pair = f2(scale_after, scale_after), ref_pair = f2(-m_ref, -m_ref);
+      uint64_t ps[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
 #pragma unroll
       for (int c = 0; c < PAGE; c += 2) {
         // a masked score is -1e30: 2^(that * scale - m_ref) is exactly zero
-        const float p0 = ex2(fmaf(__uint_as_float(v[c]), scale_after, -m_ref)), p1 = ex2(fmaf(__uint_as_float(v[c + 1]), scale_after, -m_ref));
-        ps[(c >> 1) & 3] += p0 + p1;
+        const float2 x = halves(fma_f2(f2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), scale_pair, ref_pair));
+        const float p0 = ex2(x.x), p1 = ex2(x.y);
+        ps[(c >> 1) & 1] = add_f2(ps[(c >> 1) & 1], f2(p0, p1));
         __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-        pk[c >> 1] = *reinterpret_cast<uint32_t*>(&pp);
+        pk[(c >> 1) & (WIDE ? 31 : 3)] = *reinterpret_cast<uint32_t*>(&pp);
         if (WIDE) {
           __nv_bfloat162 pr = __floats2bfloat162_rn(p0 - __bfloat162float(pp.x), p1 - __bfloat162float(pp.y));
-          pl[c >> 1] = *reinterpret_cast<uint32_t*>(&pr);
+          pl[WIDE ? c >> 1 : 0] = *reinterpret_cast<uint32_t*>(&pr);
+        } else if ((c & 7) == 6) {      // eight weights: a 16-byte piece of the row
+          *reinterpret_cast<uint4*>(sp + r * 128 + (((c >> 3) ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
       }
-      l += (ps[0] + ps[1]) + (ps[2] + ps[3]);
-      // P[bsel] was last read by the product of page i-2
-      if (i >= 2 && !mbar_wait(&pv_done[bsel], ((i - 2) >> 1) & 1, abort_flag)) { atomicExch(status, 18); ok = false; break; }
-      tc_fence_after();
       if (WIDE) {
-        tmem_st32(t_s0 + 64 * bsel + lane_base, pk);
-        tmem_st32(t_s0 + 64 * bsel + 32 + lane_base, pl);
-      } else {
-        tmem_st32(t_p0 + 32 * bsel + lane_base, pk);
+        tc_fence_after();
+        tmem_st32(t_s, pk);
+        tmem_st32(t_s + 32, pl);
+        tmem_st_wait();
       }
-      tmem_st_wait();
+      const float2 sums = halves(add_f2(ps[0], ps[1]));
+      l += sums.x + sums.y;
       const int key_end = pooled ? nb_tile : key_hi;
       if (key0 + PAGE > key_end) {
         // the page with the end of the sequence (or of the pooled blocks): its value columns beyond it become zero
@@ -338,33 +426,37 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             for (int e = max(0, n_valid - cc * 8); e < 8; e++) piece[e] = __float2bfloat16_rn(0.f);
           }
         }
-        fence_proxy_async_smem();
+        if (WIDE) fence_proxy_async_smem();
       }
+      if (!WIDE) fence_proxy_async_smem();      // P (and the zeros) before the product reads them
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[bsel]);   // one arrival per softmax warp
     }
     if (ok) {
-      if (!mbar_wait(&pv_done[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, abort_flag)) { atomicExch(status, 20); ok = false; }
+      if (!mbar_wait(&pv_done[(n_it - 1) & (SB - 1)], ((n_it - 1) / SB) & 1, abort_flag)) { atomicExch(status, 20); ok = false; }
     }
     if (ok) {
       tc_fence_after();
       float inv = l > 0.f ? 1.0f / l : 0.f;
       if (!POOLED && sinks) inv = sink_quotient(m_used * 0.6931471805599453f, l, sinks[h0 + g]);
       if (gate && !gate_elem && row_valid) inv *= head_gate(gate, m_base + pi, gate_stride, h0 + g, 0, VD, 0);
-      uint4* orow = reinterpret_cast<uint4*>(out + ((m_base + pi) * nh + h0 + g) * VD);
-      uint32_t o[VD];
-      tmem_ld32(t_o + lane_base, o);
-      if (VD > 32) tmem_ld32(t_o + lane_base + 32, o + (VD > 32 ? 32 : 0));
-      tmem_ld_wait();
-      if (row_valid) {
+      constexpr int OW = WIDE ? VD : 32;      // numbers of the row at a time
 #pragma unroll
-        for (int c = 0; c < VD; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * inv);
+      for (int d0 = 0; d0 < VD; d0 += OW) {
+        uint4* orow = reinterpret_cast<uint4*>(out + ((m_base + pi) * nh + h0 + g) * VD + d0);
+        uint32_t o[OW];
+        tmem_ld32(t_o + lane_base + d0, o);
+        if (OW > 32) tmem_ld32(t_o + lane_base + 32, o + (OW > 32 ? 32 : 0));
+        tmem_ld_wait();
+        if (!row_valid) continue;
+#pragma unroll
+        for (int c = 0; c < OW; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * inv);
         if (gate && gate_elem) {
-          const bf16* grow = gate + (m_base + pi) * (size_t)gate_stride + (h0 + g) * VD;
+          const bf16* grow = gate + (m_base + pi) * (size_t)gate_stride + (h0 + g) * VD + d0;
           if ((((uintptr_t)grow) & 15) == 0) {
 #pragma unroll
-            for (int c = 0; c < VD; c += 8) {
+            for (int c = 0; c < OW; c += 8) {
               const uint4 w = *reinterpret_cast<const uint4*>(grow + c);
               const bf16* z = reinterpret_cast<const bf16*>(&w);
 #pragma unroll
@@ -373,7 +465,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
           } else {
 #pragma unroll
-            for (int c = 0; c < VD; c++)
+            for (int c = 0; c < OW; c++)
               o[c] = __float_as_uint(__fdividef(__uint_as_float(o[c]), 1.0f + __expf(-__bfloat162float(grow[c]))));
           }
         }
@@ -381,16 +473,16 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           // values were cached turned by their positions: the sum is turned back by the query's (pairs c, c + VD/2)
           const float fpos = (float)qpos;
 #pragma unroll
-          for (int c = 0; c < VD / 2; c++) {
+          for (int c = 0; c < OW / 2; c++) {
             float sn, cs;
             sincosf(fpos * freq_v[c], &sn, &cs);
-            const float a = __uint_as_float(o[c]), bb = __uint_as_float(o[c + VD / 2]);
+            const float a = __uint_as_float(o[c]), bb = __uint_as_float(o[c + OW / 2]);
             o[c] = __float_as_uint(a * cs + bb * sn);
-            o[c + VD / 2] = __float_as_uint(bb * cs - a * sn);
+            o[c + OW / 2] = __float_as_uint(bb * cs - a * sn);
           }
         }
 #pragma unroll
-        for (int c = 0; c < VD; c += 8) {
+        for (int c = 0; c < OW; c += 8) {
           uint4 w;
           uint32_t* wp = reinterpret_cast<uint32_t*>(&w);
 #pragma unroll
@@ -405,7 +497,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) tmem_dealloc(tmem, 256);
+  if (warp == 4) tmem_dealloc(tmem, AtcShape<WIDE>::COLUMNS);
 }
 
 LEB_API int leb_attention_prefill_tc_supported(int nh, int nkv, int hd, int page_size) {
@@ -446,7 +538,7 @@ static int launch_attention_prefill_tc(const char* who, void* out, const void* q
   }
   dim3 grid(nkv, ceil_div(max_qlen, TP), B);
   LEB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "%s: grid too large", who);
-  const size_t smem = 1024 + 128 * 64 * 2 + ATC_STAGES * (64 + VD) * 64 * 2;
+  const size_t smem = 1024 + 128 * 64 * 2 + AtcShape<WIDE>::STAGES * (64 + VD) * 64 * 2 + (WIDE ? 0 : 128 * 64 * 2);
 #define LEB_ATC(GS_)                                                                                              \
   {                                                                                                               \
     static bool set = false;                                                                                      \
