@@ -31,11 +31,11 @@ __device__ __forceinline__ void store_value_tile(
     const int* __restrict__ row_pos, const int* __restrict__ seq_slot, int M, int nkv, int hd,
     int page_size, int v_norm, float eps, int vin) {      // hd: the head's width in the pool; vin <= hd: in v_in (the rest is stored as zeros)
   constexpr int LD = VT_DIMS + (sizeof(CT) == 2 ? 2 : 1);     // odd number of 32-bit words
-  __shared__ CT tile[VT_ROWS * LD];
+  __shared__ __align__(16) CT tile[VT_ROWS * LD];
   __shared__ long long dst[VT_ROWS];                          // element offset of (row, dim 0), or -1
   __shared__ float rs[VT_ROWS];                               // 1 / root mean square of the row's head, or 1
   const int kvh = t % nkv, m0 = (t / nkv) * VT_ROWS;
-  if (threadIdx.x < VT_ROWS) {
+  if (threadIdx.x < VT_ROWS) {      // (the blocks of every launch have 256 threads)
     int m = m0 + threadIdx.x;
     long long off = -1;
     if (m < M) {
@@ -46,6 +46,36 @@ __device__ __forceinline__ void store_value_tile(
       }
     }
     dst[threadIdx.x] = off;
+  }
+  // Heads of 64 as they are (bfloat16): 16 bytes a thread in, and where eight rows are eight positions of a page from a
+  // multiple of eight on, as in most of a prompt, 16 bytes a thread out.
+  if (sizeof(T) == 2 && sizeof(CT) == 2 && hd == VT_DIMS && vin == hd && !v_norm && kv_stride % 8 == 0 &&
+      (((uintptr_t)v_in | (uintptr_t)v_pool) & 15) == 0) {
+    const int r = threadIdx.x >> 3, c = threadIdx.x & 7;      // 256 threads: 32 rows of eight pieces
+    if (m0 + r < M) {
+      const uint4 v = *reinterpret_cast<const uint4*>(v_in + (size_t)(m0 + r) * kv_stride + (size_t)kvh * vin + c * 8);
+      uint32_t* t = reinterpret_cast<uint32_t*>(tile + r * LD + c * 8);      // rows are an odd number of words apart
+      t[0] = v.x, t[1] = v.y, t[2] = v.z, t[3] = v.w;
+    }
+    __syncthreads();
+    const int d = threadIdx.x & 63, r0 = (threadIdx.x >> 6) * 8;
+    const long long first = dst[r0];
+    bool run = first >= 0 && first % 8 == 0;
+#pragma unroll
+    for (int e = 1; e < 8; e++) run = run && dst[r0 + e] == first + e;
+    // (eight positions from a multiple of eight on lie in one page: pages are multiples of eight positions, checked below)
+    if (run && page_size % 8 == 0) {
+      uint4 o;
+      CT* op = reinterpret_cast<CT*>(&o);
+#pragma unroll
+      for (int e = 0; e < 8; e++) op[e] = tile[(r0 + e) * LD + d];
+      *reinterpret_cast<uint4*>(v_pool + first + (size_t)d * page_size) = o;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        if (dst[r0 + e] >= 0) v_pool[dst[r0 + e] + (size_t)d * page_size] = tile[(r0 + e) * LD + d];
+    }
+    return;
   }
   // values divided by their root mean square over the head (no weight) where the layer asks for it
   for (int r = threadIdx.x >> 5; r < VT_ROWS; r += blockDim.x >> 5) {
@@ -259,6 +289,116 @@ __global__ void __launch_bounds__(ROPE_WARPS * 32) qk_rope_store_lanes_kernel(
   }
 }
 
+// The same for steps of many rows (bfloat16, split halves over a whole head of 64, 16-byte aligned rows): bound by memory,
+// so a thread moves 16 bytes at a time.  Four neighbouring lanes hold a head, each eight numbers of its first half
+// and the eight they turn with; a block takes R rows and forms their sines and cosines once, in shared
+// memory, for all heads (the kernel above: 2 bytes a lane and access, and sines once per warp).  Operations and their order are
+// those of the kernel above (of its butterfly over 32 lanes two steps are over lanes here, three over a lane's own
+// numbers), so the results are the same bit for bit.
+template <int R>
+__global__ void __launch_bounds__(256) qk_rope_store_many_kernel(
+    bf16* __restrict__ q_out, const bf16* __restrict__ q_in, int q_stride, const bf16* __restrict__ k_in,
+    const bf16* __restrict__ v_in, int kv_stride, bf16* __restrict__ k_pool, bf16* __restrict__ v_pool,
+    const int* __restrict__ block_table, int bt_width,
+    const int* __restrict__ row_seq, const int* __restrict__ row_pos, const int* __restrict__ seq_slot,
+    const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float eps,
+    const float* __restrict__ inv_freq, int M, int nh, int nkv, int page_size, int vd, int v_norm, int vin,
+    float temp_coef, float temp_every) {
+  constexpr int HD = 64, HALF = 32;
+  __shared__ __align__(16) float cs[R][2][HALF];
+  __shared__ long long kdst[R];
+  __shared__ float factor[R];
+  pdl_trigger();   // the kernel after this one may start and wait (see common.cuh)
+  pdl_wait();
+  const int groups = (M + R - 1) / R;
+  if ((int)blockIdx.x >= groups) {
+    store_value_tile<bf16, bf16>(blockIdx.x - groups, v_in, kv_stride, v_pool, block_table, bt_width, row_seq, row_pos,
+                                 seq_slot, M, nkv, vd, page_size, v_norm, eps, vin);
+    return;
+  }
+  const int m0 = blockIdx.x * R, rows = min(R, M - m0);
+  for (int i = threadIdx.x; i < rows * HALF; i += 256) {
+    const int r = i / HALF, p = i % HALF;
+    const float th = inv_freq ? (float)row_pos[m0 + r] * inv_freq[p] : 0.f;     // no rotation: turned by zero
+    cs[r][0][p] = cosf(th);
+    cs[r][1][p] = sinf(th);
+  }
+  if ((int)threadIdx.x < rows) {
+    const int m = m0 + threadIdx.x, b = row_seq[m], pos = row_pos[m];
+    long long off = -1;
+    if (k_in && seq_slot[b] >= 0) {
+      const int page = block_table[(size_t)b * bt_width + pos / page_size];
+      if (page >= 0) off = ((long long)page * nkv * page_size + pos % page_size) * HD;
+    }
+    kdst[threadIdx.x] = off;
+    factor[threadIdx.x] = query_temperature(pos, temp_coef, temp_every);
+  }
+  __syncthreads();
+  const int d0 = 8 * (threadIdx.x & 3);
+  float wq[16], wk[16];
+#pragma unroll
+  for (int e = 0; e < 16; e++) {
+    const int d = d0 + (e & 7) + (e >> 3) * HALF;
+    wq[e] = q_norm_w ? q_norm_w[d] : 1.f;
+    wk[e] = k_norm_w ? k_norm_w[d] : 1.f;
+  }
+  const int per_row = nh + (k_in ? nkv : 0), total = rows * per_row;
+#pragma unroll 2
+  for (int i0 = threadIdx.x / 4; i0 < (total + 7) / 8 * 8; i0 += 64) {     // whole warps together: the shuffles take all lanes
+    const bool in = i0 < total;
+    const int r = in ? i0 / per_row : 0, head = in ? i0 - r * per_row : 0;
+    const bool is_q = head < nh;
+    const bf16* src = is_q ? q_in + (size_t)(m0 + r) * q_stride + (size_t)head * HD
+                           : k_in + (size_t)(m0 + r) * kv_stride + (size_t)(head - nh) * HD;
+    const uint4 lo = *reinterpret_cast<const uint4*>(src + d0), hi = *reinterpret_cast<const uint4*>(src + HALF + d0);
+    const bf16 *le = reinterpret_cast<const bf16*>(&lo), *he = reinterpret_cast<const bf16*>(&hi);
+    float a[8], b[8], ss[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      a[e] = to_f32(le[e]);
+      b[e] = to_f32(he[e]);
+      ss[e] = fmaf(b[e], b[e], a[e] * a[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++) ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 2);
+#pragma unroll
+    for (int e = 0; e < 8; e++) ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 1);
+    const float sum = ((ss[0] + ss[4]) + (ss[2] + ss[6])) + ((ss[1] + ss[5]) + (ss[3] + ss[7]));
+    if (!in || (!is_q && kdst[r] < 0)) continue;
+    if (is_q ? q_norm_w != nullptr : k_norm_w != nullptr) {
+      const float inv = 1.0f / sqrtf(sum / (float)HD + eps);
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        a[e] = a[e] * inv * (is_q ? wq[e] : wk[e]);
+        b[e] = b[e] * inv * (is_q ? wq[e + 8] : wk[e + 8]);
+      }
+    }
+    const float f = is_q ? factor[r] : 1.f;
+    uint4 olo, ohi;
+    uint32_t *lp = reinterpret_cast<uint32_t*>(&olo), *hp = reinterpret_cast<uint32_t*>(&ohi);
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      float x[2], y[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const float c = cs[r][0][d0 + e + u], sn = cs[r][1][d0 + e + u];
+        x[u] = a[e + u] * c - b[e + u] * sn;
+        y[u] = a[e + u] * sn + b[e + u] * c;
+        if (is_q) {
+          x[u] *= f;
+          y[u] *= f;
+        }
+      }
+      __nv_bfloat162 px = __floats2bfloat162_rn(x[0], x[1]), py = __floats2bfloat162_rn(y[0], y[1]);
+      lp[e >> 1] = *reinterpret_cast<uint32_t*>(&px);
+      hp[e >> 1] = *reinterpret_cast<uint32_t*>(&py);
+    }
+    bf16* dst = is_q ? q_out + ((size_t)(m0 + r) * nh + head) * HD : k_pool + kdst[r] + (size_t)(head - nh) * page_size * HD;
+    *reinterpret_cast<uint4*>(dst + d0) = olo;
+    *reinterpret_cast<uint4*>(dst + HALF + d0) = ohi;
+  }
+}
+
 // The same job where q and k are normed over their whole projected row (all heads at once, a weight per number of the
 // row) instead of head by head.  Block (m, 0): row m's q, block (m, 1): its k (sum of squares, norm, rotation, q out or
 // cache write); blocks (x >= M, 0): value tiles as above.
@@ -449,6 +589,20 @@ LEB_API int leb_qk_rope_store(void* q_out, const void* q_in, int q_stride, const
   int total = nh + (k_in ? nkv : 0);
   dim3 block(32 * ROPE_WARPS);
   if (dtype == LEB_BF16 && (inv_freq ? neox && rope_dim == hd : temp_coef != 0.f) && hin == hd && (hd == 64 || hd == 128)) {
+    // From some hundred rows on the launch is bound by memory, not by its start: 16 bytes a thread, where rows and
+    // pages allow it (40 heads of 64, values included: 200 rows 12.7 -> 10.7 us a launch, 2,048 25.1 -> 14.8, 16,384
+    // 169 -> 85, of which the bytes alone would take 31; below 128 rows the start of the launch is most of both).
+    if (hd == 64 && M >= 128 && q_stride % 8 == 0 && kv_stride % 8 == 0 &&
+        (((uintptr_t)q_out | (uintptr_t)q_in | (uintptr_t)k_in | (uintptr_t)k_pool) & 15) == 0) {
+      const bool big = M >= 8 * sm_count();      // eight rows a block once that leaves every SM one
+      const dim3 grid(ceil_div(M, big ? 8 : 2) + tiles);
+      leb_launch(big ? qk_rope_store_many_kernel<8> : qk_rope_store_many_kernel<2>, grid, block, 0, st,
+          (bf16*)q_out, (const bf16*)q_in, q_stride, (const bf16*)k_in, (const bf16*)v_in, kv_stride,
+          (bf16*)k_pool, (bf16*)v_pool, block_table, bt_width, row_seq, row_pos, seq_slot, q_norm_w,
+          k_norm_w, eps, inv_freq, M, nh, nkv, page_size, vd, v_norm, vin, temp_coef, temp_every);
+      LEB_CHECK_LAUNCH("leb_qk_rope_store");
+      return 0;
+    }
     // heads per warp: one while the launch is small, up to all of a row's over 8 warps
     int per_warp = 1;
     const long long n_sm = sm_count();

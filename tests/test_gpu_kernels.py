@@ -469,6 +469,47 @@ def test_qk_rope_store(dtype, nh, nkv, hd, rope_dim, lens):
         r0 += n
 
 
+@pytest.mark.parametrize("lens,nh,nkv,weights,rotate", [([128], 4, 2, True, True), ([60, 69], 5, 5, True, True),
+                                                        ([1, 200, 3], 32, 8, True, True), ([700, 485], 8, 2, True, True),
+                                                        ([129], 3, 1, False, True), ([130], 4, 4, True, False)])
+def test_qk_rope_store_of_many_rows_gives_the_bits_of_few(lens, nh, nkv, weights, rotate):
+    """Steps of 128 rows and more (blocks of two rows, from 8 rows an SM on of eight) against the same rows in steps of at most
+    60: q, the cached keys and the cached values, bit for bit.  Odd lengths, starts off the multiples of eight (values leave
+    in single numbers there and in runs of eight elsewhere), a padding sequence in front."""
+    hd, page, eps = 64, 64, 1e-4
+    M = sum(lens)
+    qkv = gen(M, (nh + 2 * nkv) * hd, seed=30, dtype=torch.bfloat16).to(DEV)
+    qn, kn = ((1 + 0.1 * gen(hd, seed=31)).to(DEV), (1 + 0.1 * gen(hd, seed=32)).to(DEV)) if weights else (None, None)
+    inv = torch.pow(torch.tensor(12345.0, dtype=torch.float64), -torch.arange(32, dtype=torch.float64) / 32).float().to(DEV) \
+        if rotate else None
+    pos0 = [0, 62, 5][:len(lens)]
+    slots = [-1, 0, 1] if len(lens) == 3 else list(range(len(lens)))
+    width = max(-(-(p + n) // page) for p, n in zip(pos0, lens))
+    n_pages = len(lens) * width + 1
+    table = np.random.default_rng(5).permutation(n_pages)[:len(lens) * width].astype(np.int32).reshape(len(lens), width)
+
+    def run(pieces):
+        """pieces: [(sequence, first row, rows)] per step"""
+        kp = torch.zeros(n_pages, nkv, page, hd, device=DEV, dtype=torch.bfloat16)
+        vp = torch.zeros(n_pages, nkv, hd, page, device=DEV, dtype=torch.bfloat16)
+        out = torch.zeros(M, nh * hd, device=DEV, dtype=torch.bfloat16)
+        for step in pieces:
+            lo = sum(lens[:step[0][0]]) + step[0][1]
+            n = sum(c for _, _, c in step)
+            batch = builder().build([slots[b] for b, _, _ in step], [[0] * c for _, _, c in step],
+                                    [pos0[b] + f for b, f, _ in step], [], {0: table[[b for b, _, _ in step]]})
+            r = qkv[lo:lo + n]
+            K().qk_rope_store(out[lo:lo + n], r[:, :nh * hd], r[:, nh * hd:(nh + nkv) * hd], r[:, (nh + nkv) * hd:], kp, vp,
+                              batch.tables[0], batch, qn, kn, eps, inv, hd if rotate else 0, True, nh, nkv, hd, page,
+                              **({} if rotate else {"temperature": (0.3, 7.0)}))
+        return out, kp, vp
+
+    whole = run([[(b, 0, n) for b, n in enumerate(lens)]])
+    parts = run([[(b, f, min(60, n - f))] for b, n in enumerate(lens) for f in range(0, n, 60)])
+    for a, b in zip(whole, parts):
+        assert torch.equal(a, b)
+
+
 # ---- attention ---------------------------------------------------------------------------------------
 def plain_attention(q, k, v, qpos, window, scale):
     """q [Tq, nh, hd], k/v [Tk, nkv, hd] (positions 0..Tk-1), qpos [Tq]."""
