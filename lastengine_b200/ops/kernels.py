@@ -1740,9 +1740,10 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
         return
     if scale is not None:
         raise KernelError("linear: a split norm goes with the decode products of up to SKINNY_M rows only")
-    if (not streaming and group_offsets is None and M >= PAIRS_MIN_ROWS and (N >= 4096 or K >= 4096)
+    if (not streaming and group_offsets is None and M >= PAIRS_MIN_ROWS
+            and (N >= 4096 or K >= 4096 or -(-M // 256) * -(-N // 256) >= PAIRS_MIN_TILES)
             and linear_tc2(out, x, w, epilogue)):
-        return      # many rows and a large weight matrix: 256 x 256 tiles on pairs of SMs
+        return      # many rows and a large weight matrix, or many tiles: 256 x 256 tiles on pairs of SMs
     if tc is not None and not streaming and group_offsets is None and M > SMALL_M and tc(out, x, w, epilogue):
         return
     if (not streaming and group_offsets is not None and E <= 256 and M > 16 * E and w.is_contiguous()
@@ -1982,6 +1983,10 @@ def linear_tc(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int
 
 
 PAIRS_MIN_ROWS = 1024   # rows from which the paired kernel is used (measured: 3-9% faster there, slower on small products)
+# ... and, for matrices of less than 4,096 either way, the tiles of 256 x 256 from which it is.  K = 2,048, a float sum: 64 tiles
+# (2,048 x 2,048) 19.9 us unpaired and 20.6 paired; 128 tiles 34.1 and 32.4; 192 tiles 49.7 and 46.4; 512 tiles 133 and 119;
+# bfloat16 results 29.3 and 29.4 at 128, 107.7 and 99.5 at 512.
+PAIRS_MIN_TILES = 128
 
 
 def linear_tc2(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = STORE) -> bool:
