@@ -109,6 +109,7 @@ def _declare(L) -> None:
         "leb_heads_to_rows": [P, P, I, I, I, I, P],
         "leb_latent_attention": [P, I, P, P, P, P, I, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P],
         "leb_latent_attention_mma_supported": [I, I, I],
+        "leb_latent_attention_mma_few": [I, I, I, I, I],
         "leb_gemm_bf16_any": [P, I, P, P, I, I, I, I, I, I, P, I, S, P],
         "leb_gated_residual": [P, P, P, I, I, P, P, I, P, F, I, I, P],
         "leb_stream_add": [P, P, P, I, I, P],
@@ -1336,20 +1337,26 @@ def _read_length(max_kvlen: int, window: int = 0, chunk: int = 0) -> int:
     return n
 
 
-def latent_attention_splits(batch, H: int, mma: bool = False, rank: int = 0, window: int = 0, chunk: int = 0) -> int:
+def latent_attention_few(H: int, rank: int, rot: int, page_size: int, wide: bool) -> bool:
+    """Whether the tensor-core latent attention of a decode step runs its kernel of 16 query vectors."""
+    return bool(lib().leb_latent_attention_mma_few(int(H), int(rank), int(rot), int(page_size), int(wide)))
+
+
+def latent_attention_splits(batch, H: int, mma: bool = False, rank: int = 0, window: int = 0, chunk: int = 0, few: bool = False) -> int:
     """Pieces the key range of a decode step is cut into so that the blocks fill the SMs (1 for prompts).
     The tensor-core kernel takes up to 64 heads in a block that is alone on its SM, the general one 8 in
     blocks of which an SM holds several; a piece is 128 cached rows (measured at 2,048 positions:
     16 pieces of 128 rows are the fastest cut at batch 1 and 8 for latents of 256 and of 512), 64 where a row
     reads up to 1,024 (a step of three such layers at batch 8: 0.377 -> 0.367 ms in a window of 1,024, 0.247 ->
     0.236 ms in one of 512).  A window seldom starts on a tile's border: it reaches into one tile more, which
-    gets a piece of its own instead of doubling the length of every piece."""
+    gets a piece of its own instead of doubling the length of every piece.  `few`: the kernel of 16 query vectors runs,
+    whose tiles are 64 rows: a piece is one of them."""
     if batch.max_qlen != 1:
         return 1
     blocks = batch.n_seqs * -(-H // (64 if mma else 8))
     want = max(1, ((1 if mma else 2) * sm_count()) // max(1, blocks))
     n = _read_length(batch.max_kvlen, window, chunk)
-    piece = 64 if n <= 1024 and n < batch.max_kvlen else 128
+    piece = 64 if few or (n <= 1024 and n < batch.max_kvlen) else 128
     spare = 63 if n < batch.max_kvlen else 0
     return int(max(1, min(want, -(-(n + spare) // piece), 64)))
 

@@ -347,6 +347,44 @@ def test_decoding_with_the_key_range_cut_into_pieces_for_the_blocks(dtype):
         assert H.rel_err(torch.cat(got[j]), want[j][-4:]) < TOL[dtype]
 
 
+@pytest.mark.parametrize("H_,rank,rot,window,wide", [(1, 64, 0, 0, False), (5, 128, 16, 0, False), (16, 512, 64, 0, False),
+                                                     (16, 192, 64, 100, False), (9, 512, 128, 70, True), (16, 256, 32, 0, True)])
+@pytest.mark.parametrize("splits", [1, 3, 16])
+def test_latent_decode_of_few_heads(H_, rank, rot, window, wide, splits):
+    """The decode kernel of up to 16 query vectors: lengths at the borders of its tiles of 64, pieces without a row, a padding
+    sequence, windows that begin inside a tile, with and without a sink.  Weights and results are bfloat16 (2^-9 each
+    of the largest value; `wide` weights 2^-17): 8e-3 of the largest result bounds both."""
+    from lastengine_b200.engine.batch import BatchBuilder
+    assert K().latent_attention_few(H_, rank, rot, 64, wide)
+    assert not K().latent_attention_few(17, rank, rot, 64, wide) and not K().latent_attention_few(H_, 96, rot, 64, wide)
+    g = torch.Generator().manual_seed(rank + rot)
+    lens, page, scale = [1, 63, 64, 65, 700, 128, 9], 64, (rank + rot) ** -0.5
+    B, width = len(lens), 11
+    slots = list(range(B - 1)) + [-1]
+    pool = torch.randn(B * width + 1, page, rank + rot, generator=g).to(torch.bfloat16)
+    table = np.random.default_rng(3).permutation(B * width + 1)[:B * width].astype(np.int32).reshape(B, width)
+    qt = torch.randn(H_, B, rank, generator=g).to(torch.bfloat16)
+    qr = torch.randn(B, H_, rot, generator=g).to(torch.bfloat16)
+    sink = torch.randn(H_, generator=g) if H_ != 5 else None
+    batch = BatchBuilder(torch.device(DEV)).build(slots, [[0]] * B, [n - 1 for n in lens], [], {0: table})
+    out = torch.full((H_, B, rank), float("nan"), device=DEV, dtype=torch.bfloat16)
+    scratch = torch.empty(B * H_ * splits * (rank + 2), device=DEV) if splits > 1 else None
+    K().latent_attention(out, qt.to(DEV), qr.to(DEV), pool.to(DEV), batch.tables[0], batch, None if sink is None else sink.to(DEV),
+                         rank, rot, page, scale, n_splits=splits, scratch=scratch, window=window, wide=wide)
+    for b, n in enumerate(lens):
+        if slots[b] < 0:
+            assert not out[:, b].any()
+            continue
+        rows = pool[table[b].astype(np.int64)].reshape(-1, rank + rot)[:n].double()
+        lo = max(0, n - window) if window else 0
+        s = (torch.cat([qt[:, b], qr[b]], -1).double() @ rows[lo:].T) * scale
+        if sink is not None:
+            s = torch.cat([s, sink.double()[:, None]], -1)
+        want = torch.softmax(s, -1)[:, :n - lo] @ rows[lo:, :rank]
+        got = out[:, b].double().cpu()
+        assert float((got - want).abs().max() / want.abs().max()) < 8e-3
+
+
 def test_a_layer_reads_the_rows_another_layer_cached():
     D = 40
     m0 = lat(2, 16, 8, 24, 24, 32, 0.2, 5000.0)
