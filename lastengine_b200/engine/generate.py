@@ -50,7 +50,9 @@ class GenerationResult:
 class Backend(Protocol):
     def start(self, prompts: list[list[int]], u01: list[float] | None,
               histories: list[list[int]] | None) -> tuple[list[int], list[int]]:
-        """Allocates a slot per prompt, runs all prompts in one step; returns (slots, first tokens)."""
+        """Allocates a slot per prompt, runs all prompts in one step; returns (slots, first tokens).  A
+        backend with a true attribute `start_lookahead` also takes `lookahead` as `decode` does: the first
+        decode step's, under the same promise."""
 
     def decode(self, slots: list[int], tokens: list[int], u01: list[float] | None,
                histories: list[list[int]]) -> list[int]:
@@ -135,7 +137,8 @@ class GenerationLoop:
             t0 = self.clock()
             u = [r.rng.next() for r in batch] if draw else None
             slots, toks = self.backend.start([r.prompt for r in batch], u,
-                                             [r.history for r in batch] if want_hist else None)
+                                             [r.history for r in batch] if want_hist else None,
+                                             **self._lookahead(batch, draw, "start_lookahead"))
             stats.prefill_ms += (self.clock() - t0) * 1e3
             stats.prefill_tokens += sum(len(r.prompt) for r in batch)
             for r, s in zip(batch, slots):
@@ -152,6 +155,13 @@ class GenerationLoop:
                 raise
             stats.decode_ms += (self.clock() - t1) * 1e3
         return GenerationResult([r.out for r in reqs], [r.reason or "length" for r in reqs], stats)
+
+    def _lookahead(self, active, draw, which: str = "lookahead") -> dict:
+        """What a backend that runs ahead is told with a step whose uniform numbers are drawn already."""
+        if not getattr(self.backend, which, False):
+            return {}
+        return {"lookahead": ([r.rng.peek() for r in active] if draw else None,
+                              [len(r.out) + 1 < r.budget for r in active])}
 
     def _decode_batch(self, active, toks, stats, draw, want_hist):
         """One batch from its first tokens until its last request has ended."""
@@ -173,12 +183,8 @@ class GenerationLoop:
             if not active:
                 break
             u = [r.rng.next() for r in active] if draw else None
-            kw = {}
-            if getattr(self.backend, "lookahead", False):
-                kw["lookahead"] = ([r.rng.peek() for r in active] if draw else None,
-                                   [len(r.out) + 1 < r.budget for r in active])
             toks = self.backend.decode([r.slot for r in active], [r.out[-1] for r in active], u,
-                                       [r.history for r in active] if want_hist else None, **kw)
+                                       [r.history for r in active] if want_hist else None, **self._lookahead(active, draw))
             stats.decode_steps += 1
             stats.decode_tokens += len(active)
         return active
@@ -194,6 +200,7 @@ class EngineBackend:
         self.sampler = Sampler(sampling, engine.device)
         self._torch = torch
         self._host = torch.empty(1025, dtype=torch.int32, pin_memory=True)
+        self._starting: list[int] | None = None           # the slots of the prompts whose step is on the device
         self.d2h_bytes = 0
 
     def _choose(self, logits, u01_dev, histories) -> list[int]:
@@ -215,11 +222,15 @@ class EngineBackend:
             self.sampler.sample(out, logits, u01_dev)
             self._host[:1].copy_(kernels.status_and_tokens(dev, 0), non_blocking=True)
             self._host[1:n + 1].copy_(out, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
+        self._read_soon()
         self.d2h_bytes = (n + 1) * 4
         vals = self._host[:n + 1].tolist()
         kernels.raise_on_status(vals[0], dev)
         return vals[1:]
+
+    def _read_soon(self) -> None:
+        """Called once the copy of a step's tokens to the host is on the stream; returns when they have arrived."""
+        self._torch.cuda.current_stream().synchronize()
 
     def _step(self, slots, tokens, u01, histories) -> list[int]:
         import numpy as np
@@ -238,6 +249,7 @@ class EngineBackend:
 
     def start(self, prompts, u01, histories):
         slots = [self.engine.new_sequence() for _ in prompts]
+        self._starting = slots
         try:
             return slots, self._step(slots, prompts, u01, histories)
         except Exception:

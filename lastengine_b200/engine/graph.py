@@ -11,6 +11,7 @@ steps cannot move what a graph points at.
 from __future__ import annotations
 
 import gc
+from dataclasses import replace
 
 import numpy as np
 import torch
@@ -227,7 +228,7 @@ class GraphBackend(EngineBackend):
     tokens are those they would have got without it.
     """
 
-    lookahead = True
+    lookahead = start_lookahead = True
 
     def __init__(self, engine, sampling: SamplingParams, max_batch: int = 64, max_seq_len: int | None = None):
         super().__init__(engine, sampling)
@@ -239,12 +240,19 @@ class GraphBackend(EngineBackend):
         # pages), not the cache's capacity: the decode attention chooses its split for the width,
         # and a short sequence in a large cache must not be split and merged for lengths it has not.
         store = engine.__dict__.setdefault("_decode_graphs", {})
-        self.graphs: dict = store.setdefault(sampling, {})
+        # The seed is not baked in (the numbers it gives come with every step): calls that differ in it alone share
+        # their graphs, which are also found under the last call's own parameters.
+        self.graphs: dict = store.setdefault(replace(sampling, seed=None), {})
+        for k in [k for k in store if k.seed is not None]:
+            store.pop(k, None)
+        store[sampling] = self.graphs
         self.h2d_bytes = 0
         self._ahead: _StepInFlight | None = None
         self._launched = 0
         self._held: list[tuple[int, list[int]]] = []     # (step number to wait for, slots to give back)
         self._fed: dict[int, int] = {}                    # slot -> the token the next step was given on the device
+        self._starting: list[int] | None = None           # the slots of the prompts whose step is on the device
+        self._start_lookahead = None                      # what `start` was told of the step after it
 
     def _chosen(self, n: int) -> torch.Tensor:
         """Where the steps put their chosen tokens: the buffer behind the device's status word (one
@@ -386,9 +394,10 @@ class GraphBackend(EngineBackend):
             grow = g.stage_prompts(slots, prompts, u01)
             g.launch()
             eng.cache.commit(grow)
-            host = self._hosts[0]
+            host = self._host
             host[:n + 1].copy_(kernels.status_and_tokens(eng.device, n), non_blocking=True)
-            torch.cuda.current_stream().synchronize()
+            self._starting = slots
+            self._read_soon()
             vals = host[:n + 1].tolist()
             kernels.raise_on_status(vals[0], eng.device)
             self.h2d_bytes = g.builder.last_h2d_bytes
@@ -397,10 +406,46 @@ class GraphBackend(EngineBackend):
             eng.release(slots)
             raise
 
-    def start(self, prompts, u01, histories):
+    def _read_soon(self) -> None:
+        """The first decode step is staged and launched before the prompts' tokens are waited for: it takes
+        them on the device, and the host's part of it (0.2 ms) runs under the prompts' kernels."""
+        slots, look = self._starting, self._start_lookahead
+        if slots is None or look is None:
+            super()._read_soon()
+            return
+        copied = torch.cuda.Event()
+        copied.record()
+        self._start_lookahead = None
+        next_u01, goes_on = look
+        keep = [i for i, c in enumerate(goes_on) if c]
+        if keep:
+            try:
+                self._ahead = self._launch([slots[i] for i in keep], None,
+                                           [next_u01[i] for i in keep] if next_u01 is not None else None, keep)
+            except CacheFull:
+                self._ahead = None      # no room to run ahead: the first step is staged when it is asked for
+        copied.synchronize()
+
+    def start(self, prompts, u01, histories, lookahead=None):
+        """`lookahead` as in `decode`, for the first decode step.  Runs ahead only where the prompts' tokens lie in the
+        buffer that the decode steps take theirs from, and no penalties wait for them on the host."""
         self._drain()
-        captured = self._start_captured(prompts, u01)
-        slots, toks = captured if captured is not None else super().start(prompts, u01, histories)
+        b = bucket_for(max(1, len(prompts)))
+        self._starting = None
+        self._start_lookahead = lookahead if (b <= kernels.RESULT_TOKENS and not self.sampler.params.has_penalties
+                                              and lookahead is not None
+                                              and (lookahead[0] is not None or not self.sampler.needs_uniform())) else None
+        try:
+            captured = self._start_captured(prompts, u01)
+            slots, toks = captured if captured is not None else super().start(prompts, u01, histories)
+        except BaseException:
+            # the step ahead belongs to slots that have been given back: nothing of it is read, and it has ended
+            self._ahead = None
+            torch.cuda.synchronize(self.engine.device)
+            raise
+        finally:
+            self._starting = self._start_lookahead = None
+        self._fed = dict(zip(slots, toks)) if self._ahead is not None else {}
         h = self._history()
         if h is not None:
             # the rings of the new sequences: their last tokens, the first chosen one among them

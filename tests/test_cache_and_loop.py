@@ -322,6 +322,32 @@ def test_loop_look_ahead_is_a_promise_it_keeps(temperature):
     assert a == g.next() and g.peek() != a
 
 
+class LookingAheadFromTheStart(LookingAhead):
+    """... and the one the loop gives with the prompts, for the first decode step."""
+    start_lookahead = True
+
+    def start(self, prompts, u01, histories, lookahead=None):
+        slots, toks = super().start(prompts, u01, histories)
+        assert lookahead is not None
+        nu, goes_on = lookahead
+        self.promised = (dict(zip(slots, nu)) if nu is not None else None,
+                         {s for s, c in zip(slots, goes_on) if c}, dict(zip(slots, toks)))
+        return slots, toks
+
+
+@pytest.mark.parametrize("temperature", [0.0, 0.8])
+@pytest.mark.parametrize("budget", [1, 2, 4])
+def test_loop_look_ahead_begins_with_the_prompts(temperature, budget):
+    script = {0: [5, 6, 99, 7], 1: [99], 2: [1, 2, 3, 4, 5, 6], 3: [8, 8, 8, 8, 8, 8], 4: [9, 99]}
+    prompts, sp = [[0, 50], [1], [2, 50, 51], [3], [4, 1, 2, 3]], SamplingParams(temperature=temperature, seed=3)
+    logs = []
+    for kind in (LookingAheadFromTheStart, Scripted):
+        be = kind(script)
+        res = GenerationLoop(be, sp, max_new_tokens=budget, stop_token_ids=[99], max_batch=3).run(prompts)
+        logs.append((res.tokens, be.log))
+    assert logs[0] == logs[1]
+
+
 def test_plan_batches_respects_cache_room():
     assert plan_batches([10, 10, 10], [5, 5, 5], max_batch=2, token_budget=1000, page=64) == [[0, 1], [2]]
     assert plan_batches([60, 60, 60], [10, 10, 10], max_batch=8, token_budget=256, page=64) == [[0, 1], [2]]

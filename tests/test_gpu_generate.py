@@ -57,6 +57,30 @@ def test_greedy_generation_matches_plain(name, cfg, lens, steps, dtype, bf16, ga
     eng.cache.check()
 
 
+@pytest.mark.parametrize("lens,room", [([5, 20, 33], 2048), ([300, 280], 2048), ([40, 24], 128)])
+def test_first_decode_step_runs_ahead_of_the_prompts_tokens(lens, room, dirs):
+    """The first decode step is launched before the prompts' tokens are read (captured prompts, and uncaptured ones of more
+    rows): requests that end at their first token, by a stop token or by their budget, leave as they do without graphs,
+    and so do calls without room to run ahead."""
+    from lastengine_b200 import Engine, SamplingParams
+    eng = Engine.from_pretrained(dirs["A"], dtype="float32", max_tokens=room)
+    prompts = H.requests_for(TINY_A, lens, 51)
+    greedy = SamplingParams(temperature=0.0)
+    first = [t[0] for t in eng.generate(prompts, greedy, max_new_tokens=1, stop_token_ids=[]).tokens]
+    for sp in (greedy, SamplingParams(temperature=0.9, seed=5)):
+        for new, stop in ((1, []), (2, []), (5, first[:1]), (5, first), (24, [])):
+            a = eng.generate(prompts, sp, max_new_tokens=new, stop_token_ids=stop, use_graphs=True)
+            b = eng.generate(prompts, sp, max_new_tokens=new, stop_token_ids=stop, use_graphs=False)
+            assert a.tokens == b.tokens and a.finish_reasons == b.finish_reasons
+            assert eng.cache.slots.n_held == 0
+    # calls that differ in their seed alone share their captured graphs
+    n = len(eng._decode_graphs[SamplingParams(temperature=0.9)])
+    eng.generate(prompts, SamplingParams(temperature=0.9, seed=6), max_new_tokens=2, stop_token_ids=[])
+    assert len(eng._decode_graphs[SamplingParams(temperature=0.9)]) == n
+    assert sum(k.seed is not None for k in eng._decode_graphs) == 1
+    eng.cache.check()
+
+
 def test_sampling_is_seeded_and_independent_of_batching(dirs):
     from lastengine_b200 import Engine, SamplingParams
     eng = Engine.from_pretrained(dirs["A"], dtype="float32", max_tokens=1024)
