@@ -114,7 +114,7 @@ __global__ void shortconv_rows_bf16x8_kernel(bf16* __restrict__ y, const bf16* _
 // rows and keeps the last LC-1 products B*x in registers, so each row's B, C and x are loaded
 // once instead of LC times.  Taps, bias and order of the sum are those of the kernels above, so
 // the results are the same bit for bit.
-constexpr int CONV_CHUNK = 8;
+constexpr int CONV_CHUNK = 8, CONV_BATCH = 4;
 
 __device__ __forceinline__ void conv_mul8(float* o, const uint4& a, const uint4& b) {
   const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a);
@@ -155,51 +155,64 @@ __global__ void __launch_bounds__(128) shortconv_rows_bf16x8_chunk_kernel(
       for (int e = 0; e < 8; e++) hist[k][e] = 0.f;
     }
   }
+  // Rows in batches: the loads of a batch, and where its rows stand in their sequences, go out together (clamped to the last
+  // row, so that none hangs on a branch); row by row, each waited for its own chain of them (2,048 channels: 16,384 rows
+  // 80 -> 68 us, 9,681 54 -> 45, 2,048 16 -> 15 with the state's kernel).
 #pragma unroll
-  for (int rr = 0; rr < CONV_CHUNK; rr++) {
-    const int m = m0 + rr;
-    if (m >= M) break;
-    const bf16* r = bcx + (size_t)m * 3 * D;
-    const uint4 Bv = *reinterpret_cast<const uint4*>(r + ch0);
-    const uint4 Cv = *reinterpret_cast<const uint4*>(r + D + ch0);
-    const uint4 Xv = *reinterpret_cast<const uint4*>(r + 2 * D + ch0);
-    const int b = row_seq[m];
-    const int slot = seq_slot[b];
-    const int i = m - seq_qstart[b];
-    float cur[8], acc[8];
-    conv_mul8(cur, Bv, Xv);
+  for (int r0 = 0; r0 < CONV_CHUNK; r0 += CONV_BATCH) {
+    if (m0 + r0 >= M) break;
+    uint4 Bv[CONV_BATCH], Cv[CONV_BATCH], Xv[CONV_BATCH];
+    int slot[CONV_BATCH], at[CONV_BATCH];
 #pragma unroll
-    for (int e = 0; e < 8; e++) acc[e] = bs[e];
+    for (int u = 0; u < CONV_BATCH; u++) {
+      const int m = min(m0 + r0 + u, M - 1);
+      const bf16* r = bcx + (size_t)m * 3 * D;
+      Bv[u] = *reinterpret_cast<const uint4*>(r + ch0);
+      Cv[u] = *reinterpret_cast<const uint4*>(r + D + ch0);
+      Xv[u] = *reinterpret_cast<const uint4*>(r + 2 * D + ch0);
+      const int b = row_seq[m];
+      slot[u] = seq_slot[b];
+      at[u] = m - seq_qstart[b];
+    }
 #pragma unroll
-    for (int j = 0; j < LC - 1; j++) {
-      const int src = i - (LC - 1) + j;  // row of this sequence in this step; negative: before it
-      if (src >= 0) {
+    for (int u = 0; u < CONV_BATCH; u++) {
+      const int m = m0 + r0 + u;
+      if (m >= M) break;
+      float cur[8], acc[8];
+      conv_mul8(cur, Bv[u], Xv[u]);
 #pragma unroll
-        for (int e = 0; e < 8; e++) acc[e] += wt[j][e] * hist[j][e];
-      } else if (slot >= 0) {
+      for (int e = 0; e < 8; e++) acc[e] = bs[e];
 #pragma unroll
-        for (int e = 0; e < 8; e++)
-          acc[e] += wt[j][e] * state[((size_t)slot * D + ch0 + e) * (LC - 1) + (LC - 1) + src];
+      for (int j = 0; j < LC - 1; j++) {
+        const int src = at[u] - (LC - 1) + j;  // row of this sequence in this step; negative: before it
+        if (src >= 0) {
+#pragma unroll
+          for (int e = 0; e < 8; e++) acc[e] += wt[j][e] * hist[j][e];
+        } else if (slot[u] >= 0) {
+#pragma unroll
+          for (int e = 0; e < 8; e++)
+            acc[e] += wt[j][e] * state[((size_t)slot[u] * D + ch0 + e) * (LC - 1) + (LC - 1) + src];
+        }
       }
+      const __nv_bfloat162* Cp = reinterpret_cast<const __nv_bfloat162*>(&Cv[u]);
+      uint4 o;
+      uint32_t* op = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float2 cf = __bfloat1622float2(Cp[e]);
+        __nv_bfloat162 v = __floats2bfloat162_rn(cf.x * (acc[2 * e] + wt[LC - 1][2 * e] * cur[2 * e]),
+                                                 cf.y * (acc[2 * e + 1] + wt[LC - 1][2 * e + 1] * cur[2 * e + 1]));
+        op[e] = *reinterpret_cast<uint32_t*>(&v);
+      }
+      if (slot[u] < 0) o = make_uint4(0, 0, 0, 0);  // padding row
+      *reinterpret_cast<uint4*>(y + (size_t)m * D + ch0) = o;
+#pragma unroll
+      for (int k = 0; k + 1 < LC - 1; k++)
+#pragma unroll
+        for (int e = 0; e < 8; e++) hist[k][e] = hist[k + 1][e];
+#pragma unroll
+      for (int e = 0; e < 8; e++) hist[LC - 2][e] = cur[e];
     }
-    const __nv_bfloat162* Cp = reinterpret_cast<const __nv_bfloat162*>(&Cv);
-    uint4 o;
-    uint32_t* op = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const float2 cf = __bfloat1622float2(Cp[e]);
-      __nv_bfloat162 v = __floats2bfloat162_rn(cf.x * (acc[2 * e] + wt[LC - 1][2 * e] * cur[2 * e]),
-                                               cf.y * (acc[2 * e + 1] + wt[LC - 1][2 * e + 1] * cur[2 * e + 1]));
-      op[e] = *reinterpret_cast<uint32_t*>(&v);
-    }
-    if (slot < 0) o = make_uint4(0, 0, 0, 0);  // padding row
-    *reinterpret_cast<uint4*>(y + (size_t)m * D + ch0) = o;
-#pragma unroll
-    for (int k = 0; k + 1 < LC - 1; k++)
-#pragma unroll
-      for (int e = 0; e < 8; e++) hist[k][e] = hist[k + 1][e];
-#pragma unroll
-    for (int e = 0; e < 8; e++) hist[LC - 2][e] = cur[e];
   }
 }
 
