@@ -52,14 +52,14 @@ __device__ __forceinline__ void latent_cache_row(const T* __restrict__ lat, int 
                                                  const float* __restrict__ inv_freq, int rot_dims, int neox, int rank, int rot,
                                                  int page_size, float* red) {
   const int b = row_seq[m], pos = row_pos[m];
+  if (seq_slot[b] < 0) return;      // a padding sequence touches no cache
+  const int page = block_table[(size_t)b * bt_width + pos / page_size];      // (on its way under the sum)
   float ss = 0.f;
   for (int i = threadIdx.x; i < rank; i += blockDim.x) {
     const float v = to_f32(lat[i]);
     ss += v * v;
   }
   ss = block_sum(ss, red);
-  if (seq_slot[b] < 0) return;      // a padding sequence touches no cache
-  const int page = block_table[(size_t)b * bt_width + pos / page_size];
   if (page < 0) return;
   const float r = 1.0f / sqrtf(ss / (float)rank + eps);
   CT* dst = pool + ((size_t)page * page_size + pos % page_size) * (size_t)(rank + rot);
@@ -95,7 +95,8 @@ __device__ __forceinline__ void latent_split_row(T* __restrict__ qn, T* __restri
   }
 }
 
-// One block per row.  in [M, ld_in]: columns [0, q_rank) the query latent before its norm, then
+// Two blocks per row (one without a cache write): the query latent's norm, and the cache row, side by side (a
+// step of few rows waits for their chains of loads and block sums, not for bytes: 8 rows 12.7 -> 8.6 us).  in [M, ld_in]: columns [0, q_rank) the query latent before its norm, then
 // (own_kv) `rank` columns of the key/value latent before its norm and `rot` columns of the shared
 // key part before its rotation.  Leaves cq [M, q_rank] = rmsnorm(.) * wq and, for rows of live
 // sequences, the cache row [c | k^r] at the row's position.
@@ -111,16 +112,18 @@ latent_prep_kernel(T* __restrict__ cq, const T* __restrict__ in, int ld_in, CT* 
   pdl_wait();
   const int m = blockIdx.x;
   const T* row = in + (size_t)m * ld_in;
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < q_rank; i += blockDim.x) {
-    const float v = to_f32(row[i]);
-    ss += v * v;
+  if (blockIdx.y == 0) {
+    float ss = 0.f;
+    for (int i = threadIdx.x; i < q_rank; i += blockDim.x) {
+      const float v = to_f32(row[i]);
+      ss += v * v;
+    }
+    ss = block_sum(ss, red);
+    const float r = 1.0f / sqrtf(ss / (float)q_rank + eps);
+    for (int i = threadIdx.x; i < q_rank; i += blockDim.x)
+      cq[(size_t)m * q_rank + i] = from_f32<T>(to_f32(row[i]) * r * wq[i]);
+    return;
   }
-  ss = block_sum(ss, red);
-  const float r = 1.0f / sqrtf(ss / (float)q_rank + eps);
-  for (int i = threadIdx.x; i < q_rank; i += blockDim.x)
-    cq[(size_t)m * q_rank + i] = from_f32<T>(to_f32(row[i]) * r * wq[i]);
-  if (!pool) return;
   latent_cache_row<T, CT>(row + q_rank, m, pool, block_table, bt_width, row_seq, row_pos, seq_slot, wkv, eps, inv_freq, rot_dims,
                           neox, rank, rot, page_size, red);
 }
@@ -426,11 +429,11 @@ LEB_API int leb_latent_prep(void* cq, const void* in, int ld_in, int dtype, void
               "leb_latent_prep: %d rotated dimensions of %d", rot_dims, rot);
   LebPlainLaunches plain(true);
   if (dtype == LEB_F32)
-    leb_launch(latent_prep_kernel<float, float>, dim3(M), dim3(128), 0, st, (float*)cq, (const float*)in, ld_in,
+    leb_launch(latent_prep_kernel<float, float>, dim3(M, pool ? 2 : 1), dim3(256), 0, st, (float*)cq, (const float*)in, ld_in,
                (float*)pool, block_table, bt_width, row_seq, row_pos, seq_slot, wq, wkv, eps, inv_freq, rot_dims, neox,
                q_rank, rank, rot, page_size);
   else if (dtype == LEB_BF16)
-    leb_launch(latent_prep_kernel<bf16, bf16>, dim3(M), dim3(128), 0, st, (bf16*)cq, (const bf16*)in, ld_in,
+    leb_launch(latent_prep_kernel<bf16, bf16>, dim3(M, pool ? 2 : 1), dim3(256), 0, st, (bf16*)cq, (const bf16*)in, ld_in,
                (bf16*)pool, block_table, bt_width, row_seq, row_pos, seq_slot, wq, wkv, eps, inv_freq, rot_dims, neox,
                q_rank, rank, rot, page_size);
   else
