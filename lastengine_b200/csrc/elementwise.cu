@@ -90,12 +90,17 @@ rmsnorm_bf16_vec_kernel(bf16* __restrict__ out, const float* __restrict__ x, con
                         const int* __restrict__ rows, int D, float eps) {
   __shared__ float red[33];
   pdl_trigger();   // the kernel after this one may start and wait (see common.cuh)
+  const float4* w4 = reinterpret_cast<const float4*>(w);
+  const int n4 = D >> 2;
+  float4 v[CH], ww[CH];
+#pragma unroll
+  for (int c = 0; c < CH; c++) {      // the weights do not depend on the kernel before this one (1% of a step with a norm kernel per sublayer)
+    const int i = threadIdx.x + c * 256;
+    if (i < n4) ww[c] = w4[i];
+  }
   pdl_wait();
   const int m = blockIdx.x;
   const float4* xi = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[m] : m) * D);
-  const float4* w4 = reinterpret_cast<const float4*>(w);
-  const int n4 = D >> 2;
-  float4 v[CH];
   float s = 0.f;
 #pragma unroll
   for (int c = 0; c < CH; c++) {
@@ -112,9 +117,8 @@ rmsnorm_bf16_vec_kernel(bf16* __restrict__ out, const float* __restrict__ x, con
   for (int c = 0; c < CH; c++) {
     const int i = threadIdx.x + c * 256;
     if (i < n4) {
-      const float4 ww = w4[i];
-      __nv_bfloat162 lo = __floats2bfloat162_rn(v[c].x * r * ww.x, v[c].y * r * ww.y);
-      __nv_bfloat162 hi = __floats2bfloat162_rn(v[c].z * r * ww.z, v[c].w * r * ww.w);
+      __nv_bfloat162 lo = __floats2bfloat162_rn(v[c].x * r * ww[c].x, v[c].y * r * ww[c].y);
+      __nv_bfloat162 hi = __floats2bfloat162_rn(v[c].z * r * ww[c].z, v[c].w * r * ww[c].w);
       o[i] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
     }
   }
