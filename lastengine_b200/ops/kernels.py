@@ -7,6 +7,7 @@ the built library, or with tensors that are not on a CUDA device, raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_size_t, c_void_p
 
 import torch
@@ -1337,6 +1338,7 @@ def _read_length(max_kvlen: int, window: int = 0, chunk: int = 0) -> int:
     return n
 
 
+@functools.lru_cache(maxsize=256)
 def latent_attention_few(H: int, rank: int, rot: int, page_size: int, wide: bool) -> bool:
     """Whether the tensor-core latent attention of a decode step runs its kernel of 16 query vectors."""
     return bool(lib().leb_latent_attention_mma_few(int(H), int(rank), int(rot), int(page_size), int(wide)))
