@@ -20,7 +20,10 @@
 //
 // Block = 4 warps.  A block owns one sequence, one kv head, a chunk of HC <= 8 of its query
 // heads, QT rows (QT*HC <= 32 "query vectors") and one split of the key range.  Per tile of 32
-// keys, lane = key for q.k, lane = dimension for p.v.
+// keys, lane = key for q.k, lane = dimension for p.v.  A warp takes its up to 8 vectors through both products
+// together, so that a key's or value's number from shared memory meets 8 of them and theirs come four at a time:
+// vector by vector, with two shared loads to a multiply-add, the loads bound it (32-bit prompts of 190 and 333 rows, 32
+// heads of 64 over 8: 273 -> 155 us a layer; their decode step 121 -> 25 with twice the splits).
 #include "common.cuh"
 
 #define ATT_WARPS 4
@@ -37,7 +40,7 @@ attention_kernel(T* __restrict__ out, float* __restrict__ part, const T* __restr
                  const T* __restrict__ gate, int gate_stride, int gate_elem, int nh, int nkv, int hd, int vd,
                  int page_size, int window, int chunk, float scale, const float* __restrict__ slopes,
                  const float* __restrict__ sinks, int QT, int HC, int n_splits) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int G = nh / nkv;
   const int n_hc = (G + HC - 1) / HC;
@@ -54,10 +57,10 @@ attention_kernel(T* __restrict__ out, float* __restrict__ part, const T* __restr
   const int R = QT * HC;
   const int KS = hd + 1;  // stride of a staged key row: lanes read different rows, same column
 
-  float* q_s = sm;                 // [R][hd]
+  float* p_s = sm;                 // [ATT_WARPS][ATT_RPW][32]
+  float* q_s = p_s + ATT_WARPS * ATT_RPW * 32;   // [R][hd]
   float* k_s = q_s + R * hd;       // [32][hd + 1]
   float* v_s = k_s + 32 * KS;      // [32][vd]
-  float* p_s = v_s + 32 * vd;      // [ATT_WARPS][32]
 
   if (slot < 0) {  // padding sequence: defined output, no cache access
     for (int r = warp; r < R; r += ATT_WARPS) {
@@ -106,62 +109,138 @@ attention_kernel(T* __restrict__ out, float* __restrict__ part, const T* __restr
     for (int jj = 0; jj < HDL; jj++) acc[ri][jj] = 0.f;
   }
 
+  const int kk0 = threadIdx.x / hd, d0 = threadIdx.x % hd, kk_step = 32 * ATT_WARPS / hd, d_step = 32 * ATT_WARPS % hd;
+  const int kk_step4 = 128 * ATT_WARPS / hd, d_step4 = 128 * ATT_WARPS % hd;
+  const bool wide = (hd & 3) == 0 && (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;      // (pages are multiples of 32 positions)
   for (int tile = t_lo; tile < t_hi; tile++) {
     const int key0 = tile * 32;
     const int page = block_table[(size_t)b * bt_width + key0 / page_size];
     const size_t base = (((size_t)(page < 0 ? 0 : page) * nkv + kvh) * page_size + key0 % page_size) * hd;
     const size_t vbase = ((size_t)(page < 0 ? 0 : page) * nkv + kvh) * vd * page_size + key0 % page_size;
     __syncthreads();  // the previous tile has been consumed (and q_s is written, first time round)
-    for (int idx = threadIdx.x; idx < 32 * hd; idx += blockDim.x) {
-      int kk = idx / hd, d = idx - kk * hd;
-      float kv = 0.f;
-      if (page >= 0 && key0 + kk < kv_len) kv = to_f32(k_pool[base + idx]);  // beyond the sequence the pool holds stale bits
-      k_s[kk * KS + d] = kv;
-    }
-    for (int idx = threadIdx.x; idx < 32 * vd; idx += blockDim.x) {
-      int d = idx / 32, kk = idx - d * 32;                         // values are stored [dim][position]
-      float vv = 0.f;
-      if (page >= 0 && key0 + kk < kv_len) vv = to_f32(v_pool[vbase + (size_t)d * page_size + kk]);
-      v_s[kk * vd + d] = vv;
+    if (sizeof(CT) == 4 && wide) {
+      // four numbers a load, four loads in flight: a tile waits for two trips to L2 where single numbers took four and more
+      const int n4 = 32 * hd / 4;
+      int kk = 4 * threadIdx.x / hd, d = 4 * threadIdx.x % hd;
+#pragma unroll 4
+      for (int idx = threadIdx.x; idx < n4; idx += 32 * ATT_WARPS) {
+        const float4 kv = page >= 0 && key0 + kk < kv_len ? load4(k_pool + base + 4 * idx) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float* ks = k_s + kk * KS + d;
+        ks[0] = kv.x, ks[1] = kv.y, ks[2] = kv.z, ks[3] = kv.w;
+        kk += kk_step4;
+        d += d_step4;
+        if (d >= hd) d -= hd, kk++;
+      }
+#pragma unroll 4
+      for (int idx = threadIdx.x; idx < 8 * vd; idx += 32 * ATT_WARPS) {
+        const int dim = idx / 8, k4 = (idx & 7) * 4, left = page >= 0 ? kv_len - key0 - k4 : 0;      // live positions of the four
+        const float4 vv = left > 0 ? load4(v_pool + vbase + (size_t)dim * page_size + k4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float* vs = v_s + k4 * vd + dim;
+        vs[0] = left > 0 ? vv.x : 0.f, vs[vd] = left > 1 ? vv.y : 0.f, vs[2 * vd] = left > 2 ? vv.z : 0.f, vs[3 * vd] = left > 3 ? vv.w : 0.f;
+      }
+    } else {
+      int kk = kk0, d = d0;      // idx / hd and idx % hd, kept up without dividing
+#pragma unroll 8
+      for (int idx = threadIdx.x; idx < 32 * hd; idx += 32 * ATT_WARPS) {
+        float kv = 0.f;
+        if (page >= 0 && key0 + kk < kv_len) kv = to_f32(k_pool[base + idx]);  // beyond the sequence the pool holds stale bits
+        k_s[kk * KS + d] = kv;
+        kk += kk_step;
+        d += d_step;
+        if (d >= hd) d -= hd, kk++;
+      }
+#pragma unroll 8
+      for (int idx = threadIdx.x; idx < 32 * vd; idx += 32 * ATT_WARPS) {
+        int dim = idx / 32, pos = idx - dim * 32;                         // values are stored [dim][position]
+        float vv = 0.f;
+        if (page >= 0 && key0 + pos < kv_len) vv = to_f32(v_pool[vbase + (size_t)dim * page_size + pos]);
+        v_s[pos * vd + dim] = vv;
+      }
     }
     __syncthreads();
+    const float* kr = k_s + lane * KS;
+    float s[ATT_RPW], corr[ATT_RPW];
+#pragma unroll
+    for (int ri = 0; ri < ATT_RPW; ri++) s[ri] = 0.f;
+    if ((hd & 3) == 0) {
+      for (int d = 0; d < hd; d += 4) {
+        const float k0 = kr[d], k1 = kr[d + 1], k2 = kr[d + 2], k3 = kr[d + 3];
+#pragma unroll
+        for (int ri = 0; ri < ATT_RPW; ri++) {
+          const int r = warp + ri * ATT_WARPS;
+          if (r >= R) break;
+          const float4 qv = load4(q_s + r * hd + d);
+          s[ri] += qv.x * k0;
+          s[ri] += qv.y * k1;
+          s[ri] += qv.z * k2;
+          s[ri] += qv.w * k3;
+        }
+      }
+    } else {
+      for (int d = 0; d < hd; d++) {
+        const float k0 = kr[d];
+#pragma unroll
+        for (int ri = 0; ri < ATT_RPW; ri++) {
+          const int r = warp + ri * ATT_WARPS;
+          if (r >= R) break;
+          s[ri] += q_s[r * hd + d] * k0;
+        }
+      }
+    }
+    float* pw = p_s + warp * ATT_RPW * 32;
 #pragma unroll
     for (int ri = 0; ri < ATT_RPW; ri++) {
       const int r = warp + ri * ATT_WARPS;
       if (r >= R) break;
       const int i = r / HC, j = r % HC;
-      if (i >= nrows || j >= nheads) continue;
       const int qpos = pos0 + row_lo + i;
       const int lo = first_key(qpos, window, chunk);
-      if (key0 > qpos || key0 + 31 < lo) continue;   // the whole tile lies after this row, or before what it reads
-      const float* qv = q_s + r * hd;
-      const float* kr = k_s + lane * KS;
-      float s = 0.f;
-      for (int d = 0; d < hd; d++) s += qv[d] * kr[d];
-      s *= scale;
+      corr[ri] = 1.f;
+      // an idle vector, or the whole tile lies after this row or before what it reads: its sums stay as they are
+      if (i >= nrows || j >= nheads || key0 > qpos || key0 + 31 < lo) {
+        pw[ri * 32 + lane] = 0.f;
+        continue;
+      }
+      float sc = s[ri] * scale;
       const int kp = key0 + lane;
-      if (slopes) s -= slopes[kvh * G + hc * HC + j] * (float)(qpos - kp);
+      if (slopes) sc -= slopes[kvh * G + hc * HC + j] * (float)(qpos - kp);
       const bool valid = kp <= qpos && kp >= lo;
-      s = valid ? s : ATT_NEG;
-      const float mn = fmaxf(mx[ri], warp_max(s));
-      const float p = valid ? expf(s - mn) : 0.f;
-      const float corr = expf(mx[ri] - mn);
-      l[ri] = l[ri] * corr + warp_sum(p);
+      sc = valid ? sc : ATT_NEG;
+      const float mn = fmaxf(mx[ri], warp_max(sc));
+      const float p = valid ? expf(sc - mn) : 0.f;
+      corr[ri] = expf(mx[ri] - mn);
+      l[ri] = l[ri] * corr[ri] + warp_sum(p);
       mx[ri] = mn;
-      p_s[warp * 32 + lane] = p;
-      __syncwarp();
+      pw[ri * 32 + lane] = p;
+    }
+    __syncwarp();
 #pragma unroll
-      for (int jj = 0; jj < HDL; jj++) {
-        const int d = lane + 32 * jj;
-        if (d < vd) {
-          float a = 0.f;
-#pragma unroll 8
-          for (int kk = 0; kk < 32; kk++) a += p_s[warp * 32 + kk] * v_s[kk * vd + d];
-          acc[ri][jj] = acc[ri][jj] * corr + a;
+    for (int jj = 0; jj < HDL; jj++) {
+      const int d = lane + 32 * jj;
+      if (d >= vd) continue;
+      float a[ATT_RPW];
+#pragma unroll
+      for (int ri = 0; ri < ATT_RPW; ri++) a[ri] = 0.f;
+#pragma unroll 2
+      for (int kk = 0; kk < 32; kk += 4) {
+        const float v0 = v_s[kk * vd + d], v1 = v_s[(kk + 1) * vd + d], v2 = v_s[(kk + 2) * vd + d], v3 = v_s[(kk + 3) * vd + d];
+#pragma unroll
+        for (int ri = 0; ri < ATT_RPW; ri++) {
+          if (warp + ri * ATT_WARPS >= R) break;
+          const float4 pv = load4(pw + ri * 32 + kk);
+          a[ri] += pv.x * v0;
+          a[ri] += pv.y * v1;
+          a[ri] += pv.z * v2;
+          a[ri] += pv.w * v3;
         }
       }
-      __syncwarp();
+#pragma unroll
+      for (int ri = 0; ri < ATT_RPW; ri++) {
+        if (warp + ri * ATT_WARPS >= R) break;
+        acc[ri][jj] = acc[ri][jj] * corr[ri] + a[ri];
+      }
     }
+    __syncwarp();
   }
 
 #pragma unroll
@@ -253,7 +332,7 @@ static int launch_attention(void* out, float* part, const void* q, const void* k
   if (QT > max_qlen) QT = max_qlen;
   const int R = QT * HC;
   const int n_hc = ceil_div(G, HC);
-  size_t smem = ((size_t)R * hd + 32 * (hd + 1) + 32 * vd + ATT_WARPS * 32) * sizeof(float);
+  size_t smem = ((size_t)R * hd + 32 * (hd + 1) + 32 * vd + ATT_WARPS * ATT_RPW * 32) * sizeof(float);
   auto kern = attention_kernel<T, CT, HDL>;
   static size_t smem_set = 0;
   if (smem > 48 * 1024 && smem > smem_set) {

@@ -1399,7 +1399,8 @@ def sm_count() -> int:
     return n
 
 
-def attention_splits(batch, nkv: int, G: int, sm_count: int | None = None, hd: int = 64, chunk: int = 0, window: int = 0) -> int:
+def attention_splits(batch, nkv: int, G: int, sm_count: int | None = None, hd: int = 64, chunk: int = 0, window: int = 0,
+                     general: bool = False) -> int:
     """How many blocks share one sequence's key range in a decode step (1 for prompts).
 
     Measured on B200 (head size 64, 8 kv heads, times with the merge of the splits): a block has a
@@ -1409,7 +1410,9 @@ def attention_splits(batch, nkv: int, G: int, sm_count: int | None = None, hd: i
     positions 6 splits, 384 blocks, take 14.7 us a layer and 7 splits, 448 blocks, 18.8 us); and
     when the sequences alone fill the GPU twice over, splitting pays only for long ranges (64
     sequences of 640 positions: 20.3 us unsplit, 27.4 us in 4 splits; of 4,096 positions: 110 us
-    unsplit, 89 us in 4 splits).
+    unsplit, 89 us in 4 splits).  The general kernel (`general`: 32-bit caches) takes several times as long over a
+    position as the tensor-core kernel: beyond 128 positions half as many of them make a split worth its start (two sequences
+    of 190 and 333: 87 -> 25 us a layer with the wider loads of its tiles).
     """
     if batch.max_qlen != 1:
         return 1
@@ -1422,6 +1425,8 @@ def attention_splits(batch, nkv: int, G: int, sm_count: int | None = None, hd: i
     if per >= 2 * sm_count:
         return 1 if kv < 2048 else min(4, kv // 1024)
     least = 128 if per * 8 <= sm_count else 256       # one or two sequences: latency counts, shorter blocks pay
+    if general and kv > 128:
+        least //= 2
     return max(1, min(slots // per, kv // least, 32))
 
 

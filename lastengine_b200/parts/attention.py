@@ -272,7 +272,8 @@ class AttentionMixer(Mixer):
             kernels.qk_rope_store(q, qn, kn, vn, kp, vp, cache.block_table, batch, None, None, self.eps,
                                   None, 0, True, nh, nkv, hd, cache.page_size)
         o = ws.get("attn.o", (M, nh * kvd), env.dtype)
-        n_splits = kernels.attention_splits(batch, nkv, nh // nkv, hd=khd, chunk=self.chunk, window=self.window)
+        n_splits = kernels.attention_splits(batch, nkv, nh // nkv, hd=khd, chunk=self.chunk, window=self.window,
+                                            general=env.is_float32)
         scratch = None
         if n_splits > 1:
             scratch = ws.get("attn.part", (M * nh * n_splits * (max(khd, kvd) + 2),), torch.float32)
