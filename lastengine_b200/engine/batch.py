@@ -56,6 +56,14 @@ class BatchBuilder:
             self._host = torch.empty(cap, dtype=torch.int32, pin_memory=self.device.type == "cuda")
             self._dev = torch.empty(cap, dtype=torch.int32, device=self.device)
 
+    def _send(self, n: int) -> None:
+        """The first n words of the staging buffer to the device."""
+        if self.device.type == "cuda":
+            from ..ops import kernels
+            kernels.stage_words(self._dev, self._host, n)
+        else:
+            self._dev[:n].copy_(self._host[:n])
+
     def build(self, slots: list[int], tokens: list[list[int]] | list[np.ndarray], pos0: list[int],
               logit_rows: list[int], tables: dict[int, np.ndarray],
               u01: np.ndarray | None = None, feed: np.ndarray | None = None) -> StepBatch:
@@ -89,7 +97,7 @@ class BatchBuilder:
         host = self._host.numpy()
         for o, p in zip(offs, pieces):
             host[o:o + p.size] = p
-        self._dev[:total].copy_(self._host[:total], non_blocking=True)
+        self._send(total)
         if self.device.type == "cuda":
             if self._copied is None:
                 self._copied = torch.cuda.Event()
@@ -130,6 +138,6 @@ class BatchBuilder:
         if self._copied is not None:
             self._copied.synchronize()
         n = self.total if n_ints is None else n_ints
-        self._dev[:n].copy_(self._host[:n], non_blocking=True)
+        self._send(n)
         self._copied.record()
         self.last_h2d_bytes = n * 4

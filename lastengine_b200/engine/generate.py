@@ -216,7 +216,7 @@ class EngineBackend:
             self.sampler.apply_penalties(logits, histories)
         if n <= kernels.RESULT_TOKENS:
             self.sampler.sample(kernels.result_tokens(dev), logits, u01_dev)
-            self._host[:n + 1].copy_(kernels.status_and_tokens(dev, n), non_blocking=True)
+            kernels.stage_words(self._host, kernels.status_and_tokens(dev, n), n + 1)
         else:                                      # more rows than the shared buffer holds: two copies
             out = torch.empty(n, dtype=torch.int32, device=dev)
             self.sampler.sample(out, logits, u01_dev)

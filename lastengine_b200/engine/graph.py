@@ -310,7 +310,7 @@ class GraphBackend(EngineBackend):
             self._hosts[self._launched % 2]
         # the status word and the tokens: one copy where they lie together
         if n <= kernels.RESULT_TOKENS:
-            host[:n + 1].copy_(kernels.status_and_tokens(eng.device, n), non_blocking=True)
+            kernels.stage_words(host, kernels.status_and_tokens(eng.device, n), n + 1)
         else:
             host[:1].copy_(kernels.status_and_tokens(eng.device, 0), non_blocking=True)
             host[1:n + 1].copy_(out[:n], non_blocking=True)
@@ -395,7 +395,7 @@ class GraphBackend(EngineBackend):
             g.launch()
             eng.cache.commit(grow)
             host = self._host
-            host[:n + 1].copy_(kernels.status_and_tokens(eng.device, n), non_blocking=True)
+            kernels.stage_words(host, kernels.status_and_tokens(eng.device, n), n + 1)
             self._starting = slots
             self._read_soon()
             vals = host[:n + 1].tolist()

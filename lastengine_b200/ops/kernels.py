@@ -94,6 +94,7 @@ def _declare(L) -> None:
     P, I, F, S, LL = c_void_p, c_int, c_float, c_size_t, ctypes.c_longlong
     sig = {
         "leb_embed": [P, P, I, P, I, I, I, F, P],
+        "leb_stage_words": [P, P, I, P],
         "leb_rmsnorm": [P, I, P, P, P, I, I, F, I, P],
         "leb_swiglu": [P, I, P, I, I, I, P],
         "leb_gather_rows": [P, P, I, P, P, I, I, I, P],
@@ -1949,6 +1950,21 @@ def result_tokens(device: torch.device) -> torch.Tensor:
 def status_and_tokens(device: torch.device, n: int) -> torch.Tensor:
     """The status word followed by the first n chosen tokens: what one copy brings to the host."""
     return _status_block(device)[_STATUS_AT:_STATUS_AT + 1 + n]
+
+
+STAGE_WORDS = 4096      # words up to which a block moves them between pinned memory and the device; the copy engine takes more
+
+
+def stage_words(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
+    """The first n int32 of `src` into `dst` on the current stream, one of the two in pinned host memory: up to STAGE_WORDS
+    by a kernel that reads or writes the host's memory itself, more of them as an asynchronous copy."""
+    host, dev = (dst, src) if src.is_cuda else (src, dst)
+    assert dst.dtype == src.dtype == torch.int32 and dst.is_contiguous() and src.is_contiguous() and dev.is_cuda
+    assert n <= dst.numel() and n <= src.numel()
+    if n > STAGE_WORDS or not host.is_pinned():
+        dst[:n].copy_(src[:n], non_blocking=True)
+        return
+    _check(lib().leb_stage_words(dst.data_ptr(), src.data_ptr(), int(n), _stream()))
 
 
 def raise_on_status(value: int, device: torch.device) -> None:
