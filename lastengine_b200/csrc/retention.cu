@@ -24,7 +24,9 @@ __global__ void __launch_bounds__(RPT >= 64 ? 1024 : 512) retention_recurrent_ke
     const int* __restrict__ seq_qlen, int H, int d, int e) {
   extern __shared__ float sm[];
   pdl_trigger();
-  pdl_wait();
+  // What the step brought (ahead of its first kernel), the state (written a step ago) and the first row's sines do
+  // not depend on the kernel before this one: they are fetched and formed under its end (1.4% of a decode step of one
+  // sequence on six layers, with the same in the rotation's kernel).
   const int b = blockIdx.y, h = blockIdx.x;
   const int slot = seq_slot[b];
   const int n = seq_qlen ? seq_qlen[b] : 1;
@@ -45,6 +47,13 @@ __global__ void __launch_bounds__(RPT >= 64 ? 1024 : 512) retention_recurrent_ke
   float* sp = slot >= 0 ? state + (((size_t)slot * H + h) * d) * e : nullptr;
 #pragma unroll
   for (int r = 0; r < RPT; r++) S[r] = (sp && r0 + r < d) ? sp[(size_t)(r0 + r) * e + c] : 0.f;
+  float cs0 = 1.f, sn0 = 0.f;
+  if (tid < rot) {
+    const float th = (float)pos0 * inv_freq[tid < half ? tid : tid - half];
+    cs0 = cosf(th);
+    sn0 = sinf(th);
+  }
+  pdl_wait();
 
   for (int i = 0; i < n; i++) {
     const size_t m = (size_t)q0 + i;
@@ -56,8 +65,12 @@ __global__ void __launch_bounds__(RPT >= 64 ? 1024 : 512) retention_recurrent_ke
       float qa = to_f32(qr[j]), ka = to_f32(kr[j]);
       if (j < rot) {
         const int p = j < half ? j : j - half;
-        const float th = pos * inv_freq[p];
-        const float cs = cosf(th), sn = sinf(th);
+        float cs = cs0, sn = sn0;
+        if (i > 0 || j != tid) {
+          const float th = pos * inv_freq[p];
+          cs = cosf(th);
+          sn = sinf(th);
+        }
         const int jo = j < half ? j + half : j - half;
         const float qb = to_f32(qr[jo]), kb = to_f32(kr[jo]);
         if (j < half) { qa = qa * cs - qb * sn; ka = ka * cs - kb * sn; }

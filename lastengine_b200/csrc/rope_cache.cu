@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(ROPE_WARPS * 32) qk_rope_store_lanes_kernel(
     float temp_coef, float temp_every) {
   constexpr int HD = EPL * 32, NP = EPL / 2, U = 4;
   pdl_trigger();   // the kernel after this one may start and wait (see common.cuh)
-  pdl_wait();
   if ((int)blockIdx.x >= M) {
+    pdl_wait();
     if (blockIdx.y == 0)
       store_value_tile<T, CT>(blockIdx.x - M, v_in, kv_stride, v_pool, block_table, bt_width, row_seq, row_pos,
                               seq_slot, M, nkv, vd, page_size, v_norm, eps, vin);
@@ -219,7 +219,12 @@ __global__ void __launch_bounds__(ROPE_WARPS * 32) qk_rope_store_lanes_kernel(
   const int m = blockIdx.x;
   const int total = nh + (k_in ? nkv : 0);
   const int h0 = (blockIdx.y * ROPE_WARPS + warp) * per_warp;
-  if (h0 >= total) return;
+  if (h0 >= total) {
+    pdl_wait();      // a kernel counts as complete when its blocks are: none may finish before its predecessor has
+    return;
+  }
+  // What the step brought (ahead of its first kernel) and the weights do not depend on the kernel before this
+  // one: positions, pages, sines and weights are formed under its end, and only q and k are waited for.
   const int h1 = min(h0 + per_warp, total);
   const int b = row_seq[m], pos = row_pos[m];
   long long kdst = -1;
@@ -240,6 +245,7 @@ __global__ void __launch_bounds__(ROPE_WARPS * 32) qk_rope_store_lanes_kernel(
     wk[e] = k_norm_w ? k_norm_w[lane + 32 * e] : 1.f;
   }
   const float factor = query_temperature(pos, temp_coef, temp_every);
+  pdl_wait();
   for (int hb = h0; hb < h1; hb += U) {
     float x[U][EPL];
 #pragma unroll
