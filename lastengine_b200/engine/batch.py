@@ -14,6 +14,8 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from ..ops import kernels
+
 
 @dataclass
 class StepBatch:
@@ -46,23 +48,27 @@ class BatchBuilder:
 
     def __init__(self, device: torch.device):
         self.device = device
-        self._host: torch.Tensor | None = None
+        self._host: kernels.PinnedWords | None = None
         self._dev: torch.Tensor | None = None
-        self._copied: torch.cuda.Event | None = None   # the last copy out of the staging buffer
 
     def _ensure(self, n: int) -> None:
-        if self._host is None or self._host.numel() < n:
+        if self._host is None or self._host.words.numel() < n:
             cap = max(1024, int(n * 1.5))
-            self._host = torch.empty(cap, dtype=torch.int32, pin_memory=self.device.type == "cuda")
+            self._host = kernels.PinnedWords(cap, self.device)
             self._dev = torch.empty(cap, dtype=torch.int32, device=self.device)
+
+    def wait(self) -> None:
+        """Until the last step's words have left the staging buffer, which may then be changed."""
+        if self._host is not None:
+            self._host.wait()
 
     def _send(self, n: int) -> None:
         """The first n words of the staging buffer to the device."""
         if self.device.type == "cuda":
-            from ..ops import kernels
-            kernels.stage_words(self._dev, self._host, n)
+            kernels.stage_words(self._dev, self._host.words, n)
+            self._host.mark()
         else:
-            self._dev[:n].copy_(self._host[:n])
+            self._dev[:n].copy_(self._host.words[:n])
 
     def build(self, slots: list[int], tokens: list[list[int]] | list[np.ndarray], pos0: list[int],
               logit_rows: list[int], tables: dict[int, np.ndarray],
@@ -91,17 +97,12 @@ class BatchBuilder:
         for p in pieces:
             offs.append(total)
             total += (p.size + 3) // 4 * 4
-        if self._copied is not None:
-            self._copied.synchronize()   # the previous step's copy has read the staging buffer
+        self.wait()
         self._ensure(total + 4)
-        host = self._host.numpy()
+        host = self._host.words.numpy()
         for o, p in zip(offs, pieces):
             host[o:o + p.size] = p
         self._send(total)
-        if self.device.type == "cuda":
-            if self._copied is None:
-                self._copied = torch.cuda.Event()
-            self._copied.record()
         self.last_h2d_bytes = total * 4
         names = ["tokens", "row_seq", "row_pos", "seq_slot", "seq_pos0", "seq_qstart", "seq_qlen", "logit_rows"]
         names += (["u01"] if u01 is not None else []) + (["feed"] if feed is not None else [])
@@ -130,14 +131,12 @@ class BatchBuilder:
     def host_view(self, name: str) -> np.ndarray:
         """The staged copy of one piece of the last built step (int32; `u01` as raw bits)."""
         o, n = self.layout[name]
-        return self._host.numpy()[o:o + n]
+        return self._host.words.numpy()[o:o + n]
 
     def resend(self, n_ints: int | None = None) -> None:
         """Copies the staging buffer (or its first `n_ints` words) to the device again, after
         the caller changed pieces of it in place.  The device addresses stay what they were."""
-        if self._copied is not None:
-            self._copied.synchronize()
+        self.wait()
         n = self.total if n_ints is None else n_ints
         self._send(n)
-        self._copied.record()
         self.last_h2d_bytes = n * 4

@@ -195,11 +195,12 @@ class EngineBackend:
 
     def __init__(self, engine, sampling: SamplingParams):
         import torch
+        from ..ops import kernels
         from ..sampling.sampler import Sampler
         self.engine = engine
         self.sampler = Sampler(sampling, engine.device)
         self._torch = torch
-        self._host = torch.empty(1025, dtype=torch.int32, pin_memory=True)
+        self._host = kernels.PinnedWords(1025, engine.device)
         self._starting: list[int] | None = None           # the slots of the prompts whose step is on the device
         self.d2h_bytes = 0
 
@@ -210,27 +211,29 @@ class EngineBackend:
         from ..ops import kernels
         torch, dev = self._torch, self.engine.device
         n = logits.shape[0]
-        if n + 1 > self._host.numel():
-            self._host = torch.empty(2 * n + 1, dtype=torch.int32, pin_memory=True)
+        if n + 1 > self._host.words.numel():
+            self._host = kernels.PinnedWords(2 * n + 1, dev)
+        host = self._host.words
         if histories is not None:
             self.sampler.apply_penalties(logits, histories)
         if n <= kernels.RESULT_TOKENS:
             self.sampler.sample(kernels.result_tokens(dev), logits, u01_dev)
-            kernels.stage_words(self._host, kernels.status_and_tokens(dev, n), n + 1)
+            kernels.stage_words(host, kernels.status_and_tokens(dev, n), n + 1)
         else:                                      # more rows than the shared buffer holds: two copies
             out = torch.empty(n, dtype=torch.int32, device=dev)
             self.sampler.sample(out, logits, u01_dev)
-            self._host[:1].copy_(kernels.status_and_tokens(dev, 0), non_blocking=True)
-            self._host[1:n + 1].copy_(out, non_blocking=True)
+            host[:1].copy_(kernels.status_and_tokens(dev, 0), non_blocking=True)
+            host[1:n + 1].copy_(out, non_blocking=True)
         self._read_soon()
         self.d2h_bytes = (n + 1) * 4
-        vals = self._host[:n + 1].tolist()
+        vals = host[:n + 1].tolist()
         kernels.raise_on_status(vals[0], dev)
         return vals[1:]
 
     def _read_soon(self) -> None:
         """Called once the copy of a step's tokens to the host is on the stream; returns when they have arrived."""
-        self._torch.cuda.current_stream().synchronize()
+        self._host.mark()
+        self._host.wait()
 
     def _step(self, slots, tokens, u01, histories) -> list[int]:
         import numpy as np

@@ -151,8 +151,7 @@ class DecodeGraph:
         page = cache.page_size
         pos = bb.host_view("seq_pos0")
         grow = {}
-        if bb._copied is not None:
-            bb._copied.synchronize()          # the last copy has read the buffer we are about to change
+        bb.wait()
         new_page = [i for i in range(n) if (int(pos[i]) + 1) % page == 0]
         if new_page:
             cache.reserve({slots[i]: 1 for i in new_page})
@@ -211,8 +210,8 @@ class DecodeGraph:
 class _StepInFlight:
     """A launched decode step whose chosen tokens the host has not read yet."""
 
-    def __init__(self, number: int, slots: list[int], host: torch.Tensor, event: torch.cuda.Event):
-        self.number, self.slots, self.host, self.event = number, slots, host, event
+    def __init__(self, number: int, slots: list[int], host: kernels.PinnedWords):
+        self.number, self.slots, self.host = number, slots, host
 
 
 class GraphBackend(EngineBackend):
@@ -306,32 +305,31 @@ class GraphBackend(EngineBackend):
         g.cache_version = eng.cache.state_version
         n = len(slots)
         self._launched += 1
-        host = torch.empty(n + 1, dtype=torch.int32, pin_memory=True) if n > 1024 else \
-            self._hosts[self._launched % 2]
+        # (two buffers take turns: a step's is written again when the step after the next is launched, with this one's tokens read)
+        host = kernels.PinnedWords(n + 1, eng.device) if n > 1024 else self._hosts[self._launched % 2]
         # the status word and the tokens: one copy where they lie together
         if n <= kernels.RESULT_TOKENS:
-            kernels.stage_words(host, kernels.status_and_tokens(eng.device, n), n + 1)
+            kernels.stage_words(host.words, kernels.status_and_tokens(eng.device, n), n + 1)
         else:
-            host[:1].copy_(kernels.status_and_tokens(eng.device, 0), non_blocking=True)
-            host[1:n + 1].copy_(out[:n], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
+            host.words[:1].copy_(kernels.status_and_tokens(eng.device, 0), non_blocking=True)
+            host.words[1:n + 1].copy_(out[:n], non_blocking=True)
+        host.mark()
         self.h2d_bytes = g.builder.last_h2d_bytes
         self.d2h_bytes = (n + 1) * 4
-        return _StepInFlight(self._launched, list(slots), host, ev)
+        return _StepInFlight(self._launched, list(slots), host)
 
     @property
     def _hosts(self):
         h = self.__dict__.get("_host_pair")
         if h is None:
-            h = self.__dict__["_host_pair"] = [torch.empty(1025, dtype=torch.int32, pin_memory=True) for _ in range(2)]
+            h = self.__dict__["_host_pair"] = [kernels.PinnedWords(1025, self.engine.device) for _ in range(2)]
         return h
 
     def _wait(self, step: _StepInFlight, check: bool = True) -> list[int]:
         """The step's tokens, once it has finished.  The status word came with them: a kernel that
         gave up on a bounded wait in this step raises KernelError here (`check`)."""
-        step.event.synchronize()
-        vals = step.host[:len(step.slots) + 1].tolist()
+        step.host.wait()
+        vals = step.host.words[:len(step.slots) + 1].tolist()
         toks = vals[1:]
         still = []
         for number, slots in self._held:
@@ -394,7 +392,7 @@ class GraphBackend(EngineBackend):
             grow = g.stage_prompts(slots, prompts, u01)
             g.launch()
             eng.cache.commit(grow)
-            host = self._host
+            host = self._host.words
             kernels.stage_words(host, kernels.status_and_tokens(eng.device, n), n + 1)
             self._starting = slots
             self._read_soon()
@@ -413,8 +411,7 @@ class GraphBackend(EngineBackend):
         if slots is None or look is None:
             super()._read_soon()
             return
-        copied = torch.cuda.Event()
-        copied.record()
+        self._host.mark()
         self._start_lookahead = None
         next_u01, goes_on = look
         keep = [i for i, c in enumerate(goes_on) if c]
@@ -424,7 +421,7 @@ class GraphBackend(EngineBackend):
                                            [next_u01[i] for i in keep] if next_u01 is not None else None, keep)
             except CacheFull:
                 self._ahead = None      # no room to run ahead: the first step is staged when it is asked for
-        copied.synchronize()
+        self._host.wait()
 
     def start(self, prompts, u01, histories, lookahead=None):
         """`lookahead` as in `decode`, for the first decode step.  Runs ahead only where the prompts' tokens lie in the

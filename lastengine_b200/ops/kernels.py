@@ -6,6 +6,7 @@ the built library, or with tensors that are not on a CUDA device, raises.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import functools
 from ctypes import c_float, c_int, c_size_t, c_void_p
@@ -1957,7 +1958,8 @@ STAGE_WORDS = 4096      # words up to which a block moves them between pinned me
 
 def stage_words(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
     """The first n int32 of `src` into `dst` on the current stream, one of the two in pinned host memory: up to STAGE_WORDS
-    by a kernel that reads or writes the host's memory itself, more of them as an asynchronous copy."""
+    by a kernel that reads or writes the host's memory itself, more of them as an asynchronous copy.  The host's side
+    belongs to a PinnedWords whose `mark` follows the call: torch's allocator does not know of the kernel."""
     host, dev = (dst, src) if src.is_cuda else (src, dst)
     assert dst.dtype == src.dtype == torch.int32 and dst.is_contiguous() and src.is_contiguous() and dev.is_cuda
     assert n <= dst.numel() and n <= src.numel()
@@ -1965,6 +1967,50 @@ def stage_words(dst: torch.Tensor, src: torch.Tensor, n: int) -> None:
         dst[:n].copy_(src[:n], non_blocking=True)
         return
     _check(lib().leb_stage_words(dst.data_ptr(), src.data_ptr(), int(n), _stream()))
+
+
+class PinnedWords:
+    """int32 words of host memory (pinned where the device is a GPU) that go over to the device or come from it.
+
+    torch's allocator of pinned memory keeps a dropped block back until the copies it knows of have ended; of a kernel that
+    reads or writes the block it knows nothing, and would hand it to the next owner under that kernel.  So `mark`
+    records an event behind every transfer, and an object that is dropped leaves its block and event in `_left` until the
+    event has passed, which is looked at when the next object is made: dropping itself makes no call to the
+    driver, since the garbage collector may do it while a stream captures."""
+
+    _left: collections.deque = collections.deque()      # (words, event) of dropped objects
+
+    def __init__(self, n: int, device: torch.device):
+        self.event = None                                # behind the last transfer
+        self.give_back()
+        self.words = torch.empty(n, dtype=torch.int32, pin_memory=device.type == "cuda")
+
+    def mark(self):
+        """An event behind the transfer that was just put on the current stream."""
+        if self.event is None:
+            self.event = torch.cuda.Event()
+        self.event.record()
+        return self.event
+
+    def wait(self) -> None:
+        """Until the last transfer has ended and the words may be changed."""
+        if self.event is not None:
+            self.event.synchronize()
+
+    def __del__(self):
+        if self.event is not None:
+            self._left.append((self.words, self.event))
+
+    @classmethod
+    def give_back(cls) -> None:
+        """Lets go of the blocks of dropped objects whose transfers have ended."""
+        for _ in range(len(cls._left)):
+            try:
+                kept = cls._left.popleft()
+            except IndexError:                           # another thread took it
+                return
+            if not kept[1].query():
+                cls._left.append(kept)
 
 
 def raise_on_status(value: int, device: torch.device) -> None:

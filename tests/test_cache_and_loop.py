@@ -199,6 +199,41 @@ def test_xorshift_matches_the_reference_recurrence():
     assert all(0.0 <= XorShift64(3).next() < 1.0 for _ in range(3))
 
 
+class Behind:
+    """An event that passes when the test says so."""
+
+    def __init__(self):
+        self.passed = False
+
+    def query(self):
+        return self.passed
+
+
+def test_a_dropped_staging_buffer_is_kept_until_its_transfer_has_ended():
+    """A kernel may still read the words of a builder, or write a step's tokens, when their owner is dropped: the block
+    must not go back to the allocator before (it would be the next owner's, and change under the kernel)."""
+    import weakref
+    from lastengine_b200.engine.batch import BatchBuilder
+    from lastengine_b200.ops.kernels import PinnedWords
+    cpu = torch.device("cpu")
+    b = BatchBuilder(cpu)
+    assert b.build([0], [[7, 8]], [3], [1], {}).tokens.tolist() == [7, 8]
+    held = weakref.ref(b._host.words)
+    b._host.event = behind = Behind()
+    del b
+    PinnedWords.give_back()
+    assert held() is not None
+    PinnedWords(4, cpu)                       # another one is made, the transfer still runs
+    assert held() is not None
+    behind.passed = True
+    PinnedWords(4, cpu)
+    assert held() is None
+    idle = PinnedWords(4, cpu)                # nothing was transferred: nothing is kept
+    held = weakref.ref(idle.words)
+    del idle
+    assert held() is None
+
+
 class Scripted:
     """A backend that plays tokens from a script: request r's i-th token is script[r][i]."""
 

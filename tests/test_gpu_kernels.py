@@ -510,6 +510,44 @@ def test_qk_rope_store_of_many_rows_gives_the_bits_of_few(lens, nh, nkv, weights
         assert torch.equal(a, b)
 
 
+# ---- words between host and device ---------------------------------------------------------------------
+def test_words_of_dropped_owners_stay_until_the_device_is_through_with_them():
+    """Builders and result buffers dropped while their transfers wait behind other work: every step finds its own words, and
+    what a late transfer brings to the host lands in no other owner's buffer."""
+    dev = torch.device(DEV)
+    torch.cuda._sleep(100_000_000)
+    steps = [builder().build([0], [list(range(100 * i, 100 * i + 40))], [i], [39], {}) for i in range(20)]
+    for i in range(4):
+        w = K().PinnedWords(1025, dev)
+        K().stage_words(w.words, torch.full((1025,), i, dtype=torch.int32, device=DEV), 1025)
+        w.mark()
+    del w
+    mine = [K().PinnedWords(1025, dev) for _ in range(4)]
+    for m in mine:
+        m.words.fill_(-1)
+    torch.cuda.synchronize()
+    for i, b in enumerate(steps):
+        assert b.tokens.tolist() == list(range(100 * i, 100 * i + 40)) and b.row_pos.tolist() == list(range(i, i + 40))
+    assert all(bool((m.words == -1).all()) for m in mine)
+
+
+@pytest.mark.parametrize("n", [1, 3, 255, 256, 257, 4095, 4096, 4097])
+def test_stage_words_both_ways(n):
+    """Up to 4,096 words by a kernel (of 256 or 1,024 threads), more by a copy: all of them arrive and nothing beyond them."""
+    dev = torch.device(DEV)
+    host, back = K().PinnedWords(5000, dev), K().PinnedWords(5000, dev)
+    host.words.copy_(torch.arange(5000, dtype=torch.int32) * 7 - 3)
+    back.words.fill_(-9)
+    d = torch.full((5000,), -5, dtype=torch.int32, device=DEV)
+    K().stage_words(d, host.words, n)
+    host.mark()
+    K().stage_words(back.words, d, n)
+    back.mark()
+    back.wait()
+    assert torch.equal(back.words[:n], host.words[:n]) and bool((back.words[n:] == -9).all())
+    assert bool((d[n:] == -5).all())
+
+
 # ---- attention ---------------------------------------------------------------------------------------
 def plain_attention(q, k, v, qpos, window, scale):
     """q [Tq, nh, hd], k/v [Tk, nkv, hd] (positions 0..Tk-1), qpos [Tq]."""
