@@ -735,8 +735,10 @@ LEB_API int leb_weighted_pair_sum(float* out, const float* y1, const float* bias
 // decoding is 0.4 to 2 ms between two such copies, and each handover from kernels to the engine and back leaves
 // the device idle for longer than the words take over the bus (32 to 64 decode steps a call: 36.8 -> 36.4 ms on a dense model of
 // 1.2B, 18.4 -> 18.2 and 27.7 -> 27.4 on smaller ones).
-// Kernels read the step's tables ahead of their own waits, counting on what brings them to have finished before the
-// step's first kernel starts: so it says nothing to its successor (no pdl_trigger) and is launched plainly.
+// Kernels read the step's tables ahead of their own waits, counting on what brings them to be complete and visible before
+// the step's first kernel starts: so it is launched plainly, and to the device it brings words only where the launch of
+// a graph follows, which waits for all of it (a kernel with the programmatic attribute behind it would wait for its
+// blocks to end, and its own successors for nothing more).
 __global__ void stage_words_kernel(int* __restrict__ dst, const int* __restrict__ src, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }

@@ -44,10 +44,18 @@ class StepBatch:
 
 
 class BatchBuilder:
-    """Lays a step out in a pinned staging buffer and copies it to the device in one go."""
+    """Lays a step out in a pinned staging buffer and copies it to the device in one go.
 
-    def __init__(self, device: torch.device):
+    Kernels read the step's tables, and what earlier steps left in the cache, ahead of their own wait for the kernel before
+    them: they count on the step's first kernel starting after everything before it is complete and visible.  A copy by
+    the copy engine gives that to whatever is launched next, and so does the launch of a graph.  A kernel that brings the
+    words gives it to a graph only: a kernel launched behind it with the programmatic attribute may start when its
+    blocks have ended, and let its own successors start.  So the words go over by a kernel (which is quicker for a
+    few of them) where `replayed` says that the launch of a graph follows, and by the copy engine otherwise."""
+
+    def __init__(self, device: torch.device, replayed: bool = False):
         self.device = device
+        self.replayed = bool(replayed)
         self._host: kernels.PinnedWords | None = None
         self._dev: torch.Tensor | None = None
 
@@ -64,11 +72,12 @@ class BatchBuilder:
 
     def _send(self, n: int) -> None:
         """The first n words of the staging buffer to the device."""
-        if self.device.type == "cuda":
+        if self.replayed and self.device.type == "cuda":
             kernels.stage_words(self._dev, self._host.words, n)
-            self._host.mark()
         else:
-            self._dev[:n].copy_(self._host.words[:n])
+            self._dev[:n].copy_(self._host.words[:n], non_blocking=True)
+        if self.device.type == "cuda":
+            self._host.mark()
 
     def build(self, slots: list[int], tokens: list[list[int]] | list[np.ndarray], pos0: list[int],
               logit_rows: list[int], tables: dict[int, np.ndarray],

@@ -55,7 +55,7 @@ class DecodeGraph:
         self.engine, self.sampler, self.bucket, self.width = engine, sampler, bucket, table_width
         self.self_feeding, self.fed = self_feeding, fed
         self.ws = workspace if workspace is not None else Workspace(engine.device)
-        self.builder = BatchBuilder(engine.device)
+        self.builder = BatchBuilder(engine.device, replayed=True)
         self.out = out if out is not None else torch.zeros(bucket, dtype=torch.int32, device=engine.device)
         self.graph: torch.cuda.CUDAGraph | None = None
         self.batch = None
@@ -181,6 +181,7 @@ class DecodeGraph:
         eng.env.workspace = self.ws
         try:
             if self.graph is None or self.ws_generation != self.ws.generation:
+                torch.cuda.current_stream().synchronize()      # the staged words are there (see BatchBuilder: no graph follows them yet)
                 self._run(self.batch)            # warm-up: loads kernels, sizes the scratch memory
                 torch.cuda.current_stream().synchronize()
                 before = kernels.launch_count()

@@ -234,6 +234,27 @@ def test_a_dropped_staging_buffer_is_kept_until_its_transfer_has_ended():
     assert held() is None
 
 
+def test_the_uncaptured_run_of_a_graph_waits_for_its_staged_words(monkeypatch):
+    """Words for a graph are brought by a kernel, which the kernels of an uncaptured run could overtake: the run before the
+    capture starts when they are there, a replay right away."""
+    from contextlib import nullcontext
+    from types import SimpleNamespace
+    from lastengine_b200.engine import graph as G
+    calls = []
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: SimpleNamespace(synchronize=lambda: calls.append("wait")))
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: SimpleNamespace(replay=lambda: calls.append("replay")))
+    monkeypatch.setattr(torch.cuda, "graph", lambda g: nullcontext())
+    monkeypatch.setattr(G.kernels, "launch_count", lambda: 0)
+    eng = SimpleNamespace(device=torch.device("cpu"), env=SimpleNamespace(workspace=None))
+    g = G.DecodeGraph(eng, None, 1, 1)
+    assert g.builder.replayed
+    monkeypatch.setattr(g, "_run", lambda batch: calls.append("run"))
+    g.launch()
+    assert calls == ["wait", "run", "wait", "run"]      # the uncaptured run, then the captured one
+    g.launch()
+    assert calls[4:] == ["replay"]
+
+
 class Scripted:
     """A backend that plays tokens from a script: request r's i-th token is script[r][i]."""
 

@@ -531,6 +531,22 @@ def test_words_of_dropped_owners_stay_until_the_device_is_through_with_them():
     assert all(bool((m.words == -1).all()) for m in mine)
 
 
+@pytest.mark.parametrize("replayed", [False, True])
+def test_steps_are_brought_by_a_kernel_only_where_a_graph_follows(replayed):
+    """Behind the copy engine any kernel may start; behind a kernel of ours the next one could start before its words are
+    visible, unless a graph's launch stands between."""
+    from lastengine_b200.engine.batch import BatchBuilder
+    b = BatchBuilder(torch.device(DEV), replayed=replayed)
+    n = K().launch_count()
+    step = b.build([0], [[5, 6, 7]], [2], [2], {})
+    assert K().launch_count() - n == int(replayed)
+    assert step.tokens.tolist() == [5, 6, 7] and step.row_pos.tolist() == [2, 3, 4]
+    b.host_view("tokens")[:] = [8, 9, 10]
+    b.resend()
+    assert K().launch_count() - n == 2 * int(replayed)
+    assert step.tokens.tolist() == [8, 9, 10]
+
+
 @pytest.mark.parametrize("n", [1, 3, 255, 256, 257, 4095, 4096, 4097])
 def test_stage_words_both_ways(n):
     """Up to 4,096 words by a kernel (of 256 or 1,024 threads), more by a copy: all of them arrive and nothing beyond them."""
