@@ -444,53 +444,55 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       constexpr int OW = WIDE ? VD : 32;      // numbers of the row at a time
 #pragma unroll
       for (int d0 = 0; d0 < VD; d0 += OW) {
+        __syncwarp();      // rows beyond the sequence left the branch below early: the loads take the whole warp
         uint4* orow = reinterpret_cast<uint4*>(out + ((m_base + pi) * nh + h0 + g) * VD + d0);
         uint32_t o[OW];
         tmem_ld32(t_o + lane_base + d0, o);
         if (OW > 32) tmem_ld32(t_o + lane_base + 32, o + (OW > 32 ? 32 : 0));
         tmem_ld_wait();
-        if (!row_valid) continue;
+        if (row_valid) {
 #pragma unroll
-        for (int c = 0; c < OW; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * inv);
-        if (gate && gate_elem) {
-          const bf16* grow = gate + (m_base + pi) * (size_t)gate_stride + (h0 + g) * VD + d0;
-          if ((((uintptr_t)grow) & 15) == 0) {
+          for (int c = 0; c < OW; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * inv);
+          if (gate && gate_elem) {
+            const bf16* grow = gate + (m_base + pi) * (size_t)gate_stride + (h0 + g) * VD + d0;
+            if ((((uintptr_t)grow) & 15) == 0) {
 #pragma unroll
-            for (int c = 0; c < OW; c += 8) {
-              const uint4 w = *reinterpret_cast<const uint4*>(grow + c);
-              const bf16* z = reinterpret_cast<const bf16*>(&w);
+              for (int c = 0; c < OW; c += 8) {
+                const uint4 w = *reinterpret_cast<const uint4*>(grow + c);
+                const bf16* z = reinterpret_cast<const bf16*>(&w);
 #pragma unroll
-              for (int e = 0; e < 8; e++)
-                o[c + e] = __float_as_uint(__fdividef(__uint_as_float(o[c + e]), 1.0f + __expf(-__bfloat162float(z[e]))));
+                for (int e = 0; e < 8; e++)
+                  o[c + e] = __float_as_uint(__fdividef(__uint_as_float(o[c + e]), 1.0f + __expf(-__bfloat162float(z[e]))));
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < OW; c++)
+                o[c] = __float_as_uint(__fdividef(__uint_as_float(o[c]), 1.0f + __expf(-__bfloat162float(grow[c]))));
             }
-          } else {
-#pragma unroll
-            for (int c = 0; c < OW; c++)
-              o[c] = __float_as_uint(__fdividef(__uint_as_float(o[c]), 1.0f + __expf(-__bfloat162float(grow[c]))));
           }
-        }
-        if (POOLED && freq_v) {
-          // values were cached turned by their positions: the sum is turned back by the query's (pairs c, c + VD/2)
-          const float fpos = (float)qpos;
+          if (POOLED && freq_v) {
+            // values were cached turned by their positions: the sum is turned back by the query's (pairs c, c + VD/2)
+            const float fpos = (float)qpos;
 #pragma unroll
-          for (int c = 0; c < OW / 2; c++) {
-            float sn, cs;
-            sincosf(fpos * freq_v[c], &sn, &cs);
-            const float a = __uint_as_float(o[c]), bb = __uint_as_float(o[c + OW / 2]);
-            o[c] = __float_as_uint(a * cs + bb * sn);
-            o[c + OW / 2] = __float_as_uint(bb * cs - a * sn);
+            for (int c = 0; c < OW / 2; c++) {
+              float sn, cs;
+              sincosf(fpos * freq_v[c], &sn, &cs);
+              const float a = __uint_as_float(o[c]), bb = __uint_as_float(o[c + OW / 2]);
+              o[c] = __float_as_uint(a * cs + bb * sn);
+              o[c + OW / 2] = __float_as_uint(bb * cs - a * sn);
+            }
           }
-        }
 #pragma unroll
-        for (int c = 0; c < OW; c += 8) {
-          uint4 w;
-          uint32_t* wp = reinterpret_cast<uint32_t*>(&w);
+          for (int c = 0; c < OW; c += 8) {
+            uint4 w;
+            uint32_t* wp = reinterpret_cast<uint32_t*>(&w);
 #pragma unroll
-          for (int e = 0; e < 4; e++) {
-            __nv_bfloat162 pp = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e]), __uint_as_float(o[c + 2 * e + 1]));
-            wp[e] = *reinterpret_cast<uint32_t*>(&pp);
+            for (int e = 0; e < 4; e++) {
+              __nv_bfloat162 pp = __floats2bfloat162_rn(__uint_as_float(o[c + 2 * e]), __uint_as_float(o[c + 2 * e + 1]));
+              wp[e] = *reinterpret_cast<uint32_t*>(&pp);
+            }
+            orow[c / 8] = w;
           }
-          orow[c / 8] = w;
         }
       }
     }

@@ -755,6 +755,44 @@ def test_attention_long_prompts_on_tcgen05(nh, nkv, window):
         assert err(out[650].view(nh, hd)[0], vs[0][far, 0].double()) < 1e-2     # the far key's value, alone
 
 
+@pytest.mark.parametrize("nh,nkv", [(4, 4), (4, 2), (8, 2), (8, 1)])
+@pytest.mark.parametrize("gate", ["none", "head", "number", "number, unaligned"])
+@pytest.mark.parametrize("wide", [False, True])
+def test_prompt_attention_of_part_tiles_with_gates(nh, nkv, gate, wide):
+    """Last tiles whose warps hold rows of the sequence beside rows beyond it (1 to 127 of 128), which part ways before
+    the second half of a row is read from tensor memory; with every form of the output gate, whose 16-byte loads are a
+    branch of their own.  Results are bfloat16 and weights one or two bfloat16 terms: the tolerance of the other prompts."""
+    hd, page, dtype = 64, 64, torch.bfloat16
+    lens = [2, 33, 70, 131, 45]
+    width, M = 3, sum(lens)
+    table = np.random.default_rng(11).permutation(len(lens) * width).astype(np.int32).reshape(len(lens), width)
+    pk = torch.full((table.size, nkv, page, hd), float("nan"), dtype=dtype)
+    pv = torch.full((table.size, nkv, hd, page), float("nan"), dtype=dtype)
+    q = gen(M, nh, hd, seed=190, dtype=dtype)
+    want, r0 = [], 0
+    width_g = 0 if gate == "none" else nh if gate == "head" else nh * hd
+    g_all = gen(M, width_g + 8, seed=191, dtype=dtype)
+    off = 3 if gate.endswith("unaligned") else 0
+    g = g_all[:, off:off + width_g]
+    for b, n in enumerate(lens):
+        k, v = gen(n, nkv, hd, seed=192 + b, dtype=dtype), gen(n, nkv, hd, seed=292 + b, dtype=dtype)
+        for t in range(n):
+            pk[table[b, t // page], :, t % page] = k[t]
+            pv[table[b, t // page], :, :, t % page] = v[t]
+        w = plain_attention(q[r0:r0 + n].double(), k.double(), v.double(), torch.arange(n), 0, 0.125)
+        if width_g:
+            w = w * torch.sigmoid(g[r0:r0 + n].double()).reshape(n, nh, -1)
+        want.append(w)
+        r0 += n
+    batch = builder().build(list(range(len(lens))), [[0] * n for n in lens], [0] * len(lens), [], {0: table})
+    out = torch.full((M + 1, nh * hd), float("nan"), device=DEV, dtype=dtype)
+    K().attention(out[:M], q.reshape(M, nh * hd).to(DEV), pk.to(DEV), pv.to(DEV), batch.tables[0], batch, nh, nkv, hd, page, 0,
+                  0.125, gate=g_all.to(DEV)[:, off:off + width_g] if width_g else None, wide=wide)
+    K().check_device_status()
+    assert err(out[:M].view(M, nh, hd), torch.cat(want)) < 8e-3
+    assert bool(out[M].isnan().all())
+
+
 @pytest.mark.parametrize("dtype,nh,nkv,hd", [(torch.float32, 6, 2, 48), (torch.bfloat16, 6, 2, 64), (torch.bfloat16, 6, 2, 48),
                                              (torch.bfloat16, 8, 2, 64), (torch.bfloat16, 8, 1, 64)])
 def test_attention_batch_of_unequal_sequences(dtype, nh, nkv, hd):
