@@ -188,6 +188,8 @@ attention_kernel(T* __restrict__ out, float* __restrict__ part, const T* __restr
       }
     }
     float* pw = p_s + warp * ATT_RPW * 32;
+    unsigned live = 0;      // the warp's vectors that read something of this tile: the others' sums stay as they are, whatever
+                            // its values hold (zero times an infinity among them would not)
 #pragma unroll
     for (int ri = 0; ri < ATT_RPW; ri++) {
       const int r = warp + ri * ATT_WARPS;
@@ -195,12 +197,9 @@ attention_kernel(T* __restrict__ out, float* __restrict__ part, const T* __restr
       const int i = r / HC, j = r % HC;
       const int qpos = pos0 + row_lo + i;
       const int lo = first_key(qpos, window, chunk);
-      corr[ri] = 1.f;
-      // an idle vector, or the whole tile lies after this row or before what it reads: its sums stay as they are
-      if (i >= nrows || j >= nheads || key0 > qpos || key0 + 31 < lo) {
-        pw[ri * 32 + lane] = 0.f;
-        continue;
-      }
+      // an idle vector, or the whole tile lies after this row or before what it reads
+      if (i >= nrows || j >= nheads || key0 > qpos || key0 + 31 < lo) continue;
+      live |= 1u << ri;
       float sc = s[ri] * scale;
       const int kp = key0 + lane;
       if (slopes) sc -= slopes[kvh * G + hc * HC + j] * (float)(qpos - kp);
@@ -237,7 +236,7 @@ attention_kernel(T* __restrict__ out, float* __restrict__ part, const T* __restr
 #pragma unroll
       for (int ri = 0; ri < ATT_RPW; ri++) {
         if (warp + ri * ATT_WARPS >= R) break;
-        acc[ri][jj] = acc[ri][jj] * corr[ri] + a[ri];
+        if (live >> ri & 1) acc[ri][jj] = acc[ri][jj] * corr[ri] + a[ri];
       }
     }
     __syncwarp();

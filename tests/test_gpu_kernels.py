@@ -680,6 +680,35 @@ def test_attention_prompt_and_decode(dtype, nh, nkv, hd, window):
         assert err(out.view(n, nh, hd), want) < tol, (q0, n, splits)
 
 
+@pytest.mark.parametrize("dtype,nh,nkv,hd", [(torch.float32, 4, 4, 64), (torch.float32, 8, 2, 64), (torch.float32, 3, 1, 48),
+                                             (torch.bfloat16, 4, 4, 48)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("window", [0, 40])
+def test_values_of_tiles_a_row_does_not_read_do_not_reach_it(dtype, nh, nkv, hd, bad, window):
+    """The general kernel takes rows of several positions through a tile of 32 keys together.  A value that is not finite, at
+    the last position (of a tile of its own) or at one that a window has left behind, must stay out of the rows whose
+    tiles it does not lie in."""
+    page, Tk = 64, 97
+    k, v = gen(Tk, nkv, hd, seed=60, dtype=dtype), gen(Tk, nkv, hd, seed=61, dtype=dtype)
+    q = gen(Tk, nh, hd, seed=62, dtype=dtype)
+    tables = {0: np.array([[1, 0]], dtype=np.int32)}
+    scale = 1 / math.sqrt(hd)
+    want = plain_attention(q.double(), k.double(), v.double(), torch.arange(Tk), window, scale)
+    batch = builder().build([0], [[0] * Tk], [0], [], tables)
+    # position 96 lies in the tile from 96 on, which rows below 96 do not read; position 0 in the first tile, which rows from
+    # 71 on (71 - 40 + 1 = 32) do not read through the window
+    for at, clean in ((Tk - 1, slice(0, 96)), (0, slice(71, Tk) if window else slice(0, 0))):
+        w = v.clone()
+        w[at] = bad
+        kp, vp = fill_cache(k, w, [1, 0], nkv, hd, page, dtype)
+        out = torch.zeros(Tk, nh * hd, device=DEV, dtype=dtype)
+        K().attention(out, q.reshape(Tk, nh * hd).to(DEV), kp, vp, batch.tables[0], batch, nh, nkv, hd, page, window, scale)
+        got = out.view(Tk, nh, hd)[clean]
+        assert bool(got.isfinite().all())
+        assert clean.stop == 0 or err(got, want[clean]) < (2e-5 if dtype == torch.float32 else 8e-3)
+        assert not bool(out.view(Tk, nh, hd)[at].isfinite().any())      # ... and reaches the row whose own it is
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_far_key_and_window_edge(dtype):
     """One early key is made to dominate: among hundreds of keys the output must be its value;
