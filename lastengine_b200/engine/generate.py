@@ -23,7 +23,8 @@ from ..sampling.params import SamplingParams, XorShift64
 @dataclass
 class GenerationStats:
     """prefill tok/s = prompt tokens / prefill time; decode tok/s = tokens after each request's
-    first / decode time (src/server/mod.rs:270-286)."""
+    first / decode time (src/server/mod.rs:270-286).  The prefill ends when the prompts' tokens are there: what a backend
+    does for the first decode step before it hands them out (`Backend.ahead_s`) is decode time."""
     prefill_tokens: int = 0
     prefill_ms: float = 0.0
     decode_tokens: int = 0
@@ -52,7 +53,8 @@ class Backend(Protocol):
               histories: list[list[int]] | None) -> tuple[list[int], list[int]]:
         """Allocates a slot per prompt, runs all prompts in one step; returns (slots, first tokens).  A
         backend with a true attribute `start_lookahead` also takes `lookahead` as `decode` does: the first
-        decode step's, under the same promise."""
+        decode step's, under the same promise; its `ahead_s` is then how many seconds of the last call it went on
+        with that step after the prompts' tokens were there."""
 
     def decode(self, slots: list[int], tokens: list[int], u01: list[float] | None,
                histories: list[list[int]]) -> list[int]:
@@ -139,12 +141,12 @@ class GenerationLoop:
             slots, toks = self.backend.start([r.prompt for r in batch], u,
                                              [r.history for r in batch] if want_hist else None,
                                              **self._lookahead(batch, draw, "start_lookahead"))
-            stats.prefill_ms += (self.clock() - t0) * 1e3
+            t1 = self.clock() - getattr(self.backend, "ahead_s", 0.0)
+            stats.prefill_ms += (t1 - t0) * 1e3
             stats.prefill_tokens += sum(len(r.prompt) for r in batch)
             for r, s in zip(batch, slots):
                 r.slot = s
             active = batch
-            t1 = self.clock()
             try:
                 active = self._decode_batch(active, toks, stats, draw, want_hist)
             except BaseException:

@@ -11,6 +11,7 @@ steps cannot move what a graph points at.
 from __future__ import annotations
 
 import gc
+import time
 from dataclasses import replace
 
 import numpy as np
@@ -253,6 +254,9 @@ class GraphBackend(EngineBackend):
         self._fed: dict[int, int] = {}                    # slot -> the token the next step was given on the device
         self._starting: list[int] | None = None           # the slots of the prompts whose step is on the device
         self._start_lookahead = None                      # what `start` was told of the step after it
+        self.ahead_s = 0.0                                # Backend.ahead_s
+        self._clock = [torch.cuda.Event(enable_timing=True) for _ in range(2)]      # `start` begins; its tokens are there
+        self._begun = 0.0                                 # the host's time of the first
 
     def _chosen(self, n: int) -> torch.Tensor:
         """Where the steps put their chosen tokens: the buffer behind the device's status word (one
@@ -413,8 +417,11 @@ class GraphBackend(EngineBackend):
             super()._read_soon()
             return
         self._host.mark()
+        begun, there = self._clock
+        there.record()
         self._start_lookahead = None
         next_u01, goes_on = look
+        t = time.perf_counter()
         keep = [i for i, c in enumerate(goes_on) if c]
         if keep:
             try:
@@ -422,6 +429,9 @@ class GraphBackend(EngineBackend):
                                            [next_u01[i] for i in keep] if next_u01 is not None else None, keep)
             except CacheFull:
                 self._ahead = None      # no room to run ahead: the first step is staged when it is asked for
+        now = time.perf_counter()
+        if there.query():               # some of that (all of it where the step was captured first) came after the tokens
+            self.ahead_s = min(now - t, max(0.0, now - self._begun - begun.elapsed_time(there) * 1e-3))
         self._host.wait()
 
     def start(self, prompts, u01, histories, lookahead=None):
@@ -430,9 +440,13 @@ class GraphBackend(EngineBackend):
         self._drain()
         b = bucket_for(max(1, len(prompts)))
         self._starting = None
+        self.ahead_s = 0.0
         self._start_lookahead = lookahead if (b <= kernels.RESULT_TOKENS and not self.sampler.params.has_penalties
                                               and lookahead is not None
                                               and (lookahead[0] is not None or not self.sampler.needs_uniform())) else None
+        if self._start_lookahead is not None:
+            self._begun = time.perf_counter()
+            self._clock[0].record()
         try:
             captured = self._start_captured(prompts, u01)
             slots, toks = captured if captured is not None else super().start(prompts, u01, histories)

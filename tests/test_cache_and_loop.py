@@ -404,6 +404,26 @@ def test_loop_look_ahead_begins_with_the_prompts(temperature, budget):
     assert logs[0] == logs[1]
 
 
+def test_what_a_backend_does_for_the_first_step_is_decode_time():
+    """A backend that goes on with the first decode step after the prompts' tokens are there says for how long: the rates
+    are then those of a backend that does the same work in `decode`."""
+    now = [0.0]
+
+    class Timed(LookingAheadFromTheStart):
+        def start(self, *a, **kw):
+            now[0] += 2.0 + 0.25          # the prompts, then the first step's staging
+            self.ahead_s = 0.25
+            return super().start(*a, **kw)
+
+        def decode(self, *a, **kw):
+            now[0] += 1.0
+            return super().decode(*a, **kw)
+
+    res = GenerationLoop(Timed({0: [5, 6, 7], 1: [8, 9, 3]}), SamplingParams(temperature=0.0), max_new_tokens=3, max_batch=1,
+                         clock=lambda: now[0]).run([[0, 50], [1]])
+    assert res.stats.prefill_ms == 2 * 2000 and res.stats.decode_ms == 2 * 2250
+
+
 def test_plan_batches_respects_cache_room():
     assert plan_batches([10, 10, 10], [5, 5, 5], max_batch=2, token_budget=1000, page=64) == [[0, 1], [2]]
     assert plan_batches([60, 60, 60], [10, 10, 10], max_batch=8, token_budget=256, page=64) == [[0, 1], [2]]

@@ -81,6 +81,20 @@ def test_first_decode_step_runs_ahead_of_the_prompts_tokens(lens, room, dirs):
     eng.cache.check()
 
 
+def test_prefill_time_is_the_prompts_own(dirs):
+    """The first decode step runs ahead of the prompts' tokens, and is captured there in an engine's first call (its prompts'
+    step having been captured by a call of one token): the reported prefill time does not grow by that."""
+    from lastengine_b200 import Engine, SamplingParams
+    eng = Engine.from_pretrained(dirs["A"], dtype="float32", max_tokens=1024)
+    prompts, greedy = H.requests_for(TINY_A, [5, 20], 51), SamplingParams(temperature=0.0)
+    for _ in range(3):
+        alone = eng.generate(prompts, greedy, max_new_tokens=1, stop_token_ids=[])
+    first = eng.generate(prompts, greedy, max_new_tokens=8, stop_token_ids=[])      # captures the decode step
+    assert first.stats.prefill_ms < first.stats.decode_ms       # a capture takes far longer than a prompt's replay
+    again = eng.generate(prompts, greedy, max_new_tokens=8, stop_token_ids=[])
+    assert again.tokens == first.tokens and [t[:1] for t in again.tokens] == alone.tokens
+
+
 def test_sampling_is_seeded_and_independent_of_batching(dirs):
     from lastengine_b200 import Engine, SamplingParams
     eng = Engine.from_pretrained(dirs["A"], dtype="float32", max_tokens=1024)
