@@ -332,12 +332,10 @@ static int launch_attention(void* out, float* part, const void* q, const void* k
   const int R = QT * HC;
   const int n_hc = ceil_div(G, HC);
   size_t smem = ((size_t)R * hd + 32 * (hd + 1) + 32 * vd + ATT_WARPS * ATT_RPW * 32) * sizeof(float);
-  auto kern = attention_kernel<T, CT, HDL>;
-  static size_t smem_set = 0;
-  if (smem > 48 * 1024 && smem > smem_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr auto kern = attention_kernel<T, CT, HDL>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = leb_allow_smem<kern>();
     if (e != cudaSuccess) return leb_fail("leb_attention: shared memory %zu: %s", smem, cudaGetErrorString(e));
-    smem_set = smem;
   }
   dim3 grid(ceil_div(max_qlen, QT), nkv * n_hc, B * n_splits);
   LEB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "leb_attention: grid too large (%u, %u)", grid.y, grid.z);

@@ -9,6 +9,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #define LEB_API extern "C" __attribute__((visibility("default")))
 
 // element type codes shared with the Python side
@@ -197,6 +199,19 @@ __device__ __forceinline__ float sink_quotient(float m, float l, float sink) {
 }
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+// Allows a kernel all of a block's 227 KB of dynamic shared memory.  The limit belongs to a device's copy of the kernel, so it
+// is raised once on each device that launches it.
+template <auto KERNEL>
+static inline cudaError_t leb_allow_smem() {
+  static std::atomic<bool> allowed[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev >= 0 && dev < 64 && allowed[dev].load(std::memory_order_relaxed))) return e;
+  e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) allowed[dev].store(true, std::memory_order_relaxed);
+  return e;
+}
 
 // SMs of the current device, asked once per device (device_info.cu); launch shapes that are
 // chosen for "a wave of blocks" use it.

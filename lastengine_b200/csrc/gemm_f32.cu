@@ -297,7 +297,7 @@ template <int MT>
 static int launch_f32_stream(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldc,
                              int accumulate, cudaStream_t st) {
   constexpr int smem = F32Stream<MT>::SMEM;
-  static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_stream_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t set = leb_allow_smem<gemm_f32_stream_kernel<MT>>();
   LEB_REQUIRE(set == cudaSuccess, "leb_gemm_f32: %s", cudaGetErrorString(set));
   const int tiles = ceil_div(N, F32S_ROWS), sms = sm_count();
   const int blocks = ceil_div(tiles, ceil_div(tiles, sms));        // as many tiles for every block
@@ -310,8 +310,8 @@ template <int BM, int BN, int WM, int WN, int WK, bool VEC>
 static int launch_f32_tile(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldc, int accumulate,
                            const int* group_offsets, int groups, size_t w_group_stride, cudaStream_t st) {
   constexpr int smem = F32Tile<BM, BN, WK>::SMEM;
-  auto kernel = gemm_f32_tile_kernel<BM, BN, WM, WN, WK, VEC>;
-  static const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr auto kernel = gemm_f32_tile_kernel<BM, BN, WM, WN, WK, VEC>;
+  const cudaError_t set = leb_allow_smem<kernel>();
   LEB_REQUIRE(set == cudaSuccess, "leb_gemm_f32: %s", cudaGetErrorString(set));
   const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, BN);
   LEB_REQUIRE(tiles < (1ll << 24) && groups <= 65535, "leb_gemm_f32: too many tiles (%lld) or groups (%d)", tiles, groups);

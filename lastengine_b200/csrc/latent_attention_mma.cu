@@ -623,8 +623,8 @@ static int launch_latent_few(bf16* out, float* part, const bf16* qt, const bf16*
                              const int* seq_qstart, const int* seq_qlen, const float* sink, int M, int B, int H, int rank,
                              int rot, int page_size, int window, int chunk, float scale, int n_splits, cudaStream_t st) {
   const size_t smem = lm_few_smem_bytes(rank + rot, WIDE);
-  auto kern = latent_attention_mma_few_kernel<NT, WIDE>;
-  static const cudaError_t set = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  constexpr auto kern = latent_attention_mma_few_kernel<NT, WIDE>;
+  const cudaError_t set = leb_allow_smem<kern>();
   LEB_REQUIRE(set == cudaSuccess, "leb_latent_attention_mma: %s", cudaGetErrorString(set));
   leb_launch(kern, dim3(B * n_splits), dim3(256), smem, st, out, part, qt, qr, pool, block_table, bt_width, seq_slot, seq_pos0,
              seq_qstart, seq_qlen, sink, M, H, rank, rot, page_size, window, chunk, scale, n_splits);
