@@ -1089,10 +1089,12 @@ def test_linear_tc_pairs(M, N, K_):
 
 @pytest.mark.parametrize("M,N,K_", [(17, 2048, 2048), (64, 352, 128), (100, 6144, 64), (33, 11264, 192), (128, 100, 200),
                                     (1, 128, 64), (16, 48, 72), (48, 2048, 5632), (64, 65536, 256),
-                                    (65, 2048, 2048), (96, 352, 5632), (90, 100, 200), (97, 6144, 136)])
+                                    (65, 2048, 2048), (96, 352, 5632), (90, 100, 200), (97, 6144, 136),
+                                    (24, 100, 1024), (24, 100, 1280), (24, 100, 2048), (24, 100, 2304), (24, 100, 4096), (24, 100, 4352), (40, 100, 8192)])
 def test_linear_skinny(M, N, K_):
     """The swapped-operand tcgen05 product with K sliced over blocks: store, add to residual, both
-    result types, sizes that leave partial tiles and slices."""
+    result types, sizes that leave partial tiles and slices; 4 and 5, 8 and 9, 16 and 17, and 32 slices (the second
+    kernel asks for up to 4, 8 or 16 at a time)."""
     x, w = gen(M, K_, seed=120, dtype=torch.bfloat16), gen(N, K_, seed=121, scale=0.05, dtype=torch.bfloat16)
     want = x.double() @ w.double().T
     out = torch.full((M, N), float("nan"), device=DEV)
