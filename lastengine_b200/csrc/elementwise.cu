@@ -84,7 +84,11 @@ __global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x
 
 // The same norm for bfloat16 output with 16-byte loads: a thread keeps its CH float4 pieces of
 // the row in registers between the sum and the product, so the row is read once.
-template <int CH>
+// EARLY: the weights, which do not depend on the kernel before this one, are fetched before the wait for it (1% of a step
+// with a norm kernel per sublayer).  They take registers until the end, so fewer blocks fit an SM: rows of more than 2,048
+// numbers are normed so where one or two waves do and that makes none more (512 rows of 4,096 3.7 -> 2.8 us, of 8,192 4.3 and
+// 5.0; 4,096 rows of 4,096 13.5 and 14.7, of 5,120 20.8 and 23.6).
+template <int CH, bool EARLY>
 __global__ void __launch_bounds__(256)
 rmsnorm_bf16_vec_kernel(bf16* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
                         const int* __restrict__ rows, int D, float eps) {
@@ -94,9 +98,9 @@ rmsnorm_bf16_vec_kernel(bf16* __restrict__ out, const float* __restrict__ x, con
   const int n4 = D >> 2;
   float4 v[CH], ww[CH];
 #pragma unroll
-  for (int c = 0; c < CH; c++) {      // the weights do not depend on the kernel before this one (1% of a step with a norm kernel per sublayer)
+  for (int c = 0; c < CH; c++) {
     const int i = threadIdx.x + c * 256;
-    if (i < n4) ww[c] = w4[i];
+    if (EARLY && i < n4) ww[c] = w4[i];
   }
   pdl_wait();
   const int m = blockIdx.x;
@@ -117,11 +121,26 @@ rmsnorm_bf16_vec_kernel(bf16* __restrict__ out, const float* __restrict__ x, con
   for (int c = 0; c < CH; c++) {
     const int i = threadIdx.x + c * 256;
     if (i < n4) {
+      if (!EARLY) ww[c] = w4[i];
       __nv_bfloat162 lo = __floats2bfloat162_rn(v[c].x * r * ww[c].x, v[c].y * r * ww[c].y);
       __nv_bfloat162 hi = __floats2bfloat162_rn(v[c].z * r * ww[c].z, v[c].w * r * ww[c].w);
       o[i] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
     }
   }
+}
+
+template <int CH>
+static void launch_rmsnorm_vec(bf16* out, const float* x, const float* w, const int* rows, int M, int D, float eps, cudaStream_t st) {
+  auto resident = [](void (*kern)(bf16*, const float*, const float*, const int*, int, float)) {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, 0) == cudaSuccess && n > 0 ? n : 1;
+  };
+  static const int early = resident(rmsnorm_bf16_vec_kernel<CH, true>), late = resident(rmsnorm_bf16_vec_kernel<CH, false>);
+  const int sms = sm_count();
+  const int waves = ceil_div(M, early * sms);
+  const bool first = CH <= 2 || (waves <= 2 && waves <= ceil_div(M, late * sms));
+  leb_launch(first ? rmsnorm_bf16_vec_kernel<CH, true> : rmsnorm_bf16_vec_kernel<CH, false>, dim3(M), dim3(256), 0, st, out, x, w, rows,
+             D, eps);
 }
 
 LEB_API int leb_rmsnorm(void* out, int out_dtype, const float* x, const float* w, const int* rows,
@@ -131,10 +150,10 @@ LEB_API int leb_rmsnorm(void* out, int out_dtype, const float* x, const float* w
       ((uintptr_t)w % 16) == 0 && ((uintptr_t)out % 8) == 0) {
     const int ch = ceil_div(D / 4, 256);
     bf16* o = (bf16*)out;
-    if (ch <= 1) leb_launch(rmsnorm_bf16_vec_kernel<1>, dim3(M), dim3(256), 0, st, o, x, w, rows, D, eps);
-    else if (ch <= 2) leb_launch(rmsnorm_bf16_vec_kernel<2>, dim3(M), dim3(256), 0, st, o, x, w, rows, D, eps);
-    else if (ch <= 4) leb_launch(rmsnorm_bf16_vec_kernel<4>, dim3(M), dim3(256), 0, st, o, x, w, rows, D, eps);
-    else leb_launch(rmsnorm_bf16_vec_kernel<8>, dim3(M), dim3(256), 0, st, o, x, w, rows, D, eps);
+    if (ch <= 1) launch_rmsnorm_vec<1>(o, x, w, rows, M, D, eps, st);
+    else if (ch <= 2) launch_rmsnorm_vec<2>(o, x, w, rows, M, D, eps, st);
+    else if (ch <= 4) launch_rmsnorm_vec<4>(o, x, w, rows, M, D, eps, st);
+    else launch_rmsnorm_vec<8>(o, x, w, rows, M, D, eps, st);
     LEB_CHECK_LAUNCH("leb_rmsnorm");
     return 0;
   }

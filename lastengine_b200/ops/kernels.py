@@ -264,7 +264,8 @@ def embed(x: torch.Tensor, table: torch.Tensor, tokens: torch.Tensor, scale: flo
 
 def rmsnorm(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, eps: float,
             rows: torch.Tensor | None = None, add: bool = False) -> None:
-    """out = x * rsqrt(mean(x^2) + eps) * w  (out += ... when add).  x is float."""
+    """out = x * rsqrt(mean(x^2) + eps) * w  (out += ... when add).  x is float.  (`w` may be fetched ahead of the wait for the
+    kernel launched before: it must not be what that kernel writes.)"""
     _cuda(out, "rmsnorm.out")
     _cuda(x, "rmsnorm.x", torch.float32)
     _cuda(w, "rmsnorm.w", torch.float32)

@@ -64,6 +64,17 @@ def test_rmsnorm(D):
     assert err(res, r0.cpu().double() + want) < 1e-6
 
 
+@pytest.mark.parametrize("D", [2052, 4096, 8192])
+def test_rmsnorm_of_many_rows_gives_the_bits_of_few(D):
+    """Few rows fetch the weights ahead of the wait for the kernel before, many do not (more than fit the SMs at once)."""
+    x, w = gen(3001, D, seed=2, dtype=torch.float32).to(DEV), (1 + 0.1 * gen(D, seed=3)).to(DEV)
+    many, few = (torch.empty(3001, D, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    K().rmsnorm(many, x, w, 1e-3)
+    for r in range(0, 3001, 100):
+        K().rmsnorm(few[r:r + 100], x[r:r + 100], w, 1e-3)
+    assert torch.equal(many, few)
+
+
 def test_swiglu():
     gu = gen(9, 2 * 37, seed=5, scale=2.0)
     want = P.silu(gu[:, :37].double()) * gu[:, 37:].double()
