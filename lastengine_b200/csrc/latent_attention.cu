@@ -42,9 +42,39 @@ __device__ __forceinline__ void rotate_unit(CT* __restrict__ dst, const T* __res
   dst[ib] = from_f32<CT>(v * c + u * s);
 }
 
+// Sum of the squares of n numbers by the whole block, in the order of 256 threads: in a block of 128 each of them stands
+// for two, so that a row has the same bits from either.
+template <typename T, int THREADS>
+__device__ __forceinline__ float row_squares(const T* __restrict__ x, int n, float* red) {
+  static_assert(THREADS == 128 || THREADS == 256, "a thread is one or two of 256");
+  constexpr bool two = THREADS == 128;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool second = two && n > 128;
+  float a = 0.f, b = 0.f;
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const float v = to_f32(x[i]), u = second && i + 128 < n ? to_f32(x[i + 128]) : 0.f;
+    a += v * v;
+    b += u * u;
+  }
+  a = warp_sum(a);
+  if (second) b = warp_sum(b);
+  __syncthreads();      // `red` may still be read from an earlier call
+  if (lane == 0) {
+    red[warp] = a;
+    if (two) red[warp + 4] = b;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const float t = warp_sum(lane < 8 ? red[lane] : 0.f);
+    if (lane == 0) red[32] = t;
+  }
+  __syncthreads();
+  return red[32];
+}
+
 // The cache row [c | k^r] of row m: lat = `rank` numbers of the latent before its norm, then `rot` of the shared key part
 // before its rotation.  By the whole block; rows of padding sequences touch no cache.
-template <typename T, typename CT>
+template <typename T, typename CT, int THREADS>
 __device__ __forceinline__ void latent_cache_row(const T* __restrict__ lat, int m, CT* __restrict__ pool,
                                                  const int* __restrict__ block_table, int bt_width,
                                                  const int* __restrict__ row_seq, const int* __restrict__ row_pos,
@@ -54,17 +84,12 @@ __device__ __forceinline__ void latent_cache_row(const T* __restrict__ lat, int 
   const int b = row_seq[m], pos = row_pos[m];
   if (seq_slot[b] < 0) return;      // a padding sequence touches no cache
   const int page = block_table[(size_t)b * bt_width + pos / page_size];      // (on its way under the sum)
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < rank; i += blockDim.x) {
-    const float v = to_f32(lat[i]);
-    ss += v * v;
-  }
-  ss = block_sum(ss, red);
+  const float ss = row_squares<T, THREADS>(lat, rank, red);
   if (page < 0) return;
   const float r = 1.0f / sqrtf(ss / (float)rank + eps);
   CT* dst = pool + ((size_t)page * page_size + pos % page_size) * (size_t)(rank + rot);
-  for (int i = threadIdx.x; i < rank; i += blockDim.x) dst[i] = from_f32<CT>(to_f32(lat[i]) * r * wkv[i]);
-  for (int t = threadIdx.x; t < rot - rot_dims / 2; t += blockDim.x)
+  for (int i = threadIdx.x; i < rank; i += THREADS) dst[i] = from_f32<CT>(to_f32(lat[i]) * r * wkv[i]);
+  for (int t = threadIdx.x; t < rot - rot_dims / 2; t += THREADS)
     rotate_unit<T, CT>(dst + rank, lat + rank, t, (float)pos, inv_freq, rot_dims, neox);
 }
 
@@ -95,13 +120,13 @@ __device__ __forceinline__ void latent_split_row(T* __restrict__ qn, T* __restri
   }
 }
 
-// Two blocks per row (one without a cache write): the query latent's norm, and the cache row, side by side (a
-// step of few rows waits for their chains of loads and block sums, not for bytes: 8 rows 12.7 -> 8.6 us).  in [M, ld_in]: columns [0, q_rank) the query latent before its norm, then
-// (own_kv) `rank` columns of the key/value latent before its norm and `rot` columns of the shared
-// key part before its rotation.  Leaves cq [M, q_rank] = rmsnorm(.) * wq and, for rows of live
-// sequences, the cache row [c | k^r] at the row's position.
-template <typename T, typename CT>
-__global__ void __launch_bounds__(256)
+// in [M, ld_in]: columns [0, q_rank) the query latent before its norm, then (own_kv) `rank` columns of the key/value
+// latent before its norm and `rot` columns of the shared key part before its rotation.  Leaves cq [M, q_rank] = rmsnorm(.) * wq
+// and, for rows of live sequences, the cache row [c | k^r] at the row's position.  A step of few rows waits for the two
+// chains of loads and block sums, not for bytes: the query latent and the cache row have a block of 256 threads each.
+// One of many rows is bound by the blocks it starts: a block of 128 does both (LEB_PREP_FEW below has the times).
+template <typename T, typename CT, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 latent_prep_kernel(T* __restrict__ cq, const T* __restrict__ in, int ld_in, CT* __restrict__ pool,
                    const int* __restrict__ block_table, int bt_width, const int* __restrict__ row_seq,
                    const int* __restrict__ row_pos, const int* __restrict__ seq_slot,
@@ -113,18 +138,12 @@ latent_prep_kernel(T* __restrict__ cq, const T* __restrict__ in, int ld_in, CT* 
   const int m = blockIdx.x;
   const T* row = in + (size_t)m * ld_in;
   if (blockIdx.y == 0) {
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < q_rank; i += blockDim.x) {
-      const float v = to_f32(row[i]);
-      ss += v * v;
-    }
-    ss = block_sum(ss, red);
-    const float r = 1.0f / sqrtf(ss / (float)q_rank + eps);
-    for (int i = threadIdx.x; i < q_rank; i += blockDim.x)
+    const float r = 1.0f / sqrtf(row_squares<T, THREADS>(row, q_rank, red) / (float)q_rank + eps);
+    for (int i = threadIdx.x; i < q_rank; i += THREADS)
       cq[(size_t)m * q_rank + i] = from_f32<T>(to_f32(row[i]) * r * wq[i]);
-    return;
+    if (THREADS == 256 || !pool) return;
   }
-  latent_cache_row<T, CT>(row + q_rank, m, pool, block_table, bt_width, row_seq, row_pos, seq_slot, wkv, eps, inv_freq, rot_dims,
+  latent_cache_row<T, CT, THREADS>(row + q_rank, m, pool, block_table, bt_width, row_seq, row_pos, seq_slot, wkv, eps, inv_freq, rot_dims,
                           neox, rank, rot, page_size, red);
 }
 
@@ -157,7 +176,7 @@ latent_rows_kernel(T* __restrict__ qn, T* __restrict__ qr, const T* __restrict__
   if (blockIdx.y == 0)
     latent_split_row<T>(qn, qr, row, m, (float)row_pos[m], inv_freq, rot_dims, neox, M, H, dim, dim_p, rot, wide != 0);
   else
-    latent_cache_row<T, T>(row + H * (dim + rot), m, pool, block_table, bt_width, row_seq, row_pos, seq_slot, wkv, eps, inv_freq,
+    latent_cache_row<T, T, 256>(row + H * (dim + rot), m, pool, block_table, bt_width, row_seq, row_pos, seq_slot, wkv, eps, inv_freq,
                            rot_dims, neox, rank, rot, page_size, red);
 }
 
@@ -417,6 +436,9 @@ LEB_API int leb_latent_rows(void* qn, void* qr, const void* in, int ld_in, int d
   return 0;
 }
 
+// Rows up to which the query latent and the cache row have a block each.  One block of 128 against two of 256, us a launch: 64 rows of
+// 1,536 + 512 numbers 5.0 and 3.7, 512 rows 5.4 and 4.7, 768 rows 5.6 and 6.5, 8,192 rows 24.6 and 40.4; rows of 384 + 128 cross at 600.
+#define LEB_PREP_FEW 592
 LEB_API int leb_latent_prep(void* cq, const void* in, int ld_in, int dtype, void* pool, const int* block_table,
                             int bt_width, const int* row_seq, const int* row_pos, const int* seq_slot,
                             const float* wq, const float* wkv, float eps, const float* inv_freq, int rot_dims,
@@ -428,12 +450,14 @@ LEB_API int leb_latent_prep(void* cq, const void* in, int ld_in, int dtype, void
   LEB_REQUIRE(rot_dims >= 0 && rot_dims <= rot && rot_dims % 2 == 0 && (rot_dims == 0 || inv_freq),
               "leb_latent_prep: %d rotated dimensions of %d", rot_dims, rot);
   LebPlainLaunches plain(true);
+  const bool few = M <= LEB_PREP_FEW;
+  const dim3 grid(M, pool && few ? 2 : 1), block(few ? 256 : 128);
   if (dtype == LEB_F32)
-    leb_launch(latent_prep_kernel<float, float>, dim3(M, pool ? 2 : 1), dim3(256), 0, st, (float*)cq, (const float*)in, ld_in,
+    leb_launch(few ? latent_prep_kernel<float, float, 256> : latent_prep_kernel<float, float, 128>, grid, block, 0, st, (float*)cq, (const float*)in, ld_in,
                (float*)pool, block_table, bt_width, row_seq, row_pos, seq_slot, wq, wkv, eps, inv_freq, rot_dims, neox,
                q_rank, rank, rot, page_size);
   else if (dtype == LEB_BF16)
-    leb_launch(latent_prep_kernel<bf16, bf16>, dim3(M, pool ? 2 : 1), dim3(256), 0, st, (bf16*)cq, (const bf16*)in, ld_in,
+    leb_launch(few ? latent_prep_kernel<bf16, bf16, 256> : latent_prep_kernel<bf16, bf16, 128>, grid, block, 0, st, (bf16*)cq, (const bf16*)in, ld_in,
                (bf16*)pool, block_table, bt_width, row_seq, row_pos, seq_slot, wq, wkv, eps, inv_freq, rot_dims, neox,
                q_rank, rank, rot, page_size);
   else

@@ -347,6 +347,40 @@ def test_decoding_with_the_key_range_cut_into_pieces_for_the_blocks(dtype):
         assert H.rel_err(torch.cat(got[j]), want[j][-4:]) < TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("q_rank,rank,rot", [(384, 128, 32), (100, 40, 8), (257, 129, 6), (1536, 512, 64)])
+def test_latent_preparation_of_many_rows_gives_the_bits_of_few(dtype, q_rank, rank, rot):
+    """The query latent and the cache row by a block each (256 threads), or in a step of many rows by one block (of 128) both:
+    the same sums in the same order.  A padding sequence among the rows."""
+    from lastengine_b200.engine.batch import BatchBuilder
+    g = torch.Generator().manual_seed(q_rank)
+    M, page = 2100, 64
+    lens = [700, 650, 750]
+    proj = torch.randn(M, q_rank + rank + rot + 8, generator=g).to(dtype).to(DEV)[:, :q_rank + rank + rot]
+    wq, wkv, inv = (torch.randn(n, generator=g).to(DEV) for n in (q_rank, rank, rot // 2))
+    table = np.random.default_rng(3).permutation(36).astype(np.int32).reshape(3, 12)
+
+    def run(step):
+        cq = torch.empty(M, q_rank, device=DEV, dtype=dtype)
+        pool = torch.zeros(36, page, rank + rot, device=DEV, dtype=dtype)
+        for lo in range(0, 750, step):
+            n = [max(0, min(step, m - lo)) for m in lens]
+            at = [0, 700, 1350]
+            for i in range(3) if step < 750 else (None,):
+                seqs = [i] if i is not None else [0, 1, 2]
+                if not sum(n[j] for j in seqs):
+                    continue
+                b = BatchBuilder(torch.device(DEV)).build([-1 if j == 1 else j for j in seqs], [[0] * n[j] for j in seqs],
+                                                          [lo] * len(seqs), [], {0: table[seqs]})
+                r0 = at[seqs[0]] + lo
+                rows = slice(r0, r0 + sum(n[j] for j in seqs))
+                K().latent_prep(cq[rows], proj[rows], pool, b.tables[0], b, wq, wkv, 1e-5, inv, rot, rank, rot, page)
+        return cq, pool
+
+    for a, b in zip(run(750), run(90)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("H_,rank,rot,window,wide", [(1, 64, 0, 0, False), (5, 128, 16, 0, False), (16, 512, 64, 0, False),
                                                      (16, 192, 64, 100, False), (9, 512, 128, 70, True), (16, 256, 32, 0, True)])
 @pytest.mark.parametrize("splits", [1, 3, 16])
