@@ -315,13 +315,14 @@ __global__ void __launch_bounds__(256) qk_rope_store_many_kernel(
   __shared__ long long kdst[R];
   __shared__ float factor[R];
   pdl_trigger();   // the kernel after this one may start and wait (see common.cuh)
-  pdl_wait();
   const int groups = (M + R - 1) / R;
   if ((int)blockIdx.x >= groups) {
+    pdl_wait();
     store_value_tile<bf16, bf16>(blockIdx.x - groups, v_in, kv_stride, v_pool, block_table, bt_width, row_seq, row_pos,
                                  seq_slot, M, nkv, vd, page_size, v_norm, eps, vin);
     return;
   }
+  // (positions, pages and sines do not depend on the kernel before this one, as in the kernel above)
   const int m0 = blockIdx.x * R, rows = min(R, M - m0);
   for (int i = threadIdx.x; i < rows * HALF; i += 256) {
     const int r = i / HALF, p = i % HALF;
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(256) qk_rope_store_many_kernel(
     kdst[threadIdx.x] = off;
     factor[threadIdx.x] = query_temperature(pos, temp_coef, temp_every);
   }
+  pdl_wait();
   __syncthreads();
   const int d0 = 8 * (threadIdx.x & 3);
   float wq[16], wk[16];
@@ -597,8 +599,10 @@ LEB_API int leb_qk_rope_store(void* q_out, const void* q_in, int q_stride, const
   if (dtype == LEB_BF16 && (inv_freq ? neox && rope_dim == hd : temp_coef != 0.f) && hin == hd && (hd == 64 || hd == 128)) {
     // From some hundred rows on the launch is bound by memory, not by its start: 16 bytes a thread, where rows and
     // pages allow it (40 heads of 64, values included: 200 rows 12.7 -> 10.7 us a launch, 2,048 25.1 -> 14.8, 16,384
-    // 169 -> 85, of which the bytes alone would take 31; below 128 rows the start of the launch is most of both).
-    if (hd == 64 && M >= 128 && q_stride % 8 == 0 && kv_stride % 8 == 0 &&
+    // 169 -> 85, of which the bytes alone would take 31; below 128 rows the start of the launch is most of both).  Queries
+    // alone have no values to transpose, and a block waits once for its sines: from 16,384 of them on (with the attention and
+    // the product behind them 190 rows of 8 heads 16.6 us by the lanes and 17.4 so, 520 of 32 39.9 both ways, 800 of 32 31.6 and 30.1).
+    if (hd == 64 && M >= 128 && (k_in || (long long)M * nh >= 16384) && q_stride % 8 == 0 && kv_stride % 8 == 0 &&
         (((uintptr_t)q_out | (uintptr_t)q_in | (uintptr_t)k_in | (uintptr_t)k_pool) & 15) == 0) {
       const bool big = M >= 8 * sm_count();      // eight rows a block once that leaves every SM one
       const dim3 grid(ceil_div(M, big ? 8 : 2) + tiles);

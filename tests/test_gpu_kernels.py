@@ -521,6 +521,26 @@ def test_qk_rope_store_of_many_rows_gives_the_bits_of_few(lens, nh, nkv, weights
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("M,nh", [(600, 32), (520, 32), (190, 8), (2100, 8)])
+def test_rotation_of_queries_alone_on_both_sides_of_its_line(M, nh):
+    """Queries without keys: from 16,384 of them on the kernel of many rows, below it the lanes; the bits of steps of 60 rows."""
+    q = gen(M, nh * 64, seed=30, dtype=torch.bfloat16).to(DEV)
+    qn = (1 + 0.1 * gen(64, seed=31)).to(DEV)
+    inv = torch.pow(torch.tensor(12345.0, dtype=torch.float64), -torch.arange(32, dtype=torch.float64) / 32).float().to(DEV)
+    table = {0: np.arange(-(-M // 64), dtype=np.int32)[None]}
+
+    def run(step):
+        out = torch.zeros(M, nh * 64, device=DEV, dtype=torch.bfloat16)
+        for lo in range(0, M, step):
+            n = min(step, M - lo)
+            b = builder().build([0], [[0] * n], [lo], [], table)
+            K().qk_rope_store(out[lo:lo + n], q[lo:lo + n], None, None, None, None, b.tables[0], b, qn, None, 1e-4, inv, 64, True, nh,
+                              1, 64, 64)
+        return out
+
+    assert torch.equal(run(M), run(60))
+
+
 # ---- words between host and device ---------------------------------------------------------------------
 def test_words_of_dropped_owners_stay_until_the_device_is_through_with_them():
     """Builders and result buffers dropped while their transfers wait behind other work: every step finds its own words, and
