@@ -293,6 +293,91 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
   }
 }
 
+// ---- few k, and operands without whole 16-byte vectors: blocks by the SM --------------------------------
+// A block of 256 threads computes 64 x 64 outputs, 4 x 4 a thread, from 16 k at a time that single loads bring to shared memory.
+// Nothing overlaps inside a block; four or five of them share an SM and overlap each other.  It takes any alignment, a
+// stage is 16 k, and a block costs nothing where it has no rows: where K is a chunk or three it is ahead of the
+// tiles above, whose warps share out chunks that are not there (300 rows x 2,048 x 128: 15 us, 59 in tiles of 64 x 64 over four
+// chunks; 64 experts of one row, 512 x 512: 87 and 121), and of their 4-byte copies where vectors are broken (300 x 771 x 301:
+// 20 and 33 us).  CHUNKS: K is more than one chunk (the sums over chunks take 16 registers, and one of five blocks).  Launched
+// plainly: with the programmatic attribute its blocks came to the SMs unevenly (1,100 x 1,024 x 1,024: 103 and 160 us).
+#define F32_BM 64
+#define F32_BN 64
+#define F32_BK 16
+template <bool CHUNKS>
+__global__ void __launch_bounds__(256)
+gemm_f32_plain_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                      int M, int N, int K, int lda, int ldc, int accumulate,
+                      const int* __restrict__ group_offsets, size_t w_group_stride) {
+  __shared__ float As[F32_BK][F32_BM + 4];
+  __shared__ float Ws[F32_BK][F32_BN + 4];
+  int row_begin = 0, row_end = M;
+  if (group_offsets) {
+    row_begin = group_offsets[blockIdx.z];
+    row_end = group_offsets[blockIdx.z + 1];
+    W += (size_t)blockIdx.z * w_group_stride;
+  }
+  const int m0 = row_begin + blockIdx.y * F32_BM;
+  if (m0 >= row_end) return;
+  const int n0 = blockIdx.x * F32_BN;
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;
+  const int lrow = tid >> 2, lk = (tid & 3) * 4;  // loader: row of the tile, first of 4 k
+  float acc[4][4], total[CHUNKS ? 4 : 1][CHUNKS ? 4 : 1];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = total[CHUNKS ? i : 0][CHUNKS ? j : 0] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += F32_BK) {
+    {
+      const int r = m0 + lrow;
+      const float* src = A + (size_t)r * lda + k0 + lk;
+#pragma unroll
+      for (int e = 0; e < 4; e++) As[lk + e][lrow] = (r < row_end && k0 + lk + e < K) ? src[e] : 0.f;
+      const int n = n0 + lrow;
+      const float* wsrc = W + (size_t)n * K + k0 + lk;
+#pragma unroll
+      for (int e = 0; e < 4; e++) Ws[lk + e][lrow] = (n < N && k0 + lk + e < K) ? wsrc[e] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < F32_BK; kk++) {
+      float a[4], w[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
+#pragma unroll
+      for (int j = 0; j < 4; j++) w[j] = Ws[kk][tx * 4 + j];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+    }
+    __syncthreads();
+    if (CHUNKS && (k0 + F32_BK) % F32_CHUNK == 0) {      // a chunk is done
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          total[CHUNKS ? i : 0][CHUNKS ? j : 0] += acc[i][j];
+          acc[i][j] = 0.f;
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int r = m0 + ty * 4 + i;
+    if (r >= row_end) continue;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int n = n0 + tx * 4 + j;
+      if (n >= N) continue;
+      float* c = C + (size_t)r * ldc + n;
+      const float sum = (CHUNKS ? total[CHUNKS ? i : 0][CHUNKS ? j : 0] : 0.f) + acc[i][j];
+      *c = accumulate ? *c + sum : sum;
+    }
+  }
+}
+
 template <int MT>
 static int launch_f32_stream(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldc,
                              int accumulate, cudaStream_t st) {
@@ -322,6 +407,47 @@ static int launch_f32_tile(float* C, const float* A, const float* W, int M, int 
   return 0;
 }
 
+// Which kernel takes a product (0-4: tiles in the order below, F32_PLAIN, F32_STREAM): the one whose blocks take the SM with most of
+// them least, in nanoseconds measured on B200 (9 to 2,048 rows, 16 to 11,264 columns, K from 16 to 2,048; 4 to 64 groups): a
+// fixed part, and per block of an SM a part of its own and one per round, of `wk` chunks of k (the plain kernel: of 16 k).  Over 967
+// such sizes the choice takes 0.46 (up to 16 rows), 0.62 (more; 0.83 with broken vectors) and 0.56 (groups) of the time of blocks of
+// 64 x 64 throughout, and above 1.1 of it at ten small sizes (by 0.3 to 2.4 us).  Groups count as many equally large ones as can
+// have rows; blocks of groups without any cost their start.
+enum { F32_PLAIN = 5, F32_STREAM = 6 };
+struct F32Cost {
+  int bm, bn, wk, fixed, block, round;
+};
+static int f32_choice(int M, int N, int K, int groups, bool vec, int sms) {      // groups: 0 for a product that is not grouped
+  static const F32Cost whole[5] = {{128, 128, 1, 0, 10500, 14600}, {64, 64, 4, 100, 1250, 18800}, {32, 32, 8, 1350, 0, 12200},
+                                   {64, 16, 8, 1400, 0, 12550}, {32, 16, 8, 1500, 0, 7600}};
+  static const F32Cost broken[5] = {{128, 128, 1, 0, 5000, 20500}, {64, 64, 4, 0, 1900, 22800}, {32, 32, 8, 1500, 1700, 13400},
+                                    {64, 16, 8, 1100, 1900, 14500}, {32, 16, 8, 1500, 2400, 7700}};
+  if (groups == 0 && M <= 8 && vec) return F32_STREAM;      // (measured up to 16 rows; up to 8 it is ahead or within 0.4 us everywhere)
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const long long live = groups > M ? M : groups < 1 ? 1 : groups, rows = up(M, live), chunks = up(K, F32_CHUNK);
+  auto per_sm = [&](int bm, int bn) { return up(live * up(rows, bm) * up(N, bn), sms); };
+  auto idle = [&](long long blocks, long long busy) { const long long n = up(blocks, sms) - busy; return n > 0 ? n : 0; };
+  int pick = F32_PLAIN;
+  const long long steps = up(K, F32_BK), per = per_sm(F32_BM, F32_BN), m_tiles = up(M, F32_BM);
+  const long long apart = per * (vec ? 230 + 870 * steps : 230 + 775 * steps), alone = up(per, 4) * steps * (vec ? 970 : 890);
+  long long best = (vec ? 1850 : 2100) + (apart > alone ? apart : alone) + 370 * idle(m_tiles * up(N, F32_BN) * (groups > 1 ? groups : 1), per);
+  if (groups > 1 && rows > F32_BM) best = best * 14 / 10;      // live blocks come to an SM in clusters
+  if (m_tiles > 65535) best = 1ll << 60;
+  const F32Cost* cost = vec ? whole : broken;
+  for (int i = 0; i < 5; i++) {
+    if (groups > 1 && (i == 0 || i == 3)) continue;
+    const F32Cost& c = cost[i];
+    const long long n = per_sm(c.bm, c.bn), all = up(M, c.bm) * up(N, c.bn), blocks = up(all, up(all, sms)) * (groups > 1 ? groups : 1);
+    const long long t = c.fixed + n * (c.block + c.round * up(chunks, c.wk)) + 600 * idle(blocks, n);
+    if (t < best) best = t, pick = i;
+  }
+  if (vec && groups == 0 && M <= 16 && 1000 + up(up(N, F32S_ROWS), sms) * 8300 * up(chunks, 16) <= best) pick = F32_STREAM;
+  return pick;
+}
+LEB_API int leb_gemm_f32_choice(int M, int N, int K, int groups, int vec, int sms) {
+  return M > 0 && N > 0 && K > 0 && sms > 0 ? f32_choice(M, N, K, groups, vec != 0, sms) : -1;
+}
+
 LEB_API int leb_gemm_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda,
                          int ldc, int accumulate, const int* group_offsets, int n_groups,
                          size_t w_group_stride, cudaStream_t st) {
@@ -329,28 +455,22 @@ LEB_API int leb_gemm_f32(float* C, const float* A, const float* W, int M, int N,
   LEB_REQUIRE(K > 0, "leb_gemm_f32: K must be positive");
   // 16-byte loads: rows of both operands begin on 16 bytes and hold whole vectors
   const bool vec = K % 4 == 0 && lda % 4 == 0 && w_group_stride % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
-  if (!group_offsets && M <= 16 && vec) {
+  const int groups = group_offsets ? n_groups : 1;
+  const int pick = f32_choice(M, N, K, group_offsets ? (n_groups > 0 ? n_groups : 1) : 0, vec, sm_count());
+  if (pick == F32_STREAM) {
     if (M == 1) return launch_f32_stream<1>(C, A, W, M, N, K, lda, ldc, accumulate, st);
     if (M == 2) return launch_f32_stream<2>(C, A, W, M, N, K, lda, ldc, accumulate, st);
     if (M <= 4) return launch_f32_stream<4>(C, A, W, M, N, K, lda, ldc, accumulate, st);
     if (M <= 8) return launch_f32_stream<8>(C, A, W, M, N, K, lda, ldc, accumulate, st);
     return launch_f32_stream<16>(C, A, W, M, N, K, lda, ldc, accumulate, st);
   }
-  const int groups = group_offsets ? n_groups : 1;
-  int pick = 0;
-  if (group_offsets) {
-    pick = M <= 32 * groups ? 4 : M <= 128 * groups ? 2 : 1;      // by the rows a group has on average
-  } else {
-    // The tile whose waves of one block per SM take least; the weights are a wave's measured microseconds per
-    // 2,048 of K.  (2,048 rows x 5,632 x 2,048 runs fastest in the largest tiles, 64 rows x 2,048 x 2,048
-    // in 28 us in tiles of 32 x 32, 31 in 64 x 16, 79 in 64 x 64 and 235 in 128 x 128.)
-    const int bm[5] = {128, 64, 32, 64, 32}, bn[5] = {128, 64, 32, 16, 16}, cost[5] = {2400, 790, 265, 275, 168};
-    long long best = -1;
-    for (int i = 0; i < 5; i++) {
-      const long long tiles = (long long)ceil_div(M, bm[i]) * ceil_div(N, bn[i]);
-      const long long t = (tiles + sm_count() - 1) / sm_count() * cost[i];
-      if (best < 0 || t < best) best = t, pick = i;
-    }
+  if (pick == F32_PLAIN) {
+    const dim3 grid(ceil_div(N, F32_BN), ceil_div(M, F32_BM), groups);
+    LEB_REQUIRE(groups <= 65535, "leb_gemm_f32: too many groups (%d)", groups);
+    (K > F32_CHUNK ? gemm_f32_plain_kernel<true> : gemm_f32_plain_kernel<false>)<<<grid, 256, 0, st>>>(
+        C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, w_group_stride);
+    LEB_CHECK_LAUNCH("leb_gemm_f32");
+    return 0;
   }
 #define LEB_F32_TILE(BM, BN, WM, WN, WK)                                                                                     \
   return vec ? launch_f32_tile<BM, BN, WM, WN, WK, true>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st) \

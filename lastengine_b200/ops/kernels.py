@@ -120,6 +120,7 @@ def _declare(L) -> None:
         "leb_retention": [P, P, P, P, P, I, I, P, P, P, I, F, F, P, P, P, P, I, I, I, I, I, P],
         "leb_retention_chunked": [P, P, P, P, P, I, I, P, P, P, P, I, F, F, P, P, P, P, I, I, I, I, I, P],
         "leb_retention_chunked_supported": [I, I],
+        "leb_gemm_f32_choice": [I, I, I, I, I, I],
         "leb_gemm_f32": [P, P, P, I, I, I, I, I, I, P, I, S, P],
         "leb_gemm_bf16_small": [P, I, P, P, I, I, I, I, I, I, P, I, S, I, P],
         "leb_gemm_bf16_stream": [P, I, P, P, I, I, I, I, I, I, P, I, I, F, P, P, P, P],
@@ -1691,6 +1692,8 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
     where a few hundred rows and a long K leave most SMs without a tile), from PAIRS_MIN_ROWS rows
     and large matrices 256 x 256 tiles on pairs of SMs; `streaming` asks for the register-fed
     weight-streaming kernel (the one that also serves grouped products) whatever the row count.
+    Kernels of a few rows fetch W ahead of their wait for the kernel launched before them: `w` must not be what that
+    kernel writes (a model's weights never are).
     """
     _cuda(x, "linear.x", contiguous=False)
     _cuda(w, "linear.w", x.dtype)

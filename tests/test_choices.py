@@ -1,0 +1,23 @@
+"""Which kernel a call takes, where that depends on sizes alone (no GPU)."""
+import pytest
+
+from lastengine_b200.ops import kernels
+
+
+@pytest.mark.parametrize("sms", [132, 148])
+def test_every_kernel_of_the_32_bit_product_is_chosen_somewhere(sms):
+    """... and only where it can run: the stream (6) takes up to 16 ungrouped rows of whole vectors, grouped products the
+    tiles 1, 2 and 4 or the blocks of 64 x 64 (5)."""
+    choice = kernels.lib().leb_gemm_f32_choice
+    sizes = [1, 3, 9, 16, 17, 36, 130, 523, 1757, 2557, 4000]
+    seen = {}
+    for groups in (0, 1, 3, 64):
+        for M in sizes:
+            for N in sizes:
+                for K in (4, 128, 132, 301, 1024, 5632):
+                    for vec in (0, 1) if K % 4 == 0 else (0,):
+                        k = choice(M, N, K, groups, vec, sms)
+                        seen.setdefault((min(groups, 2), vec), set()).add(k)
+                        assert 0 <= k <= 6 and (k != 6 or (groups == 0 and vec and M <= 16)) and (groups < 2 or k in (1, 2, 4, 5))
+    assert seen[0, 1] == set(range(7)) and seen[0, 0] == set(range(6)) and seen[2, 0] == seen[2, 1] == {1, 2, 4, 5}
+    assert choice(0, 1, 1, 0, 1, sms) == -1 and choice(1, 1, 0, 0, 1, sms) == -1

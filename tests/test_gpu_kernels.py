@@ -107,8 +107,7 @@ def test_linear_f32(M, N, K_):
 @pytest.mark.parametrize("M", [1, 2, 4, 8, 9, 16, 17, 32, 33, 64, 65, 129, 300])
 @pytest.mark.parametrize("N,K_", [(17, 4), (50, 124), (2400, 128), (36, 132), (130, 2052), (4111, 260), (33, 4100), (40, 301)])
 def test_linear_f32_sums(M, N, K_):
-    """Every kernel of the 32-bit product (the stream up to 16 rows, tiles of five sizes, sizes without whole 16-byte
-    vectors): part tiles, part chunks of k, more chunks than a round holds, rows with a stride, and the same bits
+    """The 32-bit product around the borders of its kernels' tiles (every one of them runs in the test below): part tiles, part chunks of k, more chunks than a round holds, rows with a stride, and the same bits
     whatever the row count.  A chunk of up to 128 products and a sum over K/128 chunks: each rounding is at most 2^-24
     of a partial sum, so 2^-24 * (128 + K/128) of sum |x w| bounds every element."""
     x, w = gen(M, K_ + 12, seed=6)[:, :K_], gen(N, K_, seed=7)
@@ -131,6 +130,65 @@ def test_linear_f32_sums(M, N, K_):
     grouped = torch.full((M, N), float("nan"), device=DEV)
     K().linear(grouped, xd, w3, group_offsets=offs)
     assert torch.equal(grouped[:M // 3], out[:M // 3]) and torch.equal(grouped[M // 3:], out[M // 3:] * 0.5)
+
+
+# (rows, columns, inner size, kernel as leb_gemm_f32_choice numbers them: 0 tiles of 128 x 128, 1 of 64 x 64, 2 of 32 x 32, 3 of 64 x 16,
+# 4 of 32 x 16, 5 blocks of 64 x 64 by the SM, 6 the stream), the same on GPUs of 144 to 152 SMs; inner sizes that are no
+# multiple of four have no whole 16-byte vectors
+F32_KERNELS = [(69, 10244, 252, 0), (145, 6821, 252, 0), (65, 11264, 516, 0), (288, 650, 416, 1), (1031, 300, 1028, 1),
+               (133, 767, 268, 2), (300, 300, 1028, 2), (2557, 36, 200, 3), (1757, 65, 300, 3), (33, 17, 132, 4), (138, 3, 204, 4),
+               (300, 2048, 128, 5), (523, 1500, 4, 5), (67, 65, 100, 5), (9, 1, 1084, 6), (8, 300, 60, 6), (16, 17, 2388, 6),
+               (340, 5111, 118, 0), (606, 3455, 510, 0), (9, 5311, 443, 1), (627, 305, 477, 1), (170, 643, 329, 2), (2502, 35, 283, 3),
+               (27, 5, 737, 4), (300, 771, 301, 5), (964, 2, 5, 5)]
+F32_GROUPED = [(1000, 512, 512, 1), (300, 768, 516, 2), (40, 512, 1028, 4), (64, 64, 64, 5), (300, 1023, 61, 5)]
+
+
+@pytest.mark.parametrize("M,N,K_,kind", F32_KERNELS)
+def test_linear_f32_every_kernel(M, N, K_, kind):
+    """Each kernel of the 32-bit product, where the choice takes it, with and without whole 16-byte vectors: against 64 bits
+    (the bound of the test above) and the bits of its rows alone, which another kernel computes."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert K().lib().leb_gemm_f32_choice(M, N, K_, 0, int(K_ % 4 == 0), sms) == kind
+    xd, wd = gen(M, K_, seed=6).to(DEV), gen(N, K_, seed=7).to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K().linear(out, xd, wd)
+    want = xd.double() @ wd.double().T
+    bound = 2.0 ** -24 * (min(K_, 128) + K_ / 128 + 2) * (xd.double().abs() @ wd.double().abs().T)
+    assert bool(((out.double() - want).abs() <= bound).all())
+    for m in (0, M // 2, M - 1):
+        one = torch.empty(1, N, device=DEV)
+        K().linear(one, xd[m:m + 1], wd)
+        assert torch.equal(one[0], out[m])
+    base = gen(M, N, seed=8).to(DEV)
+    b0 = base.clone()
+    K().linear(base, xd, wd, K().ACCUMULATE)
+    assert torch.equal(base, b0 + out)
+
+
+@pytest.mark.parametrize("M,N,K_,kind", F32_GROUPED)
+def test_linear_f32_every_grouped_kernel(M, N, K_, kind):
+    """... and the kernels that take products grouped by expert: unequal groups, an empty one and a single row among
+    them, the bits of the ungrouped product."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert K().lib().leb_gemm_f32_choice(M, N, K_, 4, int(K_ % 4 == 0), sms) == kind
+    xd, wd = gen(M, K_, seed=6).to(DEV), gen(N, K_, seed=7).to(DEV)
+    plain = torch.empty(M, N, device=DEV)
+    K().linear(plain, xd, wd)
+    at = [0, M // 3, M // 3, M - 1, M]
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K().linear(out, xd, torch.stack([wd, wd * 4, wd * 2, wd * 0.5]), group_offsets=torch.tensor(at, dtype=torch.int32, device=DEV))
+    for e, f in enumerate((1, 4, 2, 0.5)):
+        assert torch.equal(out[at[e]:at[e + 1]], plain[at[e]:at[e + 1]] * f)
+
+
+def test_one_f32_group_is_its_rows_alone():
+    """A single group may begin and end inside the rows: up to 8 of them, where the ungrouped product streams its weights."""
+    x, w = gen(6, 64, seed=6).to(DEV), gen(40, 64, seed=7).to(DEV)
+    out = torch.full((6, 40), -7.0, device=DEV)
+    K().linear(out, x, w[None], group_offsets=torch.tensor([2, 5], dtype=torch.int32, device=DEV))
+    whole = torch.empty(6, 40, device=DEV)
+    K().linear(whole, x, w)
+    assert torch.equal(out[2:5], whole[2:5]) and bool((out[:2] == -7).all()) and bool((out[5:] == -7).all())
 
 
 @pytest.mark.parametrize("M", [1, 5, 8, 9, 33, 64, 65, 200])
