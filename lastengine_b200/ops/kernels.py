@@ -1760,9 +1760,7 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
         return
     if scale is not None:
         raise KernelError("linear: a split norm goes with the decode products of up to SKINNY_M rows only")
-    if (not streaming and group_offsets is None and M >= PAIRS_MIN_ROWS
-            and (N >= 4096 or K >= 4096 or -(-M // 256) * -(-N // 256) >= PAIRS_MIN_TILES)
-            and linear_tc2(out, x, w, epilogue)):
+    if not streaming and group_offsets is None and pairs_take(M, N, K) and linear_tc2(out, x, w, epilogue):
         return      # many rows and a large weight matrix, or many tiles: 256 x 256 tiles on pairs of SMs
     if tc is not None and not streaming and group_offsets is None and M > SMALL_M and tc(out, x, w, epilogue):
         return
@@ -2063,10 +2061,24 @@ def linear_tc(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int
 
 
 PAIRS_MIN_ROWS = 1024   # rows from which the paired kernel is used (measured: 3-9% faster there, slower on small products)
-# ... and, for matrices of less than 4,096 either way, the tiles of 256 x 256 from which it is.  K = 2,048, a float sum: 64 tiles
-# (2,048 x 2,048) 19.9 us unpaired and 20.6 paired; 128 tiles 34.1 and 32.4; 192 tiles 49.7 and 46.4; 512 tiles 133 and 119;
-# bfloat16 results 29.3 and 29.4 at 128, 107.7 and 99.5 at 512.
+# ... and, for matrices of less than 4,096 either way, the tiles of 256 x 256 from which it is, where K is long enough or the product
+# fills PAIRS_FULL_TILES whole ones.  Both kernels in turn over 1,024 to 32,768 rows, 257 to 4,000 columns and K from 64 to 4,000, from
+# 128 tiles on: 0.94 of the unpaired one's time on average and never more than 1.02 of it.  K = 2,048, a float sum: 64 tiles
+# (2,048 x 2,048) 19.9 us unpaired and 20.6 paired; 128 tiles 34.1 and 32.4; 512 tiles 133 and 119.  Below, 128 to 160 tiles of
+# few k or of part columns are 1.03 to 1.08 times as slow paired (32,768 x 257 x 256: 30.7 and 33.2).
 PAIRS_MIN_TILES = 128
+PAIRS_MIN_K = 1024
+PAIRS_FULL_TILES = 192
+
+
+def pairs_take(M: int, N: int, K: int) -> bool:
+    """Whether a product of so many rows, columns and inner size runs on the paired kernel (if its operands suit it)."""
+    if M < PAIRS_MIN_ROWS:
+        return False
+    if N >= 4096 or K >= 4096:
+        return True
+    return (-(-M // 256) * -(-N // 256) >= PAIRS_MIN_TILES
+            and (K >= PAIRS_MIN_K or M * N >= PAIRS_FULL_TILES * 256 * 256))
 
 
 def linear_tc2(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = STORE) -> bool:

@@ -4,6 +4,16 @@ import pytest
 from lastengine_b200.ops import kernels
 
 
+def test_pairs_take_many_rows_of_large_or_long_products():
+    assert not kernels.pairs_take(1023, 8192, 8192)                        # too few rows, whatever the matrix
+    assert kernels.pairs_take(1024, 4096, 64) and kernels.pairs_take(1024, 64, 4096)
+    assert kernels.pairs_take(4096, 2048, 1024)                             # 128 tiles of a long K
+    assert not kernels.pairs_take(4096, 2048, 1016)                         # ... of a short one
+    assert not kernels.pairs_take(3840, 2048, 2048)                         # 120 tiles
+    assert kernels.pairs_take(6144, 2048, 128) and not kernels.pairs_take(6143, 2048, 128)     # 192 whole tiles, whatever K
+    assert not kernels.pairs_take(32768, 257, 256)                          # 256 tiles, half of them columns that are not there
+
+
 @pytest.mark.parametrize("sms", [132, 148])
 def test_every_kernel_of_the_32_bit_product_is_chosen_somewhere(sms):
     """... and only where it can run: the stream (6) takes up to 16 ungrouped rows of whole vectors, grouped products the

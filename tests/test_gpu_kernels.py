@@ -1176,6 +1176,24 @@ def test_linear_tc_pairs(M, N, K_):
     K().check_device_status()
 
 
+@pytest.mark.parametrize("M,N,K_", [(6144, 2040, 264), (16200, 300, 1032), (32767, 257, 1024), (16200, 300, 1016), (4000, 2056, 1032)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_linear_of_many_tiles_of_a_narrow_matrix(M, N, K_, dtype):
+    """Matrices of less than 4,096 either way on both sides of the line from which their products run on pairs of SMs, with part
+    tiles of rows, columns and k.  Sums of K_ bfloat16 products in float; a bfloat16 result is rounded once more."""
+    x, w = gen(M, K_, seed=120, dtype=torch.bfloat16).to(DEV), gen(N, K_, seed=121, scale=0.05, dtype=torch.bfloat16).to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV, dtype=dtype)
+    K().linear(out, x, w)
+    K().check_device_status()
+    want = (x.double() @ w.double().T).cpu()
+    assert err(out, want) < (2e-5 if dtype == torch.float32 else 5e-3)
+    if dtype == torch.float32:
+        base = gen(M, N, seed=122).to(DEV)
+        b0 = base.clone()
+        K().linear(base, x, w, K().ACCUMULATE)
+        assert err(base, b0.cpu().double() + want) < 2e-5
+
+
 @pytest.mark.parametrize("M,N,K_", [(17, 2048, 2048), (64, 352, 128), (100, 6144, 64), (33, 11264, 192), (128, 100, 200),
                                     (1, 128, 64), (16, 48, 72), (48, 2048, 5632), (64, 65536, 256),
                                     (65, 2048, 2048), (96, 352, 5632), (90, 100, 200), (97, 6144, 136),
