@@ -1356,12 +1356,16 @@ def latent_attention_splits(batch, H: int, mma: bool = False, rank: int = 0, win
     reads up to 1,024 (a step of three such layers at batch 8: 0.377 -> 0.367 ms in a window of 1,024, 0.247 ->
     0.236 ms in one of 512).  A window seldom starts on a tile's border: it reaches into one tile more, which
     gets a piece of its own instead of doubling the length of every piece.  `few`: the kernel of 16 query vectors runs,
-    whose tiles are 64 rows: a piece is one of them."""
+    whose tiles are 64 rows: a piece is one of them.  Two tiles are not cut apart from 128 query vectors on: what the pieces
+    leave and the merge reads again costs more than the second tile (16 heads of 512 + 64, 65 to 128 rows: 8 sequences 11.9 us
+    in two pieces and 11.7 in one, 64 sequences 21.3 and 11.9)."""
     if batch.max_qlen != 1:
         return 1
     blocks = batch.n_seqs * -(-H // (64 if mma else 8))
     want = max(1, ((1 if mma else 2) * sm_count()) // max(1, blocks))
     n = _read_length(batch.max_kvlen, window, chunk)
+    if few and n <= 128 and batch.n_seqs * H >= 128:
+        return 1
     piece = 64 if few or (n <= 1024 and n < batch.max_kvlen) else 128
     spare = 63 if n < batch.max_kvlen else 0
     return int(max(1, min(want, -(-(n + spare) // piece), 64)))

@@ -1,4 +1,6 @@
 """Which kernel a call takes, where that depends on sizes alone (no GPU)."""
+from types import SimpleNamespace
+
 import pytest
 
 from lastengine_b200.ops import kernels
@@ -12,6 +14,17 @@ def test_pairs_take_many_rows_of_large_or_long_products():
     assert not kernels.pairs_take(3840, 2048, 2048)                         # 120 tiles
     assert kernels.pairs_take(6144, 2048, 128) and not kernels.pairs_take(6143, 2048, 128)     # 192 whole tiles, whatever K
     assert not kernels.pairs_take(32768, 257, 256)                          # 256 tiles, half of them columns that are not there
+
+
+@pytest.mark.parametrize("heads,seqs,length,pieces", [(16, 8, 64, 1), (16, 8, 65, 1), (16, 64, 128, 1), (16, 7, 128, 2), (8, 16, 100, 1),
+                                                      (16, 8, 129, 3), (16, 64, 129, 2), (16, 1, 4096, 64), (16, 256, 4096, 1)])
+def test_pieces_of_the_latent_decode_kernel_of_few_heads(monkeypatch, heads, seqs, length, pieces):
+    """A piece is a tile of 64 rows as long as the blocks fit the SMs; two tiles stay together from 128 query vectors on."""
+    monkeypatch.setattr(kernels, "sm_count", lambda: 148)
+    step = SimpleNamespace(max_qlen=1, n_seqs=seqs, max_kvlen=length)
+    assert kernels.latent_attention_splits(step, heads, True, 512, few=True) == pieces
+    step.max_qlen = 2
+    assert kernels.latent_attention_splits(step, heads, True, 512, few=True) == 1
 
 
 @pytest.mark.parametrize("sms", [132, 148])
