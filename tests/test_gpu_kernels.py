@@ -769,6 +769,33 @@ def test_attention_prompt_and_decode(dtype, nh, nkv, hd, window):
         assert err(out.view(n, nh, hd), want) < tol, (q0, n, splits)
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (3, 1, 20), (16, 2, 128)])
+@pytest.mark.parametrize("window", [0, 40])
+def test_general_attention_loads_16_bytes_or_single_numbers(nh, nkv, hd, window):
+    """32-bit caches on 16-byte addresses (four numbers a load) and off them (single numbers): the same bits, for a prompt, a
+    continued one and a step of one row whole and in splits; unused places of the pages hold NaN."""
+    page, Tk, pages = 64, 150, [3, 0, 5]
+    k, v = gen(Tk, nkv, hd, seed=40), gen(Tk, nkv, hd, seed=41)
+    kp, vp = fill_cache(k, v, pages, nkv, hd, page, torch.float32)
+
+    def off(t):
+        b = torch.empty(t.numel() + 1, device=DEV)
+        b[1:] = t.reshape(-1)
+        return b[1:].view(t.shape)
+
+    assert kp.data_ptr() % 16 == 0 and off(kp).data_ptr() % 16 == 4
+    for q0, n, splits in ((0, 150, 1), (100, 37, 1), (149, 1, 1), (149, 1, 4)):
+        q = gen(n, nh * hd, seed=42 + n).to(DEV)
+        batch = builder().build([0], [[0] * n], [q0], [], {0: np.array([pages], dtype=np.int32)})
+        got = []
+        for a, b in ((kp, vp), (off(kp), off(vp)), (kp, off(vp))):
+            out = torch.full((n, nh * hd), float("nan"), device=DEV)
+            scratch = torch.empty(n * nh * splits * (hd + 2), device=DEV) if splits > 1 else None
+            K().attention(out, q, a, b, batch.tables[0], batch, nh, nkv, hd, page, window, hd ** -0.5, n_splits=splits, scratch=scratch)
+            got.append(out)
+        assert bool(got[0].isfinite().all()) and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("dtype,nh,nkv,hd", [(torch.float32, 4, 4, 64), (torch.float32, 8, 2, 64), (torch.float32, 3, 1, 48),
                                              (torch.bfloat16, 4, 4, 48)])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
