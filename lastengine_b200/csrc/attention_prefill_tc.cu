@@ -7,19 +7,20 @@
 //
 //   S[128, 64]  = Q[128, 64] . K_page[64, 64]^T        tcgen05.mma, both operands in shared memory
 //   P           = exp2(S * scale * log2 e - m)          128 threads, one row each, S read from
-//                                                       tensor memory, P written back there (bf16)
-//   O[128, 64] += P[128, 64] . V_page[64, 64]           tcgen05.mma, P from tensor memory, V from
-//                                                       shared memory
+//                                                       tensor memory, P to shared memory (bf16; as
+//                                                       two terms back to tensor memory)
+//   O[128, 64] += P[128, 64] . V_page[64, 64]           tcgen05.mma, V from shared memory
 //
 // Q, the key page [position][dim] and the value page [dim][position] (the cache stores values
 // transposed) are all K-major tiles with rows of 128 bytes, which TMA brings in under the
 // 128-byte swizzle straight from the paged cache: no gather, no transposition.
 //
 // Roles: warps 0-3 softmax (thread r owns row r of S, P and O), warp 4 TMA producer, warp 5 issues
-// the MMAs.  What bounds it is the special function unit: 64 exponentials a row and page are 512 cycles of a
-// scheduler's share, more than the products (320) or the other instructions of the row.  The unit stays busy where
-// enough rows are in their exponentials, so three blocks share an SM (112 registers a thread, 128 columns of
-// tensor memory, 64 KB of shared memory), and a row's chain is kept short: a row of S is taken into registers
+// the MMAs.  The largest share of a page is the special function unit's: 64 exponentials a row are 512 cycles of a
+// scheduler's share, more than the products (320) or the other instructions of the row.  No pipe is full (8,192 rows: that
+// unit 55% of its rate, the tensor cores 47%, issue slots 49%): what is left is the latency of a row's chain from scores to
+// weights, which other rows' work has to cover.  So three blocks share an SM (96 registers a thread, 128 columns of
+// tensor memory, 64 KB of shared memory), and the chain is kept short: a row of S is taken into registers
 // whole, whereupon the next page's scores are issued into the same columns, and P goes to the second product
 // through shared memory (swizzled as the TMA tiles are); the thread that issues the products takes what they need from
 // uniform registers.  Per layer of 32 heads over 8: 16,384 rows 2.13 -> 1.75 ms (629 TFLOP/s), 8,192 0.54 -> 0.49,
@@ -225,8 +226,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // Barriers and tensor memory are set up (a block of the next kernel, let in from here on, cannot take the columns
-  // this one still waits for); now q and the cache must be complete.
+  // Barriers and tensor memory are set up; now q and the cache must be complete.  (The next kernel is let in when this one ends.
+  // From here on it could be, its blocks no longer being able to take columns that one here waits for, but with a
+  // rotation before and a product behind it that measured 0.94 to 1.0 of the time at up to 100 rows and 1.0 to 1.03 from 1,024 on.)
   pdl_wait();
   const uint32_t tmem = tmem_slot;
   // O | S (WIDE: S0 S1) in columns; WIDE has P over the S it came from

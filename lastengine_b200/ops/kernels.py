@@ -1420,7 +1420,8 @@ def attention_splits(batch, nkv: int, G: int, sm_count: int | None = None, hd: i
     sequences of 640 positions: 20.3 us unsplit, 27.4 us in 4 splits; of 4,096 positions: 110 us
     unsplit, 89 us in 4 splits).  The general kernel (`general`: 32-bit caches) takes several times as long over a
     position as the tensor-core kernel: beyond 128 positions half as many of them make a split worth its start (two sequences
-    of 190 and 333: 87 -> 25 us a layer with the wider loads of its tiles).
+    of 190 and 333: 87 -> 25 us a layer with the wider loads of its tiles; 1 to 64 sequences of 100 to 8,000 positions, seven
+    layouts of heads: 0.18 to 0.83 of the time before both).
     """
     if batch.max_qlen != 1:
         return 1
