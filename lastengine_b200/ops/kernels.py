@@ -1364,10 +1364,10 @@ def latent_attention_splits(batch, H: int, mma: bool = False, rank: int = 0, win
     blocks = batch.n_seqs * -(-H // (64 if mma else 8))
     want = max(1, ((1 if mma else 2) * sm_count()) // max(1, blocks))
     n = _read_length(batch.max_kvlen, window, chunk)
-    if few and n <= 128 and batch.n_seqs * H >= 128:
-        return 1
     piece = 64 if few or (n <= 1024 and n < batch.max_kvlen) else 128
     spare = 63 if n < batch.max_kvlen else 0
+    if few and n + spare <= 128 and batch.n_seqs * H >= 128:
+        return 1
     return int(max(1, min(want, -(-(n + spare) // piece), 64)))
 
 

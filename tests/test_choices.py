@@ -23,6 +23,9 @@ def test_pieces_of_the_latent_decode_kernel_of_few_heads(monkeypatch, heads, seq
     monkeypatch.setattr(kernels, "sm_count", lambda: 148)
     step = SimpleNamespace(max_qlen=1, n_seqs=seqs, max_kvlen=length)
     assert kernels.latent_attention_splits(step, heads, True, 512, few=True) == pieces
+    # a window of 128 reaches into a third tile, one of 65 into no more than two
+    assert kernels.latent_attention_splits(SimpleNamespace(max_qlen=1, n_seqs=8, max_kvlen=4096), 16, True, 512, window=128, few=True) == 3
+    assert kernels.latent_attention_splits(SimpleNamespace(max_qlen=1, n_seqs=8, max_kvlen=4096), 16, True, 512, window=65, few=True) == 1
     step.max_qlen = 2
     assert kernels.latent_attention_splits(step, heads, True, 512, few=True) == 1
 
