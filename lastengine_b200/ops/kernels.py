@@ -1027,7 +1027,8 @@ def retention(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     """Decayed linear attention of the step's rows with the per-sequence state [slots, H, d, e] (float):
     q and k rotated on their first `rot` dimensions, k scaled, S = decay S + k v^T, o = S^T q,
     o divided by its root mean square per head and multiplied by silu(g).  q, k [M, H*d] and v, g
-    [M, H*e] are column slices of one projection."""
+    [M, H*e] are column slices of one projection.  (The state and the step's tables may be fetched ahead of the wait for the
+    kernel launched before: between two calls on one state lies a copy or a graph's launch, as BatchBuilder's steps have it.)"""
     _cuda(out, "retention.out")
     M = out.shape[0]
     assert out.shape == (M, H * e)
@@ -1164,6 +1165,8 @@ def qk_rope_store(q_out: torch.Tensor, q_in: torch.Tensor, k_in: torch.Tensor | 
     width of a head in q_in/k_in and in v_in where heads are stored wider than they are (hd in q_out
     and the key pool, vd in the value pool; the rest of a stored head is zeros, the norms run over the
     head as it comes).  `temperature` = (coef, every): q at position p times 1 + coef ln(floor((p + 1) / every) + 1).
+    (The step's tables may be read ahead of the wait for the kernel launched before: a copy or a graph's launch lies
+    between what writes them and the step, as BatchBuilder's steps have it.)
     """
     vd = hd if vd is None else int(vd)
     hd_in = hd if hd_in is None else int(hd_in)
