@@ -7,8 +7,7 @@
 //
 //   S[128, 64]  = Q[128, 64] . K_page[64, 64]^T        tcgen05.mma, both operands in shared memory
 //   P           = exp2(S * scale * log2 e - m)          128 threads, one row each, S read from
-//                                                       tensor memory, P to shared memory (bf16; as
-//                                                       two terms back to tensor memory)
+//                                                       tensor memory, P to shared memory or back (bf16)
 //   O[128, 64] += P[128, 64] . V_page[64, 64]           tcgen05.mma, V from shared memory
 //
 // Q, the key page [position][dim] and the value page [dim][position] (the cache stores values
@@ -27,8 +26,8 @@
 // 2,048 55.7 -> 52 us, against two blocks per SM with two buffers of S and P in tensor memory.  Measured beside it:
 // four blocks of 80 registers that read S in halves 0.50 ms at 8,192 rows; P over S in tensor memory 0.53 (three
 // blocks) and 0.67 (four, with spills); weights against the maximum so far before this page's is known: no change.
-// Weights as two bfloat16 terms (WIDE) go back to tensor memory over the scores they came from; those kernels run two
-// blocks per SM with two buffers of S.
+// Weights as two bfloat16 terms (WIDE) go back to tensor memory over the scores they came from; those kernels, and the one for
+// steps of few tiles (`atc_few_tiles`), run two blocks per SM with two buffers of S and P over the S it came from.
 // The running maximum is only moved when it grew by more than 8 (a factor 256): exponentials stay
 // bounded, the row sum uses the same reference, and the quotient at the end is exact; moving it
 // means rescaling O in tensor memory, which then happens a few times per row instead of once
@@ -43,12 +42,12 @@
 #include "tc_common.cuh"
 
 #define ATC_THREADS 192
-template <bool WIDE>
+template <bool DEEP>
 struct AtcShape {
-  static constexpr int BLOCKS = WIDE ? 2 : 3;        // per SM
-  static constexpr int STAGES = WIDE ? 4 : 2;        // pages of keys and values on their way
-  static constexpr int S_BUFS = WIDE ? 2 : 1;
-  static constexpr int COLUMNS = WIDE ? 256 : 128;   // of tensor memory
+  static constexpr int BLOCKS = DEEP ? 2 : 3;        // per SM
+  static constexpr int STAGES = DEEP ? 4 : 2;        // pages of keys and values on their way
+  static constexpr int S_BUFS = DEEP ? 2 : 1;
+  static constexpr int COLUMNS = DEEP ? 256 : 128;   // of tensor memory
 };
 #define ATC_NEG (-1e30f)
 
@@ -145,8 +144,9 @@ __device__ __forceinline__ int atc_blocks_seen(int qpos, int window, int pool) {
 
 // WIDE: the weights as two terms as POOLED has them, for layers without pooled blocks too.
 // GS query heads per kv head (1, 2, 4, 8): a tile is GS heads x 128/GS positions; VD: width of a value head (64 or 32)
-template <int GS, bool POOLED, bool WIDE, int VD>
-__global__ void __launch_bounds__(ATC_THREADS, AtcShape<WIDE>::BLOCKS)
+// DEEP: two blocks per SM, two buffers of S, P over the S it came from (WIDE always).
+template <int GS, bool POOLED, bool WIDE, bool DEEP, int VD>
+__global__ void __launch_bounds__(ATC_THREADS, AtcShape<DEEP>::BLOCKS)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_pk,
                             const __grid_constant__ CUtensorMap map_pv, bf16* __restrict__ out,
@@ -157,14 +157,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int nh, int nkv, int window, int chunk, int pool, float scale, const float* __restrict__ head_scale,
                             const float* __restrict__ freq_v, const float* __restrict__ slopes,
                             const float* __restrict__ sinks, int* __restrict__ status) {
-  constexpr int HD = 64, PAGE = 64, TP = 128 / GS, NS = AtcShape<WIDE>::STAGES, SB = AtcShape<WIDE>::S_BUFS;
+  constexpr int HD = 64, PAGE = 64, TP = 128 / GS, NS = AtcShape<DEEP>::STAGES, SB = AtcShape<DEEP>::S_BUFS;
   constexpr int Q_BYTES = 128 * HD * 2, KV_BYTES = PAGE * HD * 2, V_BYTES = VD * PAGE * 2;
   extern __shared__ uint8_t atc_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)atc_raw + 1023) & ~(uintptr_t)1023);   // swizzled tiles want 1024
   uint8_t* sq = smem;
   uint8_t* sk = sq + Q_BYTES;
   uint8_t* sv = sk + NS * KV_BYTES;
-  uint8_t* sp = sv + NS * V_BYTES;                 // P (not WIDE)
+  static_assert(DEEP || !WIDE, "weights of two terms go back over the scores");
+  uint8_t* sp = sv + NS * V_BYTES;                 // P (not DEEP)
   __shared__ uint64_t q_full, k_full[NS], v_full[NS], k_empty[NS], v_empty[NS], s_full[SB], s_free, p_full[SB], pv_done[SB];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_s;
@@ -220,7 +221,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 4) {
-    tmem_alloc(&tmem_slot, AtcShape<WIDE>::COLUMNS);
+    tmem_alloc(&tmem_slot, AtcShape<DEEP>::COLUMNS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -231,7 +232,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   // rotation before and a product behind it that measured 0.94 to 1.0 of the time at up to 100 rows and 1.0 to 1.03 from 1,024 on.)
   pdl_wait();
   const uint32_t tmem = tmem_slot;
-  // O | S (WIDE: S0 S1) in columns; WIDE has P over the S it came from
+  // O | S (DEEP: S0 S1) in columns; DEEP has P over the S it came from
   const uint32_t t_o = tmem, t_s0 = tmem + 64;
   // instruction descriptor: float accumulate, bfloat16 operands, both K-major, N = 64, M = 128
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
@@ -297,12 +298,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       tc_fence_after();
       if (elect_lane()) {
         const uint64_t va = v_desc + s * (V_BYTES / 16);
-        if (WIDE) {
-          const uint32_t t_p = tm + 64 + 64 * (i & 1);   // hi in the scores' first 32 columns, lo in the next 32
+        if (DEEP) {
+          const uint32_t t_p = tm + 64 + 64 * (i & 1);   // the scores' first 32 columns (WIDE: hi there, lo in the next 32)
 #pragma unroll
           for (int kk = 0; kk < PAGE / 16; kk++) umma_bf16_ts(tm, t_p + kk * 8, va + kk * 2, IDESC_PV, (i > 0 || kk > 0));
 #pragma unroll
-          for (int kk = 0; kk < PAGE / 16; kk++) umma_bf16_ts(tm, t_p + 32 + kk * 8, va + kk * 2, IDESC_PV, 1);
+          for (int kk = 0; kk < (WIDE ? PAGE / 16 : 0); kk++) umma_bf16_ts(tm, t_p + 32 + kk * 8, va + kk * 2, IDESC_PV, 1);
         } else {
 #pragma unroll
           for (int kk = 0; kk < PAGE / 16; kk++) umma_bf16(tm, p_desc + kk * 2, va + kk * 2, IDESC_PV, (i > 0 || kk > 0));
@@ -387,9 +388,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         l *= f;
         if (move) m_used = m_new;
       }
-      // P of the pages before (WIDE: of page i-2, which lay where this one goes) has been read
+      // P of the pages before (DEEP: of page i-2, which lay where this one goes) has been read
       if (i >= SB && !mbar_wait(&pv_done[bsel], ((i - SB) / SB) & 1, abort_flag)) { atomicExch(status, 18); ok = false; break; }
-      uint32_t pk[WIDE ? 32 : 4], pl[WIDE ? 32 : 1];
+      uint32_t pk[DEEP ? 32 : 4], pl[WIDE ? 32 : 1];
       const float m_ref = m_used > 0.5f * ATC_NEG ? m_used : 0.f;
       const uint64_t scale_pair = f2(scale_after, scale_after), ref_pair = f2(-m_ref, -m_ref);
       uint64_t ps[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
@@ -400,18 +401,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const float p0 = ex2(x.x), p1 = ex2(x.y);
         ps[(c >> 1) & 1] = add_f2(ps[(c >> 1) & 1], f2(p0, p1));
         __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-        pk[(c >> 1) & (WIDE ? 31 : 3)] = *reinterpret_cast<uint32_t*>(&pp);
+        pk[(c >> 1) & (DEEP ? 31 : 3)] = *reinterpret_cast<uint32_t*>(&pp);
         if (WIDE) {
           __nv_bfloat162 pr = __floats2bfloat162_rn(p0 - __bfloat162float(pp.x), p1 - __bfloat162float(pp.y));
           pl[WIDE ? c >> 1 : 0] = *reinterpret_cast<uint32_t*>(&pr);
-        } else if ((c & 7) == 6) {      // eight weights: a 16-byte piece of the row
+        }
+        if (!DEEP && (c & 7) == 6) {      // eight weights: a 16-byte piece of the row
           *reinterpret_cast<uint4*>(sp + r * 128 + (((c >> 3) ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
       }
-      if (WIDE) {
+      if (DEEP) {
         tc_fence_after();
         tmem_st32(t_s, pk);
-        tmem_st32(t_s + 32, pl);
+        if (WIDE) tmem_st32(t_s + 32, pl);
         tmem_st_wait();
       }
       const float2 sums = halves(add_f2(ps[0], ps[1]));
@@ -428,9 +430,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             for (int e = max(0, n_valid - cc * 8); e < 8; e++) piece[e] = __float2bfloat16_rn(0.f);
           }
         }
-        if (WIDE) fence_proxy_async_smem();
+        if (DEEP) fence_proxy_async_smem();
       }
-      if (!WIDE) fence_proxy_async_smem();      // P (and the zeros) before the product reads them
+      if (!DEEP) fence_proxy_async_smem();      // P (and the zeros) before the product reads them
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[bsel]);   // one arrival per softmax warp
@@ -443,7 +445,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       float inv = l > 0.f ? 1.0f / l : 0.f;
       if (!POOLED && sinks) inv = sink_quotient(m_used * 0.6931471805599453f, l, sinks[h0 + g]);
       if (gate && !gate_elem && row_valid) inv *= head_gate(gate, m_base + pi, gate_stride, h0 + g, 0, VD, 0);
-      constexpr int OW = WIDE ? VD : 32;      // numbers of the row at a time
+      constexpr int OW = DEEP ? VD : 32;      // numbers of the row at a time
 #pragma unroll
       for (int d0 = 0; d0 < VD; d0 += OW) {
         __syncwarp();      // rows beyond the sequence left the branch below early: the loads take the whole warp
@@ -501,7 +503,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) tmem_dealloc(tmem, AtcShape<WIDE>::COLUMNS);
+  if (warp == 4) tmem_dealloc(tmem, AtcShape<DEEP>::COLUMNS);
 }
 
 LEB_API int leb_attention_prefill_tc_supported(int nh, int nkv, int hd, int page_size) {
@@ -510,7 +512,18 @@ LEB_API int leb_attention_prefill_tc_supported(int nh, int nkv, int hd, int page
   return G == 1 || G == 2 || G == 4 || G == 8;
 }
 
-template <bool POOLED, bool WIDE, int VD>
+// Whether a step has so few tiles that a tile's own chain of pages takes the time, not the SMs' pipes: up to 2.5 an SM.  Two blocks per
+// SM with two buffers of S are then ahead of three with one.  us of the form before both, of three blocks, of two; 148 SMs:
+// 124 tiles 12.4, 14.8, 11.0; 192 36.6, 38.1, 30.7; 336 24.1, 26.8, 20.5; 392 17.2, 14.8, 15.3; 420 20.4, 16.3, 18.0; 1,304 56.9, 46.7,
+// 50.6; 2,424 148, 116, 129; below 100 tiles 0.95 of either.  The same bits from both.
+static bool atc_few_tiles(int M, int B, int nh, int nkv, int max_qlen) {
+  if (nkv <= 0 || nh < nkv || nh / nkv > 128) return false;      // (refused below)
+  const int TP = 128 / (nh / nkv);
+  const long long per_head = (long long)ceil_div(max_qlen, TP) * B, by_rows = (long long)M / TP + B;
+  return (per_head < by_rows ? per_head : by_rows) * nkv * 2 <= 5ll * sm_count();
+}
+
+template <bool POOLED, bool WIDE, bool DEEP, int VD>
 static int launch_attention_prefill_tc(const char* who, void* out, const void* q, int q_stride, int M, const void* k_pool,
                                        const void* v_pool, int n_pages, const int* block_table, int bt_width,
                                        const void* pk_pool, const void* pv_pool, int n_pooled_pages, const int* pool_table,
@@ -542,16 +555,16 @@ static int launch_attention_prefill_tc(const char* who, void* out, const void* q
   }
   dim3 grid(nkv, ceil_div(max_qlen, TP), B);
   LEB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "%s: grid too large", who);
-  const size_t smem = 1024 + 128 * 64 * 2 + AtcShape<WIDE>::STAGES * (64 + VD) * 64 * 2 + (WIDE ? 0 : 128 * 64 * 2);
+  const size_t smem = 1024 + 128 * 64 * 2 + AtcShape<DEEP>::STAGES * (64 + VD) * 64 * 2 + (DEEP ? 0 : 128 * 64 * 2);
 #define LEB_ATC(GS_)                                                                                              \
   {                                                                                                               \
     static bool set = false;                                                                                      \
     if (!set) {                                                                                                   \
-      if (cudaFuncSetAttribute(attention_prefill_tc_kernel<GS_, POOLED, WIDE, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
+      if (cudaFuncSetAttribute(attention_prefill_tc_kernel<GS_, POOLED, WIDE, DEEP, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
         return leb_fail("%s: %zu bytes of shared memory per block refused", who, smem);                         \
       set = true;                                                                                                 \
     }                                                                                                             \
-    leb_launch(attention_prefill_tc_kernel<GS_, POOLED, WIDE, VD>, grid, dim3(ATC_THREADS), smem, st,                       \
+    leb_launch(attention_prefill_tc_kernel<GS_, POOLED, WIDE, DEEP, VD>, grid, dim3(ATC_THREADS), smem, st,                       \
         mq, mk, mv, mpk, mpv, (bf16*)out, block_table, bt_width, pool_table, pt_width, seq_slot, seq_pos0, seq_qstart, \
         seq_qlen, (const bf16*)gate, gate_stride, gate_elem, nh, nkv, window, chunk, pooled ? pool : 0, scale, head_scale, freq_v, slopes, \
         sinks, status); \
@@ -581,7 +594,9 @@ LEB_API int leb_attention_prefill_tc(void* out, const void* q, int q_stride, int
 #define LEB_ATC_ARGS "leb_attention_prefill_tc", out, q, q_stride, M, k_pool, v_pool, n_pages, block_table, bt_width, nullptr, \
                      nullptr, 0, nullptr, 0, seq_slot, seq_pos0, seq_qstart, seq_qlen, gate, gate_stride, gate_elem, B, nh, nkv, \
                      hd, page_size, window, chunk, 0, scale, nullptr, nullptr, slopes, sinks, max_qlen, status, st
-  return wide ? launch_attention_prefill_tc<false, true, 64>(LEB_ATC_ARGS) : launch_attention_prefill_tc<false, false, 64>(LEB_ATC_ARGS);
+  if (wide) return launch_attention_prefill_tc<false, true, true, 64>(LEB_ATC_ARGS);
+  return atc_few_tiles(M, B, nh, nkv, max_qlen) ? launch_attention_prefill_tc<false, false, true, 64>(LEB_ATC_ARGS)
+                                                : launch_attention_prefill_tc<false, false, false, 64>(LEB_ATC_ARGS);
 #undef LEB_ATC_ARGS
 }
 
@@ -600,7 +615,7 @@ LEB_API int leb_attention_pooled_tc(void* out, const void* q, int q_stride, int 
 #define LEB_APT_ARGS "leb_attention_pooled_tc", out, q, q_stride, M, k_pool, v_pool, n_pages, block_table, bt_width, pk_pool, \
                      pv_pool, n_pooled_pages, pool_table, pt_width, seq_slot, seq_pos0, seq_qstart, seq_qlen, nullptr, 0, 0, B, nh, \
                      nkv, hd, page_size, window, 0, pool, 1.0f, head_scale, freq_v, nullptr, nullptr, max_qlen, status, st
-  const int rc = vd == 64 ? launch_attention_prefill_tc<true, true, 64>(LEB_APT_ARGS) : launch_attention_prefill_tc<true, true, 32>(LEB_APT_ARGS);
+  const int rc = vd == 64 ? launch_attention_prefill_tc<true, true, true, 64>(LEB_APT_ARGS) : launch_attention_prefill_tc<true, true, true, 32>(LEB_APT_ARGS);
 #undef LEB_APT_ARGS
   return rc;
 }

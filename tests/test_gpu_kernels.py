@@ -900,6 +900,29 @@ def test_attention_long_prompts_on_tcgen05(nh, nkv, window):
         assert err(out[650].view(nh, hd)[0], vs[0][far, 0].double()) < 1e-2     # the far key's value, alone
 
 
+@pytest.mark.parametrize("nh,nkv,window", [(8, 8, 0), (16, 8, 0), (32, 8, 0), (32, 8, 100), (64, 8, 0)])
+def test_prompt_attention_of_few_tiles_gives_the_bits_of_many(nh, nkv, window):
+    """Steps of few tiles run two blocks an SM with two buffers of scores, others three with one: a prompt alone and among others."""
+    hd, page, n, width, B = 64, 64, 333, 6, 40
+    table = np.random.default_rng(12).permutation(B * width).astype(np.int32).reshape(B, width)
+    pk, pv = (gen(B * width, nkv, page, hd, seed=s, dtype=torch.bfloat16).to(DEV) for s in (395, 396))
+    q = gen(B * n, nh * hd, seed=397, dtype=torch.bfloat16).to(DEV)
+    # beyond 2.5 tiles an SM for sure (40 prompts), and for sure not (one): 333 rows are 3 tiles of 128 and more, times 8 heads
+    assert B * 3 * nkv > 2.5 * 160 and -(-n * (nh // nkv) // 128) * nkv <= 2.5 * 132
+
+    def run(seqs):
+        batch = builder().build(list(range(len(seqs))), [[0] * n] * len(seqs), [0] * len(seqs), [], {0: table[seqs]})
+        out = torch.empty(len(seqs) * n, nh * hd, device=DEV, dtype=torch.bfloat16)
+        rows = torch.cat([q[i * n:(i + 1) * n] for i in seqs])
+        K().attention(out, rows, pk, pv, batch.tables[0], batch, nh, nkv, hd, page, window, 0.125)
+        K().check_device_status()
+        return out
+
+    many = run(list(range(B)))
+    for i in (0, 17, 39):
+        assert torch.equal(run([i]), many[i * n:(i + 1) * n])
+
+
 @pytest.mark.parametrize("nh,nkv", [(4, 4), (4, 2), (8, 2), (8, 1)])
 @pytest.mark.parametrize("gate", ["none", "head", "number", "number, unaligned"])
 @pytest.mark.parametrize("wide", [False, True])
