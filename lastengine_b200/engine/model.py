@@ -104,6 +104,10 @@ class Model:
     def forward(self, batch, cache) -> torch.Tensor:
         """Runs the step's rows through every scheduled layer; returns float logits
         [batch.n_logit_rows, vocab] (a view of workspace memory, valid until the next step)."""
+        with kernels.product_chain(self.env.workspace, batch.n_rows, self.env.dtype):
+            return self._forward(batch, cache)
+
+    def _forward(self, batch, cache) -> torch.Tensor:
         env, ws = self.env, self.env.workspace
         M, D = batch.n_rows, self.hidden_size
         x = ws.get("model.x", (M, D), torch.float32)

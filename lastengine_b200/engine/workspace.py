@@ -18,6 +18,7 @@ class Workspace:
         self.device = device
         self._bufs: dict[str, torch.Tensor] = {}
         self._views: dict[tuple, torch.Tensor] = {}    # (name, shape, dtype) -> the view handed out last time
+        self._words: dict[str, torch.Tensor] = {}
         self.generation = 0
         self.frozen = False
 
@@ -46,6 +47,15 @@ class Workspace:
         view = buf[:n * esize].view(dtype).view(*shape)
         self._views[key] = view
         return view
+
+    def zeroed(self, name: str, n: int) -> torch.Tensor:
+        """n int32 words, 0 when they are made: never moved, never handed out under another shape."""
+        buf = self._words.get(name)
+        if buf is None:
+            if self.frozen:
+                raise RuntimeError(f"workspace '{name}' would be made while a graph is captured")
+            buf = self._words[name] = torch.zeros(n, dtype=torch.int32, device=self.device)
+        return buf
 
     def nbytes(self) -> int:
         return sum(b.numel() for b in self._bufs.values())

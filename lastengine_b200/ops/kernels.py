@@ -7,8 +7,10 @@ the built library, or with tensors that are not on a CUDA device, raises.
 from __future__ import annotations
 
 import collections
+import contextlib
 import ctypes
 import functools
+import threading
 from ctypes import c_float, c_int, c_size_t, c_void_p
 
 import torch
@@ -23,11 +25,84 @@ _timer = None      # a KernelTimer while one is active
 
 
 def lib():
+    """The library, for a call that may launch: products that wait in this thread's chain are launched first."""
+    if _chain.ops:
+        _chain.flush()
+    return _library()
+
+
+def _library():
     global _lib
     if _lib is None:
         _lib = _build.load()
         _declare(_lib)
     return _lib if _timer is None else _timer.proxy
+
+
+class _Chain(threading.local):
+    """The products of a step that wait to be launched as one kernel (`product_chain`); one per thread."""
+
+    def __init__(self):
+        self.open = False
+        self.ops = []        # per product the call that launches it alone
+        self.sync = None     # the grid barrier's words
+        self.rows = 0
+        self.device = None
+
+    def flush(self) -> None:
+        """Launches what waits: CHAIN_MIN products or more as one kernel, fewer as they would be without a chain."""
+        ops, self.ops = self.ops, []
+        L = _library()
+        if len(ops) < CHAIN_MIN:
+            L.leb_chain_drop()
+            for alone in ops:
+                alone()
+            return
+        _check(L.leb_chain_run(_ptr(self.sync), _ptr(_status_word(self.device)), _stream()))
+
+
+_chain = _Chain()
+
+
+@contextlib.contextmanager
+def product_chain(workspace, rows: int, dtype: torch.dtype):
+    """Inside, consecutive products of a step of SMALL_M + 1 to SKINNY_M bfloat16 rows (dense ones, the conv mixer's decode step among them)
+    wait for one another in the host's memory and run as ONE resident kernel (csrc/product_chain.cu) as soon as
+    anything else is launched through this module, and at the end.  Nothing but calls of this module may launch work that
+    touches the products' operands in between, as is so inside a model's forward pass.  `workspace` owns the barrier's words:
+    steps that share it run one after the other."""
+    c = _chain
+    if dtype != torch.bfloat16 or not SMALL_M < rows <= SKINNY_M or c.open or _library().leb_chain_clusters(rows) <= 0:
+        yield
+        return
+    c.sync = workspace.zeroed("chain.sync", 2)
+    c.device = workspace.device
+    c.rows, c.open = rows, True
+    try:
+        yield
+        if c.ops:
+            c.flush()
+    finally:
+        c.open = False
+        if c.ops:            # the step raised: what waited is not run
+            c.ops = []
+            _library().leb_chain_drop()
+
+
+def _chained(out, x, w, M, N, K, epilogue, scale_args, emit_args, alone, conv=(None, None, None, None, None, 0)) -> bool:
+    """Adds a product to this thread's chain; False where it is not one the chain takes."""
+    c = _chain
+    if M != c.rows or N >= SKINNY_MAX_N or not w.is_contiguous() or x.data_ptr() % 16 != 0 or w.data_ptr() % 16 != 0:
+        return False
+    if (epilogue >> 8) >= PLAIN_ACT_BASE and (epilogue & 255) == STORE and out.dtype != torch.bfloat16:
+        return False
+    L = _library()
+    if len(c.ops) >= L.leb_chain_max_ops():
+        c.flush()
+    _check(L.leb_chain_add(_ptr(out), _dt(out, "linear.out"), _ptr(x), _ptr(w), M, N, K, x.stride(0), out.stride(0), epilogue,
+                           *scale_args, *emit_args, *conv))
+    c.ops.append(alone)
+    return True
 
 
 class KernelTimer:
@@ -125,6 +200,11 @@ def _declare(L) -> None:
         "leb_gemm_bf16_small": [P, I, P, P, I, I, I, I, I, I, P, I, S, I, P],
         "leb_gemm_bf16_stream": [P, I, P, P, I, I, I, I, I, I, P, I, I, F, P, P, P, P],
         "leb_gemm_bf16_stream_grouped": [P, I, P, P, I, I, I, I, I, I, P, I, S, P],
+        "leb_chain_max_ops": [],
+        "leb_chain_clusters": [I],
+        "leb_chain_drop": [],
+        "leb_chain_add": [P, I, P, P, I, I, I, I, I, I, P, I, I, F, P, P, P, P, P, P, P, P, I],
+        "leb_chain_run": [P, P, P],
         "leb_gemm_bf16_stream_conv": [P, P, P, I, I, I, I, I, P, P, P, P, P, I, P, I, I, F, P],
         "leb_gemm_bf16_tc_grouped": [P, I, P, P, I, I, I, I, I, I, P, I, P, P],
         "leb_gemm_bf16_tc2": [P, I, P, P, I, I, I, I, I, I, P, P],
@@ -1103,7 +1183,7 @@ CONV_FUSED_MAX_LC = 5    # conv lengths the fused decode kernel takes
 
 def shortconv_decode_fused(y: torch.Tensor, h: torch.Tensor, w_in: torch.Tensor, w: torch.Tensor,
                            bias: torch.Tensor | None, state: torch.Tensor, batch, Lc: int,
-                           scale: "SplitNorm | None" = None) -> bool:
+                           scale: "SplitNorm | None" = None, chain: bool = True) -> bool:
     """The conv mixer's in_proj and convolution of a decode step without a kernel of the
     convolution's own: y = conv(h . w_in^T), state updated.  Up to SMALL_M sequences it is the epilogue
     of the weight stream (one launch); up to SKINNY_M sequences the second kernel of the sliced
@@ -1115,11 +1195,25 @@ def shortconv_decode_fused(y: torch.Tensor, h: torch.Tensor, w_in: torch.Tensor,
             and batch.max_qlen == 1 and M == batch.n_seqs and 2 <= Lc <= CONV_FUSED_MAX_LC and K % 8 == 0
             and h.stride(0) % 8 == 0 and h.stride(1) == 1 and y.stride(1) == 1):
         return False
+    slices = 1
     if M > SMALL_M:
-        L = lib()
-        slices = L.leb_gemm_bf16_skinny_slices(3 * D, K)
+        slices = _library().leb_gemm_bf16_skinny_slices(3 * D, K)
         if slices < 2 or 3 * D >= SKINNY_MAX_N or not _tma_ok(h, w_in, K) or not w_in.is_contiguous():
             return False
+    if chain and _chain.open:
+        _cuda(h, "shortconv.h", contiguous=False)
+        _cuda(w_in, "shortconv.w_in", torch.bfloat16)
+        _cuda(w, "shortconv.w", torch.float32)
+        _cuda(state, "shortconv.state", torch.float32)
+        assert w_in.shape == (3 * D, K) and w.numel() == D * Lc and state.shape[1:] == (D, Lc - 1)
+        if bias is not None:
+            _cuda(bias, "shortconv.bias", torch.float32)
+        if _chained(y, h, w_in, M, 3 * D, K, STORE, _scale_args(scale, M, K), (None, None, None),
+                    lambda: shortconv_decode_fused(y, h, w_in, w, bias, state, batch, Lc, scale=scale, chain=False),
+                    (_ptr(w), _ptr(bias), _ptr(state), _ptr(batch.row_seq), _ptr(batch.seq_slot), Lc)):
+            return True
+    if M > SMALL_M:
+        L = lib()
         _cuda(w_in, "shortconv.w_in", torch.bfloat16)
         _cuda(w, "shortconv.w", torch.float32)
         _cuda(state, "shortconv.state", torch.float32)
@@ -1688,7 +1782,7 @@ def _scale_args(scale: "SplitNorm | None", M: int, K: int):
 
 def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = STORE,
            group_offsets: torch.Tensor | None = None, rows_hint: int = 0, streaming: bool = False,
-           scale: SplitNorm | None = None, emit: SplitNorm | None = None) -> None:
+           scale: SplitNorm | None = None, emit: SplitNorm | None = None, chain: bool = True) -> None:
     """out (+)= x . w^T  with w [N, K] (or [E, N, K] with group_offsets [E+1] over the rows).
 
     float32 operands run on the CUDA cores in true 32-bit; bfloat16 operands on the tensor
@@ -1701,7 +1795,8 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
     and large matrices 256 x 256 tiles on pairs of SMs; `streaming` asks for the register-fed
     weight-streaming kernel (the one that also serves grouped products) whatever the row count.
     Kernels of a few rows fetch W ahead of their wait for the kernel launched before them: `w` must not be what that
-    kernel writes (a model's weights never are).
+    kernel writes (a model's weights never are).  Inside a `product_chain` such products may wait for the ones
+    that follow (`chain`).
     """
     _cuda(x, "linear.x", contiguous=False)
     _cuda(w, "linear.w", x.dtype)
@@ -1723,6 +1818,18 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
     assert out.shape == (M, n_out), f"linear: out is {tuple(out.shape)}, expected {(M, n_out)}"
     if M == 0:
         return
+    if (chain and _chain.open and group_offsets is None and not streaming and x.dtype == torch.bfloat16 and K % 8 == 0 and lda % 8 == 0
+            and (emit is None or epilogue == ACCUMULATE)):
+        ev = eg = es = None
+        if emit is not None:
+            assert emit.values.shape == (M, N) and emit.ssq.shape == (M, -(-N // 16))
+            assert emit.values.is_contiguous() and emit.ssq.is_contiguous() and emit.weight.numel() == N
+            ev, eg, es = _ptr(emit.values), _ptr(emit.weight), _ptr(emit.ssq)
+        if _chained(out, x, w, M, N, K, epilogue, _scale_args(scale, M, K), (ev, eg, es),
+                    lambda: linear(out, x, w, epilogue, scale=scale, emit=emit, chain=False)):
+            if emit is not None:
+                emit.filled = True
+            return
     L = lib()
     if x.dtype == torch.float32:
         if gated:
@@ -2101,6 +2208,7 @@ def linear_tc2(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: in
     return True
 
 
+CHAIN_MIN = 2    # consecutive products from which a chain of them runs as one kernel
 SKINNY_M = 128   # rows up to which W is the wide tcgen05 operand and K is sliced over blocks
 SKINNY_MAX_N = 128 * 296   # from here on N alone gives every SM several tiles and the persistent kernel streams W better
 _skinny_ws: dict[int, list[torch.Tensor]] = {}

@@ -1279,3 +1279,100 @@ def test_linear_skinny_swiglu(M, F, D):
     K().check_device_status()
     assert err(out, want) < 6e-3
 
+
+def _gate(name, g, u):
+    if name == "silu":
+        return P.silu(g) * u
+    if name == "gelu_tanh":
+        return 0.5 * g * (1 + torch.tanh(math.sqrt(2 / math.pi) * (g + 0.044715 * g ** 3))) * u
+    g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
+    return g * torch.sigmoid(1.702 * g) * (u + 1)
+
+
+@pytest.mark.parametrize("M,D,F,gate", [(17, 64, 16, "silu"), (32, 2048, 5632, "silu"), (33, 104, 176, "gelu_tanh"), (64, 2048, 7168, "silu"),
+                                        (48, 520, 1040, "clamped"), (65, 1000, 2000, "silu"), (96, 328, 4224, "gelu_tanh"),
+                                        (97, 264, 96, "clamped"), (128, 2048, 1536, "silu")])
+def test_product_chain(M, D, F, gate):
+    """Products of a step run as one resident kernel: convolution, sum with the next norm's half, gated epilogue, store with and
+    without an activation, float and bfloat16, twice over (a second layer reads what the first wrote); rows at the edges of
+    the paddings, K of one block and of part blocks, tiles of every height, padding sequences.  Each product against
+    64 bits from the inputs it had; a product that adds up to K terms of bfloat16 in float is off by at most 2e-5 of the largest,
+    a bfloat16 result by half a step more (8 significant bits: at most 2^-8 of the value), the convolution by that of its three
+    projections and of its own."""
+    import types
+    from lastengine_b200.engine.workspace import Workspace
+    from lastengine_b200.parts.ffn import fuse_gate_up
+    k = K()
+    ws, b16, f32 = Workspace(torch.device(DEV)), torch.bfloat16, torch.float32
+    if k.lib().leb_gemm_bf16_skinny_slices(3 * D, D) < 2:
+        conv_fits = False        # the convolution alone needs two slices: the chain then begins without it
+    else:
+        conv_fits = True
+    slot = torch.arange(M, dtype=torch.int32).flip(0)
+    slot[M // 2] = -1
+    batch = types.SimpleNamespace(max_qlen=1, n_seqs=M, row_seq=torch.arange(M, dtype=torch.int32, device=DEV), seq_slot=slot.to(DEV))
+    act = {"silu": k.SILU, "gelu_tanh": k.GELU_TANH, "clamped": k.CLAMPED_SIGMOID}[gate]
+    gated = k.gated_epilogue(act, 7.0 if gate == "clamped" else 0.0, 1.702 if gate == "clamped" else 1.0)
+    W = {n: gen(r, c, seed=i, scale=c ** -0.5, dtype=b16) for i, (n, (r, c)) in enumerate(
+        {"in": (3 * D, D), "o": (D, D), "g": (F, D), "u": (F, D), "down": (D, F), "head": (F, D)}.items())}
+    taps, bias, norm = gen(D, 3, seed=20), gen(D, seed=21, scale=0.1), 1 + gen(D, seed=22, scale=0.1)
+    dev = {n: t.to(DEV) for n, t in W.items()}
+    dev["gu"] = fuse_gate_up(W["g"], W["u"], True).to(DEV)
+    h, x0, st0 = gen(M, D, seed=23, dtype=b16), gen(M, D, seed=24), gen(M, D, 2, seed=25)
+    x, st, hd = x0.to(DEV), st0.to(DEV), h.to(DEV)
+    buf = lambda *shape, dtype=b16: torch.full(shape, float("nan"), dtype=dtype, device=DEV)  # noqa: E731
+    steps, inp, scale = [], hd, None
+    before = k.launch_count()
+    with k.product_chain(ws, M, b16):
+        for layer in range(2):
+            y = buf(M, D)
+            if conv_fits:
+                assert k.shortconv_decode_fused(y, inp, dev["in"], taps.to(DEV), bias.to(DEV), st, batch, 3, scale=scale)
+            else:
+                k.linear(y, inp, dev["o"], scale=scale)
+            mid = k.SplitNorm(buf(M, D), buf(M, -(-D // 16), dtype=f32), norm.to(DEV), 1e-5)
+            k.linear(x, y, dev["o"], k.ACCUMULATE, emit=mid)
+            a = buf(M, F)
+            k.linear(a, mid.values, dev["gu"], gated, scale=mid)
+            nxt = k.SplitNorm(buf(M, D), buf(M, -(-D // 16), dtype=f32), norm.to(DEV), 1e-5)
+            k.linear(x, a, dev["down"], k.ACCUMULATE, emit=nxt)
+            steps.append((inp, scale, y, mid, a, nxt))
+            inp, scale = nxt.values, nxt
+        z, zf = buf(M, F), buf(M, F, dtype=f32)
+        k.linear(z, inp, dev["head"], k.plain_act_epilogue(k.PLAIN_ACTIVATIONS["relu_squared"]), scale=scale)
+        k.linear(zf, inp, dev["head"], scale=scale)
+    k.check_device_status()
+    assert k.launch_count() - before == 1
+    assert ws.zeroed("chain.sync", 2).tolist() == [0, 0]
+
+    def rows(values, sc):      # the rows a product read: with a split norm, values times the rows' factor
+        v = values.double().cpu()
+        return v if sc is None else v / torch.sqrt(sc.ssq.double().cpu().sum(-1, keepdim=True) / D + 1e-5)
+    want_x, state = x0.double(), st0.double()
+    for inp, sc, y, mid, a, nxt in steps:
+        v = rows(inp, sc)
+        if conv_fits:
+            b, c, u = (v @ W["in"].double().T).chunk(3, -1)
+            on = slot >= 0
+            bx = b.to(b16).double() * u.to(b16).double()
+            old = state[slot.clamp(min=0).long()]
+            conv = old[:, :, 0] * taps[:, 0].double() + old[:, :, 1] * taps[:, 1].double() + bx * taps[:, 2].double() + bias.double()
+            want = torch.where(on[:, None], c.to(b16).double() * conv, torch.zeros(()).double())
+            state = state.clone()
+            state[slot[on].long()] = torch.stack([old[:, :, 1], bx], -1)[on]
+            assert err(y, want) < 4 * 2 ** -8
+        else:
+            assert err(y, v @ W["o"].double().T) < 2 ** -8 + 2e-5
+        want_x = want_x + y.double().cpu() @ W["o"].double().T
+        assert err(mid.values, want_x * norm.double()) < 2 ** -8 + 2e-5
+        v = rows(mid.values, mid)
+        assert err(a, _gate(gate, v @ W["g"].double().T, v @ W["u"].double().T)) < 2 ** -8 + 1e-4
+        want_x = want_x + a.double().cpu() @ W["down"].double().T
+        assert err(nxt.values, want_x * norm.double()) < 2 ** -8 + 2e-5
+        assert err(nxt.ssq.sum(-1), (want_x ** 2).sum(-1)) < 1e-4
+    assert err(x, want_x) < 2e-5
+    if conv_fits:
+        assert err(st, state) < 2 * 2 ** -8
+    v = rows(steps[-1][5].values, steps[-1][5]) @ W["head"].double().T
+    assert err(zf, v) < 2e-5 and err(z, torch.clamp(v, min=0) ** 2) < 2 ** -8 + 4e-5
+
