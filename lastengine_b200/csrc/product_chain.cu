@@ -166,13 +166,6 @@ __device__ __forceinline__ bool pc_wait_grid(const unsigned* count, unsigned tar
   *abort_flag = 1;
   return false;
 }
-// One lane of a warp whose lanes are together: the loops that issue copies and products are walked by whole warps, so that
-// what those instructions take is uniform (see attention_prefill_tc.cu).
-__device__ __forceinline__ bool pc_elect() {
-  uint32_t e;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-  return e != 0;
-}
 // Whether all 256 threads of the summing warps say yes: a wait that ran out in one of them ends all of them together.
 __device__ __forceinline__ bool pc_all_summing(bool ok) {
   uint32_t r;
@@ -329,7 +322,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
           }
           if (gave_up) break;
           const uint32_t bar = b_wfull + 8 * (stage % PC_STAGES), bit = 1u << (stage % PC_STAGES);
-          if (pc_elect()) {
+          if (elect_lane()) {
             pc_expect(bar, here * rows * 128);
             for (int u = 0; u < here; u++) {
               const int k = (sl.lo + kb + u) * TC_BK;
@@ -361,7 +354,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
       const int n_tiles = sl.n_tiles;
       const CUtensorMap* map = &args.map[o].x;
       if (sl.first < n_tiles) {
-        if (pc_elect()) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
+        if (elect_lane()) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
         __syncwarp();
         // the activations of product o are there once every block has finished product o - 1; they were written by
         // ordinary stores and are read by the copy unit
@@ -374,7 +367,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
           for (int kb = 0; kb < sl.n; kb += 2) {
             if (!pc_wait_warp(b_xempty + 8 * s, ph, abort_flag)) { gave_up = 43; break; }
             const int here = min(2, sl.n - kb);
-            if (pc_elect()) {
+            if (elect_lane()) {
               pc_expect(b_xfull + 8 * s, here * X_BYTES);
               for (int u = 0; u < here; u++) pc_load(a_x + (2 * s + u) * X_BYTES, map, b_xfull + 8 * s, (sl.lo + kb + u) * TC_BK, 0);
             }
@@ -409,7 +402,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
           tc_fence_after();
           const int here = min(2, sl.n - kb);
           const int slot2 = slot + 1 >= NW ? 0 : slot + 1;
-          if (pc_elect()) {
+          if (elect_lane()) {
             const uint64_t da = w_desc + (uint64_t)(slot * (PC_SLOT / 16)), db = x_desc + (uint64_t)(2 * x * (X_BYTES / 16));
 #pragma unroll
             for (int k = 0; k < TC_BK / 16; k++)
