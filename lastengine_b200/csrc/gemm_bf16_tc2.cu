@@ -21,6 +21,9 @@
 // The loops that issue copies and MMAs are walked by whole warps and one elected lane issues: walked by one lane alone, every
 // operand of an MMA had to be moved to a uniform register first, which together with the waits took longer than the MMAs.
 // 16,384 rows x 11,264 x 2,048: 512 -> 481 us (1,570 TFLOP/s), 2,048 rows 67.4 -> 63.9.
+// Tiles are dealt in bands of T2_BAND row tiles, down a band's rows first: a wave of 74 pairs then works on about 8 row tiles
+// and 9 column tiles, 17 slabs of operands instead of 65, and what A holds beyond L2 is read from memory once and not once per
+// column tile.  16,384 x 2,048 x 5,632 (A 184 MB): 310 -> 267 us; x 6,144 x 2,048 276 -> 269.  Bands of 16: 271, 270.
 //
 // Every wait on an mbarrier is bounded; a wait that gives up sets the status word and every role
 // leaves its loop.  Both blocks always meet at a cluster barrier before they free tensor memory
@@ -29,6 +32,7 @@
 
 #define T2_THREADS 192
 #define T2_STAGES 6
+#define T2_BAND 8
 #define T2_BN 256
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -95,6 +99,12 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const int nk = (K + TC_BK - 1) / TC_BK;
   const int m_tiles = (M + 255) / 256, n_tiles = (N + BN - 1) / BN;
   const int num_tiles = m_tiles * n_tiles;
+  // the row and the column tile of a tile
+  auto place = [&](int tile, int& mt, int& nt) {
+    const int band = tile / (T2_BAND * n_tiles), r = tile - band * (T2_BAND * n_tiles), rows = min(T2_BAND, m_tiles - band * T2_BAND);
+    nt = r / rows;
+    mt = band * T2_BAND + r - nt * rows;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -125,8 +135,9 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     uint32_t s = 0, ph = 1;
     bool ok = true;
     for (int tile = pair; tile < num_tiles && ok; tile += n_pairs) {
-      const int nt = tile / m_tiles;
-      const int m0 = (tile % m_tiles) * 256 + 128 * (int)rank, n0 = nt * BN + 128 * (int)rank;
+      int mt, nt;
+      place(tile, mt, nt);
+      const int m0 = mt * 256 + 128 * (int)rank, n0 = nt * BN + 128 * (int)rank;
       int kk = (nt * 5) % nk;              // tiles that share rows of A start at different k
       for (int kb = 0; kb < nk; kb++) {
         if (!mbar_wait_warp(&empty[s], ph, abort_flag)) { ok = false; break; }
@@ -176,7 +187,9 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const uint32_t acc_empty0 = map_to_rank(smem_u32(&acc_empty[0]), 0);
     uint32_t t = 0;
     for (int tile = pair; tile < num_tiles; tile += n_pairs, t++) {
-      const int m0 = (tile % m_tiles) * 256 + 128 * (int)rank, n0 = (tile / m_tiles) * BN;
+      int mt, nt;
+      place(tile, mt, nt);
+      const int m0 = mt * 256 + 128 * (int)rank, n0 = nt * BN;
       const uint32_t buf = t & 1;
       const int row_base = m0 + quad * 32;
       // adding epilogue with 16-byte rows: a lane's eight old values (rows lane/8 + 4j, four columns
