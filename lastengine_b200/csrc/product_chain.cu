@@ -511,13 +511,24 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
       __syncwarp();
       if (!pc_all_summing(there)) { gave_up = 47; break; }
       // the rows' factors of a split norm (1 without one): a warp takes rows ew, ew + 8, ...; the convolution's slots
-#pragma unroll 1
-      for (int r = ew; r < R; r += 8) {
-        float s = 0.f;
-        if (op.ssq_in && m0 + r < M)
-          for (int p = lane; p < op.parts_in; p += 32) s += __ldcg(op.ssq_in + (size_t)(m0 + r) * op.parts_in + p);
+      constexpr int RW = (R + 7) / 8;      // (all loads first: one after the other they would be eight trips to L2)
+      float part[RW][4];
+#pragma unroll
+      for (int i = 0; i < RW; i++)
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+          const int r = ew + 8 * i;
+          part[i][p] = op.ssq_in && r < R && m0 + r < M && lane + 32 * p < op.parts_in
+                           ? __ldcg(op.ssq_in + (size_t)(m0 + r) * op.parts_in + lane + 32 * p) : 0.f;
+        }
+#pragma unroll
+      for (int i = 0; i < RW; i++) {
+        const int r = ew + 8 * i;
+        float s = (part[i][0] + part[i][1]) + (part[i][2] + part[i][3]);
+        if (op.ssq_in && r < R && m0 + r < M)
+          for (int p = lane + 128; p < op.parts_in; p += 32) s += __ldcg(op.ssq_in + (size_t)(m0 + r) * op.parts_in + p);
         s = warp_sum(s);
-        if (lane == 0) {
+        if (lane == 0 && r < R) {
           row_scale[r] = op.ssq_in ? 1.0f / sqrtf(s / (float)op.d_in + op.eps) : 1.f;
           row_slot[r] = kind == 3 && m0 + r < M ? op.seq_slot[op.row_seq[m0 + r]] : -1;
         }
