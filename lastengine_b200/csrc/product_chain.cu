@@ -20,12 +20,13 @@
 // and x rows of 32 channels), each optionally scaled by a split norm.
 //
 // What bounds it: four products of a conv layer at 64 rows (width 2,048, 7,168 wide inside, 122 MB of weights, 18.6 us at the copy
-// rate) take 41 us here and 67 as eight launches of the sliced product and its second kernel; 36 and 43 at 32 rows, 64 and 71
-// at 128 (5,632 wide).  The stream runs at the memory's rate while there is room in the ring; the chain of a
+// rate) take 41 us here and 67 as eight launches of the sliced product and its second kernel; 36 and 43 at 32 rows, 52 and 62
+// at 96, 58 and 71 at 128 (5,632 wide).  The stream runs at the memory's rate while there is room in the ring; the chain of a
 // product (grid barrier 1.3 us, activations 0.7, last k-blocks 0.5 to 2, exchange 0.7, sums and stores 1, each once per
 // product) is longer than what the ring holds.  A cluster of 8 halves a block's k-blocks, but only 15 such clusters fit the
 // chip (120 blocks against 132 in 33 clusters of 4) and 16 tiles then take two rounds: 57 us.  Two buffers for the exchange
-// against two more weight slots: 47.2 and 50.9 us, with the second the senders wait for their credits.  Epilogues unrolled
+// against two more weight slots: 47.2 and 50.9 us, with the second the senders wait for their credits.  From 65 rows on a tile is exchanged in two
+// parts, so that two buffers fit: 128 rows 64 -> 58 us, 96 rows 55 -> 52; at 64 rows the second exchange costs more (46 -> 52).  Epilogues unrolled
 // over all of a thread's outputs (128 KB of instructions) against loops: 47.2 and 45.8.
 //
 // All blocks wait for one another, so they must all be resident: the launch is cooperative.  Every wait is bounded
@@ -191,17 +192,18 @@ __device__ __noinline__ void pc_act_call(float* z, int act) {
   for (int e = 0; e < 4; e++) z[e] = plain_act(z[e], act);
 }
 
-// By MP: weight slots of 16 KB, stages of two k-blocks of activations (MP x 256 bytes), buffers for a cluster's partial tile (MP x 512).
+// By MP: weight slots of 16 KB, stages of two k-blocks of activations (MP x 256 bytes), parts in which a partial tile is exchanged
+// (an owner's first rows, then its last), buffers for such a part of the cluster's partial tiles (MP x 512 / parts bytes).
 template <int MP> struct ChainRing;
-template <> struct ChainRing<32> { static constexpr int NW = 9, NX = 4, RB = 2; };
-template <> struct ChainRing<64> { static constexpr int NW = 7, NX = 2, RB = 2; };
-template <> struct ChainRing<96> { static constexpr int NW = 7, NX = 2, RB = 1; };
-template <> struct ChainRing<128> { static constexpr int NW = 5, NX = 2, RB = 1; };
+template <> struct ChainRing<32> { static constexpr int NW = 9, NX = 4, H = 1, RB = 2; };
+template <> struct ChainRing<64> { static constexpr int NW = 7, NX = 2, H = 1, RB = 2; };
+template <> struct ChainRing<96> { static constexpr int NW = 7, NX = 2, H = 2, RB = 2; };
+template <> struct ChainRing<128> { static constexpr int NW = 5, NX = 2, H = 2, RB = 2; };
 
 template <int MP>
 static constexpr size_t chain_smem() {
   typedef ChainRing<MP> Ring;
-  return (size_t)Ring::NW * PC_SLOT + (size_t)Ring::NX * MP * 256 + (size_t)Ring::RB * MP * 512 + 1024 /* alignment */ +
+  return (size_t)Ring::NW * PC_SLOT + (size_t)Ring::NX * MP * 256 + (size_t)Ring::RB * MP * 512 / Ring::H + 1024 /* alignment */ +
          sizeof(ChainOp) * PC_MAX_OPS + 8 * (2 * PC_STAGES + 2 * Ring::NX + 4 + 3 * Ring::RB) + 4 * (MP / 4) * 2 + 80;
 }
 
@@ -209,8 +211,8 @@ template <int MP>
 __global__ void __launch_bounds__(PC_THREADS, 1)
 product_chain_kernel(const __grid_constant__ ChainArgs args) {
   typedef ChainRing<MP> Ring;
-  constexpr int NW = Ring::NW, NX = Ring::NX, RB = Ring::RB, R = MP / PC_CLUSTER;
-  constexpr int X_BYTES = MP * 128, RECV = MP * 512;     // RECV: 4 slices of [R / 4][128][4] floats
+  constexpr int NW = Ring::NW, NX = Ring::NX, H = Ring::H, RB = Ring::RB, R = MP / PC_CLUSTER, RH = R / H;
+  constexpr int X_BYTES = MP * 128, RECV = MP * 512 / H;     // RECV: 4 slices of [RH / 4][128][4] floats
   constexpr uint32_t ACC_COLS = MP <= 32 ? 32 : (MP <= 64 ? 64 : 128), TMEM_COLS = 2 * ACC_COLS;
   extern __shared__ uint8_t smem_raw[];
   // the same offset in every block of the cluster (addresses of peers' buffers are formed from this block's)
@@ -433,7 +435,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
       for (int o = 0; o < n_ops && !gave_up; o++) {
         const Share sl = share_of(o);
         const int n_tiles = sl.n_tiles;
-        for (int t = sl.first; t < n_tiles; t += n_clusters, q++) {
+        for (int i = 0, parts = sl.first < n_tiles ? H * ((n_tiles - sl.first + n_clusters - 1) / n_clusters) : 0; i < parts; i++, q++) {
           const int rb = q % RB;
           if (!pc_wait_warp(b_taken + 8 * rb, (q / RB) & 1, abort_flag)) { gave_up = 49; break; }
           if (lane < PC_CLUSTER) pc_arrive_remote(pc_mapa(b_credit + 8 * rb, lane));
@@ -447,31 +449,39 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
     int r = 0, q = 0;
     for (int o = 0; o < n_ops && !gave_up; o++) {
       const Share sl = share_of(o);
-      for (int t = sl.first; t < sl.n_tiles; t += n_clusters, q++) {
-        if (sl.n == 0) continue;
-        const int rb = q % RB;
+      for (int t = sl.first; t < sl.n_tiles && !gave_up; t += n_clusters) {
+        if (sl.n == 0) {
+          q += H;
+          continue;
+        }
         bool ok = pc_wait<false>(b_acc_full + 8 * (r & 1), (r >> 1) & 1, abort_flag);
-        // the owners have taken what lay in this buffer
-        if (ok && q >= RB) ok = pc_wait<true>(b_credit + 8 * rb, ((q / RB) - 1) & 1, abort_flag);
-        if (!__all_sync(0xffffffffu, ok)) { gave_up = 46; break; }
-        tc_fence_after();
-        if (quad * 32 < sl.rows) {
-          const uint32_t base = a_r + rb * RECV + (uint32_t)rank * (R * 512) + (uint32_t)(quad * 32 + lane) * 16, bar = b_recv + 8 * rb;
-          const uint32_t src = tmem_acc + (r & 1) * ACC_COLS + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
-          for (int to = 0; to < n_owners; to++) {
-            uint32_t v[R];
+        for (int h = 0; h < H; h++, q++) {
+          const int rb = q % RB;
+          // the owners have taken what lay in this buffer
+          if (ok && q >= RB) ok = pc_wait<true>(b_credit + 8 * rb, ((q / RB) - 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok) != 0;
+          if (!ok) break;
+          tc_fence_after();
+          if (quad * 32 < sl.rows) {
+            const uint32_t base = a_r + rb * RECV + (uint32_t)rank * (RH * 512) + (uint32_t)(quad * 32 + lane) * 16, bar = b_recv + 8 * rb;
+            const uint32_t src = tmem_acc + (r & 1) * ACC_COLS + ((uint32_t)(quad * 32) << 16) + h * RH;
+#pragma unroll 1
+            for (int to = 0; to < n_owners; to++) {
+              uint32_t v[RH];
 #pragma unroll
-            for (int c = 0; c < R; c += 4)
-              asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                           : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3])
-                           : "r"(src + to * R + c));
-            const uint32_t there = pc_mapa(base, to), bar_there = pc_mapa(bar, to);
-            tmem_ld_wait();
+              for (int c = 0; c < RH; c += 4)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3])
+                             : "r"(src + to * R + c));
+              const uint32_t there = pc_mapa(base, to), bar_there = pc_mapa(bar, to);
+              tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < R; c += 4) pc_send4(there + (c / 4) * 2048, bar_there, v + c);
+              for (int c = 0; c < RH; c += 4) pc_send4(there + (c / 4) * 2048, bar_there, v + c);
+            }
           }
         }
+        if (!ok) { gave_up = 46; break; }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) pc_arrive(b_acc_empty + 8 * (r & 1));
@@ -483,7 +493,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
     // column and four rows (16 bytes of every slice).  Loops over units stay loops: all of a chain's epilogues
     // unrolled are 128 KB of instructions, which come from L2 every time.
     const int tid = threadIdx.x - 256, m0 = rank * R, ew = tid >> 5;
-    constexpr int G = R / 4;
+    constexpr int G = RH / 4;           // row groups of a part
     pdl_wait();
     int q = 0;
     unsigned target = 0;
@@ -539,18 +549,18 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
       const int ps = width > 64 ? 7 : (width > 32 ? 6 : 5), n_units = G << ps;
       const int end = kind == 3 ? op.width : (kind == 2 ? op.width : op.N);     // columns of the result
 #pragma unroll 1
-      for (int t = sl.first; t < n_tiles; t += n_clusters, q++) {
-        const int rb = q % RB;
-        if (tid == 0) pc_expect(b_recv + 8 * rb, (uint32_t)active * (R * 4) * rows);
+      for (int i_part = 0, parts = H * ((n_tiles - sl.first + n_clusters - 1) / n_clusters); i_part < parts; i_part++, q++) {
+        const int t = sl.first + i_part / H * n_clusters, rb = q % RB, r0 = i_part % H * RH;
+        if (tid == 0) pc_expect(b_recv + 8 * rb, (uint32_t)active * (RH * 4) * rows);
         const float* recv = (const float*)(sr + rb * RECV);
-        // column n, rows 4 g ... 4 g + 3: the slices' shares, R * 128 floats apart, added in order
+        // column n, rows 4 g ... 4 g + 3 of the part: the slices' shares, RH * 128 floats apart, added in order
         auto sum = [&](int n, int g) {
           const float4* p = (const float4*)(recv + g * 512 + n * 4);
           float4 a = p[0];
 #pragma unroll
           for (int s = 1; s < PC_CLUSTER; s++)
             if (s < active) {
-              const float4 b = p[s * (R * 32)];
+              const float4 b = p[s * (RH * 32)];
               a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w;
             }
           return a;
@@ -558,7 +568,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
         bool waited = false;
 #pragma unroll 1
         for (int u = tid; u < n_units; u += PC_SUMMING) {        // (whole warps share u's row group)
-          const int i = u & ((1 << ps) - 1), g = u >> ps, col = t * width + i, row0 = 4 * g, m = m0 + row0;
+          const int i = u & ((1 << ps) - 1), g = u >> ps, col = t * width + i, row0 = r0 + 4 * g, m = m0 + row0;
           const bool in = i < width && col < end;
           // what does not depend on the sums is on its way while they come
           float old[4], st[4][ST_CONV_MAX_LC - 1], tap[ST_CONV_MAX_LC], extra = 0.f;      // extra: the next norm's weight, or the convolution's bias
