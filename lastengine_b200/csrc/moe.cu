@@ -227,6 +227,74 @@ moe_router_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, const 
   }
 }
 
+// The same router for few rows (decode steps): a cluster of four blocks takes a row, each a quarter of the experts, a warp one of
+// them.  One block's 262 KB of router rows (32 experts of 2,048) come to its SM in 8.4 us, most of it two trips to L2 after
+// the wait; here a warp has the whole of its router row (PRE pieces of 16 bytes a lane) in registers before it waits for the
+// row of h, and the scores go to the first block's shared memory, whose first warp chooses.  A score is summed in the order of the
+// form above: the same bits.
+#define ROUTER_CLUSTER 4
+#define ROUTER_PRE 16
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, const T* __restrict__ h,
+                      const float* __restrict__ wr, const float* __restrict__ bias, int D, int E, int k, int norm_topk, float scaling) {
+  extern __shared__ __align__(16) float sm[];  // the row of h as float [D], then s[E], c[E]
+  float* s_ = sm + D;
+  float* c_ = s_ + E;
+  const int rank = blockIdx.x % ROUTER_CLUSTER, m = blockIdx.x / ROUTER_CLUSTER;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int share = (E + ROUTER_CLUSTER - 1) / ROUTER_CLUSTER, first = rank * share + warp, end = min(E, (rank + 1) * share), n4 = D / 4;
+  pdl_trigger();
+  float4 a[ROUTER_PRE];
+#pragma unroll
+  for (int u = 0; u < ROUTER_PRE; u++)
+    a[u] = first < end && lane + 32 * u < n4 ? reinterpret_cast<const float4*>(wr + (size_t)first * D)[lane + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  pdl_wait();
+  const T* hr = h + (size_t)m * D;
+  for (int i = threadIdx.x; i < n4; i += blockDim.x) reinterpret_cast<float4*>(sm)[i] = load4(hr + 4 * i);
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // the first block is there to be written to
+  uint32_t s0, c0;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(s0) : "r"((uint32_t)__cvta_generic_to_shared(s_)));
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(c0) : "r"((uint32_t)__cvta_generic_to_shared(c_)));
+  for (int e = first; e < end; e += nw) {
+    const float4* w4 = reinterpret_cast<const float4*>(wr + (size_t)e * D);
+    float z = 0.f;
+    for (int i0 = lane; i0 < n4; i0 += 32 * ROUTER_PRE) {
+      if (e != first || i0 != lane) {
+#pragma unroll
+        for (int u = 0; u < ROUTER_PRE; u++) a[u] = i0 + 32 * u < n4 ? w4[i0 + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < ROUTER_PRE; u++) {
+        const int i = i0 + 32 * u;
+        if (i >= n4) break;
+        const float4 x = reinterpret_cast<const float4*>(sm)[i];
+        z += a[u].x * x.x;
+        z += a[u].y * x.y;
+        z += a[u].z * x.z;
+        z += a[u].w * x.w;
+      }
+    }
+    z = warp_sum(z);
+    if (lane == 0) {
+      float s, c;
+      router_score(&s, &c, z, bias ? bias[e] : 0.f, norm_topk);
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(s0 + 4 * e), "f"(s) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(c0 + 4 * e), "f"(c) : "memory");
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank != 0 || warp != 0) return;
+  if (ROUTER_GROUPED(norm_topk))
+    router_softmax_groups(s_, c_, bias, E, ROUTER_GROUPS(norm_topk), ROUTER_KEEP(norm_topk), lane,
+                          ROUTER_MODE(norm_topk) == ROUTER_SOFTMAX_GROUPED, ROUTER_GROUP_TOP(norm_topk));
+  router_choose(topk_ids + (size_t)m * k, topk_w + (size_t)m * k, c_, s_, E, k, norm_topk, scaling, lane);
+}
+
 // The same router for the many rows of a prompt: a block of 8 warps takes RB rows (kept in shared
 // memory as they come), and a warp takes four experts at a time for all RB rows, so that one
 // piece of a router row from L2 and one piece of a row of h from shared memory feed 4 x RB
@@ -353,6 +421,29 @@ LEB_API int leb_moe_router(int* topk_ids, float* topk_w, const void* h, int dtyp
       LEB_CHECK_LAUNCH("leb_moe_router");
       return 0;
     }
+  }
+  // few rows: a cluster of four blocks each, while all of them have SMs of their own
+  const size_t smem_few = ((size_t)D + 2 * E) * sizeof(float);
+  if (ROUTER_CLUSTER * M <= sm_count() && E >= 8 && D % 8 == 0 && ((uintptr_t)wr & 15) == 0 && ((uintptr_t)h & 15) == 0 && smem_few <= 48 * 1024 &&
+      (dtype == LEB_BF16 || dtype == LEB_F32)) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ROUTER_CLUSTER * M);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem_few;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ROUTER_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_leb_pdl ? 2 : 1;
+    const cudaError_t e = dtype == LEB_BF16 ? cudaLaunchKernelEx(&cfg, moe_router_few_kernel<bf16>, topk_ids, topk_w, (const bf16*)h, wr, bias, D, E, k, norm_topk, scaling)
+                                            : cudaLaunchKernelEx(&cfg, moe_router_few_kernel<float>, topk_ids, topk_w, (const float*)h, wr, bias, D, E, k, norm_topk, scaling);
+    if (e != cudaSuccess) return leb_fail("leb_moe_router: %s", cudaGetErrorString(e));
+    LEB_CHECK_LAUNCH("leb_moe_router");
+    return 0;
   }
   // rows per block: 1 while every row can have an SM of its own (a block's pace is set by one SM
   // reading the router's weights), 4 for many rows when they fit shared memory
