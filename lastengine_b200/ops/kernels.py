@@ -210,6 +210,7 @@ def _declare(L) -> None:
         "leb_gemm_bf16_tc2": [P, I, P, P, I, I, I, I, I, I, P, P],
         "leb_moe_router": [P, P, P, I, P, P, I, I, I, I, I, F, P],
         "leb_moe_align": [P, P, P, P, I, I, P],
+        "leb_moe_align_gather": [P, P, P, P, I, P, P, P, I, I, I, I, P],
         "leb_moe_combine": [P, P, P, P, I, I, I, I, P],
         "leb_penalties": [P, P, P, I, I, I, F, F, P],
         "leb_argmax": [P, P, I, I, P],
@@ -1944,6 +1945,31 @@ def moe_align(offsets: torch.Tensor, sorted_pair: torch.Tensor, pair_row: torch.
     P_ = topk_ids.numel()
     assert offsets.numel() >= E + 1 and sorted_pair.numel() >= P_ and pair_row.numel() >= P_
     _check(lib().leb_moe_align(_ptr(offsets), _ptr(sorted_pair), _ptr(pair_row), _ptr(topk_ids), P_, E, _stream()))
+
+
+MOE_FEW_PAIRS = 256      # pairs up to which order and rows come from one launch (a thread of its blocks is a pair)
+
+
+def moe_align_gather(offsets: torch.Tensor, sorted_pair: torch.Tensor, pair_row: torch.Tensor, xs: torch.Tensor,
+                     topk_ids: torch.Tensor, h: torch.Tensor, E: int, weights: torch.Tensor | None = None) -> None:
+    """`moe_align` and the rows in that order: xs[r] = h[sorted_pair[r] // k], times weights[sorted_pair[r]] where they are given."""
+    P_, D = xs.shape
+    k = topk_ids.shape[1]
+    if not (0 < P_ <= MOE_FEW_PAIRS and D * xs.element_size() % 16 == 0 and xs.data_ptr() % 16 == 0 and h.data_ptr() % 16 == 0):
+        moe_align(offsets, sorted_pair, pair_row, topk_ids, E)
+        gather_rows(xs, h, sorted_pair, div=k, weights=weights)
+        return
+    for n, t in (("offsets", offsets), ("sorted_pair", sorted_pair), ("pair_row", pair_row), ("topk_ids", topk_ids)):
+        _cuda(t, f"moe_align_gather.{n}", torch.int32)
+    _cuda(xs, "moe_align_gather.xs")
+    _cuda(h, "moe_align_gather.h", xs.dtype)
+    assert topk_ids.numel() == P_ and h.shape == (P_ // k, D)
+    assert offsets.numel() >= E + 1 and sorted_pair.numel() >= P_ and pair_row.numel() >= P_
+    if weights is not None:
+        _cuda(weights, "moe_align_gather.weights", torch.float32)
+        assert weights.numel() >= P_
+    _check(lib().leb_moe_align_gather(_ptr(offsets), _ptr(sorted_pair), _ptr(pair_row), _ptr(xs), _dt(xs, "moe_align_gather"), _ptr(topk_ids),
+                                      _ptr(h), _ptr(weights), P_, E, k, D, _stream()))
 
 
 def moe_combine(x: torch.Tensor, ys: torch.Tensor, pair_row: torch.Tensor, topk_w: torch.Tensor | None,

@@ -257,9 +257,8 @@ class SigmoidTopKMoE(FeedForward):
         offsets = ws.get("moe.offsets", (self.E + 1,), torch.int32)
         sorted_pair = ws.get("moe.sorted", (P,), torch.int32)
         pair_row = ws.get("moe.rows", (P,), torch.int32)
-        kernels.moe_align(offsets, sorted_pair, pair_row, ids, self.E)
         xs = ws.get("moe.xs", (P, self.D), env.dtype)
-        kernels.gather_rows(xs, h, sorted_pair, div=self.k, weights=wts if self.weight_input else None)
+        kernels.moe_align_gather(offsets, sorted_pair, pair_row, xs, ids, h, self.E, weights=wts if self.weight_input else None)
         a = ws.get("moe.a", (P, self.Fe), env.dtype)
         if not self.gated and kernels.takes_plain_act(xs, self.w13, n_groups=self.E):
             kernels.linear(a, xs, self.w13, kernels.plain_act_epilogue(self.act), group_offsets=offsets, rows_hint=P)

@@ -1053,6 +1053,27 @@ def test_moe_router_gives_a_row_the_same_bits_whatever_the_step(dtype, E, k, D):
     assert err(all_w[agree.to(DEV)], want_w[agree]) < 1e-5
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,k,E,D", [(1, 1, 1, 8), (1, 4, 32, 2048), (8, 4, 32, 2048), (64, 4, 32, 520), (51, 5, 256, 4100), (37, 2, 3, 72),
+                                     (65, 4, 32, 64), (9, 3, 8, 36)])
+def test_moe_align_gather(dtype, M, k, E, D):
+    """The expert-sorted order and the rows in it by one launch (up to 256 pairs, rows of whole 16-byte pieces; the last two
+    sizes are beyond): what the sort and the gather give, with and without weights on the rows; fewer pairs than experts,
+    experts without rows, more pieces than threads."""
+    g = torch.Generator().manual_seed(7 * M + k)
+    ids = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(M)]).to(torch.int32).to(DEV)
+    h, w = gen(M, D, seed=90, dtype=dtype).to(DEV), gen(M, k, seed=91).to(DEV)
+    for weights in (None, w):
+        want, got = [], []
+        for out in (want, got):
+            i32 = lambda n: torch.full((n,), -1, dtype=torch.int32, device=DEV)  # noqa: E731
+            out += [i32(E + 1), i32(M * k), i32(M * k), torch.full((M * k, D), float("nan"), dtype=dtype, device=DEV)]
+        K().moe_align(*want[:3], ids, E)
+        K().gather_rows(want[3], h, want[1], div=k, weights=weights)
+        K().moe_align_gather(*got, ids, h, E, weights=weights)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 # ---- sampling ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("V", [256, 1000, 65536])
 def test_argmax_and_sampling(V):
