@@ -12,7 +12,7 @@
 // Roles per block: warp 0 issues the TMA loads (its A half and its W half of every
 // stage; the bytes of both blocks are counted on the first block's barrier); warp 1 allocates
 // tensor memory (both blocks ask, with cta_group::2; they get the same address) and, in the first
-// block only, one thread issues the MMAs and commits them to both blocks' barriers
+// block only, issues the MMAs (the whole warp walks the loop, one elected lane issues) and commits them to both blocks' barriers
 // (tcgen05.commit with multicast); warps 2-5 read the block's accumulator rows and apply the
 // epilogue (store, add into the float residual, SwiGLU over gate/up rows interleaved in blocks
 // of 16), then tell the first block that the accumulator is free.  Two accumulators (all 512

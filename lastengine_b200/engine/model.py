@@ -44,6 +44,20 @@ class Model:
         self.stream_tables: dict[str, torch.Tensor] = {}
         self.stream_matrices: dict[str, torch.Tensor] = {}
         self.embedding_spec = self.embedding.cache_spec() if hasattr(self.embedding, "cache_spec") else None
+        # Products of a step may wait for one another on the host (kernels.product_chain).  The library's own parts touch their
+        # results through its kernels alone, which launch what waits first; of parts from elsewhere that is not known.
+        own = __package__.split(".")[0] + "."
+        self.chains = all(type(p).__module__.startswith(own) for top in (*self.blocks, self.embedding, self.final_norm, self.head)
+                          for p in self._parts_in(top))
+
+    @classmethod
+    def _parts_in(cls, part):
+        """A part and the parts it holds (attributes, and members of lists, that compute: they have `forward` or `apply`)."""
+        yield part
+        for v in vars(part).values():
+            for p in v if isinstance(v, (list, tuple)) else (v,):
+                if not isinstance(p, (torch.Tensor, type)) and (hasattr(p, "forward") or hasattr(p, "apply")):
+                    yield from cls._parts_in(p)
 
     # ---- tensors ------------------------------------------------------------------------
     def named_parts(self) -> list[tuple[str, object]]:
@@ -104,6 +118,8 @@ class Model:
     def forward(self, batch, cache) -> torch.Tensor:
         """Runs the step's rows through every scheduled layer; returns float logits
         [batch.n_logit_rows, vocab] (a view of workspace memory, valid until the next step)."""
+        if not self.chains:
+            return self._forward(batch, cache)
         with kernels.product_chain(self.env.workspace, batch.n_rows, self.env.dtype):
             return self._forward(batch, cache)
 

@@ -1910,7 +1910,8 @@ def moe_router(topk_ids: torch.Tensor, topk_w: torch.Tensor, h: torch.Tensor, wr
     `groups` equal groups of neighbours (a group's score: its largest choice score) can be chosen, weights
     are the chosen scores over their sum (+ 1e-20).  `sigmoid_groups` = (groups, keep, top): sigmoid scores, the
     bias only chooses, groups as before with a group's score the sum of its `top` largest choice scores, weights
-    the chosen scores over their sum (+ 1e-20) times `scaling`."""
+    the chosen scores over their sum (+ 1e-20) times `scaling`.  Steps of few rows fetch `wr` ahead of their wait for the kernel
+    launched before: it must not be what that kernel writes."""
     _cuda(topk_ids, "moe_router.topk_ids", torch.int32)
     _cuda(topk_w, "moe_router.topk_w", torch.float32)
     _cuda(h, "moe_router.h")

@@ -2,6 +2,7 @@
 from types import SimpleNamespace
 
 import pytest
+import torch
 
 from lastengine_b200.ops import kernels
 
@@ -47,3 +48,25 @@ def test_every_kernel_of_the_32_bit_product_is_chosen_somewhere(sms):
                         assert 0 <= k <= 6 and (k != 6 or (groups == 0 and vec and M <= 16)) and (groups < 2 or k in (1, 2, 4, 5))
     assert seen[0, 1] == set(range(7)) and seen[0, 0] == set(range(6)) and seen[2, 0] == seen[2, 1] == {1, 2, 4, 5}
     assert choice(0, 1, 1, 0, 1, sms) == -1 and choice(1, 1, 0, 0, 1, sms) == -1
+
+
+def test_products_wait_for_one_another_only_in_models_of_the_librarys_own_parts():
+    """A part from elsewhere may touch its input or result without the library's kernels: its model launches every product at once."""
+    import dataclasses
+    from lastengine_b200.engine.model import Model
+    from lastengine_b200.engine.workspace import Workspace
+    from lastengine_b200.parts.base import BuildEnv, PartSpec
+    from lastengine_b200.parts.ffn import SwiGLU
+    from lastengine_b200.registry import FEED_FORWARDS, plan_from_config
+    from tiny_configs import TINY_A
+    cpu = torch.device("cpu")
+    env = BuildEnv(device=cpu, dtype=torch.bfloat16, workspace=Workspace(cpu))
+    plan = plan_from_config(TINY_A)
+    assert Model(plan, env).chains
+
+    @FEED_FORWARDS.register("swiglu_from_elsewhere", replace=True)
+    class Elsewhere(SwiGLU):
+        pass
+    last = plan.layers[-1]
+    layers = [*plan.layers[:-1], dataclasses.replace(last, ffn=PartSpec("swiglu_from_elsewhere", last.ffn.params))]
+    assert not Model(dataclasses.replace(plan, layers=layers), env).chains

@@ -1340,7 +1340,8 @@ def test_product_chain(M, D, F, gate):
     dev = {n: t.to(DEV) for n, t in W.items()}
     dev["gu"] = fuse_gate_up(W["g"], W["u"], True).to(DEV)
     h, x0, st0 = gen(M, D, seed=23, dtype=b16), gen(M, D, seed=24), gen(M, D, 2, seed=25)
-    x, st, hd = x0.to(DEV), st0.to(DEV), h.to(DEV)
+    x, st, hd = x0.to(DEV), st0.to(DEV), torch.zeros(M, D + 16, dtype=b16, device=DEV)[:, :D]     # rows of a wider matrix
+    hd.copy_(h)
     buf = lambda *shape, dtype=b16: torch.full(shape, float("nan"), dtype=dtype, device=DEV)  # noqa: E731
     steps, inp, scale = [], hd, None
     before = k.launch_count()
@@ -1359,7 +1360,7 @@ def test_product_chain(M, D, F, gate):
             k.linear(x, a, dev["down"], k.ACCUMULATE, emit=nxt)
             steps.append((inp, scale, y, mid, a, nxt))
             inp, scale = nxt.values, nxt
-        z, zf = buf(M, F), buf(M, F, dtype=f32)
+        z, zf = buf(M, F + 24)[:, 8:8 + F], buf(M, F + 3, dtype=f32)[:, 3:]
         k.linear(z, inp, dev["head"], k.plain_act_epilogue(k.PLAIN_ACTIVATIONS["relu_squared"]), scale=scale)
         k.linear(zf, inp, dev["head"], scale=scale)
     k.check_device_status()
