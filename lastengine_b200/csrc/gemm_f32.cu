@@ -1,6 +1,6 @@
 // True 32-bit matrix product on the CUDA cores:  C[M,N] (+)= A[M,K] . W[N,K]^T.
 //
-// FFMA only: no tensor cores, no TF32, no reduced-precision mode of any kind.  An output element is
+// 32-bit fused multiply-adds only: no tensor cores, no TF32, no reduced-precision mode of any kind.  An output element is
 // summed in one fixed order whatever M is and whichever kernel runs: k is cut into chunks of F32_CHUNK, a
 // chunk is one chain of fused multiply-adds in ascending k from zero, and the chunks' sums are added in
 // ascending order.  A row's result therefore does not depend on which other rows share the launch: a
@@ -130,22 +130,17 @@ gemm_f32_stream_kernel(float* __restrict__ C, const float* __restrict__ A, const
   }
 }
 
-// ---- more rows: tiles ----------------------------------------------------------------------------------
+// ---- a few dozen rows: small tiles over many chunks ---------------------------------------------------------
 // 256 threads; a block's tile is BM x BN, and its eight warps are WM x WN x WK: WM x WN parts of the tile, and WK chunks
-// of k at a time (WK 1 for many rows; more where the tiles would leave SMs idle: a small tile over eight chunks gives a
-// few dozen rows as many blocks as a stream of the weights has).  A lane of a warp's 8 x 4 holds TM x TN sums, rows 8
-// apart and columns side by side.  Both operands lie in shared memory as rows of 32 k at a pitch of 36 floats, where
-// the 16-byte loads of eight lanes meet no bank twice, and come through a ring of cp.async stages that runs on
-// across chunks and tiles, so only a block's first loads are waited for.  Bound by the FMA pipes and the shared loads beside
-// them: 37 TFLOP/s of the 72 the pipes have at 2,048 rows x 11,264 x 2,048 (2.5 ms, 3.7 ms before in tiles of 64 x 64 with
-// 4 x 4 sums a thread); 523 rows x 2,048 x 5,632 570 -> 436 us.  Twice the warps over the largest tile (half the
-// sums a thread, half again as many shared loads) took 2.75 ms; fma.rn.f32x2 in place of single multiply-adds takes 2.4
-// cycles for two against 2.0 and gives the pipes nothing.
+// of k at a time (a small tile over eight chunks gives a few dozen rows as many blocks as a stream of the weights has).  A
+// lane of a warp's 8 x 4 holds TM x TN sums, rows 8 apart and columns side by side.  Both operands lie in shared memory as
+// rows of 32 k at a pitch of 36 floats, where the 16-byte loads of eight lanes meet no bank twice, and come through a ring of
+// cp.async stages that runs on across chunks and tiles, so only a block's first loads are waited for.
 template <int BM, int BN, int WK>
 struct F32Tile {
   static constexpr int ROWS = WK * (BM + BN);                       // rows of 32 k in a stage
   static constexpr int STAGE = ROWS * F32S_SEG;
-  static constexpr int PART = WK > 1 ? WK * BM * (BN + 4) : 0;      // chunk sums on their way to being added up
+  static constexpr int PART = WK * BM * (BN + 4);                   // chunk sums on their way to being added up
   static constexpr int STAGES = (3 * STAGE + PART) * 4 <= 220 * 1024 ? 3 : 2;
   static constexpr int SMEM = (STAGES * STAGE + PART) * 4;
 };
@@ -161,7 +156,7 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
                      const int* __restrict__ group_offsets, size_t w_group_stride) {
   using T = F32Tile<BM, BN, WK>;
   constexpr int TM = BM / WM / 8, TN = BN / WN / 4, STAGES = T::STAGES, THREADS = 32 * WM * WN * WK;
-  constexpr int SUMS = WK > 1 ? BM * BN / THREADS : 1;
+  constexpr int SUMS = BM * BN / THREADS;
   static_assert(TN % 4 == 0 && BM * BN % THREADS == 0 && T::ROWS * 8 % THREADS == 0, "whole vectors and equal shares");
   extern __shared__ __align__(16) float smem[];
   float* part = smem + STAGES * T::STAGE;
@@ -207,11 +202,11 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
     if (s < steps) issue(s);
     st_commit();
   }
-  float acc[TM][TN], total[WK > 1 ? 1 : TM][WK > 1 ? 1 : TN], sum[SUMS];
+  float acc[TM][TN], sum[SUMS];
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < TN; j++) acc[i][j] = total[WK > 1 ? 0 : i][WK > 1 ? 0 : j] = 0.f;
+    for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
 #pragma unroll
   for (int i = 0; i < SUMS; i++) sum[i] = 0.f;
   for (int s = 0; s < steps; s++) {
@@ -240,41 +235,215 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
       }
     }
     if ((s & 3) != 3) continue;
+    // WK chunks are done
+    const int round = (s >> 2) % rounds, tile = blockIdx.x + (s / (4 * rounds)) * gridDim.x;
+    const int m0 = row_begin + tile % tiles_m * BM, n0 = tile / tiles_m * BN;
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        store4(part + (wk * BM + wm * (BM / WM) + lm + 8 * i) * (BN + 4) + wn * (BN / WN) + ln * TN + j,
+               make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]));
+        acc[i][j] = acc[i][j + 1] = acc[i][j + 2] = acc[i][j + 3] = 0.f;
+      }
+    __syncthreads();      // the next write to `part` comes after the barriers of the stages between
+    const int c1 = min(WK, chunks - round * WK);
+#pragma unroll
+    for (int i = 0; i < SUMS; i++) {
+      const int e = tid + THREADS * i, m = e / BN, n = e % BN;
+      for (int c = 0; c < c1; c++) sum[i] += part[(c * BM + m) * (BN + 4) + n];
+      if (round == rounds - 1) {
+        if (m0 + m < row_end && n0 + n < N) {
+          float* c = C + (size_t)(m0 + m) * ldc + n0 + n;
+          *c = accumulate ? *c + sum[i] : sum[i];
+        }
+        sum[i] = 0.f;
+      }
+    }
+  }
+}
+
+// ---- more rows: tiles of pairs --------------------------------------------------------------------------
+// 256 threads, a tile of BM x BN, warps dealt as above (WK 1 for many rows; 4 chunks of k at a time where larger tiles would leave SMs
+// idle); a lane holds 8 x 8 sums.  Bound by the FMA pipes and what is issued beside them.  Single multiply-adds read three
+// registers an instruction, which the register ports do not bear at full rate (37 TFLOP/s of the pipes' 72 with 8 x 8 sums);
+// fma.rn.f32x2 does two an instruction and leaves every second issue slot to the loads.  Each half rounds like fmaf and goes
+// through its k in the same order, so the bits are the same.  A pair holds two rows of one k, side by side: rows (m, m + 1) times
+// columns (n, n + 1) make one pair product as they lie and one with the columns changed over, two moves for eight sums.  So
+// operands lie in shared memory by k, rows side by side, and must be turned on their way there: a thread takes 4 k of a row to
+// registers a stage ahead and stores them under four k.  (Turned by 4-byte cp.async instead, the copies took a third of
+// the time: 2.49 ms for 2,048 x 11,264 x 2,048, and 1.75 with them left out.)  Rows are XORed by their k / 4, so those stores meet
+// no bank twice; lanes of one row and of one column alternate, so a 16-byte load takes two passes over the banks and not
+// three or four; stores and loads are spread over the stage's products.  2,048 rows x 11,264 x 2,048: 2,530 -> 2,110 us
+// (45 TFLOP/s); 523 x 11,264 x 2,048 761 -> 635, x 6,144 480 -> 389; 523 x 2,048 x 5,632 437 -> 355; 1,000 x 1,000 x 1,000 86.5 -> 73.8.
+template <int BM, int BN, int WK>
+struct F32Pairs {
+  static constexpr int PITCH = BM + BN;                             // floats of one k: the tile's rows of A, then of W
+  static constexpr int STAGE = WK * 32 * PITCH;
+  static constexpr int PART = WK > 1 ? WK * BM * (BN + 4) : 0;
+  static constexpr int SMEM = (2 * STAGE + PART) * 4;
+};
+
+typedef unsigned long long f32pair;
+__device__ __forceinline__ f32pair f32_fma2(f32pair a, f32pair b, f32pair c) {
+  f32pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ float f32_lo(f32pair p) { return __uint_as_float((unsigned)p); }
+__device__ __forceinline__ float f32_hi(f32pair p) { return __uint_as_float((unsigned)(p >> 32)); }
+__device__ __forceinline__ f32pair f32_pair(float lo, float hi) {
+  return (f32pair)__float_as_uint(hi) << 32 | __float_as_uint(lo);
+}
+
+template <int BM, int BN, int WM, int WN, int WK, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN * WK, 1)
+gemm_f32_pairs_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                      int M, int N, int K, int lda, int ldc, int accumulate,
+                      const int* __restrict__ group_offsets, size_t w_group_stride) {
+  using T = F32Pairs<BM, BN, WK>;
+  constexpr int PITCH = T::PITCH, THREADS = 32 * WM * WN * WK, LOADS = WK * PITCH / 32;
+  constexpr int SUMS = WK > 1 ? BM * BN / THREADS : 1;
+  static_assert(BM == WM * 64 && BN == WN * 32 && THREADS == 256 && BM % 32 == 0, "8 x 8 sums a lane, 8 warps");
+  extern __shared__ __align__(16) float smem[];
+  float* part = smem + 2 * T::STAGE;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lm = (lane >> 1) & 7, ln = (lane & 1) | (lane >> 4) << 1;
+  const int wk = warp % WK, wn = warp / WK % WN, wm = warp / (WK * WN);
+  pdl_wait();
+  int row_begin = 0, row_end = M;
+  if (group_offsets) {
+    row_begin = group_offsets[blockIdx.z];
+    row_end = group_offsets[blockIdx.z + 1];
+    W += (size_t)blockIdx.z * w_group_stride;
+  }
+  // tiles in order of their rows first, so that blocks that run together share their weights
+  const int tiles_m = (row_end - row_begin + BM - 1) / BM, tiles = tiles_m * ((N + BN - 1) / BN);
+  const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int chunks = (K + F32_CHUNK - 1) / F32_CHUNK, rounds = (chunks + WK - 1) / WK;
+  const int steps = mine * rounds * 4;      // stages of 32 k: four to a chunk
+  if (steps <= 0) return;                   // a group without rows
+
+  // a thread brings 4 k of every 32nd row of the stage's operands
+  const int cv = lane & 7, cr = warp * 4 + (lane >> 3);
+  float4 held[LOADS];
+  struct From {
+    const float *a, *w;
+    int rows, cols, ks;      // how many rows of A, rows of W and k lie from this thread's first ones on
+  };
+  auto from = [&](int s) {
+    const int tile = blockIdx.x + (s / (4 * rounds)) * gridDim.x;
+    const int m0 = row_begin + tile % tiles_m * BM + cr, n0 = tile / tiles_m * BN + cr;
+    const int k0 = ((s >> 2) % rounds) * WK * F32_CHUNK + (s & 3) * 32 + cv * 4;
+    return From{A + (size_t)m0 * lda + k0, W + (size_t)n0 * K + k0, row_end - m0, N - n0, s < steps ? K - k0 : 0};
+  };
+  auto fetch = [&](const From& f, int l) {
+    const int c = l / (PITCH / 32), r = l % (PITCH / 32) * 32, k = f.ks - c * F32_CHUNK;
+    const bool in = r < BM ? r < f.rows : r - BM < f.cols;
+    const float* src = (r < BM ? f.a + (size_t)r * lda : f.w + (size_t)(r - BM) * K) + c * F32_CHUNK;
+    held[l] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC) {
+      if (in && k > 0) held[l] = load4(src);
+    } else {
+      if (in && k > 0) held[l].x = src[0];
+      if (in && k > 1) held[l].y = src[1];
+      if (in && k > 2) held[l].z = src[2];
+      if (in && k > 3) held[l].w = src[3];
+    }
+  };
+  auto put = [&](int s, int l) {
+    float* p = smem + (s & 1) * T::STAGE + (l / (PITCH / 32) * 32 + cv * 4) * PITCH + l % (PITCH / 32) * 32 + (cr ^ cv * 4);
+    p[0] = held[l].x;
+    p[PITCH] = held[l].y;
+    p[2 * PITCH] = held[l].z;
+    p[3 * PITCH] = held[l].w;
+  };
+  From next = from(0);
+#pragma unroll
+  for (int l = 0; l < LOADS; l++) fetch(next, l);
+#pragma unroll
+  for (int l = 0; l < LOADS; l++) put(0, l);
+  next = from(1);
+#pragma unroll
+  for (int l = 0; l < LOADS; l++) fetch(next, l);
+  // of rows (m, m + 1) and columns (n, n + 1): `same` holds (m, n) and (m + 1, n + 1), `cross` (m, n + 1) and (m + 1, n)
+  f32pair same[4][4], cross[4][4];
+  float total[WK > 1 ? 1 : 8][WK > 1 ? 1 : 8], sum[SUMS];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) same[i][j] = cross[i][j] = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) total[WK > 1 ? 0 : i][WK > 1 ? 0 : j] = 0.f;
+#pragma unroll
+  for (int i = 0; i < SUMS; i++) sum[i] = 0.f;
+  auto value = [&](int i, int j) {
+    const f32pair p = (i ^ j) & 1 ? cross[i >> 1][j >> 1] : same[i >> 1][j >> 1];
+    return i & 1 ? f32_hi(p) : f32_lo(p);
+  };
+  for (int s = 0; s < steps; s++) {
+    __syncthreads();      // stage s is there, and everyone is done with the one before it
+    next = from(s + 2);
+    const float* a = smem + (s & 1) * T::STAGE + wk * 32 * PITCH + wm * 64;
+    const float* w = smem + (s & 1) * T::STAGE + wk * 32 * PITCH + BM + wn * 32;
+#pragma unroll
+    for (int v = 0; v < 8; v++) {
+      const int am = (lm ^ v) * 4, w0n = (ln ^ v) * 4, w1n = w0n ^ 16;
+#pragma unroll
+      for (int k = v * 4; k < v * 4 + 4; k++) {
+        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(a + k * PITCH + am), a1 = *reinterpret_cast<const ulonglong2*>(a + k * PITCH + am + 32);
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(w + k * PITCH + w0n), w1 = *reinterpret_cast<const ulonglong2*>(w + k * PITCH + w1n);
+        const f32pair av[4] = {a0.x, a0.y, a1.x, a1.y}, wv[4] = {w0.x, w0.y, w1.x, w1.y};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const f32pair wx = f32_pair(f32_hi(wv[j]), f32_lo(wv[j]));
+#pragma unroll
+          for (int i = 0; i < 4; i++) same[i][j] = f32_fma2(av[i], wv[j], same[i][j]);
+#pragma unroll
+          for (int i = 0; i < 4; i++) cross[i][j] = f32_fma2(av[i], wx, cross[i][j]);
+        }
+      }
+      // a share of the next stage, and of the loads for the one after it (zeros past the last)
+#pragma unroll
+      for (int l = v * LOADS / 8; l < (v + 1) * LOADS / 8; l++) {
+        put(s + 1, l);
+        fetch(next, l);
+      }
+    }
+    if ((s & 3) != 3) continue;
     // a chunk (or WK of them) is done
     const int round = (s >> 2) % rounds, tile = blockIdx.x + (s / (4 * rounds)) * gridDim.x;
     const int m0 = row_begin + tile % tiles_m * BM, n0 = tile / tiles_m * BN;
     if (WK == 1) {
 #pragma unroll
-      for (int i = 0; i < TM; i++)
+      for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j++) {
-          total[WK > 1 ? 0 : i][WK > 1 ? 0 : j] += acc[i][j];
-          acc[i][j] = 0.f;
-        }
-      if (round < rounds - 1) continue;
+        for (int j = 0; j < 8; j++) total[WK > 1 ? 0 : i][WK > 1 ? 0 : j] += value(i, j);
+      if (round == rounds - 1) {
 #pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const int r = m0 + wm * (BM / WM) + lm + 8 * i;
+        for (int i = 0; i < 8; i++) {
+          const int r = m0 + wm * 64 + lm * 4 + (i & 3) + 32 * (i >> 2);
 #pragma unroll
-        for (int j = 0; j < TN; j++) {
-          const int n = n0 + wn * (BN / WN) + ln * TN + j;
-          float& t = total[WK > 1 ? 0 : i][WK > 1 ? 0 : j];
-          if (r < row_end && n < N) {
-            float* c = C + (size_t)r * ldc + n;
-            *c = accumulate ? *c + t : t;
+          for (int j = 0; j < 8; j++) {
+            const int n = n0 + wn * 32 + ln * 4 + (j & 3) + 16 * (j >> 2);
+            float& t = total[WK > 1 ? 0 : i][WK > 1 ? 0 : j];
+            if (r < row_end && n < N) {
+              float* c = C + (size_t)r * ldc + n;
+              *c = accumulate ? *c + t : t;
+            }
+            t = 0.f;
           }
-          t = 0.f;
         }
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < TM; i++)
+      for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j += 4) {
-          store4(part + (wk * BM + wm * (BM / WM) + lm + 8 * i) * (BN + 4) + wn * (BN / WN) + ln * TN + j,
-                 make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]));
-          acc[i][j] = acc[i][j + 1] = acc[i][j + 2] = acc[i][j + 3] = 0.f;
-        }
+        for (int j = 0; j < 8; j += 4)
+          store4(part + (wk * BM + wm * 64 + lm * 4 + (i & 3) + 32 * (i >> 2)) * (BN + 4) + wn * 32 + ln * 4 + 16 * (j >> 2),
+                 make_float4(value(i, j), value(i, j + 1), value(i, j + 2), value(i, j + 3)));
       __syncthreads();      // the next write to `part` comes after the barriers of the stages between
       const int c1 = min(WK, chunks - round * WK);
 #pragma unroll
@@ -290,6 +459,10 @@ gemm_f32_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const f
         }
       }
     }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) same[i][j] = cross[i][j] = 0;
   }
 }
 
@@ -407,20 +580,37 @@ static int launch_f32_tile(float* C, const float* A, const float* W, int M, int 
   return 0;
 }
 
+template <int BM, int BN, int WM, int WN, int WK, bool VEC>
+static int launch_f32_pairs(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldc, int accumulate,
+                           const int* group_offsets, int groups, size_t w_group_stride, cudaStream_t st) {
+  constexpr int smem = F32Pairs<BM, BN, WK>::SMEM;
+  constexpr auto kernel = gemm_f32_pairs_kernel<BM, BN, WM, WN, WK, VEC>;
+  const cudaError_t set = leb_allow_smem<kernel>();
+  LEB_REQUIRE(set == cudaSuccess, "leb_gemm_f32: %s", cudaGetErrorString(set));
+  const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, BN);
+  LEB_REQUIRE(tiles < (1ll << 24) && groups <= 65535, "leb_gemm_f32: too many tiles (%lld) or groups (%d)", tiles, groups);
+  const int sms = sm_count(), blocks = ceil_div((int)tiles, ceil_div((int)tiles, sms));
+  leb_launch(kernel, dim3(blocks, 1, groups), dim3(32 * WM * WN * WK), smem, st, C, A, W, M, N, K, lda, ldc, accumulate, group_offsets,
+             w_group_stride);
+  LEB_CHECK_LAUNCH("leb_gemm_f32");
+  return 0;
+}
+
 // Which kernel takes a product (0-4: tiles in the order below, F32_PLAIN, F32_STREAM): the one whose blocks take the SM with most of
 // them least, in nanoseconds measured on B200 (9 to 2,048 rows, 16 to 11,264 columns, K from 16 to 2,048; 4 to 64 groups): a
 // fixed part, and per block of an SM a part of its own and one per round, of `wk` chunks of k (the plain kernel: of 16 k).  Over 967
 // such sizes the choice takes 0.46 (up to 16 rows), 0.62 (more; 0.83 with broken vectors) and 0.56 (groups) of the time of blocks of
-// 64 x 64 throughout, and above 1.1 of it at ten small sizes (by 0.3 to 2.4 us).  Groups count as many equally large ones as can
+// 64 x 64 throughout, and above 1.1 of it at ten small sizes (by 0.3 to 2.4 us); the two larger tiles' figures were taken
+// again when they came to hold pairs (150 sizes of 17 to 2,048 rows: 0.91 of the time before).  Groups count as many equally large ones as can
 // have rows; blocks of groups without any cost their start.
 enum { F32_PLAIN = 5, F32_STREAM = 6 };
 struct F32Cost {
   int bm, bn, wk, fixed, block, round;
 };
 static int f32_choice(int M, int N, int K, int groups, bool vec, int sms) {      // groups: 0 for a product that is not grouped
-  static const F32Cost whole[5] = {{128, 128, 1, 0, 10500, 14600}, {64, 64, 4, 100, 1250, 18800}, {32, 32, 8, 1350, 0, 12200},
+  static const F32Cost whole[5] = {{128, 128, 1, 0, 8800, 12200}, {64, 64, 4, 6000, 600, 15800}, {32, 32, 8, 1350, 0, 12200},
                                    {64, 16, 8, 1400, 0, 12550}, {32, 16, 8, 1500, 0, 7600}};
-  static const F32Cost broken[5] = {{128, 128, 1, 0, 5000, 20500}, {64, 64, 4, 0, 1900, 22800}, {32, 32, 8, 1500, 1700, 13400},
+  static const F32Cost broken[5] = {{128, 128, 1, 0, 4200, 17100}, {64, 64, 4, 0, 1550, 18500}, {32, 32, 8, 1500, 1700, 13400},
                                     {64, 16, 8, 1100, 1900, 14500}, {32, 16, 8, 1500, 2400, 7700}};
   if (groups == 0 && M <= 8 && vec) return F32_STREAM;      // (measured up to 16 rows; up to 8 it is ahead or within 0.4 us everywhere)
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
@@ -472,13 +662,13 @@ LEB_API int leb_gemm_f32(float* C, const float* A, const float* W, int M, int N,
     LEB_CHECK_LAUNCH("leb_gemm_f32");
     return 0;
   }
-#define LEB_F32_TILE(BM, BN, WM, WN, WK)                                                                                     \
-  return vec ? launch_f32_tile<BM, BN, WM, WN, WK, true>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st) \
-             : launch_f32_tile<BM, BN, WM, WN, WK, false>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st)
-  if (pick == 0) LEB_F32_TILE(128, 128, 2, 4, 1);
-  if (pick == 1) LEB_F32_TILE(64, 64, 1, 2, 4);
-  if (pick == 2) LEB_F32_TILE(32, 32, 1, 2, 8);
-  if (pick == 3) LEB_F32_TILE(64, 16, 1, 1, 8);
-  LEB_F32_TILE(32, 16, 1, 1, 8);
+#define LEB_F32_TILE(KIND, BM, BN, WM, WN, WK)                                                                                \
+  return vec ? launch_f32_##KIND<BM, BN, WM, WN, WK, true>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st) \
+             : launch_f32_##KIND<BM, BN, WM, WN, WK, false>(C, A, W, M, N, K, lda, ldc, accumulate, group_offsets, groups, w_group_stride, st)
+  if (pick == 0) LEB_F32_TILE(pairs, 128, 128, 2, 4, 1);
+  if (pick == 1) LEB_F32_TILE(pairs, 64, 64, 1, 2, 4);
+  if (pick == 2) LEB_F32_TILE(tile, 32, 32, 1, 2, 8);
+  if (pick == 3) LEB_F32_TILE(tile, 64, 16, 1, 1, 8);
+  LEB_F32_TILE(tile, 32, 16, 1, 1, 8);
 #undef LEB_F32_TILE
 }
