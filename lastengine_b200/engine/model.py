@@ -44,20 +44,26 @@ class Model:
         self.stream_tables: dict[str, torch.Tensor] = {}
         self.stream_matrices: dict[str, torch.Tensor] = {}
         self.embedding_spec = self.embedding.cache_spec() if hasattr(self.embedding, "cache_spec") else None
-        # Products of a step may wait for one another on the host (kernels.product_chain).  The library's own parts touch their
-        # results through its kernels alone, which launch what waits first; of parts from elsewhere that is not known.
-        own = __package__.split(".")[0] + "."
-        self.chains = all(type(p).__module__.startswith(own) for top in (*self.blocks, self.embedding, self.final_norm, self.head)
-                          for p in self._parts_in(top))
+        # Products of a step may wait for one another on the host (kernels.product_chain) in a model that is built of the library's
+        # own parts throughout.  What is put into a built model, or wrapped there, is judged when it is called (kernels.run_part).
+        own = __package__.partition(".")[0]
+        self.chains = all(type(p).__module__.partition(".")[0] == own
+                          for p in self._objects_in([*self.blocks, self.embedding, self.final_norm, self.head], {}))
 
     @classmethod
-    def _parts_in(cls, part):
-        """A part and the parts it holds (attributes, and members of lists, that compute: they have `forward` or `apply`)."""
-        yield part
-        for v in vars(part).values():
-            for p in v if isinstance(v, (list, tuple)) else (v,):
-                if not isinstance(p, (torch.Tensor, type)) and (hasattr(p, "forward") or hasattr(p, "apply")):
-                    yield from cls._parts_in(p)
+    def _objects_in(cls, p, seen: dict):
+        """What can be reached from `p` through attributes and members of containers and is no plain data, whatever its
+        interface (a gate and a position encoding have no `forward`)."""
+        if isinstance(p, (list, tuple, set, frozenset, dict)):
+            held = p.values() if isinstance(p, dict) else p
+        elif type(p).__module__.partition(".")[0] in ("builtins", "torch", "numpy") or id(p) in seen:
+            return
+        else:
+            seen[id(p)] = p
+            yield p
+            held = getattr(p, "__dict__", {}).values()
+        for q in held:
+            yield from cls._objects_in(q, seen)
 
     # ---- tensors ------------------------------------------------------------------------
     def named_parts(self) -> list[tuple[str, object]]:
@@ -128,9 +134,9 @@ class Model:
         M, D = batch.n_rows, self.hidden_size
         x = ws.get("model.x", (M, D), torch.float32)
         if self.embedding_spec is not None:
-            self.embedding.forward(x, batch.tokens, batch=batch, cache=cache.view(EMBEDDING_ENTRY, True, batch.tables))
+            kernels.run_part(self.embedding.forward, x, batch.tokens, batch=batch, cache=cache.view(EMBEDDING_ENTRY, True, batch.tables))
         else:
-            self.embedding.forward(x, batch.tokens, batch=batch)
+            kernels.run_part(self.embedding.forward, x, batch.tokens, batch=batch)
         x0 = pair = None
         if self.keeps_embedding:      # the embedding output is added to the stream again later
             x0 = ws.get("model.x0", (M, D), torch.float32)
@@ -161,14 +167,14 @@ class Model:
             env.next_block_norm = after.first_reader() if hasattr(after, "first_reader") and (i + 1) not in self.stream_adds \
                 else None
             if pending is not None:
-                pending = block.forward(x, batch, view, env, pending=pending)
+                pending = kernels.run_part(block.forward, x, batch, view, env, pending=pending)
             else:
-                pending = block.forward(x, batch, view, env)
+                pending = kernels.run_part(block.forward, x, batch, view, env)
         env.next_block_norm = None
         R = batch.n_logit_rows
         logits = ws.get("model.logits", (R, self.vocab_size), torch.float32)
         if R:
             xn = ws.get("model.xn", (R, D), env.dtype)
-            self.final_norm.forward(xn, x, rows=batch.logit_rows)
-            self.head.forward(logits, xn)
+            kernels.run_part(self.final_norm.forward, xn, x, rows=batch.logit_rows)
+            kernels.run_part(self.head.forward, logits, xn)
         return logits

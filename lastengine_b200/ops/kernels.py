@@ -11,6 +11,7 @@ import contextlib
 import ctypes
 import functools
 import threading
+import types
 from ctypes import c_float, c_int, c_size_t, c_void_p
 
 import torch
@@ -69,12 +70,15 @@ def product_chain(workspace, rows: int, dtype: torch.dtype):
     """Inside, consecutive products of a step of SMALL_M + 1 to SKINNY_M bfloat16 rows (dense ones, the conv mixer's decode step among them)
     wait for one another in the host's memory and run as ONE resident kernel (csrc/product_chain.cu) as soon as
     anything else is launched through this module, and at the end.  Nothing but calls of this module may launch work that
-    touches the products' operands in between, as is so inside a model's forward pass.  `workspace` owns the barrier's words:
-    steps that share it run one after the other."""
+    touches the products' operands in between; a model's forward pass calls its parts through `run_part`, which sees to that.
+    `workspace` owns the barrier's words: steps that share it run one after the other."""
     c = _chain
     if dtype != torch.bfloat16 or not SMALL_M < rows <= SKINNY_M or c.open or _library().leb_chain_clusters(rows) <= 0:
         yield
+        if c.ops:            # inside another chain: nothing waits beyond this one's end
+            c.flush()
         return
+    outer = c.sync, c.device, c.rows      # of a chain that `run_part` holds closed meanwhile
     c.sync = workspace.zeroed("chain.sync", 2)
     c.device = workspace.device
     c.rows, c.open = rows, True
@@ -84,9 +88,39 @@ def product_chain(workspace, rows: int, dtype: torch.dtype):
             c.flush()
     finally:
         c.open = False
+        c.sync, c.device, c.rows = outer
         if c.ops:            # the step raised: what waited is not run
             c.ops = []
             _library().leb_chain_drop()
+
+
+_PACKAGE = __name__.partition(".")[0] + "."
+
+
+def is_own(method) -> bool:
+    """Whether `method` is a bound method that a class of this package has from code of this package."""
+    return (type(method) is types.MethodType and type(method.__self__).__module__.startswith(_PACKAGE)
+            and getattr(method.__func__, "__globals__", _NOWHERE)["__name__"].startswith(_PACKAGE))
+
+
+_NOWHERE = {"__name__": ""}      # a callable that is no function
+
+
+def run_part(method, *args, **kwargs):
+    """Calls a part's method: every call of a part inside a forward pass goes through here.  The library's own parts touch their
+    operands through this module alone, which launches what waits in a chain first; other code (a part registered from
+    elsewhere, a method wrapped or replaced on a class or an object) may use torch on them, so whatever waits is launched
+    before it runs, and its own products are launched at their call.  Judged at every call: parts change after a model is built."""
+    c = _chain
+    if not c.open or is_own(method):
+        return method(*args, **kwargs)
+    if c.ops:
+        c.flush()
+    c.open = False
+    try:
+        return method(*args, **kwargs)
+    finally:
+        c.open = True
 
 
 def _chained(out, x, w, M, N, K, epilogue, scale_args, emit_args, alone, conv=(None, None, None, None, None, 0)) -> bool:

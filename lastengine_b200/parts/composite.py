@@ -115,8 +115,8 @@ class ParallelMixers(Mixer):
             kl["proj"], kr["proj"] = proj[:, : self.n_left], proj[:, self.n_left:]
         if bias is not None:
             kl["add_output_bias"] = False
-        self.left.forward(h, y1, False, batch, self._view(cache, 0), env, **kl)
-        self.right.forward(h, y2, False, batch, self._view(cache, 1), env, **kr)
+        kernels.run_part(self.left.forward, h, y1, False, batch, self._view(cache, 0), env, **kl)
+        kernels.run_part(self.right.forward, h, y2, False, batch, self._view(cache, 1), env, **kr)
         if getattr(self.right, "output_bias", lambda: None)() is not None:
             raise NotImplementedError("an output bias on the right-hand mixer")
         return y1, self.a, y2, self.b, bias

@@ -1,0 +1,86 @@
+"""The resident kernel of consecutive products (csrc/product_chain.cu) and the host side that lets them wait for one another."""
+import contextlib
+
+import numpy as np
+import pytest
+import torch
+
+import harness as H
+from zekivik_configs import ALL as ZEKIVIK
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def K():
+    from lastengine_b200.ops import kernels
+    return kernels
+
+
+# ---- code from elsewhere inside a step ---------------------------------------------------------------------
+def torch_gate(block_gate, kept):
+    """The sigmoid gate in plain torch, with a copy of what it read."""
+    from lastengine_b200.parts.gate import SigmoidGate
+
+    class TorchGate(SigmoidGate):
+        def add_gated(self, x, y, h, env, z=None, next_norm=None, h_out=None):
+            z = h.float() @ self.w.float().T if z is None else z.float()
+            kept.append(y.clone())
+            x += y * torch.sigmoid(z + self.b if self.b is not None else z)
+            if h_out is not None:
+                next_norm.forward(h_out, x)
+    block_gate.__class__ = TorchGate
+
+
+def wrapped(part, kept):
+    """A part's forward as a caller wraps it to look at what goes in and comes out."""
+    own = part.forward
+
+    def forward(h, out, *a, **k):
+        kept.append(h.clone())
+        own(h, out, *a, **k)
+        kept.append(out.clone())
+    part.forward = forward
+
+
+@pytest.mark.parametrize("rows", [17, 64])
+@pytest.mark.parametrize("what", ["gate", "wrapped"])
+def test_code_from_elsewhere_reads_finished_products(what, rows, tmp_path, monkeypatch):
+    """A gate in plain torch, and a feed-forward wrapped to keep copies of its operands, put into a built model: in steps whose
+    products wait for one another they read what those products give.  Against the same model with every product launched
+    at its call; the step before it had other tokens, so that a buffer read too early holds other numbers.  Whole rows agree to
+    the rounding of a bfloat16 model (K is cut differently in a chain)."""
+    from lastengine_b200 import Engine
+    from lastengine_b200.weights import write_model_dir
+    k = K()
+    name = next(n for n, c in ZEKIVIK.items() if sum(lay["mlp"] is not None for lay in c["layers"]) > 1)
+    cfg = ZEKIVIK[name]
+    d = write_model_dir(cfg, str(tmp_path), seed=3, norm_init="random")
+    rng = np.random.default_rng(rows)
+    prompts = [rng.integers(0, cfg["vocab"], size=rows).tolist() for _ in range(2)]
+
+    def run():
+        eng = Engine.from_pretrained(d, dtype="bfloat16", max_tokens=512)
+        H.run_whole(eng, prompts[0])       # (a first step: matrices that a gate gives to a mixer have moved)
+        kept: list = []
+        for block in eng.model.blocks:
+            if what == "wrapped":
+                for part in (block.mixer, block.ffn):
+                    if part is not None:
+                        wrapped(part, kept)
+            else:
+                for gate in (block.mixer_gate, block.ffn_gate):
+                    if gate is not None:
+                        torch_gate(gate, kept)
+        H.run_whole(eng, prompts[0])
+        kept.clear()
+        logits = H.run_whole(eng, prompts[1])
+        k.check_device_status()
+        return logits, [t.float().cpu() for t in kept]
+    got = run()
+    monkeypatch.setattr(k, "product_chain", lambda *a: contextlib.nullcontext())
+    want = run()
+    assert len(got[1]) == len(want[1]) >= 2
+    for a, b in zip(got[1] + [got[0]], want[1] + [want[0]]):
+        e = (a - b).abs().amax(-1) / b.abs().max()
+        assert e.median() < H.TOL_BF16 / 3 and torch.quantile(e, 0.9) < 2 * H.TOL_BF16
