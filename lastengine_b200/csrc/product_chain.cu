@@ -450,20 +450,17 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
     for (int o = 0; o < n_ops && !gave_up; o++) {
       const Share sl = share_of(o);
       for (int t = sl.first; t < sl.n_tiles && !gave_up; t += n_clusters) {
-        if (sl.n == 0) {
-          q += H;
-          continue;
-        }
-        bool ok = pc_wait<false>(b_acc_full + 8 * (r & 1), (r >> 1) & 1, abort_flag);
+        bool ok = sl.n == 0 || pc_wait<false>(b_acc_full + 8 * (r & 1), (r >> 1) & 1, abort_flag);
 #pragma unroll 1
         for (int h = 0; h < H; h++, q++) {
           const int rb = q % RB;
-          // the owners have taken what lay in this buffer
+          // the owners have taken what lay in this buffer (a block without k-blocks waits too and sends nothing: a wait tells only odd
+          // phases from even ones, so a phase that is passed by would be taken for the one after the next)
           if (ok && q >= RB) ok = pc_wait<true>(b_credit + 8 * rb, ((q / RB) - 1) & 1, abort_flag);
           ok = __all_sync(0xffffffffu, ok) != 0;
           if (!ok) break;
           tc_fence_after();
-          if (quad * 32 < sl.rows) {
+          if (sl.n > 0 && quad * 32 < sl.rows) {
             const uint32_t base = a_r + rb * RECV + (uint32_t)rank * (RH * 512) + (uint32_t)(quad * 32 + lane) * 16, bar = b_recv + 8 * rb;
             const uint32_t src = tmem_acc + (r & 1) * ACC_COLS + ((uint32_t)(quad * 32) << 16) + h * RH;
 #pragma unroll 1
@@ -482,6 +479,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
           }
         }
         if (!ok) { gave_up = 46; break; }
+        if (sl.n == 0) continue;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) pc_arrive(b_acc_empty + 8 * (r & 1));

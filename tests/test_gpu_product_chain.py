@@ -84,3 +84,40 @@ def test_code_from_elsewhere_reads_finished_products(what, rows, tmp_path, monke
     for a, b in zip(got[1] + [got[0]], want[1] + [want[0]]):
         e = (a - b).abs().amax(-1) / b.abs().max()
         assert e.median() < H.TOL_BF16 / 3 and torch.quantile(e, 0.9) < 2 * H.TOL_BF16
+
+
+# ---- the kernel --------------------------------------------------------------------------------------------
+def gen(*shape, seed, scale=1.0, dtype=torch.bfloat16):
+    g = torch.Generator().manual_seed(seed)
+    return (scale * torch.randn(*shape, generator=g)).to(dtype).to(DEV)
+
+
+def workspace():
+    from lastengine_b200.engine.workspace import Workspace
+    return Workspace(torch.device(DEV))
+
+
+@pytest.mark.parametrize("M", [17, 64, 65, 128])
+def test_slices_without_k_between_others(M):
+    """Products of so few k that some blocks of a cluster have none (up to 192, 257 to 384, 513 to 576), of several tiles a
+    cluster, between products of many k: each against 64 bits (up to K bfloat16 terms in float), and the same bits every time."""
+    k, ws = K(), workspace()
+    inner = (2048, 64, 192, 2048, 320, 576, 128, 2048, 64, 2048)
+    outer = (64, 192, 2048, 320, 576, 128, 2048, 64, 2048, 12672)
+    W = [gen(n, kk, seed=i, scale=kk ** -0.5) for i, (n, kk) in enumerate(zip(outer, inner))]
+    h = gen(M, inner[0], seed=50)
+    first = None
+    for _ in range(20):
+        outs, x = [], h
+        with k.product_chain(ws, M, torch.bfloat16):
+            for i, w in enumerate(W):
+                outs.append(torch.empty(M, w.shape[0], device=DEV, dtype=torch.float32 if i == len(W) - 1 else torch.bfloat16))
+                k.linear(outs[-1], x, w)
+                x = outs[-1]
+        first = first or outs
+        assert all(torch.equal(a, b) for a, b in zip(first, outs))
+    k.check_device_status()
+    for x, w, y in zip([h, *first], W, first):
+        want = x.double() @ w.double().T
+        tol = 2 ** -8 + 2e-5 if y.dtype == torch.bfloat16 else 2e-5
+        assert float((y.double() - want).abs().max() / want.abs().max()) < tol
