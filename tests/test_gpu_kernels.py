@@ -1055,11 +1055,13 @@ def test_moe_router_gives_a_row_the_same_bits_whatever_the_step(dtype, E, k, D):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,k,E,D", [(1, 1, 1, 8), (1, 4, 32, 2048), (8, 4, 32, 2048), (64, 4, 32, 520), (51, 5, 256, 4100), (37, 2, 3, 72),
+                                     (1, 1, 256, 64), (4, 8, 256, 2048), (33, 1, 256, 72), (11, 1, 32, 64), (3, 4, 32, 64),
                                      (65, 4, 32, 64), (9, 3, 8, 36)])
 def test_moe_align_gather(dtype, M, k, E, D):
     """The expert-sorted order and the rows in it by one launch (up to 256 pairs, rows of whole 16-byte pieces; the last two
     sizes are beyond): what the sort and the gather give, with and without weights on the rows; fewer pairs than experts,
-    experts without rows, more pieces than threads."""
+    experts without rows, more pieces than threads; offsets counted by a thread each (up to 32 pairs for 256 experts, 11 for 32)
+    and by whole blocks."""
     g = torch.Generator().manual_seed(7 * M + k)
     ids = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(M)]).to(torch.int32).to(DEV)
     h, w = gen(M, D, seed=90, dtype=dtype).to(DEV), gen(M, k, seed=91).to(DEV)
