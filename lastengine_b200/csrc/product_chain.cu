@@ -10,10 +10,14 @@
 //
 // Split: a cluster of 4 blocks takes tiles of up to 128 weight rows; within the cluster block r takes slice r of K.  W is
 // the 128-row operand of tcgen05.mma, the activations (padded to MP rows) the narrow one, the accumulator the
-// transposed tile C^T [128 n][MP m] in tensor memory, two of them in turn.  A slice's partial tile does not go to
-// memory: the rows of A are dealt to the 4 blocks (MP / 4 each, their owners), and a block sends each owner its share
-// of the partial tile into the owner's shared memory (st.async, counted by the owner's mbarrier).  The owner adds the
-// slices in slice order and applies the epilogue.  So a result does not depend on timing, nor on the other rows.
+// transposed tile C^T[128 n][MP m] in tensor memory.  An accumulator loses in proportion to the products added up in it (2,048 x 5,632
+// with a slice of 22 k-blocks in one: 1.4e-6 from 64 bits; the product alone, in slices of ten: 5.9e-7), so it takes no more
+// k-blocks than a slice of the product alone, the next ones go to the next accumulator of a ring, and a block adds a tile's
+// accumulators up in float (4.4e-7; 0.22 to 1.00 of the error alone over 19 sizes of 64 to 14,336 columns and K from 64 to
+// 17,408).  Those before the last are read while that one fills, where the registers hold them for all owners (up to 64 rows).
+// A slice's partial tile does not go to memory: the rows of A are dealt to the 4 blocks (MP / 4 each, their owners), and a block
+// sends each owner its share of the partial tile into the owner's shared memory (st.async, counted by the owner's mbarrier).  The
+// owner adds the slices in slice order and applies the epilogue.  So a result does not depend on timing, nor on the other rows.
 //
 // Epilogues as in gemm_bf16_stream.cu: 0 store (with an activation), 1 add into float C (leaving the next norm's
 // half), 2 gated activation over interleaved weight rows, 3 the one-token gated convolution (a tile is then the B, C
@@ -69,7 +73,7 @@ struct __align__(64) ChainMaps {
 // whole warp and stays in uniform registers.
 struct __align__(16) ChainGeo {
   int blocks, n_tiles, rows, conv_width;      // k-blocks of 64 in K; tiles; weight rows of a tile; channels of a convolution (0: none)
-  int per, skip, arrivals, unused;            // k-blocks of a block's slice; tiles dealt before this product, modulo the clusters; blocks that arrive at its end
+  int per, skip, arrivals, run;               // k-blocks of a block's slice; tiles dealt before this product, modulo the clusters; blocks that arrive at its end; k-blocks added up in one accumulator
 };
 struct __align__(64) ChainArgs {
   ChainMaps map[PC_MAX_OPS];
@@ -134,6 +138,28 @@ template <bool CLUSTER>
 __device__ __forceinline__ bool pc_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return pc_passed<CLUSTER>(bar, parity) || pc_wait_long<CLUSTER>(bar, parity, abort_flag);
 }
+// N columns of a warp's 32 lanes of tensor memory.
+template <int N>
+__device__ __forceinline__ void pc_tmem_read(uint32_t* v, uint32_t src) {
+  if (N == 16)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8 % N]), "=r"(v[9 % N]), "=r"(v[10 % N]), "=r"(v[11 % N]), "=r"(v[12 % N]), "=r"(v[13 % N]), "=r"(v[14 % N]), "=r"(v[15 % N])
+                 : "r"(src));
+  else
+#pragma unroll
+    for (int c = 0; c < N; c += 4)
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3])
+                   : "r"(src + c));
+}
+// What was read is used after the wait, and not moved before it.
+template <int N>
+__device__ __forceinline__ void pc_tmem_there(uint32_t* v) {
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < N; c++) asm volatile("" : "+r"(v[c]));
+}
 // By all lanes of a warp.
 __device__ __forceinline__ bool pc_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (__all_sync(0xffffffffu, pc_passed<false>(bar, parity))) return true;
@@ -192,28 +218,29 @@ __device__ __noinline__ void pc_act_call(float* z, int act) {
   for (int e = 0; e < 4; e++) z[e] = plain_act(z[e], act);
 }
 
-// By MP: weight slots of 16 KB, stages of two k-blocks of activations (MP x 256 bytes), parts in which a partial tile is exchanged
+// By MP: accumulators in tensor memory, weight slots of 16 KB, stages of two k-blocks of activations (MP x 256 bytes), parts in which a partial tile is exchanged
 // (an owner's first rows, then its last), buffers for such a part of the cluster's partial tiles (MP x 512 / parts bytes).
 template <int MP> struct ChainRing;
-template <> struct ChainRing<32> { static constexpr int NW = 9, NX = 4, H = 1, RB = 2; };
-template <> struct ChainRing<64> { static constexpr int NW = 7, NX = 2, H = 1, RB = 2; };
-template <> struct ChainRing<96> { static constexpr int NW = 7, NX = 2, H = 2, RB = 2; };
-template <> struct ChainRing<128> { static constexpr int NW = 5, NX = 2, H = 2, RB = 2; };
+template <> struct ChainRing<32> { static constexpr int NACC = 8, NW = 9, NX = 4, H = 1, RB = 2; };
+template <> struct ChainRing<64> { static constexpr int NACC = 8, NW = 7, NX = 2, H = 1, RB = 2; };
+template <> struct ChainRing<96> { static constexpr int NACC = 4, NW = 7, NX = 2, H = 2, RB = 2; };
+template <> struct ChainRing<128> { static constexpr int NACC = 4, NW = 5, NX = 2, H = 2, RB = 2; };
 
 template <int MP>
 static constexpr size_t chain_smem() {
   typedef ChainRing<MP> Ring;
   return (size_t)Ring::NW * PC_SLOT + (size_t)Ring::NX * MP * 256 + (size_t)Ring::RB * MP * 512 / Ring::H + 1024 /* alignment */ +
-         sizeof(ChainOp) * PC_MAX_OPS + 8 * (2 * PC_STAGES + 2 * Ring::NX + 4 + 3 * Ring::RB) + 4 * (MP / 4) * 2 + 80;
+         sizeof(ChainOp) * PC_MAX_OPS + 8 * (2 * PC_STAGES + 2 * Ring::NX + 2 * Ring::NACC + 3 * Ring::RB) + 4 * (MP / 4) * 2 + 80;
 }
 
 template <int MP>
 __global__ void __launch_bounds__(PC_THREADS, 1)
 product_chain_kernel(const __grid_constant__ ChainArgs args) {
   typedef ChainRing<MP> Ring;
-  constexpr int NW = Ring::NW, NX = Ring::NX, H = Ring::H, RB = Ring::RB, R = MP / PC_CLUSTER, RH = R / H;
+  constexpr int NACC = Ring::NACC, NW = Ring::NW, NX = Ring::NX, H = Ring::H, RB = Ring::RB, R = MP / PC_CLUSTER, RH = R / H;
+  constexpr bool EARLY = MP <= 64;
   constexpr int X_BYTES = MP * 128, RECV = MP * 512 / H;     // RECV: 4 slices of [RH / 4][128][4] floats
-  constexpr uint32_t ACC_COLS = MP <= 32 ? 32 : (MP <= 64 ? 64 : 128), TMEM_COLS = 2 * ACC_COLS;
+  constexpr uint32_t ACC_COLS = MP <= 32 ? 32 : (MP <= 64 ? 64 : 128), TMEM_COLS = NACC * ACC_COLS;
   extern __shared__ uint8_t smem_raw[];
   // the same offset in every block of the cluster (addresses of peers' buffers are formed from this block's)
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -226,8 +253,8 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
   uint64_t* xfull = wempty + PC_STAGES;
   uint64_t* xempty = xfull + NX;
   uint64_t* acc_full = xempty + NX;
-  uint64_t* acc_empty = acc_full + 2;
-  uint64_t* recv_full = acc_empty + 2;
+  uint64_t* acc_empty = acc_full + NACC;
+  uint64_t* recv_full = acc_empty + NACC;
   uint64_t* credit = recv_full + RB;
   uint64_t* taken = credit + RB;
   float* row_scale = (float*)(((uintptr_t)(taken + RB) + 15) & ~(uintptr_t)15);     // [R]
@@ -255,7 +282,7 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
       mbar_init(&xfull[s], 1);
       mbar_init(&xempty[s], 1);
     }
-    for (int s = 0; s < 2; s++) {
+    for (int s = 0; s < NACC; s++) {
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_empty[s], 4);
     }
@@ -385,41 +412,68 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
     pdl_wait();
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MP >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     const uint64_t w_desc = make_desc(a_w), x_desc = make_desc(a_x);
-    int slot = 0, x = 0, xph = 0, r = 0;
-    unsigned stage = 0;
+    int slot = 0, x = 0, xph = 0;
+    unsigned stage = 0, run = 0;           // run: accumulators filled
     for (int o = 0; o < n_ops && !gave_up; o++) {
       const Share sl = share_of(o);
-      const int n_tiles = sl.n_tiles, rows = sl.rows;
+      const int n_tiles = sl.n_tiles, rows = sl.rows, most = args.geo[o].run;
       if (sl.n == 0) continue;
       const bool once = sl.n <= 2 * NX;
       const int x0 = x, xph0 = xph;
-      for (int t = sl.first; t < n_tiles && !gave_up; t += n_clusters, r++) {
-        const uint32_t acc = tmem_acc + (r & 1) * ACC_COLS;
+      for (int t = sl.first; t < n_tiles && !gave_up; t += n_clusters) {
         const bool first = !once || t == sl.first, last = !once || t + n_clusters >= n_tiles;    // who waits for, and who frees, a stage
         if (!first) x = x0, xph = xph0;
-        if (!pc_wait_warp(b_acc_empty + 8 * (r & 1), ((r >> 1) & 1) ^ 1, abort_flag)) { gave_up = 44; break; }
-        for (int kb = 0; kb < sl.n; kb += 2) {
+        int left = 0;                      // k-blocks that the accumulator still takes
+        for (int kb = 0; kb < sl.n && !gave_up; kb += 2) {
+          const int here = min(2, sl.n - kb);
+          const int slot2 = slot + 1 >= NW ? 0 : slot + 1;
+          const uint64_t da = w_desc + (uint64_t)(slot * (PC_SLOT / 16)), db = x_desc + (uint64_t)(2 * x * (X_BYTES / 16));
+          const uint64_t da2 = rows > 64 ? w_desc + (uint64_t)(slot2 * (PC_SLOT / 16)) : da + (uint64_t)(rows * 8);
+          const uint32_t begins = left == 0;
+          if (begins) {
+            if (!pc_wait_warp(b_acc_empty + 8 * (run % NACC), ((run / NACC) & 1) ^ 1, abort_flag)) { gave_up = 44; break; }
+            left = most;
+          }
+          const bool apart = left < here;      // the accumulator ends between the stage's k-blocks
+          const bool ends = left <= here || kb + 2 >= sl.n;
+          const uint32_t acc = tmem_acc + (run % NACC) * ACC_COLS, full = b_acc_full + 8 * (run % NACC), empty = b_wempty + 8 * (stage % PC_STAGES);
           if (first && !pc_wait_warp(b_xfull + 8 * x, xph, abort_flag)) { gave_up = 45; break; }
           if (!pc_wait_warp(b_wfull + 8 * (stage % PC_STAGES), (stage / PC_STAGES) & 1, abort_flag)) { gave_up = 45; break; }
           tc_fence_after();
-          const int here = min(2, sl.n - kb);
-          const int slot2 = slot + 1 >= NW ? 0 : slot + 1;
           if (elect_lane()) {
-            const uint64_t da = w_desc + (uint64_t)(slot * (PC_SLOT / 16)), db = x_desc + (uint64_t)(2 * x * (X_BYTES / 16));
 #pragma unroll
             for (int k = 0; k < TC_BK / 16; k++)
-              umma_bf16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-            if (here == 2) {
-              const uint64_t da2 = rows > 64 ? w_desc + (uint64_t)(slot2 * (PC_SLOT / 16)) : da + (uint64_t)(rows * 8);
+              umma_bf16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, !begins || k != 0);
+            if (here == 2 && !apart) {
 #pragma unroll
               for (int k = 0; k < TC_BK / 16; k++)
                 umma_bf16(acc, da2 + (uint64_t)(k * 2), db + (uint64_t)(X_BYTES / 16 + k * 2), idesc, 1);
             }
-            pc_commit(b_wempty + 8 * (stage % PC_STAGES));
-            if (last) pc_commit(b_xempty + 8 * x);
-            if (kb + 2 >= sl.n) pc_commit(b_acc_full + 8 * (r & 1));
+            if (!apart) {
+              pc_commit(empty);
+              if (last) pc_commit(b_xempty + 8 * x);
+            }
+            if (ends) pc_commit(full);
           }
           __syncwarp();
+          left -= here;
+          if (ends) left = 0, run++;
+          if (apart) {      // the stage's second k-block is the next accumulator's first
+            if (!pc_wait_warp(b_acc_empty + 8 * (run % NACC), ((run / NACC) & 1) ^ 1, abort_flag)) { gave_up = 44; break; }
+            tc_fence_after();
+            const bool whole = most == 1 || kb + 2 >= sl.n;      // it holds no other
+            if (elect_lane()) {
+#pragma unroll
+              for (int k = 0; k < TC_BK / 16; k++)
+                umma_bf16(tmem_acc + (run % NACC) * ACC_COLS, da2 + (uint64_t)(k * 2), db + (uint64_t)(X_BYTES / 16 + k * 2), idesc, k != 0);
+              pc_commit(empty);
+              if (last) pc_commit(b_xempty + 8 * x);
+              if (whole) pc_commit(b_acc_full + 8 * (run % NACC));
+            }
+            __syncwarp();
+            left = whole ? 0 : most - 1;
+            if (whole) run++;
+          }
           slot += slots_of(rows, here);
           if (slot >= NW) slot -= NW;
           stage++;
@@ -446,11 +500,43 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
     // the partial tile from tensor memory to the rows' owners; a thread holds one weight row, all activation rows
     pdl_wait();
     const int quad = warp & 3;
-    int r = 0, q = 0;
+    int q = 0;
+    unsigned run = 0;
     for (int o = 0; o < n_ops && !gave_up; o++) {
       const Share sl = share_of(o);
-      for (int t = sl.first; t < sl.n_tiles && !gave_up; t += n_clusters) {
-        bool ok = sl.n == 0 || pc_wait<false>(b_acc_full + 8 * (r & 1), (r >> 1) & 1, abort_flag);
+      int runs = 0;                        // accumulators of a tile
+      for (int k = 0; k < sl.n; k += args.geo[o].run) runs++;
+      for (int t = sl.first; t < sl.n_tiles && !gave_up; t += n_clusters, run += runs) {
+        bool ok = true;
+        const uint32_t src = tmem_acc + ((uint32_t)(quad * 32) << 16);
+        const bool has = sl.n > 0 && quad * 32 < sl.rows;
+        // what the accumulators before the last hold is added up while that one is filled, for all owners, where the registers suffice
+        uint32_t sum[EARLY ? PC_CLUSTER : 1][RH];
+        for (int j = 0; j < runs - 1 && ok; j++) {
+          ok = pc_wait<false>(b_acc_full + 8 * ((run + j) % NACC), ((run + j) / NACC) & 1, abort_flag);
+          if (EARLY && has) {
+            ok = __all_sync(0xffffffffu, ok) != 0;
+            if (!ok) break;
+            tc_fence_after();
+            if (j == 0) {
+#pragma unroll
+              for (int to = 0; to < (EARLY ? PC_CLUSTER : 1); to++) pc_tmem_read<RH>(sum[to], src + (run % NACC) * ACC_COLS + to * R);
+#pragma unroll
+              for (int to = 0; to < (EARLY ? PC_CLUSTER : 1); to++) pc_tmem_there<RH>(sum[to]);
+            } else {
+#pragma unroll
+              for (int to = 0; to < (EARLY ? PC_CLUSTER : 1); to++) {
+                uint32_t w[RH];
+                pc_tmem_read<RH>(w, src + ((run + j) % NACC) * ACC_COLS + to * R);
+                pc_tmem_there<RH>(w);
+#pragma unroll
+                for (int c = 0; c < RH; c++) sum[to][c] = __float_as_uint(__uint_as_float(sum[to][c]) + __uint_as_float(w[c]));
+              }
+            }
+          }
+        }
+        const uint32_t final = run + max(runs - 1, 0);
+        if (runs > 0 && ok) ok = pc_wait<false>(b_acc_full + 8 * (final % NACC), (final / NACC) & 1, abort_flag);
 #pragma unroll 1
         for (int h = 0; h < H; h++, q++) {
           const int rb = q % RB;
@@ -460,30 +546,50 @@ product_chain_kernel(const __grid_constant__ ChainArgs args) {
           ok = __all_sync(0xffffffffu, ok) != 0;
           if (!ok) break;
           tc_fence_after();
-          if (sl.n > 0 && quad * 32 < sl.rows) {
+          if (has) {
             const uint32_t base = a_r + rb * RECV + (uint32_t)rank * (RH * 512) + (uint32_t)(quad * 32 + lane) * 16, bar = b_recv + 8 * rb;
-            const uint32_t src = tmem_acc + (r & 1) * ACC_COLS + ((uint32_t)(quad * 32) << 16) + h * RH;
-#pragma unroll 1
-            for (int to = 0; to < n_owners; to++) {
-              uint32_t v[RH];
-#pragma unroll
-              for (int c = 0; c < RH; c += 4)
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3])
-                             : "r"(src + to * R + c));
+            auto send = [&](int to, const uint32_t* v) {
               const uint32_t there = pc_mapa(base, to), bar_there = pc_mapa(bar, to);
-              tmem_ld_wait();
 #pragma unroll
               for (int c = 0; c < RH; c += 4) pc_send4(there + (c / 4) * 2048, bar_there, v + c);
+            };
+            if (EARLY) {
+#pragma unroll
+              for (int to = 0; to < PC_CLUSTER; to++)
+                if (to < n_owners) {
+                  uint32_t v[RH];
+                  pc_tmem_read<RH>(v, src + (final % NACC) * ACC_COLS + to * R);
+                  pc_tmem_there<RH>(v);
+                  if (runs > 1) {
+#pragma unroll
+                    for (int c = 0; c < RH; c++) v[c] = __float_as_uint(__uint_as_float(sum[EARLY ? to : 0][c]) + __uint_as_float(v[c]));
+                  }
+                  send(to, v);
+                }
+            } else {
+#pragma unroll 1
+              for (int to = 0; to < n_owners; to++) {
+                uint32_t v[RH], w[RH];
+                pc_tmem_read<RH>(v, src + h * RH + (run % NACC) * ACC_COLS + to * R);
+#pragma unroll 1
+                for (int j = 1; j < runs; j++) {
+                  pc_tmem_read<RH>(w, src + h * RH + ((run + j) % NACC) * ACC_COLS + to * R);
+                  pc_tmem_there<RH>(v);
+                  pc_tmem_there<RH>(w);
+#pragma unroll
+                  for (int c = 0; c < RH; c++) v[c] = __float_as_uint(__uint_as_float(v[c]) + __uint_as_float(w[c]));
+                }
+                pc_tmem_there<RH>(v);
+                send(to, v);
+              }
             }
           }
         }
         if (!ok) { gave_up = 46; break; }
-        if (sl.n == 0) continue;
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) pc_arrive(b_acc_empty + 8 * (r & 1));
-        r++;
+        if (lane == 0)
+          for (int j = 0; j < runs; j++) pc_arrive(b_acc_empty + 8 * ((run + j) % NACC));
       }
     }
   } else if (owner) {
@@ -792,7 +898,9 @@ LEB_API int leb_chain_drop() {
   return 0;
 }
 
-// Adds a product to the chain (nothing is launched).  Arguments as leb_gemm_bf16_stream; with conv_w the product is the conv
+extern "C" int leb_gemm_bf16_skinny_slices(int N, int K);
+
+// Adds a product to the chain (nothing is launched).  2: the chain does not take it (its slices need more accumulators than there are).  Arguments as leb_gemm_bf16_stream; with conv_w the product is the conv
 // mixer's in_proj [3D, K] of a decode step (N is 3D, C is y [M, D], bfloat16) as in leb_gemm_bf16_stream_conv.
 LEB_API int leb_chain_add(void* C, int c_dtype, const void* A, const void* W, int M, int N, int K, int lda, int ldc, int epilogue,
                           const float* ssq_in, int parts_in, int d_in, float eps, void* emit_vals, const float* emit_g, float* emit_ssq,
@@ -827,9 +935,13 @@ LEB_API int leb_chain_add(void* C, int c_dtype, const void* A, const void* W, in
       if (best < 0 || cost < best) best = cost, rows = r;
     }
   }
+  // k-blocks of an accumulator: at most those of a slice of the product alone, evenly dealt over a block's slice
+  const int MP = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128));
+  const int blocks = ceil_div(K, TC_BK), per = ceil_div(blocks, PC_CLUSTER), most = ceil_div(blocks, leb_gemm_bf16_skinny_slices(N, K));
+  const int runs = ceil_div(per, most);
+  if (runs > (MP <= 64 ? ChainRing<64>::NACC : ChainRing<128>::NACC)) return 2;
   ChainOp& op = g_chain.op[g_chain_ops];
   ChainMaps& map = g_chain.map[g_chain_ops];
-  const int MP = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128));
   if (tensor_map(&map.w, W, N, K, K, kind == 3 ? PC_CONV_CH : rows)) return 1;
   if (tensor_map(&map.x, A, M, K, lda, MP)) return 1;
   op.C = C;
@@ -848,10 +960,10 @@ LEB_API int leb_chain_add(void* C, int c_dtype, const void* A, const void* W, in
   op.epilogue = kind | (act << 8);
   op.c_dtype = c_dtype;
   op.width = kind == 3 ? N / 3 : (kind == 2 ? N / 2 : N);
-  const int blocks = ceil_div(K, TC_BK), n_tiles = kind == 3 ? ceil_div(N / 3, PC_CONV_CH) : ceil_div(N, rows), dealt = max(clusters, 1);
+  const int n_tiles = kind == 3 ? ceil_div(N / 3, PC_CONV_CH) : ceil_div(N, rows), dealt = max(clusters, 1);
   const ChainGeo* before = g_chain_ops ? &g_chain.geo[g_chain_ops - 1] : nullptr;
-  g_chain.geo[g_chain_ops] = ChainGeo{blocks, n_tiles, rows, kind == 3 ? N / 3 : 0, ceil_div(blocks, PC_CLUSTER),
-                                      before ? (before->skip + before->n_tiles) % dealt : 0, min(dealt, n_tiles) * ceil_div(M, MP / PC_CLUSTER), 0};
+  g_chain.geo[g_chain_ops] = ChainGeo{blocks, n_tiles, rows, kind == 3 ? N / 3 : 0, per,
+                                      before ? (before->skip + before->n_tiles) % dealt : 0, min(dealt, n_tiles) * ceil_div(M, MP / PC_CLUSTER), ceil_div(per, runs)};
   op.parts_in = parts_in;
   op.d_in = d_in;
   op.eps = eps;

@@ -133,8 +133,11 @@ def _chained(out, x, w, M, N, K, epilogue, scale_args, emit_args, alone, conv=(N
     L = _library()
     if len(c.ops) >= L.leb_chain_max_ops():
         c.flush()
-    _check(L.leb_chain_add(_ptr(out), _dt(out, "linear.out"), _ptr(x), _ptr(w), M, N, K, x.stride(0), out.stride(0), epilogue,
-                           *scale_args, *emit_args, *conv))
+    rc = L.leb_chain_add(_ptr(out), _dt(out, "linear.out"), _ptr(x), _ptr(w), M, N, K, x.stride(0), out.stride(0), epilogue,
+                         *scale_args, *emit_args, *conv)
+    if rc == CHAIN_TAKES_NOT:
+        return False
+    _check(rc)
     c.ops.append(alone)
     return True
 
@@ -2269,6 +2272,7 @@ def linear_tc2(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: in
     return True
 
 
+CHAIN_TAKES_NOT = 2   # leb_chain_add: not a product the chain takes
 CHAIN_MIN = 2    # consecutive products from which a chain of them runs as one kernel
 SKINNY_M = 128   # rows up to which W is the wide tcgen05 operand and K is sliced over blocks
 SKINNY_MAX_N = 128 * 296   # from here on N alone gives every SM several tiles and the persistent kernel streams W better

@@ -121,3 +121,27 @@ def test_slices_without_k_between_others(M):
         want = x.double() @ w.double().T
         tol = 2 ** -8 + 2e-5 if y.dtype == torch.bfloat16 else 2e-5
         assert float((y.double() - want).abs().max() / want.abs().max()) < tol
+
+
+@pytest.mark.parametrize("N,kk", [(64, 64), (328, 4224), (512, 8192), (768, 3072), (1000, 5000), (2048, 2048), (2048, 5632), (2048, 7168),
+                                  (3072, 2048), (2560, 9728)])
+@pytest.mark.parametrize("M", [17, 64, 128])
+def test_a_chained_product_is_as_near_to_64_bits_as_one_alone(M, N, kk):
+    """K is cut otherwise in a chain, but no accumulator takes more of it than a slice of the product alone: one to eight of them in
+    a block's slice, ends between the two k-blocks of a stage, and (512 x 8,192 at 128 rows) more than a chain takes.  The same operands on
+    both sides; 1.05 for the draw of the roundings (measured: 0.22 to 1.00; with one accumulator a slice 1.4 to 8.4)."""
+    k, ws = K(), workspace()
+    W, h = gen(N, kk, seed=kk, scale=kk ** -0.5), gen(M, kk, seed=M)
+    want = h.double() @ W.double().T
+    off = {}
+    for chained in (True, False):
+        outs = [torch.empty(M, N, device=DEV) for _ in range(6)]
+        before = k.launch_count()
+        with k.product_chain(ws, M, torch.bfloat16) if chained else contextlib.nullcontext():
+            for y in outs:
+                k.linear(y, h, W)
+        assert (k.launch_count() - before == 1) == (chained and not (kk == 8192 and M == 128))
+        assert all(torch.equal(outs[0], y) for y in outs)
+        off[chained] = float((outs[0].double() - want).norm() / want.norm())
+    k.check_device_status()
+    assert off[True] <= 1.05 * off[False]
