@@ -900,7 +900,17 @@ LEB_API int leb_chain_drop() {
 
 extern "C" int leb_gemm_bf16_skinny_slices(int N, int K);
 
-// Adds a product to the chain (nothing is launched).  2: the chain does not take it (its slices need more accumulators than there are).  Arguments as leb_gemm_bf16_stream; with conv_w the product is the conv
+// Accumulators of a block's slice: each takes at most the k-blocks of a slice of the product alone.
+static int chain_runs(int N, int K) {
+  const int blocks = ceil_div(K, TC_BK);
+  return ceil_div(ceil_div(blocks, PC_CLUSTER), ceil_div(blocks, leb_gemm_bf16_skinny_slices(N, K)));
+}
+// Whether the chain takes a product of M rows: whether there are so many accumulators.
+LEB_API int leb_chain_takes(int M, int N, int K) {
+  return chain_runs(N, K) <= (M <= 64 ? ChainRing<64>::NACC : ChainRing<128>::NACC);
+}
+
+// Adds a product to the chain (nothing is launched).  Arguments as leb_gemm_bf16_stream; with conv_w the product is the conv
 // mixer's in_proj [3D, K] of a decode step (N is 3D, C is y [M, D], bfloat16) as in leb_gemm_bf16_stream_conv.
 LEB_API int leb_chain_add(void* C, int c_dtype, const void* A, const void* W, int M, int N, int K, int lda, int ldc, int epilogue,
                           const float* ssq_in, int parts_in, int d_in, float eps, void* emit_vals, const float* emit_g, float* emit_ssq,
@@ -935,11 +945,8 @@ LEB_API int leb_chain_add(void* C, int c_dtype, const void* A, const void* W, in
       if (best < 0 || cost < best) best = cost, rows = r;
     }
   }
-  // k-blocks of an accumulator: at most those of a slice of the product alone, evenly dealt over a block's slice
-  const int MP = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128));
-  const int blocks = ceil_div(K, TC_BK), per = ceil_div(blocks, PC_CLUSTER), most = ceil_div(blocks, leb_gemm_bf16_skinny_slices(N, K));
-  const int runs = ceil_div(per, most);
-  if (runs > (MP <= 64 ? ChainRing<64>::NACC : ChainRing<128>::NACC)) return 2;
+  LEB_REQUIRE(leb_chain_takes(M, N, K), "leb_chain_add: %d columns of %d numbers need more accumulators than there are at %d rows", N, K, M);
+  const int MP = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128)), blocks = ceil_div(K, TC_BK), per = ceil_div(blocks, PC_CLUSTER);
   ChainOp& op = g_chain.op[g_chain_ops];
   ChainMaps& map = g_chain.map[g_chain_ops];
   if (tensor_map(&map.w, W, N, K, K, kind == 3 ? PC_CONV_CH : rows)) return 1;
@@ -963,7 +970,7 @@ LEB_API int leb_chain_add(void* C, int c_dtype, const void* A, const void* W, in
   const int n_tiles = kind == 3 ? ceil_div(N / 3, PC_CONV_CH) : ceil_div(N, rows), dealt = max(clusters, 1);
   const ChainGeo* before = g_chain_ops ? &g_chain.geo[g_chain_ops - 1] : nullptr;
   g_chain.geo[g_chain_ops] = ChainGeo{blocks, n_tiles, rows, kind == 3 ? N / 3 : 0, per,
-                                      before ? (before->skip + before->n_tiles) % dealt : 0, min(dealt, n_tiles) * ceil_div(M, MP / PC_CLUSTER), ceil_div(per, runs)};
+                                      before ? (before->skip + before->n_tiles) % dealt : 0, min(dealt, n_tiles) * ceil_div(M, MP / PC_CLUSTER), ceil_div(per, chain_runs(N, K))};
   op.parts_in = parts_in;
   op.d_in = d_in;
   op.eps = eps;

@@ -45,7 +45,7 @@ class Model:
         self.stream_matrices: dict[str, torch.Tensor] = {}
         self.embedding_spec = self.embedding.cache_spec() if hasattr(self.embedding, "cache_spec") else None
         # Products of a step may wait for one another on the host (kernels.product_chain) in a model that is built of the library's
-        # own parts throughout.  What is put into a built model, or wrapped there, is judged when it is called (kernels.run_part).
+        # own parts throughout.  What is put into a built model, or wrapped there, is judged when it is called (kernels.guarded).
         own = __package__.partition(".")[0]
         self.chains = all(type(p).__module__.partition(".")[0] == own
                           for p in self._objects_in([*self.blocks, self.embedding, self.final_norm, self.head], {}))
@@ -134,9 +134,9 @@ class Model:
         M, D = batch.n_rows, self.hidden_size
         x = ws.get("model.x", (M, D), torch.float32)
         if self.embedding_spec is not None:
-            kernels.run_part(self.embedding.forward, x, batch.tokens, batch=batch, cache=cache.view(EMBEDDING_ENTRY, True, batch.tables))
+            kernels.guarded(self.embedding.forward)(x, batch.tokens, batch=batch, cache=cache.view(EMBEDDING_ENTRY, True, batch.tables))
         else:
-            kernels.run_part(self.embedding.forward, x, batch.tokens, batch=batch)
+            kernels.guarded(self.embedding.forward)(x, batch.tokens, batch=batch)
         x0 = pair = None
         if self.keeps_embedding:      # the embedding output is added to the stream again later
             x0 = ws.get("model.x0", (M, D), torch.float32)
@@ -167,14 +167,14 @@ class Model:
             env.next_block_norm = after.first_reader() if hasattr(after, "first_reader") and (i + 1) not in self.stream_adds \
                 else None
             if pending is not None:
-                pending = kernels.run_part(block.forward, x, batch, view, env, pending=pending)
+                pending = kernels.guarded(block.forward)(x, batch, view, env, pending=pending)
             else:
-                pending = kernels.run_part(block.forward, x, batch, view, env)
+                pending = kernels.guarded(block.forward)(x, batch, view, env)
         env.next_block_norm = None
         R = batch.n_logit_rows
         logits = ws.get("model.logits", (R, self.vocab_size), torch.float32)
         if R:
             xn = ws.get("model.xn", (R, D), env.dtype)
-            kernels.run_part(self.final_norm.forward, xn, x, rows=batch.logit_rows)
-            kernels.run_part(self.head.forward, logits, xn)
+            kernels.guarded(self.final_norm.forward)(xn, x, rows=batch.logit_rows)
+            kernels.guarded(self.head.forward)(logits, xn)
         return logits

@@ -29,7 +29,7 @@ def lib():
     """The library, for a call that may launch: products that wait in this thread's chain are launched first."""
     if _chain.ops:
         _chain.flush()
-    return _library()
+    return _library() if _lib is None or _timer is not None else _lib
 
 
 def _library():
@@ -45,20 +45,26 @@ class _Chain(threading.local):
 
     def __init__(self):
         self.open = False
-        self.ops = []        # per product the call that launches it alone
+        self.ops = []        # per product leb_chain_add's arguments, and what launches it alone (see `_chained`)
         self.sync = None     # the grid barrier's words
-        self.rows = 0
+        self.rows = self.most = 0
         self.device = None
 
     def flush(self) -> None:
         """Launches what waits: CHAIN_MIN products or more as one kernel, fewer as they would be without a chain."""
         ops, self.ops = self.ops, []
-        L = _library()
         if len(ops) < CHAIN_MIN:
-            L.leb_chain_drop()
-            for alone in ops:
-                alone()
+            for _, (out, x, w, epilogue, norm, alone) in ops:
+                if alone is not None:
+                    alone()
+                else:
+                    linear_skinny(out, x, w, epilogue, norm_args=norm)
             return
+        L = _library()
+        for args, _ in ops:
+            if L.leb_chain_add(*args):
+                L.leb_chain_drop()
+                raise KernelError(L.leb_last_error().decode())
         _check(L.leb_chain_run(_ptr(self.sync), _ptr(_status_word(self.device)), _stream()))
 
 
@@ -70,7 +76,7 @@ def product_chain(workspace, rows: int, dtype: torch.dtype):
     """Inside, consecutive products of a step of SMALL_M + 1 to SKINNY_M bfloat16 rows (dense ones, the conv mixer's decode step among them)
     wait for one another in the host's memory and run as ONE resident kernel (csrc/product_chain.cu) as soon as
     anything else is launched through this module, and at the end.  Nothing but calls of this module may launch work that
-    touches the products' operands in between; a model's forward pass calls its parts through `run_part`, which sees to that.
+    touches the products' operands in between; a model's forward pass calls its parts through `guarded`, which sees to that.
     `workspace` owns the barrier's words: steps that share it run one after the other."""
     c = _chain
     if dtype != torch.bfloat16 or not SMALL_M < rows <= SKINNY_M or c.open or _library().leb_chain_clusters(rows) <= 0:
@@ -78,67 +84,82 @@ def product_chain(workspace, rows: int, dtype: torch.dtype):
         if c.ops:            # inside another chain: nothing waits beyond this one's end
             c.flush()
         return
-    outer = c.sync, c.device, c.rows      # of a chain that `run_part` holds closed meanwhile
+    outer = c.sync, c.device, c.rows, c.most      # of a chain that `guarded` holds closed meanwhile
     c.sync = workspace.zeroed("chain.sync", 2)
     c.device = workspace.device
-    c.rows, c.open = rows, True
+    c.rows, c.most, c.open = rows, _library().leb_chain_max_ops(), True
     try:
         yield
         if c.ops:
             c.flush()
     finally:
         c.open = False
-        c.sync, c.device, c.rows = outer
-        if c.ops:            # the step raised: what waited is not run
-            c.ops = []
-            _library().leb_chain_drop()
+        c.sync, c.device, c.rows, c.most = outer
+        c.ops = []           # the step raised: what waited is not run
 
 
-_PACKAGE = __name__.partition(".")[0] + "."
+class _OwnModules(dict):
+    """Module name -> whether the module belongs to this package."""
+
+    def __missing__(self, name: str) -> bool:
+        own = self[name] = name.startswith(__name__.partition(".")[0] + ".")
+        return own
 
 
-def is_own(method) -> bool:
-    """Whether `method` is a bound method that a class of this package has from code of this package."""
-    return (type(method) is types.MethodType and type(method.__self__).__module__.startswith(_PACKAGE)
-            and getattr(method.__func__, "__globals__", _NOWHERE)["__name__"].startswith(_PACKAGE))
+_own_module = _OwnModules()
 
 
-_NOWHERE = {"__name__": ""}      # a callable that is no function
-
-
-def run_part(method, *args, **kwargs):
-    """Calls a part's method: every call of a part inside a forward pass goes through here.  The library's own parts touch their
+def guarded(method):
+    """A part's method as a forward pass calls it (all of its calls of parts go through here).  The library's own parts touch their
     operands through this module alone, which launches what waits in a chain first; other code (a part registered from
     elsewhere, a method wrapped or replaced on a class or an object) may use torch on them, so whatever waits is launched
     before it runs, and its own products are launched at their call.  Judged at every call: parts change after a model is built."""
+    if not _chain.open:
+        return method
+    if type(method) is types.MethodType and _own_module[type(method.__self__).__module__]:
+        f = method.__func__
+        if type(f) is types.FunctionType and _own_module[f.__globals__["__name__"]]:
+            return method
+    return functools.partial(_apart, method)
+
+
+def _apart(method, *args, **kwargs):
     c = _chain
-    if not c.open or is_own(method):
-        return method(*args, **kwargs)
     if c.ops:
         c.flush()
-    c.open = False
+    was, c.open = c.open, False
     try:
         return method(*args, **kwargs)
     finally:
-        c.open = True
+        c.open = was
 
 
-def _chained(out, x, w, M, N, K, epilogue, scale_args, emit_args, alone, conv=(None, None, None, None, None, 0)) -> bool:
-    """Adds a product to this thread's chain; False where it is not one the chain takes."""
+_NO_CONV = (None, None, None, None, None, 0)
+
+
+def _chained(out, x, w, M, N, K, lda, ldc, epilogue, scale, emit, conv=_NO_CONV, alone=None) -> bool:
+    """Lets a product wait in this thread's chain; False where it is not one the chain takes.  `alone`: the call that launches it by
+    itself (None: linear_skinny, which takes every product that the chain does)."""
     c = _chain
-    if M != c.rows or N >= SKINNY_MAX_N or not w.is_contiguous() or x.data_ptr() % 16 != 0 or w.data_ptr() % 16 != 0:
+    xp, wp = x.data_ptr(), w.data_ptr()
+    if M != c.rows or N >= SKINNY_MAX_N or (xp | wp) & 15 or not w.is_contiguous() or out.dtype not in _DT:
         return False
-    if (epilogue >> 8) >= PLAIN_ACT_BASE and (epilogue & 255) == STORE and out.dtype != torch.bfloat16:
+    if epilogue != STORE:
+        kind, act = epilogue & 255, epilogue >> 8
+        if kind == ACCUMULATE:
+            fits = act == 0 and out.dtype == torch.float32
+        elif kind == SWIGLU:
+            fits = N % 32 == 0 and (act in (0, 1) or act & 255 == 2)
+        else:
+            fits = kind == STORE and PLAIN_ACT_BASE <= act < PLAIN_ACT_BASE + 4 and out.dtype == torch.bfloat16
+        if not fits:
+            return False
+    if M > 64 and K >= 4096 and N <= 1536 and not _library().leb_chain_takes(M, N, K):      # (elsewhere it takes all)
         return False
-    L = _library()
-    if len(c.ops) >= L.leb_chain_max_ops():
+    norm = _scale_args(scale, M, K) + _emit_args(emit)
+    if len(c.ops) >= c.most:
         c.flush()
-    rc = L.leb_chain_add(_ptr(out), _dt(out, "linear.out"), _ptr(x), _ptr(w), M, N, K, x.stride(0), out.stride(0), epilogue,
-                         *scale_args, *emit_args, *conv)
-    if rc == CHAIN_TAKES_NOT:
-        return False
-    _check(rc)
-    c.ops.append(alone)
+    c.ops.append(((out.data_ptr(), _DT[out.dtype], xp, wp, M, N, K, lda, ldc, epilogue, *norm, *conv), (out, x, w, epilogue, norm, alone)))
     return True
 
 
@@ -240,6 +261,7 @@ def _declare(L) -> None:
         "leb_chain_max_ops": [],
         "leb_chain_clusters": [I],
         "leb_chain_drop": [],
+        "leb_chain_takes": [I, I, I],
         "leb_chain_add": [P, I, P, P, I, I, I, I, I, I, P, I, I, F, P, P, P, P, P, P, P, P, I],
         "leb_chain_run": [P, P, P],
         "leb_gemm_bf16_stream_conv": [P, P, P, I, I, I, I, I, P, P, P, P, P, I, P, I, I, F, P],
@@ -1246,9 +1268,9 @@ def shortconv_decode_fused(y: torch.Tensor, h: torch.Tensor, w_in: torch.Tensor,
         assert w_in.shape == (3 * D, K) and w.numel() == D * Lc and state.shape[1:] == (D, Lc - 1)
         if bias is not None:
             _cuda(bias, "shortconv.bias", torch.float32)
-        if _chained(y, h, w_in, M, 3 * D, K, STORE, _scale_args(scale, M, K), (None, None, None),
-                    lambda: shortconv_decode_fused(y, h, w_in, w, bias, state, batch, Lc, scale=scale, chain=False),
-                    (_ptr(w), _ptr(bias), _ptr(state), _ptr(batch.row_seq), _ptr(batch.seq_slot), Lc)):
+        if _chained(y, h, w_in, M, 3 * D, K, h.stride(0), y.stride(0), STORE, scale, None,
+                    (_ptr(w), _ptr(bias), _ptr(state), _ptr(batch.row_seq), _ptr(batch.seq_slot), Lc),
+                    lambda: shortconv_decode_fused(y, h, w_in, w, bias, state, batch, Lc, scale=scale, chain=False)):
             return True
     if M > SMALL_M:
         L = lib()
@@ -1811,11 +1833,18 @@ def split_norm_ok(M: int, dtype: torch.dtype, reader_weight: torch.Tensor | None
     return M <= SMALL_M or N < SKINNY_MAX_N
 
 
+_NO_SCALE, _NO_EMIT = (None, 0, 0, 0.0), (None, None, None)
+
+
 def _scale_args(scale: "SplitNorm | None", M: int, K: int):
     if scale is None:
-        return None, 0, 0, 0.0
+        return _NO_SCALE
     assert scale.filled and scale.values.shape == (M, K) and scale.ssq.shape[0] >= M
     return _ptr(scale.ssq), scale.ssq.shape[1], K, scale.eps
+
+
+def _emit_args(emit: "SplitNorm | None"):
+    return _NO_EMIT if emit is None else (_ptr(emit.values), _ptr(emit.weight), _ptr(emit.ssq))
 
 
 def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = STORE,
@@ -1834,7 +1863,7 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
     weight-streaming kernel (the one that also serves grouped products) whatever the row count.
     Kernels of a few rows fetch W ahead of their wait for the kernel launched before them: `w` must not be what that
     kernel writes (a model's weights never are).  Inside a `product_chain` such products may wait for the ones
-    that follow (`chain`).
+    that follow; `chain=False` is for one between two launches of other kinds, which would only wait to be launched alone.
     """
     _cuda(x, "linear.x", contiguous=False)
     _cuda(w, "linear.w", x.dtype)
@@ -1858,13 +1887,10 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
         return
     if (chain and _chain.open and group_offsets is None and not streaming and x.dtype == torch.bfloat16 and K % 8 == 0 and lda % 8 == 0
             and (emit is None or epilogue == ACCUMULATE)):
-        ev = eg = es = None
         if emit is not None:
             assert emit.values.shape == (M, N) and emit.ssq.shape == (M, -(-N // 16))
             assert emit.values.is_contiguous() and emit.ssq.is_contiguous() and emit.weight.numel() == N
-            ev, eg, es = _ptr(emit.values), _ptr(emit.weight), _ptr(emit.ssq)
-        if _chained(out, x, w, M, N, K, epilogue, _scale_args(scale, M, K), (ev, eg, es),
-                    lambda: linear(out, x, w, epilogue, scale=scale, emit=emit, chain=False)):
+        if _chained(out, x, w, M, N, K, lda, ldc, epilogue, scale, emit):
             if emit is not None:
                 emit.filled = True
             return
@@ -1896,7 +1922,7 @@ def linear(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: int = 
     if emit is not None and group_offsets is None and not streaming and M <= SKINNY_M:
         assert epilogue == ACCUMULATE and emit.values.shape == (M, N) and emit.ssq.shape == (M, -(-N // 16))
         assert emit.values.is_contiguous() and emit.ssq.is_contiguous() and emit.weight.numel() == N
-        ev, eg, es = _ptr(emit.values), _ptr(emit.weight), _ptr(emit.ssq)
+        ev, eg, es = _emit_args(emit)
     if not streaming and group_offsets is None and M <= SMALL_M:
         # the decode step: W streamed through rings of asynchronous copies in shared memory
         _check(L.leb_gemm_bf16_stream(_ptr(out), _dt(out, "linear.out"), _ptr(x), _ptr(w), M, N, K, lda, ldc,
@@ -2272,7 +2298,6 @@ def linear_tc2(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: in
     return True
 
 
-CHAIN_TAKES_NOT = 2   # leb_chain_add: not a product the chain takes
 CHAIN_MIN = 2    # consecutive products from which a chain of them runs as one kernel
 SKINNY_M = 128   # rows up to which W is the wide tcgen05 operand and K is sliced over blocks
 SKINNY_MAX_N = 128 * 296   # from here on N alone gives every SM several tiles and the persistent kernel streams W better

@@ -213,7 +213,7 @@ class AttentionMixer(Mixer):
         if w_in is None:  # q and gate rows are not adjacent once k, v are skipped: two products
             raise NotImplementedError("a gated attention layer reading another layer's cache")
         proj = ws.get("attn.proj", (M, w_in.shape[0]), env.dtype)
-        kernels.linear(proj, h, w_in, scale=scale)
+        kernels.linear(proj, h, w_in, scale=scale, chain=scale is not None)
         q_in = proj[:, : nh * hd]
         k_in = v_in = gate = None
         col = nh * hd
@@ -236,7 +236,7 @@ class AttentionMixer(Mixer):
         khd, kvd = self.khd, self.kvd
         q = ws.get("attn.q", (M, nh * khd), env.dtype)
         kp, vp = (cache.k, cache.v) if writes else (None, None)
-        rotary = kernels.run_part(self.position.fused_rotary)
+        rotary = kernels.guarded(self.position.fused_rotary)()
         raw = None
         if (rotary is not None and plain_v and khd == hd
                 and kernels.decode_attention_takes_raw(env.dtype, batch, M, nh, nkv, hd, cache.page_size, *rotary)):
@@ -268,7 +268,7 @@ class AttentionMixer(Mixer):
                 vn = ws.get("attn.vn", (M, nkv * hd), env.dtype)      # the values beside them, rows as wide as kn's
                 kernels.qk_rope_store(vn, v_in, None, None, None, None, cache.block_table, batch, None, None,
                                       self.eps, None, 0, True, nkv, nkv, hd, cache.page_size)
-            kernels.run_part(self.position.apply, qn.view(M, nh, hd), kn.view(M, nkv, hd) if writes else None, batch.row_pos)
+            kernels.guarded(self.position.apply)(qn.view(M, nh, hd), kn.view(M, nkv, hd) if writes else None, batch.row_pos)
             kernels.qk_rope_store(q, qn, kn, vn, kp, vp, cache.block_table, batch, None, None, self.eps,
                                   None, 0, True, nh, nkv, hd, cache.page_size)
         o = ws.get("attn.o", (M, nh * kvd), env.dtype)

@@ -71,7 +71,7 @@ class PreNormResidualBlock:
             return pending.values
         M, D = x.shape
         h = env.workspace.get("block.h", (M, D), env.dtype)
-        kernels.run_part(norm.forward, h, x)
+        kernels.guarded(norm.forward)(h, x)
         return h
 
     def forward(self, x: torch.Tensor, batch, cache, env, pending=None):
@@ -83,12 +83,12 @@ class PreNormResidualBlock:
         h = self._normed(self.mixer_norm, x, pending, env)
         if self.post_mixer_norm is None:
             mid = self._offer(self.mixer, self.ffn_norm, self.ffn, x, env, 0)
-            kernels.run_part(self.mixer.forward, h, x, True, batch, cache, env)
+            kernels.guarded(self.mixer.forward)(h, x, True, batch, cache, env)
         else:
             mid = None
             t = ws.get("block.t", (M, D), torch.float32)
-            kernels.run_part(self.mixer.forward, h, t, False, batch, cache, env)
-            kernels.run_part(self.post_mixer_norm.forward, x, t, add=True)
+            kernels.guarded(self.mixer.forward)(h, t, False, batch, cache, env)
+            kernels.guarded(self.post_mixer_norm.forward)(x, t, add=True)
         env.split_in = None
         h = self._normed(self.ffn_norm, x, mid, env)
         if self.post_ffn_norm is None:
@@ -97,12 +97,12 @@ class PreNormResidualBlock:
             if nxt is not None:
                 norm, consumer = nxt
                 last = self._offer(self.ffn, norm, consumer, x, env, 1)
-            kernels.run_part(self.ffn.forward, h, x, True, batch, env)
+            kernels.guarded(self.ffn.forward)(h, x, True, batch, env)
         else:
             last = None
             t = ws.get("block.t", (M, D), torch.float32)
-            kernels.run_part(self.ffn.forward, h, t, False, batch, env)
-            kernels.run_part(self.post_ffn_norm.forward, x, t, add=True)
+            kernels.guarded(self.ffn.forward)(h, t, False, batch, env)
+            kernels.guarded(self.post_ffn_norm.forward)(x, t, add=True)
         env.split_in = env.split_out = None
         return last if last is not None and last.filled else None
 
@@ -167,36 +167,36 @@ class GatedPreNormResidualBlock:
         ws = env.workspace
         env.split_in = env.split_out = None
         if self._folded is None:
-            self._folded = self.mixer_gate is not None and kernels.run_part(self.mixer_gate.give_rows_to, self.mixer)
+            self._folded = self.mixer_gate is not None and kernels.guarded(self.mixer_gate.give_rows_to)(self.mixer)
         if isinstance(pending, NormedRows) and pending.norm is self.mixer_norm and pending.values.shape == (M, D):
             h = pending.values
         else:
             h = ws.get("block.h", (M, D), env.dtype)
-            kernels.run_part(self.mixer_norm.forward, h, x)
+            kernels.guarded(self.mixer_norm.forward)(h, x)
         # the norm that reads x after each sum, and where its result goes (two buffers: h is still the gate's input)
         after_mixer = self.ffn_norm if self.ffn is not None else self._next(env)
         h2 = ws.get("block.h2" if h is ws.get("block.h", (M, D), env.dtype) else "block.h", (M, D), env.dtype)
         left = None
         if self.mixer_gate is None:
-            kernels.run_part(self.mixer.forward, h, x, True, batch, cache, env)
+            kernels.guarded(self.mixer.forward)(h, x, True, batch, cache, env)
             if self.ffn is not None:
-                kernels.run_part(self.ffn_norm.forward, h2, x)
+                kernels.guarded(self.ffn_norm.forward)(h2, x)
         else:
             y = ws.get("block.t", (M, D), torch.float32)
-            kernels.run_part(self.mixer.forward, h, y, False, batch, cache, env)
+            kernels.guarded(self.mixer.forward)(h, y, False, batch, cache, env)
             z = self.mixer.extra_out if self._folded else None
-            kernels.run_part(self.mixer_gate.add_gated, x, y, h, env, z=z, next_norm=after_mixer, h_out=h2 if after_mixer is not None else None)
+            kernels.guarded(self.mixer_gate.add_gated)(x, y, h, env, z=z, next_norm=after_mixer, h_out=h2 if after_mixer is not None else None)
             if self.ffn is None and after_mixer is not None:
                 left = NormedRows(h2, after_mixer)
         if self.ffn is None:
             return left
         after_ffn = self._next(env)
         if self.ffn_gate is None:
-            kernels.run_part(self.ffn.forward, h2, x, True, batch, env)
+            kernels.guarded(self.ffn.forward)(h2, x, True, batch, env)
             return None
         y = ws.get("block.t", (M, D), torch.float32)
-        kernels.run_part(self.ffn.forward, h2, y, False, batch, env)
-        kernels.run_part(self.ffn_gate.add_gated, x, y, h2, env, next_norm=after_ffn, h_out=h if after_ffn is not None else None)
+        kernels.guarded(self.ffn.forward)(h2, y, False, batch, env)
+        kernels.guarded(self.ffn_gate.add_gated)(x, y, h2, env, next_norm=after_ffn, h_out=h if after_ffn is not None else None)
         return NormedRows(h, after_ffn) if after_ffn is not None else None
 
 
@@ -251,11 +251,11 @@ class ParallelResidualBlock:
                 kernels.layernorm_pair(h, hf, x, self.mixer_norm.weight, self.ffn_norm.weight, self.mixer_norm.eps)
             else:
                 hf = h
-                kernels.run_part(self.mixer_norm.forward, h, x)
+                kernels.guarded(self.mixer_norm.forward)(h, x)
         y = ws.get("block.t", (M, D), torch.float32)
-        kernels.run_part(self.mixer.forward, h, y, False, batch, cache, env)
+        kernels.guarded(self.mixer.forward)(h, y, False, batch, cache, env)
         if self.ffn is not None:
-            kernels.run_part(self.ffn.forward, hf, y, True, batch, env)
+            kernels.guarded(self.ffn.forward)(hf, y, True, batch, env)
         nxt = env.next_block_norm
         after = nxt[1] if nxt is not None and isinstance(nxt[1], ParallelResidualBlock) and isinstance(nxt[0], LayerNorm) \
             and not nxt[0].has_bias else None
@@ -338,13 +338,13 @@ class PostNormResidualBlock:
         nxt = env.next_block_norm
         feeds_next = (not f32) and nxt is not None and isinstance(nxt[1], PostNormResidualBlock)
         y = ws.get("block.t", (M, D), torch.float32)
-        kernels.run_part(self.mixer.forward, h, y, False, batch, cache, env)
+        kernels.guarded(self.mixer.forward)(h, y, False, batch, cache, env)
         if self.ffn is None:
             self._sum(x, y, self.mixer_norm, other if feeds_next else None)
             return StreamRows(other) if feeds_next else None
         self._sum(x, y, self.mixer_norm, other)
         h2 = x if f32 else other
-        kernels.run_part(self.ffn.forward, h2, y, False, batch, env)
+        kernels.guarded(self.ffn.forward)(h2, y, False, batch, env)
         self._sum(x, y, self.ffn_norm, h if feeds_next else None)
         return StreamRows(h) if feeds_next else None
 
@@ -405,21 +405,21 @@ class SandwichNormResidualBlock:
             h = pending.values
         else:
             h = ws.get("block.h", (M, D), env.dtype)
-            kernels.run_part(self.mixer_norm.forward, h, x)
+            kernels.guarded(self.mixer_norm.forward)(h, x)
         other = ws.get("block.h2" if h is ws.get("block.h", (M, D), env.dtype) else "block.h", (M, D), env.dtype)
         nxt = env.next_block_norm
         after = nxt[0] if nxt is not None and isinstance(nxt[1], SandwichNormResidualBlock) else None
         follows = self.ffn_norm if self.ffn is not None else after
         if hasattr(self.mixer, "forward_parts"):
-            y, a, y2, b = kernels.run_part(self.mixer.forward_parts, h, batch, cache, env)
+            y, a, y2, b = kernels.guarded(self.mixer.forward_parts)(h, batch, cache, env)
             weighted = (a, y2, b)
         else:
             y, weighted = ws.get("block.t", (M, D), torch.float32), None
-            kernels.run_part(self.mixer.forward, h, y, False, batch, cache, env)
-        kernels.run_part(self.post_mixer_norm.add_into, x, y, follows, other if follows is not None else None, weighted)
+            kernels.guarded(self.mixer.forward)(h, y, False, batch, cache, env)
+        kernels.guarded(self.post_mixer_norm.add_into)(x, y, follows, other if follows is not None else None, weighted)
         if self.ffn is None:
             return NormedRows(other, after) if after is not None else None
         y = ws.get("block.t", (M, D), torch.float32)
-        kernels.run_part(self.ffn.forward, other, y, False, batch, env)
-        kernels.run_part(self.post_ffn_norm.add_into, x, y, after, h if after is not None else None)
+        kernels.guarded(self.ffn.forward)(other, y, False, batch, env)
+        kernels.guarded(self.post_ffn_norm.add_into)(x, y, after, h if after is not None else None)
         return NormedRows(h, after) if after is not None else None

@@ -111,12 +111,12 @@ class ParallelMixers(Mixer):
         kl, kr = {}, {}
         if self.w_in is not None:
             proj = ws.get("pair.proj", (M, self.w_in.shape[0]), torch.float32)
-            kernels.linear(proj, h, self.w_in)
+            kernels.linear(proj, h, self.w_in, chain=False)
             kl["proj"], kr["proj"] = proj[:, : self.n_left], proj[:, self.n_left:]
         if bias is not None:
             kl["add_output_bias"] = False
-        kernels.run_part(self.left.forward, h, y1, False, batch, self._view(cache, 0), env, **kl)
-        kernels.run_part(self.right.forward, h, y2, False, batch, self._view(cache, 1), env, **kr)
+        kernels.guarded(self.left.forward)(h, y1, False, batch, self._view(cache, 0), env, **kl)
+        kernels.guarded(self.right.forward)(h, y2, False, batch, self._view(cache, 1), env, **kr)
         if getattr(self.right, "output_bias", lambda: None)() is not None:
             raise NotImplementedError("an output bias on the right-hand mixer")
         return y1, self.a, y2, self.b, bias

@@ -279,4 +279,4 @@ class SigmoidTopKMoE(FeedForward):
         kernels.linear(ys, a, self.w2, group_offsets=offsets, rows_hint=P)
         kernels.moe_combine(out, ys, pair_row, None if self.weight_input else wts, accumulate, k=self.k)
         if self.shared is not None:
-            kernels.run_part(self.shared.forward, h, out, True, batch, env)
+            kernels.guarded(self.shared.forward)(h, out, True, batch, env)

@@ -66,7 +66,7 @@ class MinGRUMixer(Mixer):
         ws = env.workspace
         if proj is None:
             proj = ws.get("gru.proj", (M, 3 * W), torch.float32)
-            kernels.linear(proj, h, self.w_in)
+            kernels.linear(proj, h, self.w_in, chain=False)
         s = ws.get("gru.s", (M, W), env.dtype)
         n = kernels.min_gru_scratch(batch, W)
         scratch = ws.get("gru.pieces", (n,), torch.float32) if n else None
@@ -126,7 +126,7 @@ class MLSTMMixer(Mixer):
         f32 = torch.float32
         nq, nv = H * d, H * e
         proj = ws.get("mlstm.proj", (M, 2 * nq + 2 * nv + 2 * H), f32)
-        kernels.linear(proj, h, self.w_in)
+        kernels.linear(proj, h, self.w_in, chain=False)
         q, k = proj[:, :nq], proj[:, nq: 2 * nq]
         v, g = proj[:, 2 * nq: 2 * nq + nv], proj[:, 2 * nq + nv: 2 * nq + 2 * nv]
         gi, gf = proj[:, 2 * nq + 2 * nv: 2 * nq + 2 * nv + H], proj[:, 2 * nq + 2 * nv + H:]

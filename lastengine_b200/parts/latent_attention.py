@@ -142,7 +142,7 @@ class LatentAttentionMixer(Mixer):
         if pool.shape[-1] != rank + rd:
             raise ValueError(f"the cache rows are {pool.shape[-1]} wide, this layer reads {rank} + {rd}")
         proj = ws.get("lat.proj", (M, self.w_down.shape[0]), env.dtype)
-        kernels.linear(proj, h, self.w_down)
+        kernels.linear(proj, h, self.w_down, chain=False)
         qn = ws.get("lat.qn", (H, M, self.hd_p), env.dtype)
         qr = ws.get("lat.qr", (M, H, rd), env.dtype)
         if self.q_rank:
@@ -150,7 +150,7 @@ class LatentAttentionMixer(Mixer):
             kernels.latent_prep(cq, proj, pool if writes else None, cache.block_table, batch, self.q_norm_w,
                                 self.kv_norm_w, self.eps, self.inv_freq, self.rot_dims, rank, rd, cache.page_size, self.neox)
             q = ws.get("lat.q", (M, H * (hd + rd)), env.dtype)
-            kernels.linear(q, cq, self.w_uq)
+            kernels.linear(q, cq, self.w_uq, chain=False)
             kernels.latent_q_split(qn, qr, q, batch.row_pos, self.inv_freq, self.rot_dims, H, hd, rd, self.neox)
         else:
             kernels.latent_rows(qn, qr, proj, pool if writes else None, cache.block_table, batch, self.kv_norm_w, self.eps,

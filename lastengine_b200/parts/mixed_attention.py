@@ -115,7 +115,7 @@ class MixedHeadsAttentionMixer(Mixer):
             raise NotImplementedError("this attention keeps its own keys and values")
         if proj is None:
             proj = ws.get("mattn.proj", (M, self.w_in.shape[0]), torch.float32)
-            kernels.linear(proj, h, self.w_in)
+            kernels.linear(proj, h, self.w_in, chain=False)
         n_qkv = (nh + nkv) * hd + nkv * vd
         q = ws.get("mattn.q", (M, nh * hd), env.dtype)
         kernels.pooled_attn_prep(q, cache.k, cache.v, proj[:, :n_qkv], self.b_in, self.q_norm_w, self.k_norm_w, self.eps,

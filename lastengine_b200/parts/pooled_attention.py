@@ -106,7 +106,7 @@ class PooledWindowAttentionMixer(Mixer):
         if not cache.writable:
             raise NotImplementedError("this attention keeps its own keys and values")
         proj = ws.get("pattn.proj", (M, self.w_in.shape[0]), torch.float32)
-        kernels.linear(proj, h, self.w_in)
+        kernels.linear(proj, h, self.w_in, chain=False)
         q = ws.get("pattn.q", (M, nh * hd), env.dtype)
         kernels.pooled_attn_prep(q, cache.k, cache.v, proj, self.b_in, self.q_norm_w, self.k_norm_w, self.eps,
                                  self.freq_qk, self.rot, self.freq_v, cache.block_table, batch, nh, nkv, hd, vd,

@@ -193,7 +193,7 @@ class StateSpaceMixer(Mixer):
         ws = env.workspace
         f32 = torch.float32
         proj = ws.get("ssm.proj", (M, inner + C + H), f32)
-        kernels.linear(proj, h, self.w_in)
+        kernels.linear(proj, h, self.w_in, chain=False)
         z, dt_raw = proj[:, :inner], proj[:, inner + C:]
         xbc = ws.get("ssm.conv", (M, C), f32)
         kernels.causal_conv(xbc, proj[:, inner: inner + C], self.w_conv, cache.states[1] if self.taps > 1 else None, batch)

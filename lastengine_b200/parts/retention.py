@@ -84,7 +84,7 @@ class RetentionMixer(Mixer):
         M = h.shape[0]
         ws = env.workspace
         proj = ws.get("ret.proj", (M, self.w_in.shape[0]), env.dtype)
-        kernels.linear(proj, h, self.w_in)
+        kernels.linear(proj, h, self.w_in, chain=False)
         q, k = proj[:, : H * d], proj[:, H * d: 2 * H * d]
         v, g = proj[:, 2 * H * d: 2 * H * d + H * e], proj[:, 2 * H * d + H * e: 2 * H * (d + e)]
         if self.n_extra:

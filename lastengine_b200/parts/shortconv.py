@@ -55,7 +55,7 @@ class ShortConvMixer(Mixer):
         # a decode step of a few sequences: projection and convolution in one launch
         if not kernels.shortconv_decode_fused(y, h, self.w_in, self.w_conv, self.b_conv, cache.state, batch, self.Lc, scale=scale):
             bcx = ws.get("conv.bcx", (M, 3 * self.D), env.dtype)
-            kernels.linear(bcx, h, self.w_in, scale=scale)
+            kernels.linear(bcx, h, self.w_in, scale=scale, chain=scale is not None)
             kernels.shortconv(y, bcx, self.w_conv, self.b_conv, cache.state, batch, self.Lc)
         kernels.linear(out, y, self.w_out, kernels.ACCUMULATE if accumulate else kernels.STORE,
                        emit=emit if accumulate else None)

@@ -31,10 +31,10 @@ CPU = torch.device("cpu")
 
 
 class CountingLibrary:
-    """Every entry point does nothing and answers 0; products that wait and the launches of a chain are counted."""
+    """Every entry point does nothing and answers 0; the products and the launches of chains are counted."""
 
     def __init__(self):
-        self.waiting = self.chains = self.dropped = 0
+        self.waiting = self.chains = self.dropped = 0      # waiting: added, not launched
         self.longest = 0
 
     def leb_chain_clusters(self, rows):
@@ -42,6 +42,9 @@ class CountingLibrary:
 
     def leb_chain_max_ops(self):
         return 40
+
+    def leb_chain_takes(self, m, n, k):
+        return 1
 
     def leb_gemm_bf16_skinny_slices(self, n, k):
         return 4
@@ -249,3 +252,24 @@ def test_a_part_that_raises_leaves_no_chain_behind(library):
     del m.blocks[2].ffn.forward
     forward(m, seqs=ROWS)
     assert library.chains >= 2
+
+
+def test_products_that_are_too_few_for_a_chain_run_alone_in_their_order(library, monkeypatch):
+    ran = []
+    monkeypatch.setattr(kernels, "CHAIN_MIN", 4)
+    monkeypatch.setattr(library, "leb_gemm_bf16_skinny", lambda *a: ran.append(a[5]) or 0, raising=False)
+    x, ws = torch.zeros(ROWS, 64, dtype=torch.bfloat16), Workspace(CPU)
+    with kernels.product_chain(ws, ROWS, torch.bfloat16):
+        for n in (32, 64, 96):
+            kernels.linear(torch.zeros(ROWS, n), x, torch.zeros(n, 64, dtype=torch.bfloat16))
+        assert len(kernels._chain.ops) == 3 and not ran
+    assert ran == [32, 64, 96] and library.chains == library.longest == 0
+
+
+def test_a_product_the_chain_refuses_when_it_is_launched_leaves_none_behind(library, monkeypatch):
+    monkeypatch.setattr(library, "leb_chain_add", lambda *a: int(a[5] == 96), raising=False)
+    x, ws = torch.zeros(ROWS, 64, dtype=torch.bfloat16), Workspace(CPU)
+    with pytest.raises(kernels.KernelError, match="refused"), kernels.product_chain(ws, ROWS, torch.bfloat16):
+        for n in (32, 96):
+            kernels.linear(torch.zeros(ROWS, n), x, torch.zeros(n, 64, dtype=torch.bfloat16))
+    assert library.chains == 0 and library.dropped == 1
