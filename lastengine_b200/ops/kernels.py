@@ -51,9 +51,9 @@ class _Chain(threading.local):
         self.device = None
 
     def flush(self) -> None:
-        """Launches what waits: CHAIN_MIN products or more as one kernel, fewer as they would be without a chain."""
+        """Launches what waits: as one kernel where that pays, else as without a chain."""
         ops, self.ops = self.ops, []
-        if len(ops) < CHAIN_MIN:
+        if len(ops) == 1 or not chain_pays(self.rows, [args[5:7] for args, _ in ops]):
             for _, (out, x, w, epilogue, norm, alone) in ops:
                 if alone is not None:
                     alone()
@@ -132,6 +132,27 @@ def _apart(method, *args, **kwargs):
         return method(*args, **kwargs)
     finally:
         c.open = was
+
+
+def chain_pays(rows: int, sizes: list[tuple[int, int]]) -> bool:
+    """Whether products of `sizes` (columns, inner size) are faster as a chain than launched alone.  Ten widths of 256 to 4,096, two to
+    twelve products, 17 to 128 rows, chained and alone in turn (us):
+    - a product whose K alone is not cut has its epilogue in the first kernel's few threads there, and the chain is ahead from two
+      products on (width 2,048 and 14,336 columns, 64 rows: 32.2 and 44.9);
+    - above 96 rows it is from two on as well (97 rows, width 2,048: 21.7 and 24.0);
+    - up to 32 rows the chain's fixed part takes what two products gain (width 2,048: 16.1 and 15.1) and about what three do (the gated
+      epilogue with gelu: 0.975 of the speed of a Zekivik step); four gain from 24 rows on (32 rows, width 1,024: 23.9 and 25.0; 17: 26.8
+      and 24.7);
+    - between, two are even or ahead where the rows fill their padding (64 rows: 17.8 and 18.6, 20.4 and 20.6), and three where they do
+      not and their weights are large (33 rows, two: 18.3 and 16.5; three, width 1,024: 23.1 and 21.5)."""
+    n, padding = len(sizes), -rows % 32
+    if n < 2 or rows > 96 or (rows > 32 and padding < 16):
+        return n >= 2
+    if rows <= 32:
+        need = 5 if padding > 8 else 4
+    else:
+        need = 3 if 2 * sum(N * K for N, K in sizes) >= CHAIN_LARGE else 4
+    return n >= need or any(_library().leb_gemm_bf16_skinny_slices(N, K) == 1 for N, K in sizes)
 
 
 _NO_CONV = (None, None, None, None, None, 0)
@@ -2298,7 +2319,7 @@ def linear_tc2(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, epilogue: in
     return True
 
 
-CHAIN_MIN = 2    # consecutive products from which a chain of them runs as one kernel
+CHAIN_LARGE = 60_000_000     # bytes of weights from which three products pay as a chain (`chain_pays`)
 SKINNY_M = 128   # rows up to which W is the wide tcgen05 operand and K is sliced over blocks
 SKINNY_MAX_N = 128 * 296   # from here on N alone gives every SM several tiles and the persistent kernel streams W better
 _skinny_ws: dict[int, list[torch.Tensor]] = {}

@@ -84,6 +84,7 @@ def library(monkeypatch):
     monkeypatch.setattr(kernels, "_tc_block", {})
     monkeypatch.setattr(kernels, "_device_index", lambda d: 0)
     monkeypatch.setattr(kernels, "sm_count", lambda: 148)
+    monkeypatch.setattr(kernels, "chain_pays", lambda rows, sizes: len(sizes) >= 2)
     monkeypatch.setattr(kernels, "_tc_status", {})
     monkeypatch.setattr(kernels, "_retention_ws", {})
     monkeypatch.setattr(kernels, "_gru_piece", [64])
@@ -254,9 +255,22 @@ def test_a_part_that_raises_leaves_no_chain_behind(library):
     assert library.chains >= 2
 
 
-def test_products_that_are_too_few_for_a_chain_run_alone_in_their_order(library, monkeypatch):
+@pytest.mark.parametrize("rows,products,uncut,mb,pays", [
+    (17, 1, 0, 500, 0), (17, 1, 1, 500, 0), (17, 2, 1, 1, 1), (128, 2, 1, 1, 1), (17, 2, 0, 500, 0), (32, 2, 0, 500, 0), (32, 3, 0, 500, 0),
+    (32, 4, 0, 1, 1), (24, 4, 0, 1, 1), (23, 4, 0, 500, 0), (17, 5, 0, 1, 1), (33, 2, 0, 500, 0), (33, 3, 0, 59, 0),
+    (33, 3, 0, 61, 1), (48, 2, 0, 500, 0), (49, 2, 0, 1, 1), (64, 2, 0, 1, 1), (65, 2, 0, 500, 0), (65, 4, 0, 1, 1), (81, 2, 0, 1, 1),
+    (97, 2, 0, 1, 1), (128, 2, 0, 1, 1)])
+def test_which_products_run_as_a_chain(rows, products, uncut, mb, pays, monkeypatch):
+    """The edges of the rule: rows, products, weights, and products whose K is not cut alone."""
+    lib = CountingLibrary()
+    lib.leb_gemm_bf16_skinny_slices = lambda n, k: 1 if uncut else 4
+    monkeypatch.setattr(kernels, "_lib", lib)
+    assert kernels.chain_pays(rows, [(mb * 500_000 // products, 1)] * products) == bool(pays)
+
+
+def test_products_that_do_not_pay_as_a_chain_run_alone_in_their_order(library, monkeypatch):
     ran = []
-    monkeypatch.setattr(kernels, "CHAIN_MIN", 4)
+    monkeypatch.setattr(kernels, "chain_pays", lambda rows, sizes: False)
     monkeypatch.setattr(library, "leb_gemm_bf16_skinny", lambda *a: ran.append(a[5]) or 0, raising=False)
     x, ws = torch.zeros(ROWS, 64, dtype=torch.bfloat16), Workspace(CPU)
     with kernels.product_chain(ws, ROWS, torch.bfloat16):
