@@ -230,14 +230,22 @@ moe_router_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, const 
 // The same router for few rows (decode steps): a cluster of four blocks takes a row, each a quarter of the experts, a warp one of
 // them.  One block's 262 KB of router rows (32 experts of 2,048) come to its SM in 8.4 us, most of it two trips to L2 after
 // the wait; here a warp has the whole of its router row (PRE pieces of 16 bytes a lane) in registers before it waits for the
-// row of h, and the scores go to the first block's shared memory, whose first warp chooses.  A score is summed in the order of the
-// form above: the same bits.
+// row of h, where the caller says that the kernel launched before does not write the router's rows (`ahead`).  The scores go to
+// the first block's shared memory, whose first warp chooses.  A score is summed in the order of the form above: the same bits.
+// Those loads are written out: as plain loads of a const __restrict__ pointer the compiler takes what they read for constant and
+// moved them before the wait.
 #define ROUTER_CLUSTER 4
 #define ROUTER_PRE 16
+__device__ __forceinline__ float4 router_row_load(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
 template <typename T>
 __global__ void __launch_bounds__(256)
 moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, const T* __restrict__ h,
-                      const float* __restrict__ wr, const float* __restrict__ bias, int D, int E, int k, int norm_topk, float scaling) {
+                      const float* __restrict__ wr, const float* __restrict__ bias, int D, int E, int k, int norm_topk, float scaling,
+                      int ahead) {
   extern __shared__ __align__(16) float sm[];  // the row of h as float [D], then s[E], c[E]
   float* s_ = sm + D;
   float* c_ = s_ + E;
@@ -245,10 +253,12 @@ moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, co
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int share = (E + ROUTER_CLUSTER - 1) / ROUTER_CLUSTER, first = rank * share + warp, end = min(E, (rank + 1) * share), n4 = D / 4;
   pdl_trigger();
+  if (!ahead) pdl_wait();
   float4 a[ROUTER_PRE];
 #pragma unroll
   for (int u = 0; u < ROUTER_PRE; u++)
-    a[u] = first < end && lane + 32 * u < n4 ? reinterpret_cast<const float4*>(wr + (size_t)first * D)[lane + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+    a[u] = first < end && lane + 32 * u < n4 ? router_row_load(reinterpret_cast<const float4*>(wr + (size_t)first * D) + lane + 32 * u)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   pdl_wait();
   const T* hr = h + (size_t)m * D;
@@ -264,7 +274,7 @@ moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, co
     for (int i0 = lane; i0 < n4; i0 += 32 * ROUTER_PRE) {
       if (e != first || i0 != lane) {
 #pragma unroll
-        for (int u = 0; u < ROUTER_PRE; u++) a[u] = i0 + 32 * u < n4 ? w4[i0 + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < ROUTER_PRE; u++) a[u] = i0 + 32 * u < n4 ? router_row_load(w4 + i0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < ROUTER_PRE; u++) {
@@ -392,7 +402,7 @@ moe_router_rows_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, c
 
 LEB_API int leb_moe_router(int* topk_ids, float* topk_w, const void* h, int dtype, const float* wr,
                            const float* bias, int M, int D, int E, int k, int norm_topk,
-                           float scaling, cudaStream_t st) {
+                           float scaling, int ahead, cudaStream_t st) {
   if (M <= 0) return 0;
   LEB_REQUIRE(E >= 1 && E <= MOE_MAX_E, "leb_moe_router: %d experts outside 1..%d", E, MOE_MAX_E);
   LEB_REQUIRE(k >= 1 && k <= MOE_MAX_K && k <= E, "leb_moe_router: top-%d outside 1..min(%d, experts)", k, MOE_MAX_K);
@@ -439,8 +449,8 @@ LEB_API int leb_moe_router(int* topk_ids, float* topk_w, const void* h, int dtyp
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_leb_pdl ? 2 : 1;
-    const cudaError_t e = dtype == LEB_BF16 ? cudaLaunchKernelEx(&cfg, moe_router_few_kernel<bf16>, topk_ids, topk_w, (const bf16*)h, wr, bias, D, E, k, norm_topk, scaling)
-                                            : cudaLaunchKernelEx(&cfg, moe_router_few_kernel<float>, topk_ids, topk_w, (const float*)h, wr, bias, D, E, k, norm_topk, scaling);
+    const cudaError_t e = dtype == LEB_BF16 ? cudaLaunchKernelEx(&cfg, moe_router_few_kernel<bf16>, topk_ids, topk_w, (const bf16*)h, wr, bias, D, E, k, norm_topk, scaling, ahead)
+                                            : cudaLaunchKernelEx(&cfg, moe_router_few_kernel<float>, topk_ids, topk_w, (const float*)h, wr, bias, D, E, k, norm_topk, scaling, ahead);
     if (e != cudaSuccess) return leb_fail("leb_moe_router: %s", cudaGetErrorString(e));
     LEB_CHECK_LAUNCH("leb_moe_router");
     return 0;

@@ -288,7 +288,7 @@ def _declare(L) -> None:
         "leb_gemm_bf16_stream_conv": [P, P, P, I, I, I, I, I, P, P, P, P, P, I, P, I, I, F, P],
         "leb_gemm_bf16_tc_grouped": [P, I, P, P, I, I, I, I, I, I, P, I, P, P],
         "leb_gemm_bf16_tc2": [P, I, P, P, I, I, I, I, I, I, P, P],
-        "leb_moe_router": [P, P, P, I, P, P, I, I, I, I, I, F, P],
+        "leb_moe_router": [P, P, P, I, P, P, I, I, I, I, I, F, I, P],
         "leb_moe_align": [P, P, P, P, I, I, P],
         "leb_moe_align_gather": [P, P, P, P, I, P, P, P, I, I, I, I, P],
         "leb_moe_combine": [P, P, P, P, I, I, I, I, P],
@@ -1986,7 +1986,7 @@ _OPTIONAL_TC: list = [None]
 # ----------------------------------------------------------------------------------------------
 def moe_router(topk_ids: torch.Tensor, topk_w: torch.Tensor, h: torch.Tensor, wr: torch.Tensor,
                bias: torch.Tensor | None, norm_topk: bool, scaling: float, softmax_chosen: bool = False,
-               softmax_groups: tuple[int, int] | None = None, sigmoid_groups: tuple[int, int, int] | None = None) -> None:
+               softmax_groups: tuple[int, int] | None = None, sigmoid_groups: tuple[int, int, int] | None = None, ahead: bool = False) -> None:
     """The k experts of every row and their weights.  Default: sigmoid scores, the bias only chooses,
     weights are the chosen sigmoids (over their sum with norm_topk).  `softmax_chosen`: logits Wr h + bias,
     the k largest chosen, weights the softmax over the chosen logits alone.  `softmax_groups` = (groups, keep):
@@ -1994,8 +1994,8 @@ def moe_router(topk_ids: torch.Tensor, topk_w: torch.Tensor, h: torch.Tensor, wr
     `groups` equal groups of neighbours (a group's score: its largest choice score) can be chosen, weights
     are the chosen scores over their sum (+ 1e-20).  `sigmoid_groups` = (groups, keep, top): sigmoid scores, the
     bias only chooses, groups as before with a group's score the sum of its `top` largest choice scores, weights
-    the chosen scores over their sum (+ 1e-20) times `scaling`.  Steps of few rows fetch `wr` ahead of their wait for the kernel
-    launched before: it must not be what that kernel writes."""
+    the chosen scores over their sum (+ 1e-20) times `scaling`.  `ahead`: `wr` is not what the kernel launched before writes (a
+    model's weights never are), so steps of few rows may fetch it ahead of their wait for that kernel."""
     _cuda(topk_ids, "moe_router.topk_ids", torch.int32)
     _cuda(topk_w, "moe_router.topk_w", torch.float32)
     _cuda(h, "moe_router.h")
@@ -2019,7 +2019,7 @@ def moe_router(topk_ids: torch.Tensor, topk_w: torch.Tensor, h: torch.Tensor, wr
                               f"cannot give {k} choices")
         mode = 4 | (groups << 8) | (keep << 16) | (top << 24)
     _check(lib().leb_moe_router(_ptr(topk_ids), _ptr(topk_w), _ptr(h), _dt(h, "moe_router.h"), _ptr(wr),
-                                _ptr(bias), M, D, E, k, mode, float(scaling), _stream()))
+                                _ptr(bias), M, D, E, k, mode, float(scaling), 1 if ahead else 0, _stream()))
 
 
 def moe_align(offsets: torch.Tensor, sorted_pair: torch.Tensor, pair_row: torch.Tensor,

@@ -253,7 +253,7 @@ class SigmoidTopKMoE(FeedForward):
         kernels.moe_router(ids, wts, h, self.router_w, self.router_b, self.norm_topk, self.scaling,
                            softmax_chosen=self.router == "softmax_chosen",
                            softmax_groups=self.groups if self.router == "softmax_grouped" else None,
-                           sigmoid_groups=(*self.groups, self.group_top) if self.router == "sigmoid_grouped" else None)
+                           sigmoid_groups=(*self.groups, self.group_top) if self.router == "sigmoid_grouped" else None, ahead=True)
         offsets = ws.get("moe.offsets", (self.E + 1,), torch.int32)
         sorted_pair = ws.get("moe.sorted", (P,), torch.int32)
         pair_row = ws.get("moe.rows", (P,), torch.int32)

@@ -1053,6 +1053,30 @@ def test_moe_router_gives_a_row_the_same_bits_whatever_the_step(dtype, E, k, D):
     assert err(all_w[agree.to(DEV)], want_w[agree]) < 1e-5
 
 
+def test_moe_router_reads_weights_that_the_launch_before_it_wrote():
+    """Unless the caller says otherwise (`ahead`), router rows may come from one of the library's own kernels launched right
+    before: here a 32-bit product, which lets the router's blocks start at its beginning and writes at its end."""
+    M, E, D, k, inner = 8, 32, 2048, 4, 4096
+    h, x, w = gen(M, D, seed=30).to(DEV), gen(E, inner, seed=31, scale=inner ** -0.5).to(DEV), gen(D, inner, seed=32, scale=0.1).to(DEV)
+    wr, ids, wts = torch.empty(E, D, device=DEV), torch.empty(M, k, dtype=torch.int32, device=DEV), torch.empty(M, k, device=DEV)
+    def run():
+        K().linear(wr, x, w)
+        K().moe_router(ids, wts, h, wr, None, True, 1.0)
+    run()
+    K().linear(wr, x, w)
+    torch.cuda.synchronize()
+    K().moe_router(ids, wts, h, wr, None, True, 1.0)
+    want = ids.clone(), wts.clone()
+    graph = torch.cuda.CUDAGraph()      # the second launch right behind the first
+    with torch.cuda.graph(graph):
+        run()
+    for _ in range(20):
+        wr.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        assert torch.equal(ids, want[0]) and torch.equal(wts, want[1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,k,E,D", [(1, 1, 1, 8), (1, 4, 32, 2048), (8, 4, 32, 2048), (64, 4, 32, 520), (51, 5, 256, 4100), (37, 2, 3, 72),
                                      (1, 1, 256, 64), (4, 8, 256, 2048), (33, 1, 256, 72), (11, 1, 32, 64), (3, 4, 32, 64),
