@@ -432,9 +432,10 @@ LEB_API int leb_moe_router(int* topk_ids, float* topk_w, const void* h, int dtyp
       return 0;
     }
   }
-  // few rows: a cluster of four blocks each, while all of them have SMs of their own
+  // few rows: a cluster of four blocks each, while all of them have SMs of their own and there is enough to share out (8 experts of
+  // 256: 3.3 us against 3.05 by one block, 16 of 512 at 37 rows 3.6 and 3.4; 8 of 768 3.3 and 3.8, 24 of 512 3.2 and 3.5)
   const size_t smem_few = ((size_t)D + 2 * E) * sizeof(float);
-  if (ROUTER_CLUSTER * M <= sm_count() && E >= 8 && D % 8 == 0 && ((uintptr_t)wr & 15) == 0 && ((uintptr_t)h & 15) == 0 && smem_few <= 48 * 1024 &&
+  if (ROUTER_CLUSTER * M <= sm_count() && E >= 8 && (D >= 768 || E * D >= 12288) && D % 8 == 0 && ((uintptr_t)wr & 15) == 0 && ((uintptr_t)h & 15) == 0 && smem_few <= 48 * 1024 &&
       (dtype == LEB_BF16 || dtype == LEB_F32)) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ROUTER_CLUSTER * M);

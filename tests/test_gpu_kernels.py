@@ -1028,25 +1028,29 @@ def test_moe_router_align_combine(dtype, E, k, norm, bias, scaling):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("E,k,D", [(32, 4, 2048), (8, 2, 104), (5, 1, 72), (64, 6, 520)])
+@pytest.mark.parametrize("E,k,D", [(32, 4, 2048), (8, 2, 104), (5, 1, 72), (64, 6, 520), (10, 3, 4104), (9, 2, 768), (8, 1, 760), (23, 4, 536)])
 def test_moe_router_gives_a_row_the_same_bits_whatever_the_step(dtype, E, k, D):
-    """The router has a form for single rows and one for four rows per block (many rows): a row's
-    experts and weights are the same bits in both, so that a token is routed the same way alone, in a
-    decode batch and inside a prompt."""
+    """The router has a form of four blocks a row (up to 37 rows on 148 SMs; a quarter of the experts each, whole or not, and rows of
+    more than one round of 2,048), one of a block a row and forms of several rows a block (many rows): a row's experts and
+    weights are the same bits in all of them, so that a token is routed the same way alone, in a decode batch and
+    inside a prompt."""
     M = 700
     h = gen(M, D, seed=97, dtype=dtype).to(DEV)
     wr, b = gen(E, D, seed=98, scale=0.3).to(DEV), gen(E, seed=99, scale=0.1).to(DEV)
-    def route(rows):
+    def route(rows, ahead=False):
         ids = torch.empty(rows.shape[0], k, dtype=torch.int32, device=DEV)
         wts = torch.empty(rows.shape[0], k, device=DEV)
-        K().moe_router(ids, wts, rows, wr, b, True, 1.5)
+        K().moe_router(ids, wts, rows, wr, b, True, 1.5, ahead=ahead)
         return ids, wts
     all_ids, all_w = route(h)                                  # many rows: four per block
     some_ids, some_w = route(h[:200].contiguous())
     assert torch.equal(some_ids, all_ids[:200]) and torch.equal(some_w, all_w[:200])
-    for lo in (0, 199, 693):
-        one_ids, one_w = route(h[lo:lo + 7].contiguous())      # a row per block
-        assert torch.equal(one_ids, all_ids[lo:lo + 7]) and torch.equal(one_w, all_w[lo:lo + 7])
+    last = K().sm_count() // 4                                 # rows up to which a row has four blocks
+    for n in (1, 7, last, last + 1, 64, K().sm_count(), K().sm_count() + 1):
+        for lo in (0, 199, M - n):
+            for ahead in (False, True):
+                ids, wts = route(h[lo:lo + n].contiguous(), ahead)
+                assert torch.equal(ids, all_ids[lo:lo + n]) and torch.equal(wts, all_w[lo:lo + n])
     want_ids, want_w, _ = P.moe_route(h.double().cpu(), wr.double().cpu(), b.double().cpu(), k, True, 1.5)
     agree = (all_ids.cpu().long() == want_ids).all(dim=1)
     assert agree.float().mean() > 0.97                        # the rest: near-ties at float rounding
@@ -1246,10 +1250,11 @@ def test_shortconv_kernels_against_the_references_own():
             assert err(state[2], torch.from_numpy(g[f"state_out{case}"])) < 1e-6, (case, mode)
 
 
-@pytest.mark.parametrize("M,N,K_", [(256, 256, 64), (300, 520, 136), (129, 100, 72), (1000, 2048, 5632), (2048, 6144, 2048)])
+@pytest.mark.parametrize("M,N,K_", [(256, 256, 64), (300, 520, 136), (129, 100, 72), (1000, 2048, 5632), (2048, 6144, 2048),
+                                    (2700, 1544, 136), (4100, 520, 328)])
 def test_linear_tc_pairs(M, N, K_):
     """The product on pairs of SMs (cta_group::2, 256 x 256 tiles): tile-aligned sizes and sizes where
-    rows, columns and k run past the last tile; store, add to the residual, SwiGLU, both result types."""
+    rows, columns and k run past the last tile, a last band of fewer row tiles than eight behind whole ones among them; store, add to the residual, SwiGLU, both result types."""
     x, w = gen(M, K_, seed=100, dtype=torch.bfloat16), gen(N, K_, seed=101, scale=0.05, dtype=torch.bfloat16)
     want = x.double() @ w.double().T
     out = torch.full((M, N), float("nan"), device=DEV)
