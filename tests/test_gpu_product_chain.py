@@ -145,3 +145,138 @@ def test_a_chained_product_is_as_near_to_64_bits_as_one_alone(M, N, kk):
         off[chained] = float((outs[0].double() - want).norm() / want.norm())
     k.check_device_status()
     assert off[True] <= 1.05 * off[False]
+
+
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("Lc", [2, 3, 4, 5])
+@pytest.mark.parametrize("M,D", [(17, 520), (64, 1024), (97, 776)])
+def test_convolutions_in_a_chain(M, D, Lc, bias):
+    """The one-token convolution as a chain's epilogue for every number of taps, with and without an additive term: results and states of
+    two steps against 64 bits from the projections as bfloat16 (a projection may be rounded to either side: half a step, 2^-9 of the
+    largest, in each of the three factors), slots in another order than the rows, a padding row."""
+    import types
+    k, ws = K(), workspace()
+    w_in, w_out = gen(3 * D, D, seed=1, scale=D ** -0.5), gen(D, D, seed=2, scale=D ** -0.5)
+    taps, b = gen(D, Lc, seed=3, dtype=torch.float32), gen(D, seed=4, scale=0.1, dtype=torch.float32) if bias else None
+    slot = torch.arange(M, dtype=torch.int32).flip(0)
+    slot[M // 2] = -1
+    batch = types.SimpleNamespace(max_qlen=1, n_seqs=M, row_seq=torch.arange(M, dtype=torch.int32, device=DEV), seq_slot=slot.to(DEV))
+    state = gen(M, D, Lc - 1, seed=5, dtype=torch.float32)
+    want_state, on = state.double().cpu(), slot >= 0
+    for step in range(2):
+        h = gen(M, D, seed=6 + step)
+        y, x, before = torch.empty(M, D, dtype=torch.bfloat16, device=DEV), [torch.zeros(M, D, device=DEV) for _ in range(5)], k.launch_count()
+        with k.product_chain(ws, M, torch.bfloat16):
+            assert k.shortconv_decode_fused(y, h, w_in, taps, b, state, batch, Lc)
+            for t in x:
+                k.linear(t, y, w_out, k.ACCUMULATE)
+        assert k.launch_count() - before == 1
+        pb, pc, pu = (h.double().cpu() @ w_in.double().cpu().T).to(torch.bfloat16).double().chunk(3, -1)
+        bu, old = pb * pu, want_state[slot.clamp(min=0).long()]
+        row = torch.cat([old, bu[:, :, None]], -1)
+        conv = (row * taps.double().cpu()).sum(-1) + (b.double().cpu() if bias else 0.0)
+        want = torch.where(on[:, None], pc * conv, torch.zeros(()).double())
+        assert float((y.double().cpu() - want).abs().max() / want.abs().max()) < 4 * 2 ** -8
+        want_state = want_state.clone()
+        want_state[slot[on].long()] = row[on][:, :, 1:]
+        assert float((state.double().cpu() - want_state).abs().max() / want_state.abs().max()) < 2 * 2 ** -8
+        state.copy_(want_state)
+        assert float((x[-1].double() - y.double() @ w_out.double().T).abs().max() / x[-1].abs().max()) < 2e-5
+    k.check_device_status()
+
+
+def chain_of(k, ws, h, W, gate, norm):
+    """Six products with both halves of a split norm; the results of every one."""
+    M, D = h.shape
+    x = torch.zeros(M, D, device=DEV)
+    sp = k.SplitNorm(torch.empty(M, D, dtype=torch.bfloat16, device=DEV), torch.empty(M, -(-D // 16), device=DEV), norm, 1e-5)
+    a = torch.empty(M, gate.shape[0] // 2, dtype=torch.bfloat16, device=DEV)
+    z = [torch.empty(M, D, device=DEV) for _ in range(4)]
+    with k.product_chain(ws, M, torch.bfloat16):
+        k.linear(x, h, W, k.ACCUMULATE, emit=sp)
+        k.linear(a, sp.values, gate, k.SWIGLU, scale=sp)
+        for t in z:
+            k.linear(t, sp.values, W, scale=sp)
+    return [x, sp.values, sp.ssq, a, *z]
+
+
+@pytest.mark.parametrize("D,F", [(520, 1040), (2048, 2816)])
+def test_a_row_of_a_chain_does_not_depend_on_the_others(D, F):
+    """The same bits at every padding of the rows, alone with others' rows beside them."""
+    k, ws = K(), workspace()
+    W, gate, norm = gen(D, D, seed=1, scale=D ** -0.5), gen(2 * F, D, seed=2, scale=D ** -0.5), 1 + gen(D, seed=3, scale=0.1, dtype=torch.float32)
+    h = gen(128, D, seed=4)
+    want = chain_of(k, ws, h, W, gate, norm)
+    for M in (17, 32, 33, 64, 65, 96, 97):
+        for lo in (0, 128 - M):
+            for got, all_ in zip(chain_of(k, ws, h[lo:lo + M].contiguous(), W, gate, norm), want):
+                assert torch.equal(got, all_[lo:lo + M])
+    k.check_device_status()
+
+
+def test_chains_longer_than_the_kernel_takes_and_of_one_product():
+    """A chain that is full is launched and the next one begins (40 products); one product that leaves a norm's half is launched alone."""
+    k, ws, M, D = K(), workspace(), 40, 264
+    W, h = gen(D, D, seed=1, scale=D ** -0.5), gen(M, D, seed=2)
+    most = k.lib().leb_chain_max_ops()
+    outs, x, before = [torch.empty(M, D, dtype=torch.bfloat16, device=DEV) for _ in range(2 * most + 7)], h, k.launch_count()
+    with k.product_chain(ws, M, torch.bfloat16):
+        for y in outs:
+            k.linear(y, x, W)
+            x = y
+    assert k.launch_count() - before == 3
+    for x, y in zip([h, *outs], outs):
+        want = x.double() @ W.double().T
+        assert float((y.double() - want).abs().max() / want.abs().max()) < 2 ** -8 + 2e-5
+    results = []
+    for chained in (True, False):
+        s = torch.zeros(M, D, device=DEV)
+        sp = k.SplitNorm(torch.empty(M, D, dtype=torch.bfloat16, device=DEV), torch.empty(M, -(-D // 16), device=DEV), torch.ones(D, device=DEV), 1e-5)
+        with k.product_chain(ws, M, torch.bfloat16) if chained else contextlib.nullcontext():
+            k.linear(s, h, W, k.ACCUMULATE, emit=sp)
+        assert sp.filled
+        results.append((s, sp.values, sp.ssq))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    k.check_device_status()
+
+
+def test_a_step_that_raises_launches_nothing_and_the_next_chain_is_whole():
+    k, ws, M, D = K(), workspace(), 40, 264
+    W, h = gen(D, D, seed=1, scale=D ** -0.5), gen(M, D, seed=2)
+    y = [torch.full((M, D), 7.0, device=DEV) for _ in range(5)]
+    before = k.launch_count()
+    with pytest.raises(ValueError), k.product_chain(ws, M, torch.bfloat16):
+        for t in y:
+            k.linear(t, h, W)
+        raise ValueError
+    assert k.launch_count() == before and all(bool((t == 7).all()) for t in y)
+    with k.product_chain(ws, M, torch.bfloat16):
+        for t in y:
+            k.linear(t, h, W)
+    want = h.double() @ W.double().T
+    assert all(float((t.double() - want).abs().max() / want.abs().max()) < 2e-5 for t in y)
+    k.check_device_status()
+
+
+def test_a_chain_whose_barrier_is_never_passed_gives_up():
+    """The grid barrier's count put where no arrival brings it to its target: every block gives its bounded wait up (after about a
+    second), the status word says so, the context and the barrier's words are usable, and the next chain is right."""
+    k, ws, M, D = K(), workspace(), 40, 264
+    W, h = gen(D, D, seed=1, scale=D ** -0.5), gen(M, D, seed=2)
+    y = [torch.empty(M, D, device=DEV) for _ in range(5)]
+
+    def run():
+        with k.product_chain(ws, M, torch.bfloat16):
+            for t in y:
+                k.linear(t, h, W)
+    k.check_device_status()
+    ws.zeroed("chain.sync", 2)[0] = -1000
+    run()
+    torch.cuda.synchronize()
+    with pytest.raises(k.KernelError, match=r"role 4\d"):
+        k.check_device_status()
+    assert ws.zeroed("chain.sync", 2).tolist() == [0, 0]
+    run()
+    k.check_device_status()
+    want = h.double() @ W.double().T
+    assert all(float((t.double() - want).abs().max() / want.abs().max()) < 2e-5 for t in y)
