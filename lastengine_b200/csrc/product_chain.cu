@@ -23,15 +23,20 @@
 // half), 2 gated activation over interleaved weight rows, 3 the one-token gated convolution (a tile is then the B, C
 // and x rows of 32 channels), each optionally scaled by a split norm.
 //
-// What bounds it: four products of a conv layer at 64 rows (width 2,048, 7,168 wide inside, 122 MB of weights, 18.6 us at the copy
-// rate) take 41 us here and 67 as eight launches of the sliced product and its second kernel; 36 and 43 at 32 rows, 52 and 62
-// at 96, 58 and 71 at 128 (5,632 wide).  The stream runs at the memory's rate while there is room in the ring; the chain of a
-// product (grid barrier 1.3 us, activations 0.7, last k-blocks 0.5 to 2, exchange 0.7, sums and stores 1, each once per
-// product) is longer than what the ring holds.  A cluster of 8 halves a block's k-blocks, but only 15 such clusters fit the
-// chip (120 blocks against 132 in 33 clusters of 4) and 16 tiles then take two rounds: 57 us.  Two buffers for the exchange
-// against two more weight slots: 47.2 and 50.9 us, with the second the senders wait for their credits.  From 65 rows on a tile is exchanged in two
-// parts, so that two buffers fit: 128 rows 64 -> 58 us, 96 rows 55 -> 52; at 64 rows the second exchange costs more (46 -> 52).  Epilogues unrolled
-// over all of a thread's outputs (128 KB of instructions) against loops: 47.2 and 45.8.
+// What bounds it: the four products of a conv layer of width 2,048, chained and as launches alone, in us, a norm's launch between
+// layers:
+//   rows              32            64            96            128
+//   5,632 wide   39.7 / 42.1   44.0 / 49.2   53.6 / 59.9   58.5 / 67.7     103 MB of weights, 15.7 us at the copy rate
+//   7,168 wide   43.6 / 56.7   48.3 / 65.7   59.2 / 83.4   64.8 / 101.3    122 MB, 18.6 us
+// The stream runs at the memory's rate while there is room in the ring; the chain of a product (grid barrier 1.3 us, activations
+// 0.7, last k-blocks 0.5 to 2, exchange 0.7, sums and stores 1, each once per product) is longer than what the ring holds.  The
+// accumulators of shorter runs cost 1 to 4% of these times.
+// Variants, each beside the kernel as it was when they were tried (7,168 wide, no norm between; 64 rows where none are named).  A
+// cluster of 8 halves a block's k-blocks, but only 15 such clusters fit the chip (120 blocks against 132 in 33 clusters of 4) and 16
+// tiles then take two rounds: 57 us, against 47.  Two more weight slots in the place of the second exchange buffer: 50.9 against 47.2, the
+// senders wait for their credits.  Epilogues unrolled over all of a thread's outputs (128 KB of instructions) in the place of loops: 47.2
+// against 45.8.  A tile exchanged in two parts, so that two buffers fit: 52 against 46, but from 65 rows on, where only one fits
+// otherwise, 52 against 55 at 96 rows and 58 against 64 at 128 (5,632 wide), so it is done there.
 //
 // All blocks wait for one another, so they must all be resident: the launch is cooperative.  Every wait is bounded
 // (mbarriers and the grid barrier by their polls): a wait that runs out sets the block's abort flag and the status
