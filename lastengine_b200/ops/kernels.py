@@ -54,7 +54,7 @@ class _Chain(threading.local):
         """Launches what waits: as one kernel where that pays, else as without a chain."""
         ops, self.ops = self.ops, []
         if len(ops) == 1 or not chain_pays(self.rows, [args[5:7] for args, _ in ops]):
-            for _, (out, x, w, epilogue, norm, alone) in ops:
+            for _, (out, x, w, epilogue, norm, alone, _) in ops:
                 if alone is not None:
                     alone()
                 else:
@@ -180,7 +180,8 @@ def _chained(out, x, w, M, N, K, lda, ldc, epilogue, scale, emit, conv=_NO_CONV,
     norm = _scale_args(scale, M, K) + _emit_args(emit)
     if len(c.ops) >= c.most:
         c.flush()
-    c.ops.append(((out.data_ptr(), _DT[out.dtype], xp, wp, M, N, K, lda, ldc, epilogue, *norm, *conv), (out, x, w, epilogue, norm, alone)))
+    c.ops.append(((out.data_ptr(), _DT[out.dtype], xp, wp, M, N, K, lda, ldc, epilogue, *norm, *conv),
+                  (out, x, w, epilogue, norm, alone, (scale, emit))))      # (kept: the arguments are their addresses)
     return True
 
 

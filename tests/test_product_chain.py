@@ -2,6 +2,7 @@
 
 The models run here without a GPU: the kernel library is replaced by one that computes nothing and counts what waits."""
 import dataclasses
+import weakref
 
 import pytest
 import torch
@@ -278,6 +279,26 @@ def test_products_that_do_not_pay_as_a_chain_run_alone_in_their_order(library, m
             kernels.linear(torch.zeros(ROWS, n), x, torch.zeros(n, 64, dtype=torch.bfloat16))
         assert len(kernels._chain.ops) == 3 and not ran
     assert ran == [32, 64, 96] and library.chains == library.longest == 0
+
+
+def test_what_waits_keeps_its_operands(library):
+    """A caller may let go of them: the launch comes later and takes addresses."""
+    D, b16 = 64, torch.bfloat16
+    ws, gone = Workspace(CPU), []
+
+    def held(t):
+        gone.append(weakref.ref(t))
+        return t
+
+    def add():
+        sp = kernels.SplitNorm(held(torch.zeros(ROWS, D, dtype=b16)), held(torch.zeros(ROWS, 4)), held(torch.zeros(D)), 1e-5)
+        x, w = held(torch.zeros(ROWS, D, dtype=b16)), held(torch.zeros(D, D, dtype=b16))
+        kernels.linear(held(torch.zeros(ROWS, D)), x, w, kernels.ACCUMULATE, emit=sp)
+        kernels.linear(held(torch.zeros(ROWS, D)), sp.values, w, scale=sp)
+    with kernels.product_chain(ws, ROWS, b16):
+        add()
+        assert all(r() is not None for r in gone)
+    assert library.chains == 1 and all(r() is None for r in gone)
 
 
 def test_a_product_the_chain_refuses_when_it_is_launched_leaves_none_behind(library, monkeypatch):
