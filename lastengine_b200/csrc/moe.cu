@@ -232,20 +232,21 @@ moe_router_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, const 
 // the wait; here a warp has the whole of its router row (PRE pieces of 16 bytes a lane) in registers before it waits for the
 // row of h, where the caller says that the kernel launched before does not write the router's rows (`ahead`).  The scores go to
 // the first block's shared memory, whose first warp chooses.  A score is summed in the order of the form above: the same bits.
-// Those loads are written out: as plain loads of a const __restrict__ pointer the compiler takes what they read for constant and
-// moved them before the wait.
+// Otherwise (not AHEAD) they are fetched after the wait by loads that are written out: as plain loads of a const __restrict__ pointer
+// the compiler takes what they read for constant and moved them before the wait.
 #define ROUTER_CLUSTER 4
 #define ROUTER_PRE 16
-__device__ __forceinline__ float4 router_row_load(const float4* p) {
+template <bool AHEAD>
+__device__ __forceinline__ float4 router_row_load(const float4* __restrict__ p) {
+  if (AHEAD) return *p;
   float4 v;
   asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
   return v;
 }
-template <typename T>
+template <typename T, bool AHEAD>
 __global__ void __launch_bounds__(256)
 moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, const T* __restrict__ h,
-                      const float* __restrict__ wr, const float* __restrict__ bias, int D, int E, int k, int norm_topk, float scaling,
-                      int ahead) {
+                      const float* __restrict__ wr, const float* __restrict__ bias, int D, int E, int k, int norm_topk, float scaling) {
   extern __shared__ __align__(16) float sm[];  // the row of h as float [D], then s[E], c[E]
   float* s_ = sm + D;
   float* c_ = s_ + E;
@@ -253,11 +254,11 @@ moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, co
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int share = (E + ROUTER_CLUSTER - 1) / ROUTER_CLUSTER, first = rank * share + warp, end = min(E, (rank + 1) * share), n4 = D / 4;
   pdl_trigger();
-  if (!ahead) pdl_wait();
+  if (!AHEAD) pdl_wait();
   float4 a[ROUTER_PRE];
 #pragma unroll
   for (int u = 0; u < ROUTER_PRE; u++)
-    a[u] = first < end && lane + 32 * u < n4 ? router_row_load(reinterpret_cast<const float4*>(wr + (size_t)first * D) + lane + 32 * u)
+    a[u] = first < end && lane + 32 * u < n4 ? router_row_load<AHEAD>(reinterpret_cast<const float4*>(wr + (size_t)first * D) + lane + 32 * u)
                                              : make_float4(0.f, 0.f, 0.f, 0.f);
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   pdl_wait();
@@ -274,7 +275,7 @@ moe_router_few_kernel(int* __restrict__ topk_ids, float* __restrict__ topk_w, co
     for (int i0 = lane; i0 < n4; i0 += 32 * ROUTER_PRE) {
       if (e != first || i0 != lane) {
 #pragma unroll
-        for (int u = 0; u < ROUTER_PRE; u++) a[u] = i0 + 32 * u < n4 ? router_row_load(w4 + i0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < ROUTER_PRE; u++) a[u] = i0 + 32 * u < n4 ? router_row_load<AHEAD>(w4 + i0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < ROUTER_PRE; u++) {
@@ -450,8 +451,11 @@ LEB_API int leb_moe_router(int* topk_ids, float* topk_w, const void* h, int dtyp
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_leb_pdl ? 2 : 1;
-    const cudaError_t e = dtype == LEB_BF16 ? cudaLaunchKernelEx(&cfg, moe_router_few_kernel<bf16>, topk_ids, topk_w, (const bf16*)h, wr, bias, D, E, k, norm_topk, scaling, ahead)
-                                            : cudaLaunchKernelEx(&cfg, moe_router_few_kernel<float>, topk_ids, topk_w, (const float*)h, wr, bias, D, E, k, norm_topk, scaling, ahead);
+    cudaError_t e;
+#define LEB_ROUTER(T, AHEAD) cudaLaunchKernelEx(&cfg, moe_router_few_kernel<T, AHEAD>, topk_ids, topk_w, (const T*)h, wr, bias, D, E, k, norm_topk, scaling)
+    if (dtype == LEB_BF16) e = ahead ? LEB_ROUTER(bf16, true) : LEB_ROUTER(bf16, false);
+    else e = ahead ? LEB_ROUTER(float, true) : LEB_ROUTER(float, false);
+#undef LEB_ROUTER
     if (e != cudaSuccess) return leb_fail("leb_moe_router: %s", cudaGetErrorString(e));
     LEB_CHECK_LAUNCH("leb_moe_router");
     return 0;
